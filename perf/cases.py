@@ -122,7 +122,7 @@ def prepare(case, seed):
         weights.append(w)
         scales.append(s)
     w_scale = torch.cat(scales).cpu().numpy() if case["scaled"] else None
-    st = {"op": op, "weights": weights, "n": sum(segs[0])}
+    st = {"op": op, "weights": weights, "n": sum(segs[0]), "scales": scales}
     if op == "dequant":
         st["node"] = DequantWeightBf16(st["n"], widths=segs[0], w_scale=w_scale)
     elif op == "lmhead":
@@ -152,6 +152,54 @@ def run(st):
     if op == "argmax":
         return node(st["x"])
     return node(st["weights"][0])
+
+
+def _weight_f64(dtype, w, n, scale):
+    """The values of a stored weight, in 64 bits."""
+    if dtype != "nvfp4":
+        v = w.double()
+    else:
+        e2m1 = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device=w.device)
+        e2m1 = torch.cat([e2m1, -e2m1])
+        packed, blocks = w[:, :n // 2], w[:, n // 2:]
+        v = torch.stack([e2m1[(packed & 15).long()], e2m1[(packed >> 4).long()]], dim=-1).reshape(w.shape[0], n)
+        v = v * blocks.contiguous().view(torch.float8_e4m3fn).double().repeat_interleave(16, dim=1)
+    return v if scale is None else v * scale.double()
+
+
+def exact(case, seed):
+    st = prepare(case, seed)
+    op, dtype = case["op"], case["dtype"]
+    if op == "argmax":
+        val, idx = st["x"].double().max(dim=-1)
+        return idx, val
+    segs = _segments(case)
+
+    def bf(t):  # a rounding that the op itself is defined with
+        return t.bfloat16().double()
+
+    if op == "dequant":
+        return list(torch.split(_weight_f64(dtype, st["weights"][0], st["n"], st["scales"][0]), segs[0], dim=1))
+    if op == "shared":
+        g, u = st["g"].double(), st["u"].double()
+        x = bf(bf(g * bf(torch.sigmoid(g))) * u)
+        gate = bf(torch.sigmoid(bf(st["gx"].double() @ st["gw"].double())))
+        y = x @ _weight_f64(dtype, st["weights"][0], st["n"], st["scales"][0])
+        return st["routed"].double() + bf(y) * gate
+    x = st["x"].double()
+    if op == "lmhead":
+        best = None
+        w, n = st["weights"][0], st["n"]
+        for c0 in range(0, n, 16384):  # column blocks: the whole weight in 64 bits would be large
+            c1 = min(n, c0 + 16384)
+            block = torch.cat([w[:, c0 // 2:c1 // 2], w[:, n // 2 + c0 // 16:n // 2 + c1 // 16]], dim=1)
+            top = (x @ _weight_f64(dtype, block, c1 - c0, None)).max(dim=-1).values
+            best = top if best is None else torch.maximum(best, top)
+        return None, best, None  # the index, and the key made of it, may differ where two logits round alike
+    outs = []
+    for w, s, widths in zip(st["weights"], st["scales"], segs):
+        outs += torch.split(x @ _weight_f64(dtype, w, sum(widths), s), widths, dim=1)
+    return outs
 
 
 def work(case):
