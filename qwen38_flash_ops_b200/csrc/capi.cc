@@ -76,6 +76,7 @@ struct qfg_skinny_gemm {
   int force_slow = 0;
   int exchange_spin = qfg::kExchangeSpin;  // sharded LM head: bound of the wait for a peer's keys (iterations)
   int dense_rows = -1;  // calls with more rows take the dequantise + library GEMM branch; -1 = qfg::DenseRowsDefault(mode), 0 = never
+  qfg::DenseTcPlan dense_plan;  // bm > 0: overrides the launch shape of that branch (set_option("dense_plan", "bm,split,pair,ks"))
   unsigned long long phase_times = 0;  // device address given through set_option("phase_times", ...)
   std::string plan_spec;
   // plans already computed for this node, keyed by the shape of the call
@@ -90,8 +91,8 @@ struct qfg_skinny_gemm {
   qfg_skinny_gemm() = default;
   qfg_skinny_gemm(const qfg_skinny_gemm& o)
       : seg_outs(o.seg_outs), widths(o.widths), trigger(o.trigger), d_w_scale(o.d_w_scale), w_scale_len(o.w_scale_len),
-        pdl_wait(o.pdl_wait), force_slow(o.force_slow), exchange_spin(o.exchange_spin), dense_rows(o.dense_rows), phase_times(o.phase_times),
-        plan_spec(o.plan_spec) {}
+        pdl_wait(o.pdl_wait), force_slow(o.force_slow), exchange_spin(o.exchange_spin), dense_rows(o.dense_rows),
+        dense_plan(o.dense_plan), phase_times(o.phase_times), plan_spec(o.plan_spec) {}
 };
 
 struct qfg_dequant {
@@ -284,7 +285,13 @@ qfg::Plan ComputePlan(const qfg_skinny_gemm& op, const qfg::PlanInput& in) {
 void Run(const qfg_skinny_gemm& op, Prepared& pr, int64_t m, cudaStream_t stream, const char* name) {
   const int dense_rows = op.dense_rows < 0 ? qfg::DenseRowsDefault(pr.mode) : op.dense_rows;
   if (dense_rows > 0 && m > dense_rows && qfg::DenseEligible(pr.params)) {
-    qfg::LaunchDenseGemm(pr.mode, pr.params, m, stream);
+    if (qfg::DenseTcEligible(pr.mode, pr.params)) {
+      const qfg::DenseTcPlan plan =
+          op.dense_plan.bm > 0 ? op.dense_plan : qfg::ChooseDenseTcPlan(pr.mode, pr.params, m, pr.plan_in.sm_count);
+      qfg::LaunchDenseTc(pr.mode, pr.params, m, plan, stream);
+    } else {
+      qfg::LaunchDenseGemm(pr.mode, pr.params, m, stream);
+    }
     return;
   }
   const qfg::Plan plan = PlanFor(op, pr.plan_in, static_cast<int>(std::min<int64_t>(m, qfg::kMaxRows)));
@@ -347,6 +354,12 @@ int SetGemmOption(qfg_skinny_gemm* op, const char* key, const char* value) {
   if (k == "pdl_wait") op->pdl_wait = std::atoi(value);
   else if (k == "force_slow") op->force_slow = std::atoi(value);
   else if (k == "dense_rows") op->dense_rows = std::atoi(value);
+  else if (k == "dense_plan") {
+    qfg::DenseTcPlan plan;
+    if (std::sscanf(value, "%d,%d,%d,%d", &plan.bm, &plan.split, &plan.pair, &plan.ks) < 1)
+      return Fail(QFG_INVALID_ARGUMENT, "set_option: dense_plan is \"bm,split,pair,ks\"");
+    op->dense_plan = plan;
+  }
   else if (k == "exchange_spin") op->exchange_spin = std::max(0, std::atoi(value));
 #ifdef QFG_PHASE_TIMES
   else if (k == "phase_times") op->phase_times = std::strtoull(value, nullptr, 10);  // measurement builds only

@@ -1,13 +1,11 @@
-// Prefill-shaped SkinnyGemm calls: many rows of x against the same weights.
+// Many-row SkinnyGemm calls on layouts that the kernel of dense_tc.cu does not take (rows of x or of the weight that
+// its copies cannot address, outputs it has no alignment for).
 //
-// The streaming kernels read the weights once per eight rows, which is the right trade for decode and the
-// wrong one for hundreds of rows.  Past a row threshold the call is served the way the reference serves its
-// M > 8 calls (fused_gemm.cu:292-428, dispatch at :578-583): quantised weights (and BF16 weights with a
-// w_scale) are dequantised in column tiles into a cached BF16 buffer, w_scale folded in before the rounding,
-// and a library GEMM with FP32 accumulation produces each output slice.  cuBLAS is a plain library call here,
-// as it is in the reference; it is looked up at run time so that the decode library carries no link-time
-// dependency on it.  This branch allocates (handle, buffer) on first use and is not graph-capturable, like
-// the reference's.
+// They are served the way the reference serves its M > 8 calls (fused_gemm.cu:292-428, dispatch at :578-583):
+// quantised weights (and BF16 weights with a w_scale) are dequantised in column tiles into a cached BF16 buffer,
+// w_scale folded in before the rounding, and a library GEMM with FP32 accumulation produces each output slice.
+// cuBLAS is looked up at run time so that the library carries no link-time dependency on it.  This branch allocates
+// (handle, buffer) on first use and is not graph-capturable, like the reference's.
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 #include <dlfcn.h>

@@ -1,0 +1,879 @@
+// Calls with many rows on the tensor memory path: out[M, N] = x[M, K] @ W[K, N] with BF16, FP8 or NVFP4 weights,
+// dequantised on the way into shared memory.
+//
+// A CTA computes tiles of 128 columns of W by `bm` rows of x (bm <= 256, a multiple of 16) with tcgen05.mma: the
+// weights are the 128-row operand, read MN-major because a stored row of W is contiguous along N, and the rows of x
+// are the bm-column operand, K-major as x is stored.  Both operands are BF16 in 128-byte-swizzled shared memory,
+// 64 k per stage; the FP32 accumulators lie in tensor memory, two sets of them, so that the epilogue of a tile
+// overlaps the products of the next.  Roles by warp:
+//   0-3   epilogue: accumulators -> BF16 -> the output that owns the column
+//   4     TMA producer: the x tile of every stage, and the weight tile where the weights are BF16
+//   5     tensor memory allocation; one lane issues the MMAs
+//   6-7   FP8 / NVFP4: copy the stored weights into a ring of their own (~60 KB in flight per SM)
+//   8-23  FP8 / NVFP4: sixteen warps in two groups that take the stages in turn; a warp turns eight weight rows of a
+//         stage into BF16, w_scale folded in before the one rounding
+// Rows of x are what the dequantisation is shared by: at bm = 256 a stage takes the tensor core 512 cycles, at
+// bm <= 64 the warps of the third role and the weight stream set the pace.
+//
+// K is split over the CTAs of a cluster where the tiles alone leave SMs idle; the ranks then add their accumulators
+// through distributed shared memory in rank order.  PAIR: two CTAs of a cluster work on 256 columns with
+// cta_group::2; each holds its own 128 columns of W and half of the rows of x, which halves what the SMs fetch of x
+// from L2 (a 128 x 256 tile fetches 36 KB per 512 cycles, more than an SM's share of L2).
+//
+// What bounds it.  Few rows: the dequantising warps and the barriers between the roles, about 400 cycles a block of 64 k
+// (FP4 at 33 rows, 5120 x 17408: 24.6 us = 2.1 TB/s of weights; the dequantisation pass and the library GEMM that this
+// kernel took the place of, 86.8 us).  Many rows: the tensor core, 70-80 % of its rate (FP8, 509 rows, 5120 x 10240: 67.9 us
+// against 93.0; FP4, 2048 rows, 5120 x 17408: 309 us against 332).  The tcgen05 operands come from shared memory
+// rather than tensor memory because the rows of x per pass would be limited to 64 there, and the weights are written
+// MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
+//
+// Every wait is bounded; a CTA that gives up on one writes NaN and leaves.
+#include <cooperative_groups.h>
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
+#include <cstdlib>
+#include <stdexcept>
+#include <string>
+
+#include "qfg_internal.h"
+
+namespace qfg {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kBn = 128;           // columns of W per CTA
+constexpr int kBk = 64;            // k per block: one 128-byte swizzled row of x; a stage holds KS = 1 or 2 blocks
+constexpr int kABytes = kBn * kBk * 2;
+constexpr int kMaxStages = 8;
+constexpr int kDqWarps = 8;        // warps that fill one stage, eight weight rows each
+constexpr int kDqGroups = 2;       // groups of them, taking the stages in turn
+constexpr int kLoadWarps = 2;     // warps that copy the stored rows into the raw ring
+constexpr int kFirstDqWarp = 6 + kLoadWarps;
+constexpr int kMaxRaw = 12;
+constexpr int kSpin = 1 << 20;
+
+template <int MODE, int KS>
+struct RawRing {  // ring of stored, undequantised stages
+  static constexpr int kRows = kBk * KS;
+  static constexpr int kSlot = kRows * (MODE == kNvfp4 ? 64 + 16 : 128);
+  static constexpr int kDepth = (MODE == kNvfp4 ? 12 : 8) / KS;
+  static constexpr int kBytes = MODE == kBf16 ? 0 : kSlot * kDepth;
+};
+static_assert(RawRing<kNvfp4, 1>::kDepth <= kMaxRaw && RawRing<kFp8, 2>::kDepth >= kDqGroups, "raw ring");
+
+struct DenseSeg {
+  const uint8_t* w;
+  const float* w_scale;
+  long long pitch, total_bytes;
+  int n, tile_begin, out_begin, out_end;
+};
+
+struct DenseParams {
+  CUtensorMap xmap;
+  CUtensorMap wmap[kMaxSeg];  // stored weights (nibbles of NVFP4), where their rows are 16-byte aligned
+  CUtensorMap smap[kMaxSeg];  // NVFP4 block scales
+  DenseSeg seg[kMaxSeg];
+  uint16_t* out[kMaxOut];
+  int col_begin[kMaxOut], width[kMaxOut];
+  int nseg, M, K, ksteps, bm, m_tiles, tiles, stages, raw_tensor;
+};
+
+struct Ctl {
+  unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], raw_full[kMaxRaw], raw_empty[kMaxRaw];
+  uint32_t tmem;
+  volatile uint32_t fault;
+};
+
+// ------------------------------------------------------------------------------ PTX
+__device__ __forceinline__ uint32_t Smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void BarInit(uint32_t a, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(n) : "memory"); }
+__device__ __forceinline__ void BarArrive(uint32_t a) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(a) : "memory");
+}
+__device__ __forceinline__ uint32_t MapRank(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void BarExpect(uint32_t a, uint32_t bytes) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes) : "memory");
+}
+// arrives on the barrier of this CTA, or of the leader of its pair
+template <bool PAIR>
+__device__ __forceinline__ void BarArriveLeader(uint32_t a) {
+  if constexpr (PAIR) {
+    asm volatile("{ .reg .b32 r;\n mapa.shared::cluster.u32 r, %0, 0;\n mbarrier.arrive.shared::cluster.b64 _, [r];\n}" ::"r"(a) : "memory");
+  } else {
+    BarArrive(a);
+  }
+}
+__device__ __forceinline__ bool BarTry(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+  return ok != 0;
+}
+// the same without the pause of up to a microsecond that try_wait may take where the phase is still open
+__device__ __forceinline__ bool BarTest(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+  return ok != 0;
+}
+// false once a wait of this CTA ran out
+__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, Ctl& c) {
+  for (int i = 0; i < kSpin; ++i) {
+    if (BarTry(a, parity)) return true;
+    if ((i & 255) == 255 && c.fault) return false;
+  }
+  c.fault = 1;
+  return false;
+}
+template <bool PAIR>
+__device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  if constexpr (PAIR) {  // the barrier may be the leader's
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"(map), "r"(bar), "r"(x), "r"(y)
+                 : "memory");
+  } else {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
+                 "r"(bar), "r"(x), "r"(y)
+                 : "memory");
+  }
+}
+// one lane of a converged warp; unlike a test of the lane number it leaves the compiler's view of the operands uniform,
+// which the MMA's descriptors need (a lane test cost 80 cycles per MMA and 350 per wait)
+__device__ __forceinline__ bool ElectOne() {
+  uint32_t yes;
+  asm volatile("{ .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(yes)::"memory");
+  return yes != 0;
+}
+template <bool PAIR>
+__device__ __forceinline__ void MmaSs(uint32_t d, unsigned long long a, unsigned long long b, uint32_t idesc, bool add) {
+  if constexpr (PAIR) {
+    asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b),
+                 "r"(idesc), "r"(add ? 1 : 0)
+                 : "memory");
+  } else {
+    asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b),
+                 "r"(idesc), "r"(add ? 1 : 0)
+                 : "memory");
+  }
+}
+// arrives on the barrier (of both CTAs of a pair) when the MMAs issued so far have completed
+template <bool PAIR>
+__device__ __forceinline__ void MmaCommit(uint32_t bar) {
+  if constexpr (PAIR) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+  } else {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  }
+}
+__device__ __forceinline__ void FenceBefore() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void FenceAfter() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// 128-byte swizzle; `lbo`: distance of the 64-element groups of an MN-major operand (unused K-major), `sbo`: of the
+// groups of eight rows
+__device__ __forceinline__ unsigned long long SmemDesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return static_cast<unsigned long long>((addr >> 4) & 0x3FFF) | (static_cast<unsigned long long>(lbo >> 4) << 16) |
+         (static_cast<unsigned long long>(sbo >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void CpAsync8(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void Lds128(uint32_t a, uint32_t (&v)[4]) {
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+}
+__device__ __forceinline__ void Lds64(uint32_t a, uint32_t (&v)[2]) {
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(a));
+}
+__device__ __forceinline__ uint32_t Lds8(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void Sts128(uint32_t a, const uint32_t* v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void CvtE2m1x8(uint32_t c, uint32_t (&r)[4]) {
+  asm("{ .reg .b8 b0, b1, b2, b3;\n mov.b32 {b0, b1, b2, b3}, %4;\n cvt.rn.f16x2.e2m1x2 %0, b0;\n cvt.rn.f16x2.e2m1x2 %1, b1;\n"
+      " cvt.rn.f16x2.e2m1x2 %2, b2;\n cvt.rn.f16x2.e2m1x2 %3, b3;\n}"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(c));
+}
+__device__ __forceinline__ void CvtE4m3x4(uint32_t c, uint32_t& lo, uint32_t& hi) {
+  asm("{ .reg .b16 h0, h1;\n mov.b32 {h0, h1}, %2;\n cvt.rn.f16x2.e4m3x2 %0, h0;\n cvt.rn.f16x2.e4m3x2 %1, h1;\n}" : "=r"(lo), "=r"(hi) : "r"(c));
+}
+__device__ __forceinline__ uint32_t Hmul2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// an FP16 pair (exact products of the stored formats) as BF16, times the scales of its two columns
+template <bool SCALED>
+__device__ __forceinline__ uint32_t ToBf16(uint32_t h, float s0, float s1) {
+  float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  if constexpr (SCALED) {
+    f.x *= s0;
+    f.y *= s1;
+  }
+  const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+  return *reinterpret_cast<const uint32_t*>(&b);
+}
+
+// ------------------------------------------------------------------------------ the walk over tiles
+struct TileAt {
+  int seg, n0, m0;
+};
+// tiles of one column block follow one another (all row blocks of it, then the next), so the SMs share its weights in L2
+template <bool PAIR>
+__device__ __forceinline__ TileAt LocateDense(const DenseParams& p, int tile, int rank) {
+  TileAt t;
+  const int nt = tile / p.m_tiles;
+  t.m0 = (tile - nt * p.m_tiles) * p.bm;
+  t.seg = 0;
+#pragma unroll
+  for (int i = 1; i < kMaxSeg; ++i) t.seg += (i < p.nseg && nt >= p.seg[i].tile_begin) ? 1 : 0;
+  t.n0 = (nt - p.seg[t.seg].tile_begin) * (PAIR ? 2 * kBn : kBn) + (PAIR ? rank * kBn : 0);
+  return t;
+}
+
+// ------------------------------------------------------------------------------ loading warps
+// Stored rows -> the raw ring.  A slot holds one stage: NVFP4 [rows][64 nibble bytes], then [rows][the 16 bytes that
+// hold the row's 8 block scales, at their offset in an aligned 16]; FP8 [rows][128 bytes].  One lane's tensor
+// copies where the rows are 16-byte aligned; the rest of the NVFP4 weights (N an odd multiple of 128) in 8-byte pieces
+// by all lanes of both warps, which is slower (18 copy instructions a stage) but knows no alignment beyond 8.
+template <bool PAIR, int KS>
+__device__ __forceinline__ void LoadNvfp4Pieces(const DenseParams& p, Ctl& ctl, int lane64, int rank, int kbeg, int kcount, int first_tile,
+                                                int tile_step, uint32_t ring) {
+  using R = RawRing<kNvfp4, KS>;
+  const uint32_t full0 = Smem(&ctl.raw_full[0]), empty0 = Smem(&ctl.raw_empty[0]);
+  int slot = 0;
+  uint32_t parity = 1;
+  bool first_round = true;
+  const int c = lane64 & 7, r0 = lane64 >> 3;  // nibble piece c of rows r0 + 8 j; the scales of row lane64
+  for (int tile = first_tile; tile < p.tiles; tile += tile_step) {
+    const TileAt t = LocateDense<PAIR>(p, tile, rank);
+    const DenseSeg& sg = p.seg[t.seg];
+    const bool cols = t.n0 < sg.n;
+    const int at = sg.n / 2 + t.n0 / 16;
+    const uint8_t* nib = sg.w + (static_cast<long long>(kbeg) * R::kRows + r0) * sg.pitch + t.n0 / 2 + 8 * c;
+    const uint8_t* scl = sg.w + (static_cast<long long>(kbeg) * R::kRows + lane64) * sg.pitch + at;
+    const uint32_t nib_dst = ring + static_cast<uint32_t>(r0 * 64 + c * 8);
+    const uint32_t scl_dst = ring + static_cast<uint32_t>(R::kRows * 64 + lane64 * 16 + (at & 8));
+#pragma unroll 1
+    for (int k = 0; k < kcount; ++k) {
+      if (!first_round && !BarWait(empty0 + slot * 8, parity, ctl)) return;
+      const uint32_t base = static_cast<uint32_t>(slot) * R::kSlot;
+      const int rows = cols ? p.K - (kbeg + k) * R::kRows : 0;  // rows past K read as zero
+#pragma unroll
+      for (int j = 0; j < 8 * KS; ++j) {
+        const bool ok = r0 + 8 * j < rows;
+        CpAsync8(nib_dst + base + j * 512, ok ? nib + 8 * j * sg.pitch : sg.w, ok ? 8 : 0);
+      }
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+        const bool ok = lane64 + 64 * j < rows;
+        CpAsync8(scl_dst + base + j * 1024, ok ? scl + 64 * j * sg.pitch : sg.w, ok ? 8 : 0);
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full0 + slot * 8) : "memory");
+      nib += R::kRows * sg.pitch;
+      scl += R::kRows * sg.pitch;
+      if (++slot == R::kDepth) {
+        slot = 0;
+        parity ^= 1u;
+        first_round = false;
+      }
+    }
+  }
+}
+
+template <int MODE, bool PAIR, int KS>
+__device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int rank, int kbeg, int kcount, int first_tile, int tile_step, uint32_t ring) {
+  using R = RawRing<MODE, KS>;
+  const uint32_t full0 = Smem(&ctl.raw_full[0]), empty0 = Smem(&ctl.raw_empty[0]);
+  int slot = 0;
+  uint32_t parity = 1;
+  bool first_round = true;
+  for (int tile = first_tile; tile < p.tiles; tile += tile_step) {
+    const TileAt t = LocateDense<PAIR>(p, tile, rank);
+    const DenseSeg& sg = p.seg[t.seg];
+    const int scl = (sg.n / 2 + t.n0 / 16) & ~15;
+#pragma unroll 1
+    for (int k = 0; k < kcount; ++k) {
+      if (!first_round && !BarWait(empty0 + slot * 8, parity, ctl)) return;
+      const uint32_t dst = ring + static_cast<uint32_t>(slot) * R::kSlot, bar = full0 + slot * 8;
+      if (ElectOne()) {
+        BarExpect(bar, R::kSlot);
+        if constexpr (MODE == kNvfp4) {
+          TmaLoad<false>(dst, &p.wmap[t.seg], t.n0 / 2, (kbeg + k) * R::kRows, bar);
+          TmaLoad<false>(dst + R::kRows * 64, &p.smap[t.seg], scl, (kbeg + k) * R::kRows, bar);
+        } else {
+          TmaLoad<false>(dst, &p.wmap[t.seg], t.n0, (kbeg + k) * R::kRows, bar);
+        }
+      }
+      __syncwarp();
+      if (++slot == R::kDepth) {
+        slot = 0;
+        parity ^= 1u;
+        first_round = false;
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------ dequantising warps
+// A warp owns rows 8 w .. 8 w + 7 of its group's stages, all 128 columns.  A lane owns the 16 columns
+// 16 (q + 4 a) of two of them (rows 2 (2 i + j) + par, i = 0, 1), with q = lane % 4, par = lane / 4 % 2, j = lane / 16
+// and a = lane / 8 % 2 exclusive-or par.  That order keeps the 16-byte stores free of bank conflicts (the eight lanes of
+// a store phase are four even chunks of an even and four of an odd row, which the swizzle moves apart) and the ring's
+// loads too (the two rows' halves lie side by side in the banks).  These warps have no copies of their own in flight: the proxy fence that follows their stores waits for
+// a thread's outstanding copies as well, so a warp that did both ran at one memory latency per stage (0.55 us, whatever
+// the depth of its ring).
+template <int MODE, bool SCALED, bool PAIR, int KS>
+__device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int warp, int group, int lane, int rank, int kcount, int first_tile,
+                                            int tile_step, uint32_t ring, uint32_t stage0, uint32_t block_bytes) {
+  using R = RawRing<MODE, KS>;
+  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), rfull0 = Smem(&ctl.raw_full[0]), rempty0 = Smem(&ctl.raw_empty[0]);
+  const int q = lane & 3, par = (lane >> 2) & 1, a = ((lane >> 3) & 1) ^ par, jj = lane >> 4, g = q + 4 * a;
+  // where the lane's chunks go: row r = 4 i + 2 jj + par of the warp's eight, chunks 2 q and 2 q + 1 exclusive-or r
+  const int r0 = 2 * jj + par;
+  const uint32_t st0 = stage0 + static_cast<uint32_t>(a * (kABytes / 2) + warp * 1024 + r0 * 128 + (((2 * q) ^ r0) * 16));
+  const uint32_t row0 = static_cast<uint32_t>(warp * 8 + r0);
+  const uint32_t rd_w = ring + row0 * (MODE == kNvfp4 ? 64 : 128) + static_cast<uint32_t>(g * (MODE == kNvfp4 ? 8 : 16));
+  int stage = group % p.stages, slot = group % R::kDepth, tile = first_tile, k = group;
+  uint32_t parity = static_cast<uint32_t>(group / p.stages) & 1u, rparity = 0;
+  bool first_round = group < p.stages;
+  auto next_tile = [&]() {  // the stages alternate between the groups across tile boundaries too
+    while (k >= kcount && tile < p.tiles) {
+      k -= kcount;
+      tile += tile_step;
+    }
+  };
+  next_tile();
+  while (tile < p.tiles) {
+    const TileAt t = LocateDense<PAIR>(p, tile, rank);
+    const DenseSeg& sg = p.seg[t.seg];
+    float cs[SCALED ? 16 : 1];
+    cs[0] = 1.f;
+    if constexpr (SCALED) {
+      const int n = t.n0 + 16 * g;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) cs[i] = (sg.w_scale != nullptr && n + i < sg.n) ? __ldg(sg.w_scale + n + i) : 1.f;
+    }
+    // the scales' offset in their 16 bytes: n0 / 16 is a multiple of eight, N / 2 of sixteen
+    const uint32_t rd_s = ring + R::kRows * 64 + row0 * 16 + static_cast<uint32_t>((t.n0 >> 4) & 8) + static_cast<uint32_t>(g);
+#pragma unroll 1
+    for (; k < kcount; k += kDqGroups) {
+      // both asked at once, the answer of the second needed after the first conversions
+      const bool room = first_round || BarTest(empty0 + stage * 8, parity ^ 1u);
+      if (!BarWait(rfull0 + slot * 8, rparity, ctl)) return;
+      const uint32_t at = static_cast<uint32_t>(slot) * R::kSlot;
+      uint32_t raw[KS][2][4], sc[KS][2];
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if constexpr (MODE == kNvfp4) {
+            uint32_t v[2];
+            Lds64(rd_w + at + j * (kBk * 64) + i * 256, v);
+            raw[j][i][0] = v[0];
+            raw[j][i][1] = v[1];
+            sc[j][i] = Lds8(rd_s + at + j * (kBk * 16) + i * 64);
+          } else {
+            Lds128(rd_w + at + j * (kBk * 128) + i * 512, raw[j][i]);
+          }
+        }
+      }
+      uint32_t dst = st0 + static_cast<uint32_t>(stage * KS) * block_bytes;
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+        uint32_t o[2][8];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          uint32_t h[8];
+          if constexpr (MODE == kNvfp4) {
+            uint32_t lo[4], hi[4], s, unused;
+            CvtE4m3x4(sc[j][i] * 0x101u, s, unused);
+            CvtE2m1x8(raw[j][i][0], lo);
+            CvtE2m1x8(raw[j][i][1], hi);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              h[e] = Hmul2(lo[e], s);
+              h[4 + e] = Hmul2(hi[e], s);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) CvtE4m3x4(raw[j][i][e], h[2 * e], h[2 * e + 1]);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[i][e] = ToBf16<SCALED>(h[e], cs[SCALED ? 2 * e : 0], cs[SCALED ? 2 * e + 1 : 0]);
+        }
+        if (j == 0 && !room && !BarWait(empty0 + stage * 8, parity ^ 1u, ctl)) return;
+        // rows r0 and r0 + 4: the chunk index changes by bit 0 (second half of the columns) and bit 2 (row)
+        Sts128(dst, o[0]);
+        Sts128(dst ^ 16u, o[0] + 4);
+        Sts128((dst + 512) ^ 64u, o[1]);
+        Sts128((dst + 512) ^ 80u, o[1] + 4);
+        dst += block_bytes;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      // the raw slot is given back only here, behind stores that depend on its loads: the compiler is free to move a
+      // plain shared-memory load past an arrival, and did so (stages overwritten before they were read)
+      if (lane == 0) {
+        BarArrive(rempty0 + slot * 8);
+        BarArriveLeader<PAIR>(full0 + stage * 8);
+      }
+      slot += kDqGroups;
+      if (slot >= R::kDepth) {
+        slot -= R::kDepth;
+        rparity ^= 1u;
+      }
+      stage += kDqGroups;
+      if (stage >= p.stages) {
+        stage -= p.stages;
+        parity ^= 1u;
+        first_round = false;
+      }
+    }
+    next_tile();
+  }
+}
+
+template <int MODE>
+constexpr int DenseThreads() {
+  return 32 * (kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps * kDqGroups));
+}
+
+// SPLIT: K is split over the CTAs of the cluster, one tile per cluster.  PAIR: see above.  Never both.
+template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
+__global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const __grid_constant__ DenseParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Ctl ctl;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t smem = (Smem(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const smem_ptr = smem_raw + (smem - Smem(smem_raw));
+  const int csize = (PAIR || SPLIT) ? static_cast<int>(cg::this_cluster().num_blocks()) : 1;
+  const int rank = (PAIR || SPLIT) ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
+  const int first_tile = static_cast<int>(blockIdx.x) / csize, tile_step = static_cast<int>(gridDim.x) / csize;
+  const int kbeg = SPLIT ? rank * p.ksteps / csize : 0;
+  const int kcount = SPLIT ? (rank + 1) * p.ksteps / csize - kbeg : p.ksteps;
+  const int xrows = PAIR ? p.bm / 2 : p.bm;
+  const uint32_t block_bytes = static_cast<uint32_t>(kABytes + xrows * kBk * 2), stage_bytes = block_bytes * KS;
+  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), accf0 = Smem(&ctl.acc_full[0]), acce0 = Smem(&ctl.acc_empty[0]);
+  int acc_cols = 32;
+  while (acc_cols < 2 * p.bm) acc_cols *= 2;
+
+  if (tid == 0) {
+    for (int i = 0; i < p.stages; ++i) {
+      BarInit(full0 + i * 8, 1 + (MODE == kBf16 ? 0 : kDqWarps * (PAIR ? 2 : 1)));
+      BarInit(empty0 + i * 8, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      BarInit(accf0 + i * 8, 1);
+      BarInit(acce0 + i * 8, 4 * (PAIR ? 2 : 1));
+    }
+    for (int i = 0; MODE != kBf16 && i < RawRing<MODE, KS>::kDepth; ++i) {
+      BarInit(Smem(&ctl.raw_full[i]), MODE == kFp8 || p.raw_tensor ? 1 : 32 * kLoadWarps);
+      BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
+    }
+    ctl.fault = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 5) {
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(Smem(&ctl.tmem)), "r"(acc_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(Smem(&ctl.tmem)), "r"(acc_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+  }
+  FenceBefore();
+  __syncthreads();
+  if constexpr (PAIR) cg::this_cluster().sync();  // the leader's barriers exist before the peer arrives on them
+  FenceAfter();
+  const uint32_t tmem = ctl.tmem;
+
+  if (warp < 4) {
+    // ---- epilogue: lane = column 32 warp + lane of the tile, tensor memory columns = rows of x
+    int it = 0;
+    for (int tile = first_tile; tile < p.tiles; tile += tile_step, ++it) {
+      const int b = it & 1;
+      const bool good = BarWait(accf0 + b * 8, static_cast<uint32_t>((it >> 1) & 1), ctl);
+      FenceAfter();
+      const TileAt t = LocateDense<PAIR>(p, tile, rank);
+      const uint32_t src = tmem + (static_cast<uint32_t>(32 * warp) << 16) + static_cast<uint32_t>(b * p.bm);
+      const int n = t.n0 + 32 * warp + lane;
+      uint16_t* out = nullptr;
+      size_t width = 0;
+      if constexpr (!SPLIT) {
+        const DenseSeg& sg = p.seg[t.seg];
+        int j = sg.out_begin;
+        for (int i = j + 1; i < sg.out_end; ++i) {
+          if (n >= p.col_begin[i]) j = i;
+        }
+        width = static_cast<size_t>(p.width[j]);
+        if (n < sg.n) out = p.out[j] + static_cast<size_t>(t.m0) * width + (n - p.col_begin[j]);
+      }
+      for (int c = 0; c < p.bm; c += 16) {
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+              "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(src + static_cast<uint32_t>(c)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (!good) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = 0x7FFFFFFFu;
+        }
+        if constexpr (SPLIT) {
+          float* part = reinterpret_cast<float*>(smem_ptr) + c * kBn + 32 * warp + lane;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) part[i * kBn] = __uint_as_float(v[i]);
+        } else if (out != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            if (t.m0 + c + i < p.M) out[static_cast<size_t>(c + i) * width] = __bfloat16_as_ushort(__float2bfloat16(__uint_as_float(v[i])));
+          }
+        }
+      }
+      FenceBefore();
+      __syncwarp();
+      if (lane == 0) BarArriveLeader<PAIR>(acce0 + b * 8);
+      if (!good) break;
+    }
+  } else if (warp == 4) {
+    // ---- x (and BF16 weights)
+    int stage = 0, round = 0;
+    bool good = true;
+    const uint32_t mine = static_cast<uint32_t>(KS * (xrows * kBk * 2 + (MODE == kBf16 ? kABytes : 0)));
+    for (int tile = first_tile; tile < p.tiles && good; tile += tile_step) {
+      const TileAt t = LocateDense<PAIR>(p, tile, rank);
+      for (int k = 0; k < kcount; ++k) {
+        if (round > 0 && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) {
+          good = false;
+          break;
+        }
+        const uint32_t bar = PAIR ? MapRank(full0 + stage * 8, 0) : full0 + stage * 8;
+        const uint32_t dst = smem + static_cast<uint32_t>(stage) * stage_bytes;
+        if (ElectOne()) {
+          if (rank == 0 || !PAIR) BarExpect(full0 + stage * 8, PAIR ? 2 * mine : mine);
+#pragma unroll
+          for (int j = 0; j < KS; ++j) {
+            const int k0 = ((kbeg + k) * KS + j) * kBk;
+            const uint32_t at = dst + static_cast<uint32_t>(j) * block_bytes;
+            if constexpr (MODE == kBf16) {
+              TmaLoad<PAIR>(at, &p.wmap[t.seg], t.n0, k0, bar);
+              TmaLoad<PAIR>(at + kABytes / 2, &p.wmap[t.seg], t.n0 + 64, k0, bar);
+            }
+            TmaLoad<PAIR>(at + kABytes, &p.xmap, k0, t.m0 + (PAIR ? rank * xrows : 0), bar);
+          }
+        }
+        __syncwarp();
+        if (++stage == p.stages) {
+          stage = 0;
+          ++round;
+        }
+      }
+    }
+  } else if (warp == 5) {
+    // ---- MMAs (the leader's, for both CTAs of a pair)
+    if (!PAIR || rank == 0) {
+      // FP32 accumulators, BF16 operands, A MN-major, N = bm, M = 128 (256 across a pair)
+      const uint32_t idesc = 0x10u | (1u << 7) | (1u << 10) | (1u << 15) | (static_cast<uint32_t>(p.bm >> 3) << 17) |
+                             (static_cast<uint32_t>(PAIR ? 16 : 8) << 24);
+      const unsigned long long a0 = SmemDesc(smem, kABytes / 2, 1024), b0 = SmemDesc(smem + kABytes, 16, 1024);
+      int stage = 0, it = 0;
+      uint32_t parity = 0;
+      bool good = true, ready = false;
+      for (int tile = first_tile; tile < p.tiles && good; tile += tile_step, ++it) {
+        const int b = it & 1;
+        if (it >= 2 && !BarWait(acce0 + b * 8, static_cast<uint32_t>(((it >> 1) - 1) & 1), ctl)) break;
+        FenceAfter();
+        const uint32_t d = tmem + static_cast<uint32_t>(b * p.bm);
+        for (int k = 0; k < kcount; ++k) {
+          if (!ready && !BarWait(full0 + stage * 8, parity, ctl)) {
+            good = false;
+            break;
+          }
+          FenceAfter();
+          const uint32_t off = static_cast<uint32_t>(stage) * stage_bytes >> 4, done = empty0 + stage * 8;
+          if (++stage == p.stages) {
+            stage = 0;
+            parity ^= 1u;
+          }
+          ready = BarTest(full0 + stage * 8, parity);  // asked before the MMAs are issued, needed after
+          if (ElectOne()) {
+#pragma unroll
+            for (int j = 0; j < KS; ++j) {
+#pragma unroll
+              for (int i = 0; i < kBk / 16; ++i) {
+                const uint32_t at = off + j * (block_bytes >> 4);
+                MmaSs<PAIR>(d, a0 + at + i * (2048 >> 4), b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
+              }
+            }
+            MmaCommit<PAIR>(done);
+            if (k == kcount - 1) MmaCommit<PAIR>(accf0 + b * 8);
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else if constexpr (MODE != kBf16) {
+    const uint32_t ring = smem + static_cast<uint32_t>(p.stages) * stage_bytes;
+    if (warp < kFirstDqWarp) {
+      if (MODE == kFp8 || p.raw_tensor) {
+        if (warp == 6) LoadTensor<MODE, PAIR, KS>(p, ctl, rank, kbeg, kcount, first_tile, tile_step, ring);
+      } else if constexpr (MODE == kNvfp4) {
+        LoadNvfp4Pieces<PAIR, KS>(p, ctl, tid - 6 * 32, rank, kbeg, kcount, first_tile, tile_step, ring);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+      }
+    } else {
+      const int w = warp - kFirstDqWarp;
+      DequantRole<MODE, SCALED, PAIR, KS>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
+    }
+  }
+
+  if constexpr (SPLIT) {
+    // the ranks' sums meet: rank r finishes rows [r bm / C, (r + 1) bm / C) of the tile, adding in rank order
+    cg::cluster_group cluster = cg::this_cluster();
+    FenceBefore();
+    cluster.sync();
+    const TileAt t = LocateDense<PAIR>(p, first_tile, rank);
+    const DenseSeg& sg = p.seg[t.seg];
+    const float* part = reinterpret_cast<const float*>(smem_ptr);
+    const int r0 = rank * p.bm / csize, r1 = (rank + 1) * p.bm / csize;
+    const int c = (tid & 31) * 4, n = t.n0 + c;  // widths are multiples of eight: four columns belong to one output
+    if (n < sg.n) {
+      int j = sg.out_begin;
+      for (int i = j + 1; i < sg.out_end; ++i) {
+        if (n >= p.col_begin[i]) j = i;
+      }
+      uint16_t* const out = p.out[j] + (n - p.col_begin[j]);
+      const size_t width = static_cast<size_t>(p.width[j]);
+      for (int m = r0 + warp; m < r1 && t.m0 + m < p.M; m += static_cast<int>(blockDim.x) / 32) {
+        float4 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (r < csize) v[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, r) + m * kBn + c);
+        }
+        float4 s = v[0];
+#pragma unroll
+        for (int r = 1; r < 8; ++r) {
+          if (r < csize) {
+            s.x += v[r].x;
+            s.y += v[r].y;
+            s.z += v[r].z;
+            s.w += v[r].w;
+          }
+        }
+        uint16_t* const dst = out + static_cast<size_t>(t.m0 + m) * width;
+        dst[0] = __bfloat16_as_ushort(__float2bfloat16(s.x));
+        dst[1] = __bfloat16_as_ushort(__float2bfloat16(s.y));
+        dst[2] = __bfloat16_as_ushort(__float2bfloat16(s.z));
+        dst[3] = __bfloat16_as_ushort(__float2bfloat16(s.w));
+      }
+    }
+  }
+  if (ctl.fault) __nanosleep(100000);  // copies of a CTA that gave up may still be landing
+  FenceBefore();
+  __syncthreads();
+  if constexpr (PAIR || SPLIT) cg::this_cluster().sync();  // no CTA leaves while a peer still reads its shared memory
+  if (warp == 5) {
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(acc_cols) : "memory");
+    } else {
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(acc_cols) : "memory");
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------ host
+using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeFn Encoder() {
+  static const EncodeFn fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<EncodeFn>(f);
+  }();
+  return fn;
+}
+
+// rows x cols elements of `elem` bytes (2: BF16, boxes swizzled in 128 bytes; 1: bytes, plain), row-major
+bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols) {
+  const cuuint64_t dims[2] = {cols, rows}, strides[1] = {pitch_bytes};
+  const cuuint32_t box[2] = {box_cols, box_rows}, step[2] = {1, 1};
+  const EncodeFn fn = Encoder();
+  return fn != nullptr &&
+         fn(map, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, step,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, elem == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+constexpr int kSmemLimit = 232448 - 1024 - static_cast<int>(sizeof(Ctl)) - 64;
+
+int RawBytes(int mode) { return mode == kFp8 ? RawRing<kFp8, 1>::kBytes : mode == kNvfp4 ? RawRing<kNvfp4, 1>::kBytes : 0; }
+int BlocksFor(int mode, int xrows) { return (kSmemLimit - RawBytes(mode)) / (kABytes + xrows * kBk * 2); }
+
+template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
+cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream) {
+  static const cudaError_t configured = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                             kSmemLimit + 1024);
+  if (configured != cudaSuccess) return configured;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(static_cast<unsigned>(DenseThreads<MODE>()));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS>, p);
+}
+
+template <int MODE, bool SCALED>
+cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, int ctas, int cluster, size_t smem, cudaStream_t stream) {
+  if (pair) return ks == 2 ? LaunchOne<MODE, SCALED, true, false, 2>(p, ctas, 2, smem, stream) : LaunchOne<MODE, SCALED, true, false, 1>(p, ctas, 2, smem, stream);
+  if (cluster > 1)
+    return ks == 2 ? LaunchOne<MODE, SCALED, false, true, 2>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, true, 1>(p, ctas, cluster, smem, stream);
+  return ks == 2 ? LaunchOne<MODE, SCALED, false, false, 2>(p, ctas, 1, smem, stream) : LaunchOne<MODE, SCALED, false, false, 1>(p, ctas, 1, smem, stream);
+}
+
+}  // namespace
+
+// Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200,
+// K = 5120; us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair
+// 0.13 + 0.00098 bm (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.40 where the rows
+// are loaded in 8-byte pieces); around the blocks 4 + 0.008 bm, and 1 + 0.01 bm more where ranks add up.  More row
+// tiles than needed are tried because they can fill the last wave better (509 rows, N = 10240: 3 x 192 56 us,
+// 2 x 256 61 us).
+DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count) {
+  DenseTcPlan best;
+  double best_cost = 1e30, bytes = 0;
+  bool pieces = false;
+  for (int s = 0; s < p.nseg; ++s) {
+    bytes += static_cast<double>(p.seg[s].total_bytes);
+    pieces = pieces || (mode == kNvfp4 && p.seg[s].pitch % 16 != 0);
+  }
+  const int64_t blocks = (p.K + kBk - 1) / kBk, least = (m + 255) / 256;
+  for (int pair = 0; pair <= 1; ++pair) {
+    int64_t n_tiles = 0;
+    for (int s = 0; s < p.nseg; ++s) n_tiles += (p.seg[s].n + (pair ? 255 : 127)) / (pair ? 256 : 128);
+    const int unit = pair ? 32 : 16;
+    for (int64_t mt = least; mt <= 2 * least + 2 && mt <= m; ++mt) {
+      const int bm = static_cast<int>(((m + mt - 1) / mt + unit - 1) / unit * unit);
+      if (bm > 256 || (pair && bm < 64)) continue;
+      const int64_t tiles = n_tiles * ((m + bm - 1) / bm);
+      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : pieces ? 0.40 : 0.24);
+      for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
+        // clusters of more than two CTAs do not fill every GPC
+        const int64_t slots = pair || split == 2 ? sm_count / 2 : split == 1 ? sm_count : sm_count * 9 / (10 * split);
+        const int64_t waves = (tiles + slots - 1) / std::max<int64_t>(slots, 1);
+        if (split > 1 && waves > 1) break;
+        const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
+        const double cost = work + 4 + 0.008 * bm + (split > 1 ? 1 + 0.01 * bm : 0);
+        if (cost < best_cost) {
+          best_cost = cost;
+          best.bm = bm;
+          best.split = split;
+          best.pair = pair;
+        }
+      }
+    }
+  }
+  return best;
+}
+
+// 16-byte rows of x; weights that a tensor map describes, or NVFP4 ones in whole 128-column groups; every output a
+// multiple of eight columns.
+bool DenseTcEligible(int mode, const GemmParams& p) {
+  if (p.K % 8 != 0 || reinterpret_cast<uintptr_t>(p.x) % 16 != 0) return false;
+  for (int s = 0; s < p.nseg; ++s) {
+    const Segment& sg = p.seg[s];
+    if (reinterpret_cast<uintptr_t>(sg.w) % 16 != 0) return false;
+    if (sg.n % (mode == kNvfp4 ? 128 : mode == kFp8 ? 16 : 8) != 0) return false;
+  }
+  const int n_out = p.seg[p.nseg - 1].out_end;
+  for (int o = 0; o < n_out; ++o) {
+    if (p.out[o] == nullptr || p.width[o] % 8 != 0) return false;
+  }
+  return Encoder() != nullptr;
+}
+
+void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+  if (m > INT_MAX / 2) throw std::runtime_error("SkinnyGemm(dense): too many rows");
+  if (plan.bm < 16 || plan.bm > 256 || plan.bm % (plan.pair ? 32 : 16) != 0 || plan.split < 1 || plan.split > 8 || (plan.pair && plan.split != 1) || plan.ks < 0 || plan.ks > 2)
+    throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
+  DenseParams p = {};
+  p.nseg = g.nseg;
+  p.M = static_cast<int>(m);
+  p.K = g.K;
+  p.bm = plan.bm;
+  const int xrows = plan.pair ? p.bm / 2 : p.bm;
+  const int blocks = BlocksFor(mode, xrows), ks = plan.ks > 0 ? plan.ks : blocks >= 6 ? 2 : 1;
+  p.ksteps = (g.K + kBk * ks - 1) / (kBk * ks);
+  if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
+    throw std::runtime_error("SkinnyGemm(dense): cannot describe x to the copy engine");
+  bool scaled = false;
+  p.raw_tensor = 1;
+  int n_tiles = 0;
+  for (int s = 0; s < g.nseg; ++s) {
+    const Segment& sg = g.seg[s];
+    p.seg[s] = {sg.w, sg.w_scale, sg.pitch, sg.total_bytes, sg.n, n_tiles, sg.out_begin, sg.out_end};
+    n_tiles += (sg.n + (plan.pair ? 255 : 127)) / (plan.pair ? 256 : 128);
+    scaled = scaled || sg.w_scale != nullptr;
+    p.raw_tensor = p.raw_tensor && sg.pitch % 16 == 0;
+  }
+  for (int s = 0; s < g.nseg && p.raw_tensor; ++s) {
+    const Segment& sg = g.seg[s];
+    const uint64_t K = static_cast<uint64_t>(g.K), pitch = static_cast<uint64_t>(sg.pitch);
+    const bool ok = mode == kBf16  ? Encode(&p.wmap[s], sg.w, 2, K, static_cast<uint64_t>(sg.n), pitch, kBk, 64)
+                    : mode == kFp8 ? Encode(&p.wmap[s], sg.w, 1, K, static_cast<uint64_t>(sg.n), pitch, kBk * ks, kBn)
+                                   : Encode(&p.wmap[s], sg.w, 1, K, pitch, pitch, kBk * ks, kBn / 2) && Encode(&p.smap[s], sg.w, 1, K, pitch, pitch, kBk * ks, 16);
+    if (!ok) throw std::runtime_error("SkinnyGemm(dense): cannot describe the weight to the copy engine");
+  }
+  const int n_out = g.seg[g.nseg - 1].out_end;
+  for (int o = 0; o < n_out; ++o) {
+    p.out[o] = g.out[o];
+    p.col_begin[o] = g.col_begin[o];
+    p.width[o] = g.width[o];
+  }
+  p.m_tiles = static_cast<int>((m + p.bm - 1) / p.bm);
+  if (static_cast<int64_t>(p.m_tiles) * n_tiles > INT_MAX / 16) throw std::runtime_error("SkinnyGemm(dense): too many tiles");
+  p.tiles = p.m_tiles * n_tiles;
+  const int cluster = plan.pair ? 2 : std::min(plan.split, p.ksteps);
+  p.stages = std::min(kMaxStages, blocks / ks);
+  // the dequantising groups take the stages in turn: fewer stages than groups would run off the ring
+  if (p.stages < kDqGroups) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * (kABytes + xrows * kBk * 2) + RawBytes(mode);
+  const int slots = std::max(1, DeviceSmCount() / cluster);
+  const int ctas = cluster * (cluster > 1 && !plan.pair ? p.tiles : std::min(p.tiles, slots));
+  cudaError_t err;
+  if (mode == kBf16) {
+    err = LaunchMode<kBf16, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+  } else if (mode == kFp8) {
+    err = scaled ? LaunchMode<kFp8, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream) : LaunchMode<kFp8, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+  } else {
+    err = scaled ? LaunchMode<kNvfp4, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream)
+                 : LaunchMode<kNvfp4, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+  }
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
+}
+
+}  // namespace qfg

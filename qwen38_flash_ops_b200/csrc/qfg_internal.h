@@ -238,13 +238,25 @@ struct DequantParams {
 };
 cudaError_t LaunchDequant(const DequantParams& p, cudaStream_t stream);
 
-// dense_gemm.cc: calls with more than `dense_rows` rows (an option of the node; 0 disables the branch).
+// Calls with more than `dense_rows` rows (an option of the node; 0 disables it) leave the streaming kernels: dense_tc.cu,
+// or dense_gemm.cc for the layouts that does not take.
 // The defaults are where the branch starts to win on a B200 (K = 5120): BF16 weights need no dequantisation
 // pass, so two streaming passes already lose (N = 2048: 37.7 us against 16.3); FP8 pays 48.5 us at N = 10240
 // against 35 us per eight rows; NVFP4 pays 89 us at N = 17408, which three passes (105 us) exceed.
 constexpr int DenseRowsDefault(int mode) { return mode == kNvfp4 ? 16 : 8; }
 bool DenseEligible(const GemmParams& p);
 void LaunchDenseGemm(int mode, const GemmParams& p, int64_t m, cudaStream_t stream);  // throws std::runtime_error
+
+// dense_tc.cu: the same calls in one kernel, dequantising into shared memory.
+struct DenseTcPlan {
+  int bm = 0;     // rows of x per tile: a multiple of 16 (32 for pairs), at most 256
+  int split = 1;  // CTAs (a cluster) that share the K range of a tile
+  int pair = 0;   // two CTAs per tile of 256 columns
+  int ks = 0;     // blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room
+};
+bool DenseTcEligible(int mode, const GemmParams& p);
+DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count);
+void LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);  // throws std::runtime_error
 
 // untile_hc.cu
 cudaError_t LaunchUntileHc(bool fp8, const void* w, void* out, const float* scale, int kind, cudaStream_t stream);
