@@ -294,6 +294,13 @@ void Run(const qfg_skinny_gemm& op, Prepared& pr, int64_t m, cudaStream_t stream
     }
     return;
   }
+  const int shared_rows = op.dense_rows < 0 ? qfg::kDenseSharedRows : op.dense_rows;
+  if (pr.params.fuse && shared_rows > 0 && m > shared_rows && qfg::DenseSharedEligible(pr.mode, pr.params)) {
+    const qfg::DenseTcPlan plan =
+        op.dense_plan.bm > 0 ? op.dense_plan : qfg::ChooseDenseSharedPlan(pr.params, m, pr.plan_in.sm_count);
+    qfg::LaunchDenseShared(pr.mode, pr.params, m, plan, stream);
+    return;
+  }
   const qfg::Plan plan = PlanFor(op, pr.plan_in, static_cast<int>(std::min<int64_t>(m, qfg::kMaxRows)));
   qfg::GemmParams base = pr.params;
   int64_t done = 0;

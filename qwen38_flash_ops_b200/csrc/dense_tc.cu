@@ -133,6 +133,18 @@ __device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, Ctl& c) {
   c.fault = 1;
   return false;
 }
+// the same where what is waited for was written by another CTA of the cluster
+__device__ __forceinline__ bool BarWaitCluster(uint32_t a, uint32_t parity, Ctl& c) {
+  for (int i = 0; i < kSpin; ++i) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 255) == 255 && c.fault) return false;
+  }
+  c.fault = 1;
+  return false;
+}
 template <bool PAIR>
 __device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   if constexpr (PAIR) {  // the barrier may be the leader's
@@ -334,7 +346,7 @@ __device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int r
 // loads too (the two rows' halves lie side by side in the banks).  These warps have no copies of their own in flight: the proxy fence that follows their stores waits for
 // a thread's outstanding copies as well, so a warp that did both ran at one memory latency per stage (0.55 us, whatever
 // the depth of its ring).
-template <int MODE, bool SCALED, bool PAIR, int KS>
+template <int MODE, bool SCALED, bool PAIR, int KS, int GROUPS>
 __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int warp, int group, int lane, int rank, int kcount, int first_tile,
                                             int tile_step, uint32_t ring, uint32_t stage0, uint32_t block_bytes) {
   using R = RawRing<MODE, KS>;
@@ -368,7 +380,7 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
     // the scales' offset in their 16 bytes: n0 / 16 is a multiple of eight, N / 2 of sixteen
     const uint32_t rd_s = ring + R::kRows * 64 + row0 * 16 + static_cast<uint32_t>((t.n0 >> 4) & 8) + static_cast<uint32_t>(g);
 #pragma unroll 1
-    for (; k < kcount; k += kDqGroups) {
+    for (; k < kcount; k += GROUPS) {
       // both asked at once, the answer of the second needed after the first conversions
       const bool room = first_round || BarTest(empty0 + stage * 8, parity ^ 1u);
       if (!BarWait(rfull0 + slot * 8, rparity, ctl)) return;
@@ -429,12 +441,12 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
         BarArrive(rempty0 + slot * 8);
         BarArriveLeader<PAIR>(full0 + stage * 8);
       }
-      slot += kDqGroups;
+      slot += GROUPS;
       if (slot >= R::kDepth) {
         slot -= R::kDepth;
         rparity ^= 1u;
       }
-      stage += kDqGroups;
+      stage += GROUPS;
       if (stage >= p.stages) {
         stage -= p.stages;
         parity ^= 1u;
@@ -637,7 +649,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       }
     } else {
       const int w = warp - kFirstDqWarp;
-      DequantRole<MODE, SCALED, PAIR, KS>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
+      DequantRole<MODE, SCALED, PAIR, KS, kDqGroups>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
     }
   }
 
@@ -693,6 +705,341 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(acc_cols) : "memory");
     }
   }
+}
+
+// ------------------------------------------------------------------------------ SharedExpertDown over many rows
+// out = routed + bf16(bf16(swish_mul(g, u) @ W) * gate), gate = bf16(sigmoid(bf16(gx . gw))), in the same tiles and
+// roles.  A tile of 128 columns is one of N / 128 that need the same rows of swish_mul, so the C CTAs of a cluster
+// (neighbouring column tiles, the same rows) each evaluate 1 / C of them: a warp or two per block of 64 k compute their
+// CTA's share, store it into this CTA's stage and send it to the others' with bulk copies between shared memories,
+// which count themselves in on the receivers' barriers.  A stage is free when the MMAs of all C CTAs have read it
+// (multicast commits).  The gates are shared the same way, by the warps that have nothing to do yet.  A call is a few
+// trips to memory deep and little else, so every phase spreads over as many warps as it can: all of them finish the
+// sums (the four epilogue warps alone, 16 rows at a time, took half of a call).
+//
+// The streaming kernels that served these calls eight rows at a time took 1256 us for 777 rows of FP8 640 x 2560; this
+// one 27.  It is bound by swish_mul and latency: 0.6 us per block of 64 k at 160 rows against 0.17 us of MMAs.
+struct DenseShared {
+  DenseParams d;
+  const uint16_t *g, *u, *gx, *gw, *routed;
+  int gk, cluster;
+};
+
+constexpr int kSwishWarps = 8;  // sixteen, at 64 registers a thread, measured no faster (27.0 us, and 5-10 % slower on small calls)
+template <int MODE>
+constexpr int SharedThreads() {
+  return 32 * (kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps) + kSwishWarps);
+}
+
+__device__ __forceinline__ float RoundBf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
+__device__ __forceinline__ float SigmoidBf16(float a) {
+  const float e = expf(-fabsf(a));
+  return RoundBf16(a > 0.0f ? 1.0f / (1.0f + e) : e / (1.0f + e));
+}
+// sigmoid(a) before its rounding, for a BF16 a: exp(-|a|) as 2^y with y = -|a| h exact (h: the upper 16 bits of log2 e,
+// against the eight of a) and the rest of the exponent to first order, then a reciprocal; next to zero, where a / 4 can
+// lie on a rounding boundary to within less than an ulp, the Taylor polynomial.  Fifteen instructions where expf and an
+// IEEE division take over forty; after rounding the same for each of the 65536 inputs.
+__device__ __forceinline__ float SigmoidOfBf16(float a) {
+  const float x = fminf(fabsf(a), 256.f);  // 2^-369 is zero
+  constexpr float h = 47274.f / 32768.f, rest = 4.888495e-06f;  // log2 e = h + 7.052608e-6; that times ln 2
+  float e, r;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(x * -h));
+  e = fmaf(e, x * -rest, e);
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  const float far = (a > 0.0f ? 1.0f : e) * r, near = fmaf(a, fmaf(a * a, -1.f / 48.f, 0.25f), 0.5f);
+  return x < 0.03125f ? near : far;
+}
+__device__ __forceinline__ uint32_t PackBf16(float lo, float hi) {
+  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&b);
+}
+__device__ __forceinline__ uint32_t MulBf16x2(uint32_t a, uint32_t b) {  // one rounding, like the FP32 product rounded
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float Lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float Hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+__device__ __forceinline__ uint32_t SwishMul2(uint32_t g2, uint32_t u2) {  // two BF16 per word
+  return MulBf16x2(MulBf16x2(g2, PackBf16(SigmoidOfBf16(Lo(g2)), SigmoidOfBf16(Hi(g2)))), u2);
+}
+
+// Warps that share a block.  A barrier's parity tells a phase from the next only, so a warp must have seen a stage's
+// previous block consumed (or a later one) before it waits for the stage again: no more blocks in hand than stages.
+__device__ __forceinline__ int SwishWarpsPerBlock(int stages) { return kSwishWarps / (stages >= 8 ? 8 : stages >= 4 ? 4 : stages >= 2 ? 2 : 1); }
+
+__device__ __forceinline__ void SwishRole(const DenseShared& q, Ctl& ctl, int warp, int lane, int rank, int m0, uint32_t smem, uint32_t block_bytes) {
+  const DenseParams& p = q.d;
+  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]);
+  const int per_block = SwishWarpsPerBlock(p.stages), blocks = kSwishWarps / per_block, sub = warp / blocks;
+  const int part = p.bm / q.cluster, chunk = lane & 7, rsub = lane >> 3;
+  // this warp's rows of the tile, in groups of eight: [first, last)
+  const int first = rank * part + sub * (part >> 3) / per_block * 8, last = rank * part + (sub + 1) * (part >> 3) / per_block * 8;
+  for (int k = warp % blocks; k < p.ksteps; k += blocks) {
+    const int stage = k % p.stages, round = k / p.stages;
+    const int col = k * kBk + chunk * 8;
+    const uint32_t dst = smem + static_cast<uint32_t>(stage) * block_bytes + kABytes;
+    bool free = round == 0;
+    constexpr int kBatch = 4;
+    for (int r0 = first; r0 < last; r0 += 4 * kBatch) {
+      uint4 gv[kBatch], uv[kBatch];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int r = r0 + 4 * j + rsub, m = m0 + r;
+        gv[j] = uv[j] = make_uint4(0, 0, 0, 0);
+        if (r < last && m < p.M && col < p.K) {  // K is a multiple of eight
+          gv[j] = __ldg(reinterpret_cast<const uint4*>(q.g + static_cast<size_t>(m) * p.K + col));
+          uv[j] = __ldg(reinterpret_cast<const uint4*>(q.u + static_cast<size_t>(m) * p.K + col));
+        }
+      }
+      if (!free && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
+      free = true;
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int r = r0 + 4 * j + rsub;
+        if (r < last) {
+          const uint32_t v[4] = {SwishMul2(gv[j].x, uv[j].x), SwishMul2(gv[j].y, uv[j].y), SwishMul2(gv[j].z, uv[j].z), SwishMul2(gv[j].w, uv[j].w)};
+          Sts128(dst + static_cast<uint32_t>(r * 128 + ((chunk ^ (r & 7)) * 16)), v);
+        }
+      }
+    }
+    // a warp without rows of its own still may not count itself in on a stage that is in use
+    if (!free && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (ElectOne()) {
+      const uint32_t bytes = static_cast<uint32_t>((last - first) * 128), bar = full0 + stage * 8, src = dst + static_cast<uint32_t>(first * 128);
+      BarExpect(bar, bytes * static_cast<uint32_t>(q.cluster - 1));  // what this warp's counterparts in the other CTAs send
+      for (int i = 1; i < q.cluster && bytes > 0; ++i) {
+        const uint32_t peer = static_cast<uint32_t>((rank + i) % q.cluster);
+        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(MapRank(src, peer)), "r"(src),
+                     "r"(bytes), "r"(MapRank(bar, peer))
+                     : "memory");
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// This CTA's share of the gates, by `warps` warps, to every CTA of the cluster: asynchronous stores that count their
+// bytes in on the receiver's barrier.
+__device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, uint32_t bar, int warp, int warps, int lane, int rank, int m0) {
+  const int part = q.d.bm / q.cluster, p0 = rank * part;
+  const bool vec = reinterpret_cast<uintptr_t>(q.gx) % 16 == 0 && reinterpret_cast<uintptr_t>(q.gw) % 16 == 0 && q.gk % 8 == 0;
+  constexpr int kRows = 2, kAhead = 5;
+  for (int r0 = warp * kRows; r0 < part; r0 += warps * kRows) {
+    float acc[kRows] = {0.f, 0.f};
+    const int m = m0 + p0 + r0;
+    if (vec) {
+      const int chunks = q.gk >> 3;
+      const uint4* gw = reinterpret_cast<const uint4*>(q.gw);
+      for (int c0 = lane; c0 < chunks; c0 += 32 * kAhead) {
+        uint4 w[kAhead], x[kRows][kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const int c = c0 + 32 * i;
+          w[i] = c < chunks ? __ldg(gw + c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int j = 0; j < kRows; ++j) {
+            x[j][i] = c < chunks && m + j < q.d.M ? __ldg(reinterpret_cast<const uint4*>(q.gx + static_cast<size_t>(m + j) * q.gk) + c)
+                                                  : make_uint4(0, 0, 0, 0);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+          for (int j = 0; j < kRows; ++j) {
+            const uint32_t xx[4] = {x[j][i].x, x[j][i].y, x[j][i].z, x[j][i].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              acc[j] += Lo(xx[e]) * Lo(ww[e]);
+              acc[j] += Hi(xx[e]) * Hi(ww[e]);
+            }
+          }
+        }
+      }
+    } else {
+      for (int c = lane; c < q.gk; c += 32) {
+        const float w = __uint_as_float(static_cast<uint32_t>(q.gw[c]) << 16);
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+          if (m + j < q.d.M) acc[j] += __uint_as_float(static_cast<uint32_t>(q.gx[static_cast<size_t>(m + j) * q.gk + c]) << 16) * w;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
+    }
+    // lane = (peer, row): part is even, so both rows exist
+    const float logit = (lane & 1) ? acc[1] : acc[0];
+    const int peer = lane >> 1;
+    if (peer < q.cluster) {
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
+                       MapRank(Smem(gate + p0 + r0 + (lane & 1)), static_cast<uint32_t>(peer))),
+                   "r"(__float_as_uint(SigmoidBf16(RoundBf16(logit)))), "r"(MapRank(bar, static_cast<uint32_t>(peer)))
+                   : "memory");
+    }
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(const __grid_constant__ DenseShared q) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Ctl ctl;
+  __shared__ float gate[256];
+  __shared__ unsigned long long gate_full;
+  const DenseParams& p = q.d;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t smem = (Smem(smem_raw) + 1023u) & ~1023u;
+  const int C = q.cluster, rank = C > 1 ? static_cast<int>(cg::this_cluster().block_rank()) : 0, group = static_cast<int>(blockIdx.x) / C;
+  const int tile = ((group / p.m_tiles) * C + rank) * p.m_tiles + group % p.m_tiles;  // the columns are padded to whole clusters
+  const TileAt t = LocateDense<false>(p, tile, 0);
+  const uint32_t block_bytes = static_cast<uint32_t>(kABytes + p.bm * kBk * 2);
+  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), accf0 = Smem(&ctl.acc_full[0]);
+  int acc_cols = 32;
+  while (acc_cols < p.bm) acc_cols *= 2;
+
+  if (tid == 0) {
+    for (int i = 0; i < p.stages; ++i) {
+      BarInit(full0 + i * 8, SwishWarpsPerBlock(p.stages) + (MODE == kBf16 ? 1 : kDqWarps));
+      BarInit(empty0 + i * 8, C);
+    }
+    BarInit(accf0, 1);
+    BarInit(Smem(&gate_full), 1);
+    BarExpect(Smem(&gate_full), static_cast<uint32_t>(p.bm) * 4);
+    for (int i = 0; MODE != kBf16 && i < RawRing<MODE, 1>::kDepth; ++i) {
+      BarInit(Smem(&ctl.raw_full[i]), MODE == kFp8 || p.raw_tensor ? 1 : 32 * kLoadWarps);
+      BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
+    }
+    ctl.fault = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(Smem(&ctl.tmem)), "r"(acc_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  FenceBefore();
+  __syncthreads();
+  if (C > 1) cg::this_cluster().sync();  // every CTA's barriers exist
+  FenceAfter();
+  const uint32_t tmem = ctl.tmem;
+  constexpr int kFirstSwish = kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps);
+
+  // first the gates, by the warps that the sums need last
+  constexpr int kGateWarps = MODE == kBf16 ? 6 : 4 + kDqWarps, kSumGroups = (kFirstSwish + kSwishWarps) / 4;
+  const int gate_warp = warp < 4 ? warp : MODE == kBf16 ? (warp == 6 || warp == 7 ? warp - 2 : -1) : warp >= kFirstDqWarp && warp < kFirstSwish ? warp - 4 : -1;
+  if (gate_warp >= 0) GateRole(q, gate, Smem(&gate_full), gate_warp, kGateWarps, lane, rank, t.m0);
+
+  if (warp == 4) {
+    if constexpr (MODE == kBf16) {
+      for (int k = 0; k < p.ksteps; ++k) {
+        const int stage = k % p.stages, round = k / p.stages;
+        if (round > 0 && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) break;
+        const uint32_t dst = smem + static_cast<uint32_t>(stage) * block_bytes;
+        if (ElectOne()) {
+          BarExpect(full0 + stage * 8, kABytes);
+          TmaLoad<false>(dst, &p.wmap[0], t.n0, k * kBk, full0 + stage * 8);
+          TmaLoad<false>(dst + kABytes / 2, &p.wmap[0], t.n0 + 64, k * kBk, full0 + stage * 8);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 5) {
+    const uint32_t idesc = 0x10u | (1u << 7) | (1u << 10) | (1u << 15) | (static_cast<uint32_t>(p.bm >> 3) << 17) | (8u << 24);
+    const unsigned long long a0 = SmemDesc(smem, kABytes / 2, 1024), b0 = SmemDesc(smem + kABytes, 16, 1024);
+    for (int k = 0; k < p.ksteps; ++k) {
+      const int stage = k % p.stages, round = k / p.stages;
+      if (!BarWait(full0 + stage * 8, static_cast<uint32_t>(round & 1), ctl)) break;
+      FenceAfter();
+      const uint32_t off = static_cast<uint32_t>(stage) * block_bytes >> 4;
+      if (ElectOne()) {
+#pragma unroll
+        for (int i = 0; i < kBk / 16; ++i) MmaSs<false>(tmem, a0 + off + i * (2048 >> 4), b0 + off + i * (32 >> 4), idesc, k > 0 || i > 0);
+        if (C > 1) {
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(empty0 + stage * 8),
+                       "h"(static_cast<uint16_t>((1 << C) - 1))
+                       : "memory");
+        } else {
+          MmaCommit<false>(empty0 + stage * 8);
+        }
+        if (k == p.ksteps - 1) MmaCommit<false>(accf0);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= kFirstSwish) {
+    SwishRole(q, ctl, warp - kFirstSwish, lane, rank, t.m0, smem, block_bytes);
+  } else if (MODE != kBf16 && warp >= 6) {
+    const uint32_t ring = smem + static_cast<uint32_t>(p.stages) * block_bytes;
+    if constexpr (MODE != kBf16) {
+      if (warp >= kFirstDqWarp) {
+        // the products are exact in BF16 without w_scale, which the epilogue applies to the sums as the streaming kernels do
+        DequantRole<MODE, false, false, 1, 1>(p, ctl, warp - kFirstDqWarp, 0, lane, 0, p.ksteps, tile, p.tiles, ring, smem, block_bytes);
+      } else if (MODE == kFp8 || p.raw_tensor) {
+        if (warp == 6) LoadTensor<MODE, false, 1>(p, ctl, 0, 0, p.ksteps, tile, p.tiles, ring);
+      } else if constexpr (MODE == kNvfp4) {
+        LoadNvfp4Pieces<false, 1>(p, ctl, tid - 6 * 32, 0, 0, p.ksteps, tile, p.tiles, ring);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+      }
+    }
+  }
+
+  // the sums, by every warp: lane = column 32 (warp % 4) + lane of the tile, sixteen rows at a time
+  __syncwarp();
+  {
+    const DenseSeg& sg = p.seg[0];
+    const int quad = warp & 3, n = t.n0 + 32 * quad + lane;
+    const bool mine = n < sg.n;
+    const float scale = mine && sg.w_scale != nullptr ? __ldg(sg.w_scale + n) : 1.f;
+    const uint32_t src = tmem + (static_cast<uint32_t>(32 * quad) << 16);
+    const size_t at0 = static_cast<size_t>(t.m0) * sg.n + n;
+    uint16_t* const out = p.out[0] + at0;
+    const uint16_t* const routed = q.routed != nullptr ? q.routed + at0 : nullptr;
+    bool good = true, waited = false;
+    for (int c = 16 * (warp >> 2); c < p.bm && t.m0 + c < p.M; c += 16 * kSumGroups) {
+      uint32_t v[16], rt[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) rt[i] = mine && routed != nullptr && t.m0 + c + i < p.M ? routed[static_cast<size_t>(c + i) * sg.n] : 0;
+      if (!waited) {
+        good = BarWaitCluster(Smem(&gate_full), 0, ctl) && BarWait(accf0, 0, ctl);
+        waited = true;
+        __syncwarp();
+        FenceAfter();
+      }
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+            "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+          : "r"(src + static_cast<uint32_t>(c)));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (mine) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (t.m0 + c + i < p.M) {
+            // every step rounded to BF16 (the reference's skinny_gemm.cuh:226-240)
+            float y = RoundBf16(RoundBf16(__uint_as_float(v[i]) * scale) * gate[c + i]);
+            if (routed != nullptr) y += __uint_as_float(rt[i] << 16);
+            if (!good) y = __uint_as_float(0x7FFFFFFFu);
+            out[static_cast<size_t>(c + i) * sg.n] = __bfloat16_as_ushort(__float2bfloat16(y));
+          }
+        }
+      }
+    }
+    // a CTA leaves when its own sums are complete, and with them every copy into it: warps without rows wait too
+    if (!waited) {
+      BarWaitCluster(Smem(&gate_full), 0, ctl);
+      BarWait(accf0, 0, ctl);
+      __syncwarp();
+    }
+  }
+  if (ctl.fault) __nanosleep(100000);
+  FenceBefore();
+  __syncthreads();
+  if (C > 1) cg::this_cluster().sync();  // no CTA leaves while a peer may still write to it
+  if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(acc_cols) : "memory");
 }
 
 // ------------------------------------------------------------------------------ host
@@ -752,6 +1099,33 @@ cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, int ctas, int cl
   if (cluster > 1)
     return ks == 2 ? LaunchOne<MODE, SCALED, false, true, 2>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, true, 1>(p, ctas, cluster, smem, stream);
   return ks == 2 ? LaunchOne<MODE, SCALED, false, false, 2>(p, ctas, 1, smem, stream) : LaunchOne<MODE, SCALED, false, false, 1>(p, ctas, 1, smem, stream);
+}
+
+template <int MODE>
+cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream_t stream) {
+  static const cudaError_t configured = cudaFuncSetAttribute(DenseSharedKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - 1024);
+  if (configured != cudaSuccess) return configured;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(static_cast<unsigned>(SharedThreads<MODE>()));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(q.cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, DenseSharedKernel<MODE>, q);
+}
+
+// describes a stored weight to the copy engine
+bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int ks) {
+  const uint64_t rows = static_cast<uint64_t>(K), pitch = static_cast<uint64_t>(sg.pitch), n = static_cast<uint64_t>(sg.n);
+  if (mode == kBf16) return Encode(&p.wmap[s], sg.w, 2, rows, n, pitch, kBk, 64);
+  if (mode == kFp8) return Encode(&p.wmap[s], sg.w, 1, rows, n, pitch, kBk * ks, kBn);
+  return Encode(&p.wmap[s], sg.w, 1, rows, pitch, pitch, kBk * ks, kBn / 2) && Encode(&p.smap[s], sg.w, 1, rows, pitch, pitch, kBk * ks, 16);
 }
 
 }  // namespace
@@ -840,12 +1214,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
     p.raw_tensor = p.raw_tensor && sg.pitch % 16 == 0;
   }
   for (int s = 0; s < g.nseg && p.raw_tensor; ++s) {
-    const Segment& sg = g.seg[s];
-    const uint64_t K = static_cast<uint64_t>(g.K), pitch = static_cast<uint64_t>(sg.pitch);
-    const bool ok = mode == kBf16  ? Encode(&p.wmap[s], sg.w, 2, K, static_cast<uint64_t>(sg.n), pitch, kBk, 64)
-                    : mode == kFp8 ? Encode(&p.wmap[s], sg.w, 1, K, static_cast<uint64_t>(sg.n), pitch, kBk * ks, kBn)
-                                   : Encode(&p.wmap[s], sg.w, 1, K, pitch, pitch, kBk * ks, kBn / 2) && Encode(&p.smap[s], sg.w, 1, K, pitch, pitch, kBk * ks, 16);
-    if (!ok) throw std::runtime_error("SkinnyGemm(dense): cannot describe the weight to the copy engine");
+    if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks)) throw std::runtime_error("SkinnyGemm(dense): cannot describe the weight to the copy engine");
   }
   const int n_out = g.seg[g.nseg - 1].out_end;
   for (int o = 0; o < n_out; ++o) {
@@ -874,6 +1243,75 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
+}
+
+// SharedExpertDown: 16-byte rows of g and u as well.
+bool DenseSharedEligible(int mode, const GemmParams& p) {
+  return p.fuse && p.nseg == 1 && DenseTcEligible(mode, p) && reinterpret_cast<uintptr_t>(p.x2) % 16 == 0;
+}
+
+// Rows per tile and CTAs per cluster, by a model fitted to measured launches (us): a block of 64 k costs 0.10 + 0.0125
+// rows of swish_mul per CTA, or its MMAs and dequantisation where those take longer; around the blocks 6 + 0.02 bm +
+// 0.05 rows of the gate per CTA.  33 clusters of four, 74 of two are resident at once.
+DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) {
+  DenseTcPlan best;
+  double best_cost = 1e30;
+  const int64_t n_tiles = (p.seg[0].n + kBn - 1) / kBn;
+  const double blocks = (p.K + kBk - 1) / kBk;
+  for (int c = 1; c <= 4; c *= 2) {
+    const int64_t slots = c == 4 ? sm_count * 9 / 40 : sm_count / c, groups = (n_tiles + c - 1) / c;
+    const int unit = c == 4 ? 32 : 16;
+    for (int bm = unit; bm <= 256; bm += unit) {
+      const int64_t waves = (groups * ((m + bm - 1) / bm) + slots - 1) / slots;
+      const double block = std::max(0.10 + 0.0125 * bm / c, 0.30 + 0.0011 * bm);
+      const double cost = waves * (blocks * block + 6 + 0.02 * bm + 0.05 * bm / c);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best.bm = bm;
+        best.split = c;
+      }
+    }
+  }
+  return best;
+}
+
+void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+  const int C = plan.split;
+  if (m > INT_MAX / 2) throw std::runtime_error("SharedExpertDown: too many rows");
+  if ((C != 1 && C != 2 && C != 4) || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm % (8 * C) != 0)
+    throw std::runtime_error("SharedExpertDown: bad launch shape");
+  DenseShared q = {};
+  DenseParams& p = q.d;
+  const Segment& sg = g.seg[0];
+  p.nseg = 1;
+  p.M = static_cast<int>(m);
+  p.K = g.K;
+  p.bm = plan.bm;
+  p.ksteps = (g.K + kBk - 1) / kBk;
+  p.seg[0] = {sg.w, sg.w_scale, sg.pitch, sg.total_bytes, sg.n, 0, 0, 1};
+  p.out[0] = g.out[0];
+  p.width[0] = sg.n;
+  p.raw_tensor = sg.pitch % 16 == 0;
+  if (p.raw_tensor && !EncodeWeight(p, mode, 0, sg, g.K, 1)) throw std::runtime_error("SharedExpertDown: cannot describe the weight to the copy engine");
+  const int64_t n_tiles = ((sg.n + kBn - 1) / kBn + C - 1) / C * C, m_tiles = (m + p.bm - 1) / p.bm;
+  if (n_tiles * m_tiles > INT_MAX / 16) throw std::runtime_error("SharedExpertDown: too many tiles");
+  p.m_tiles = static_cast<int>(m_tiles);
+  p.tiles = static_cast<int>(n_tiles * m_tiles);
+  const int block = kABytes + p.bm * kBk * 2;
+  p.stages = std::min(kMaxStages, (kSmemLimit - 2048 - RawBytes(mode)) / block);
+  q.g = g.x;
+  q.u = g.x2;
+  q.gx = g.gx;
+  q.gw = g.gw;
+  q.routed = g.routed;
+  q.gk = g.gk;
+  q.cluster = C;
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode);
+  cudaError_t err = mode == kBf16  ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
+                    : mode == kFp8 ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
+                                   : LaunchShared<kNvfp4>(q, p.tiles, smem, stream);
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err != cudaSuccess) throw std::runtime_error(std::string("SharedExpertDown: ") + cudaGetErrorString(err));
 }
 
 }  // namespace qfg

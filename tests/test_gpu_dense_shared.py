@@ -1,0 +1,106 @@
+"""The many-row kernel of SharedExpertDown (csrc/dense_tc.cu) at the edges of its tiles and clusters, and its sigmoid on
+every BF16 value."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import bits, to_dev
+from oracle import oracle as O
+from qwen38_flash_ops_b200 import QfgError, SharedExpertDown
+from qwen38_flash_ops_b200 import packing as P
+
+import _util as U
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(mode, M, K, N, gk, plan, seed, gx_offset=0, g_offset=0):
+    rng = np.random.default_rng(seed)
+    bf = lambda a: P.f32_to_bf16_bits(a.astype(np.float32))
+    arr, s = U.make_weight(rng, mode, K, N, mode != 0)
+    g, u, gx = bf(rng.standard_normal((M, K)) * 0.8), bf(rng.standard_normal((M, K)) * 0.8), bf(rng.standard_normal((M, gk)) * 0.2)
+    gw, routed = bf(rng.standard_normal((gk, 1)) * 0.2), bf(rng.standard_normal((M, N)) * 0.2)
+
+    def dev(a, offset=0):
+        t = to_dev(a, "bf16")
+        if not offset:
+            return t
+        buf = torch.empty(t.numel() + offset, dtype=torch.bfloat16, device="cuda")
+        buf[offset:] = t.reshape(-1)
+        return buf[offset:].view(t.shape)
+
+    op = SharedExpertDown(w_scale=s if mode != 0 else None)
+    if plan:
+        op.set_option("dense_plan", plan)
+    out = op(dev(g, g_offset), dev(u), U.dev_weight(arr, mode), dev(gx, gx_offset), dev(gw), dev(routed))
+    torch.cuda.synchronize()
+    y, _, _, shared = O.shared_expert_down(g, u, mode, arr, N, gx, gw, routed, s if mode != 0 else None)
+    got, gf, yf = bits(out), O.bf16_to_f32(bits(out)), O.bf16_to_f32(y)
+    # FP32 sums in another order may cross a BF16 boundary: one ulp of the larger of the two terms
+    tol = np.maximum(np.maximum(np.abs(O.bf16_to_f32(routed)), np.abs(shared)), np.abs(yf)) * 2.0 ** -7 + 1e-30
+    assert np.all(np.abs(gf - yf) <= tol), f"{np.count_nonzero(np.abs(gf - yf) > tol)} outputs outside one ULP"
+    assert np.mean(got == y) > 0.97
+
+
+# rows per tile, CTAs per cluster (ranks whose warps have no rows of their own among them)
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["", "16,1", "32,4", "48,2", "96,4", "256,1", "256,4"])
+def test_tile_and_cluster_edges(cuda, mode, plan):
+    for i, (M, K, N, gk) in enumerate([(17, 256, 128, 256), (100, 648, 1152, 1024), (35, 1096, 640, 26)]):
+        _run(mode, M, K, N, gk, plan, 100 * mode + i)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_layouts_on_either_side_of_the_route(cuda, mode):
+    _run(mode, 40, 256, 128, 64, "", 7, gx_offset=1)   # gate read element by element
+    _run(mode, 40, 256, 128, 64, "", 7, g_offset=2)    # rows of g the kernel cannot read: streaming passes
+    _run(mode, 40, 260, 192, 64, "", 7)                # K off 16 bytes, N an odd number of 64
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["160,4", "256,4", "64,2", "32,1"])
+def test_repeated_calls_agree(cuda, mode, plan):
+    """A stage reused before every CTA of the cluster has read it shows as a run that differs."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    M, K, N = 300, 2560, 1152
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    if mode == 0:
+        w = mk(K, N) * 0.02
+    elif mode == 1:
+        w = mk(K, N).to(torch.float8_e4m3fn)
+    else:
+        w = torch.randint(0, 256, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)
+        w[:, N // 2:] = w[:, N // 2:] % 0x7F  # block scales: finite, not negative
+    args = (mk(M, K), mk(M, K), w, mk(M, 512), mk(512, 1), mk(M, N))
+    op = SharedExpertDown()
+    op.set_option("dense_plan", plan)
+    first = op(*args).clone()
+    assert torch.isfinite(first).all()
+    for _ in range(40):
+        assert torch.equal(op(*args), first)
+
+
+def test_swish_of_every_bf16_value_is_the_streaming_kernels(cuda):
+    """One value per row, u = 1, an identity weight and a gate of one: the output is bf16(g * bf16(sigmoid(g)))."""
+    g = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16).view(1024, 64)
+    w = torch.zeros(64, 128, device="cuda")
+    w[torch.arange(64), torch.arange(64)] = 1
+    gx, gw = torch.ones(1024, 8, device="cuda").bfloat16(), torch.full((8, 1), 10.0, device="cuda").bfloat16()
+    u, routed = torch.ones_like(g), torch.zeros(1024, 128, device="cuda").bfloat16()
+    many, few = SharedExpertDown(), SharedExpertDown()
+    few.set_option("dense_rows", 0)
+    for j in range(64):
+        gj = torch.zeros_like(g)
+        gj[:, j] = g[:, j]
+        a, b = (op(gj, u, w.bfloat16(), gx, gw, routed)[:, j] for op in (many, few))
+        assert torch.equal(torch.isnan(a), torch.isnan(b))
+        assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+
+
+def test_bad_launch_shapes(cuda):
+    z = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")
+    op = SharedExpertDown()
+    for plan in ("24,1", "272,1", "48,4", "64,3", "64,8"):
+        op.set_option("dense_plan", plan)
+        with pytest.raises(QfgError):
+            op(z(20, 64), z(20, 64), z(64, 64), z(20, 64), z(64, 1), z(20, 64))
