@@ -6,8 +6,11 @@
 //   * One cluster of up to eight CTAs per row; a CTA issues all the 16-byte loads of its share of the row at
 //     once (a scalar head and tail keep the vector body for odd vocabularies and unaligned rows), so a row
 //     costs one round trip to L2.
-//   * Candidates travel as 64-bit keys whose unsigned maximum is the winner (argmax_key.cuh): a thread packs
-//     its best pair once, a warp needs two redux.sync.max, warps meet in one shared-memory atomicMax.
+//   * The value first, the index after: a thread takes the maximum of its elements two at a time with the packed
+//     NaN-propagating maximum (half an instruction an element; carrying an index along cost five, and a dependent
+//     chain 48 elements long), warps meet in a redux and a shared-memory atomicMax, and only the threads that hold
+//     the CTA's maximum look through their registers for its first position.
+//   * Candidates travel as 64-bit keys whose unsigned maximum is the winner (argmax_key.cuh).
 //   * The CTAs of a cluster do not meet at a barrier at the end.  CTA 0 owns one mbarrier and one key slot
 //     per peer; a peer stores its key into CTA 0's shared memory, arrives on the barrier with release
 //     semantics at cluster scope, and exits; CTA 0 alone waits (bounded), folds and writes.  The one cluster
@@ -28,6 +31,10 @@ namespace {
 
 constexpr int kThreads = 512;   // 1024 threads per CTA measured slower at every row count
 constexpr int kMaxCluster = 8;
+// loads a thread has in flight: 8 CTAs x 512 threads x 6 (10) loads cover 151936 columns; ten for two-byte elements
+// measured 0.5 us slower at one row
+template <typename T>
+constexpr int kInFlight = sizeof(T) == 4 ? 10 : 6;
 constexpr int kPeerSpin = 1 << 24;  // bound of CTA 0's wait for its peers (iterations of about 30 ns)
 
 __device__ __forceinline__ float ToFloat(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -36,35 +43,56 @@ __device__ __forceinline__ float ToFloat(float v) { return v; }
 
 __device__ __forceinline__ uint32_t SharedAddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// A thread's running best.  `InOrder`: the candidate's index exceeds every index this thread has seen, so a
-// strict comparison keeps the lowest index of equal values and a NaN is never replaced; `Any`: full order.
-struct Best {
-  float v = 0.f;
-  long long i = -1;
-  __device__ __forceinline__ void InOrder(float c, long long idx) {
-    if (i < 0 || c > v || (c != c && v == v)) {
-      v = c;
-      i = idx;
-    }
+// The largest of the elements packed in 32-bit words, NaN if one is (no index yet): one instruction per word.
+template <typename T>
+struct WordMax;
+template <>
+struct WordMax<__nv_bfloat16> {
+  static constexpr uint32_t kLowest = 0xFF80FF80u;  // -infinity
+  __device__ __forceinline__ static uint32_t Max(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
   }
-  __device__ __forceinline__ void Any(float c, long long idx) {
-    const bool c_nan = c != c, v_nan = v != v;
-    const bool better = c_nan ? (!v_nan || idx < i) : (!v_nan && (c > v || (c == v && idx < i)));
-    if (i < 0 || better) {
-      v = c;
-      i = idx;
-    }
+  __device__ __forceinline__ static float Value(uint32_t w) { return Fold(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)); }
+  __device__ __forceinline__ static float Fold(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
   }
-  __device__ __forceinline__ unsigned long long Key() const { return i < 0 ? 0ull : PackKey(v, i); }
 };
+template <>
+struct WordMax<__half> {
+  static constexpr uint32_t kLowest = 0xFC00FC00u;
+  __device__ __forceinline__ static uint32_t Max(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  __device__ __forceinline__ static float Value(uint32_t w) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    return WordMax<__nv_bfloat16>::Fold(f.x, f.y);
+  }
+};
+template <>
+struct WordMax<float> {
+  static constexpr uint32_t kLowest = 0xFF800000u;
+  __device__ __forceinline__ static uint32_t Max(uint32_t a, uint32_t b) {
+    return __float_as_uint(WordMax<__nv_bfloat16>::Fold(__uint_as_float(a), __uint_as_float(b)));
+  }
+  __device__ __forceinline__ static float Value(uint32_t w) { return __uint_as_float(w); }
+};
+
+// the value half of a key: equal for equal values, for -0 and +0 and for every NaN
+__device__ __forceinline__ uint32_t ValueKey(float v) { return static_cast<uint32_t>(PackKey(v, 0) >> 32); }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict__ x, long long V,
                                                              long long* __restrict__ idx_out,
                                                              float* __restrict__ val_out) {
-  constexpr int kVecElems = 16 / sizeof(T);
-  constexpr int kInFlight = sizeof(T) == 4 ? 10 : 6;  // 8 CTAs x 512 threads x 6 (10) loads cover 151936 columns
+  constexpr int kVecElems = 16 / sizeof(T), kLoads = kInFlight<T>;
   __shared__ unsigned long long s_best;               // this CTA's best key
+  __shared__ uint32_t s_value;                        // its value half, before the index is known
   __shared__ unsigned long long s_slot[kMaxCluster];  // CTA 0: the peers' keys
   __shared__ unsigned long long s_bar;                // CTA 0: mbarrier, one arrival per peer
 
@@ -85,15 +113,18 @@ __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict
   const uint4* xv = reinterpret_cast<const uint4*>(xr + head);
 
   // ---- the first batch of loads goes out before anything else
-  uint4 q[kInFlight];
+  constexpr uint32_t kLow = WordMax<T>::kLowest;
+  const uint4 lowest = make_uint4(kLow, kLow, kLow, kLow);
+  uint4 q[kLoads];
   long long v0 = vbeg + tid;
 #pragma unroll
-  for (int k = 0; k < kInFlight; ++k) {
+  for (int k = 0; k < kLoads; ++k) {
     const long long v = v0 + static_cast<long long>(k) * kThreads;
-    q[k] = v < vend ? __ldg(xv + v) : make_uint4(0, 0, 0, 0);
+    q[k] = v < vend ? __ldg(xv + v) : lowest;
   }
   if (tid == 0) {
     s_best = 0ull;
+    s_value = 0u;
     if (c == 0 && C > 1) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(SharedAddr(&s_bar)), "r"(C - 1) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -102,35 +133,68 @@ __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict
   __syncthreads();
   if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
-  Best best;
+  // the value first: the largest of every batch of this thread, and the first batch that holds the largest of all
+  uint32_t top = 0u;  // ValueKey; 0 is below every value's
+  long long top_v0 = v0;
   for (;;) {
+    uint32_t m = kLow;
 #pragma unroll
-    for (int k = 0; k < kInFlight; ++k) {
-      const long long v = v0 + static_cast<long long>(k) * kThreads;
-      if (v < vend) {
-        const T* e = reinterpret_cast<const T*>(&q[k]);
-#pragma unroll
-        for (int j = 0; j < kVecElems; ++j) best.InOrder(ToFloat(e[j]), head + v * kVecElems + j);
-      }
+    for (int k = 0; k < kLoads; ++k) m = WordMax<T>::Max(m, WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w)));
+    const uint32_t key = v0 < vend ? ValueKey(WordMax<T>::Value(m)) : 0u;
+    if (key > top) {
+      top = key;
+      top_v0 = v0;
     }
-    v0 += static_cast<long long>(kThreads) * kInFlight;
-    if (v0 >= vend) break;  // rows longer than one batch per thread take further round trips
+    const long long next = v0 + static_cast<long long>(kThreads) * kLoads;
+    if (next >= vend) break;  // rows longer than one batch per thread take further round trips
+    v0 = next;
 #pragma unroll
-    for (int k = 0; k < kInFlight; ++k) {
+    for (int k = 0; k < kLoads; ++k) {
       const long long v = v0 + static_cast<long long>(k) * kThreads;
-      q[k] = v < vend ? __ldg(xv + v) : make_uint4(0, 0, 0, 0);
+      q[k] = v < vend ? __ldg(xv + v) : lowest;
     }
   }
-  // head goes to the first CTA, tail to the last
+  // head goes to the first CTA, tail to the last: these few elements come with their index
+  unsigned long long edge = 0ull;
   if (c == 0) {
-    for (long long i = tid; i < head; i += kThreads) best.Any(ToFloat(xr[i]), i);
+    for (long long i = tid; i < head; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
   }
   if (c == C - 1) {
-    for (long long i = head + nvec * kVecElems + tid; i < V; i += kThreads) best.Any(ToFloat(xr[i]), i);
+    for (long long i = head + nvec * kVecElems + tid; i < V; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
   }
+  const uint32_t mine = max(top, static_cast<uint32_t>(edge >> 32));
+  const uint32_t wtop = __reduce_max_sync(0xffffffffu, mine);
+  if (lane == 0 && wtop != 0u) atomicMax(&s_value, wtop);
+  __syncthreads();
 
-  const unsigned long long wkey = WarpMaxKey(best.Key());
-  if (lane == 0 && wkey != 0ull) atomicMax(&s_best, wkey);
+  // then the index, by the threads that hold the CTA's largest value (one, but for ties): their first such element
+  const uint32_t cta_top = s_value;
+  if (mine == cta_top && cta_top != 0u) {
+    unsigned long long key = static_cast<uint32_t>(edge >> 32) == cta_top ? edge : 0ull;
+    if (top == cta_top) {
+      if (top_v0 != v0) {  // not the batch in hand
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) {
+          const long long v = top_v0 + static_cast<long long>(k) * kThreads;
+          q[k] = v < vend ? __ldg(xv + v) : lowest;
+        }
+      }
+#pragma unroll
+      for (int k = kLoads - 1; k >= 0; --k) {
+        const long long v = top_v0 + static_cast<long long>(k) * kThreads;
+        const uint32_t m = WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w));
+        if (v < vend && ValueKey(WordMax<T>::Value(m)) == cta_top) {
+          const T* e = reinterpret_cast<const T*>(&q[k]);
+#pragma unroll
+          for (int j = 0; j < kVecElems; ++j) {
+            const float f = ToFloat(e[j]);
+            if (ValueKey(f) == cta_top) key = max(key, PackKey(f, head + v * kVecElems + j));  // the lower index is the larger key
+          }
+        }
+      }
+    }
+    atomicMax(&s_best, key);
+  }
   __syncthreads();
 
   // the key of a NaN carries no payload: a NaN winner's value is read back from the row, bit for bit
@@ -176,6 +240,14 @@ cudaError_t LaunchT(const T* x, int64_t rows, int64_t V, int64_t* idx, float* va
   const long long vecs = V / (16 / static_cast<long long>(sizeof(T)));
   int cluster = 1;
   while (cluster < kMaxCluster && vecs > static_cast<long long>(cluster) * kThreads * 2) cluster *= 2;
+  // Many rows fill the chip without that, and then a CTA's fixed cost (start, barriers, the exchange) is what counts:
+  // at most two CTAs per SM, or one where half the CTAs still see a row in one batch of loads (BF16, before -> after:
+  // 64 x 151936 8.7 -> 7.3 us, 128 x 151936 15.8 -> 10.7, 128 x 16384 4.25 -> 3.25).
+  const long long sms = DeviceSmCount();
+  while (cluster > 1 && (cluster * rows > 2 * sms ||
+                         (cluster * rows > sms && vecs <= static_cast<long long>(cluster / 2) * kThreads * kInFlight<T>))) {
+    cluster /= 2;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(cluster), static_cast<unsigned>(rows), 1);
   cfg.blockDim = dim3(kThreads, 1, 1);

@@ -196,3 +196,29 @@ def test_untile_hc_rejects_other_shapes(cuda):
         UntileHcBf16(0)(torch.zeros((160, 20472), dtype=torch.bfloat16, device="cuda"))
     with pytest.raises(QfgError):
         UntileHcBf16(2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,vocab", [(19, 32768), (64, 77777), (150, 16411), (300, 40000), (300, 151936)])
+def test_argmax_many_rows(cuda, dtype, rows, vocab):
+    """Row counts that shrink the cluster of a row (several batches of loads per thread), with the maximum planted in
+    early and late batches, in the scalar head and tail of unaligned rows, twice, as a NaN, and in rows of -infinity."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + vocab)
+    x = torch.randn(rows, vocab, generator=gen, device="cuda").to(dtype)
+    pos = torch.randint(0, vocab, (rows,), generator=gen, device="cuda")
+    for r in range(rows):
+        p = int(pos[r])
+        if r % 7 == 0:
+            x[r, p] = x[r, vocab - 1 - p // 2] = 100.0        # a tie, or one planted value
+        elif r % 7 == 1:
+            x[r, p:] = float("nan")
+        elif r % 7 == 2:
+            x[r] = float("-inf")
+        elif r % 7 == 3:
+            x[r, vocab - 1] = 100.0
+        elif r % 7 == 4:
+            x[r, 0] = x[r, vocab // 2] = 100.0
+        elif r % 7 == 5:
+            x[r].clamp_(max=0)                                # +0 and -0 tie
+            x[r, p] = -0.0
+    _check_argmax(x)
