@@ -67,8 +67,8 @@ def load() -> ctypes.CDLL:
     lib.qfg_version.restype = c_char_p
     lib.qfg_skinny_gemm_create.argtypes = [POINTER(c_int64), c_int, POINTER(c_int64), c_int, POINTER(c_float),
                                            c_size_t, c_int, POINTER(c_void_p)]
-    lib.qfg_skinny_gemm_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int,
-                                            POINTER(c_void_p), c_int, c_void_p]
+    # void pointers where the ops pass packed bytes for a Tensor2D or an array (structures and arrays work too)
+    lib.qfg_skinny_gemm_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int, c_void_p]
     lib.qfg_skinny_gemm_set_option.argtypes = [c_void_p, c_char_p, c_char_p]
     lib.qfg_skinny_gemm_describe.argtypes = [c_void_p, c_int64, POINTER(Tensor2D), c_int, c_char_p, c_size_t]
     lib.qfg_plan_describe.argtypes = [c_int, c_int64, POINTER(c_int64), c_int, c_int, c_int, c_char_p, c_char_p,
@@ -78,18 +78,18 @@ def load() -> ctypes.CDLL:
     lib.qfg_argmax_rows.argtypes = [c_int, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p]
     lib.qfg_dequant_create.argtypes = [c_int64, c_int64, POINTER(c_int64), c_int, POINTER(c_float), c_size_t,
                                        POINTER(c_void_p)]
-    lib.qfg_dequant_compute.argtypes = [c_void_p, POINTER(Tensor2D), POINTER(c_void_p), c_int, c_void_p]
+    lib.qfg_dequant_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p]
     lib.qfg_dequant_destroy.argtypes = [c_void_p]
     lib.qfg_dequant_destroy.restype = None
     lib.qfg_lmhead_workspace_bytes.restype = c_size_t
     lib.qfg_lmhead_create.argtypes = [POINTER(c_float), c_size_t, c_int, POINTER(c_void_p)]
-    lib.qfg_lmhead_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int64, c_int64,
+    lib.qfg_lmhead_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.qfg_lmhead_static_max_rows.restype = c_size_t
     lib.qfg_lmhead_compute_static.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int64, c_int64,
                                               c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.qfg_shared_expert_down_create.argtypes = [POINTER(c_float), c_size_t, c_int, POINTER(c_void_p)]
-    lib.qfg_shared_expert_down_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_void_p,
+    lib.qfg_shared_expert_down_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
                                                    c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]
     lib.qfg_shared_expert_down_set_option.argtypes = [c_void_p, c_char_p, c_char_p]
     lib.qfg_shared_expert_down_destroy.argtypes = [c_void_p]

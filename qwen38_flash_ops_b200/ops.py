@@ -10,6 +10,7 @@ libqfg_b200.so on the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import struct
 from ctypes import c_void_p
 
 import torch
@@ -26,18 +27,42 @@ _DTYPES = {
 }
 
 
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+# The host's part of a call is about as long as the smallest kernels (15.4 us for one SkinnyGemm before the lines below
+# were written with its time in mind, 10.6 after; 4.5 of them are the launch), so the per-call plumbing avoids what costs
+# microseconds: torch.cuda.current_stream() builds a Stream object (3.5 us; the raw handle 0.15), ctypes structures and
+# arrays are built field by field (1.6 us; one struct.pack 0.3).
+if hasattr(torch._C, "_cuda_getCurrentRawStream") and hasattr(torch._C, "_cuda_getDevice"):
+    def _stream_ptr() -> int:
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+else:
+    def _stream_ptr() -> int:
+        return torch.cuda.current_stream().cuda_stream
 
 
-def _tensor2d(w: torch.Tensor) -> Tensor2D:
+_PACK_2D = struct.Struct("Pi4xqq")  # Tensor2D
+assert _PACK_2D.size == ctypes.sizeof(Tensor2D)
+
+
+def _weight(w: torch.Tensor) -> bytes:
+    """The Tensor2D of a weight, in the bytes a foreign call takes for a pointer to it."""
     if w.dim() != 2:
         raise QfgError(_lib.QFG_INVALID_ARGUMENT, "weight must be a 2-D tensor")
     if not w.is_cuda or not w.is_contiguous():
         raise QfgError(_lib.QFG_INVALID_ARGUMENT, "weight must be a contiguous CUDA tensor")
-    if w.dtype not in _DTYPES:
+    code = _DTYPES.get(w.dtype)
+    if code is None:
         raise QfgError(_lib.QFG_INVALID_ARGUMENT, f"unsupported weight element type {w.dtype}")
-    return Tensor2D(w.data_ptr(), _DTYPES[w.dtype], w.shape[0], w.shape[1])
+    rows, cols = w.shape
+    return _PACK_2D.pack(w.data_ptr(), code, rows, cols)
+
+
+def _tensor2d(w: torch.Tensor) -> Tensor2D:
+    return Tensor2D.from_buffer_copy(_weight(w))
+
+
+def _pointers(tensors) -> bytes:
+    """An array of device pointers, as bytes."""
+    return struct.pack("%dP" % len(tensors), *[t.data_ptr() for t in tensors])
 
 
 def _require_cuda(x: torch.Tensor, what: str) -> None:
@@ -81,15 +106,17 @@ class SkinnyGemm:
         _require_cuda(x, "x")
         if x.dtype != torch.bfloat16:
             raise QfgError(_lib.QFG_INVALID_ARGUMENT, "SkinnyGemm: x must be BF16")
-        k = x.shape[-1]
+        shape = x.shape
+        k = shape[-1]
         m = x.numel() // k if k > 0 else 0
-        lead = tuple(x.shape[:-1])
         if out is None:
-            out = [torch.empty(lead + (w,), dtype=torch.bfloat16, device=x.device) for w in self.widths]
-        arr = (Tensor2D * max(len(weights), 1))(*[_tensor2d(w) for w in weights])
-        outs = (c_void_p * max(len(out), 1))(*[o.data_ptr() for o in out])
-        check(self._lib.qfg_skinny_gemm_compute(self._h, x.data_ptr(), m, k, arr, len(weights), outs, len(out),
-                                                _stream_ptr()))
+            lead, device = tuple(shape[:-1]), x.device
+            out = [torch.empty(lead + (w,), dtype=torch.bfloat16, device=device) for w in self.widths]
+        descs = b"".join([_weight(w) for w in weights])
+        code = self._lib.qfg_skinny_gemm_compute(self._h, x.data_ptr(), m, k, descs, len(weights), _pointers(out), len(out),
+                                                 _stream_ptr())
+        if code:
+            check(code)
         return out
 
     def __del__(self):
@@ -120,8 +147,9 @@ class ArgmaxRows:
             idx, val = out
             with_val = val is not None
         else:
-            idx = torch.empty(lead, dtype=torch.int64, device=x.device)
-            val = torch.empty(lead, dtype=torch.float32, device=x.device) if with_val else None
+            device = x.device
+            idx = torch.empty(lead, dtype=torch.int64, device=device)
+            val = torch.empty(lead, dtype=torch.float32, device=device) if with_val else None
         check(self._lib.qfg_argmax_rows(_DTYPES[x.dtype], x.data_ptr(), rows, vocab, idx.data_ptr(),
                                         val.data_ptr() if with_val else None, _stream_ptr()))
         return (idx, val) if with_val else idx
@@ -147,10 +175,9 @@ class DequantWeightBf16:
         self.widths = widths if widths else [int(n_cols)]
 
     def __call__(self, w: torch.Tensor, out=None):
-        t = _tensor2d(w)
+        t = _weight(w)
         outs = out if out is not None else [torch.empty((w.shape[0], wd), dtype=torch.bfloat16, device=w.device) for wd in self.widths]
-        ptrs = (c_void_p * len(outs))(*[o.data_ptr() for o in outs])
-        check(self._lib.qfg_dequant_compute(self._h, ctypes.byref(t), ptrs, len(outs), _stream_ptr()))
+        check(self._lib.qfg_dequant_compute(self._h, t, _pointers(outs), len(outs), _stream_ptr()))
         return outs
 
     def __del__(self):
@@ -181,7 +208,8 @@ class SharedExpertDown:
 
     def __call__(self, g, u, w, gx, gw, routed):
         for name, t in (("g", g), ("u", u), ("gx", gx), ("gw", gw), ("routed", routed)):
-            _require_cuda(t, name)
+            if not t.is_cuda or not t.is_contiguous():
+                _require_cuda(t, name)
             if t.dtype != torch.bfloat16:
                 raise QfgError(_lib.QFG_FAIL, f"SharedExpertDown: {name} must be BF16")
         k = w.shape[0]
@@ -191,14 +219,14 @@ class SharedExpertDown:
         if (m < 1 or g.numel() != m * k or u.numel() != m * k or routed.numel() != m * n or gx.numel() != m * gk
                 or gw.shape[-1] != 1):
             raise QfgError(_lib.QFG_FAIL, "SharedExpertDown: shape mismatch")
-        t = _tensor2d(w)
+        t = _weight(w)
         if w.dtype == torch.uint8:
             if n % 16 != 0 or w.shape[1] != n * 9 // 16:
                 raise QfgError(_lib.QFG_FAIL, "SharedExpertDown: NVFP4 weight N mismatch")
         elif w.shape[1] != n:
             raise QfgError(_lib.QFG_FAIL, "SharedExpertDown: weight N mismatch")
         out = torch.empty_like(routed)
-        check(self._lib.qfg_shared_expert_down_compute(self._h, g.data_ptr(), u.data_ptr(), m, k, ctypes.byref(t), gx.data_ptr(),
+        check(self._lib.qfg_shared_expert_down_compute(self._h, g.data_ptr(), u.data_ptr(), m, k, t, gx.data_ptr(),
                                                        gk, gw.data_ptr(), routed.data_ptr(), n, out.data_ptr(), _stream_ptr()))
         return out
 
@@ -274,7 +302,7 @@ class LmHeadArgmax:
             raise QfgError(_lib.QFG_INVALID_ARGUMENT, "LmHead: x must be BF16")
         k = x.shape[-1]
         m = x.numel() // k
-        t = _tensor2d(w)
+        t = _weight(w)
         if out is None:
             idx = torch.empty(m, dtype=torch.int64, device=x.device)
             val = torch.empty(m, dtype=torch.float32, device=x.device)
@@ -282,7 +310,7 @@ class LmHeadArgmax:
         else:
             idx, val, key = out
         lg = torch.empty((m, n), dtype=torch.bfloat16, device=x.device) if logits else None
-        check(self._lib.qfg_lmhead_compute(self._h, x.data_ptr(), m, k, ctypes.byref(t), int(n), int(col_offset),
+        check(self._lib.qfg_lmhead_compute(self._h, x.data_ptr(), m, k, t, int(n), int(col_offset),
                                            self.workspace.data_ptr(), idx.data_ptr(), val.data_ptr(), key.data_ptr(),
                                            lg.data_ptr() if logits else None, _stream_ptr()))
         return (idx, val, key, lg) if logits else (idx, val, key)
