@@ -21,11 +21,11 @@
 // from L2 (a 128 x 256 tile fetches 36 KB per 512 cycles, more than an SM's share of L2).
 //
 // What bounds it.  Few rows: the dequantising warps and the barriers between the roles, about 400 cycles a block of 64 k
-// (FP4 at 33 rows, 5120 x 17408: 24.6 us = 2.1 TB/s of weights; the dequantisation pass and the library GEMM that this
-// kernel took the place of, 86.8 us).  Many rows: the tensor core, 70-80 % of its rate (FP8, 509 rows, 5120 x 10240: 67.9 us
-// against 93.0; FP4, 2048 rows, 5120 x 17408: 309 us against 332).  The tcgen05 operands come from shared memory
-// rather than tensor memory because the rows of x per pass would be limited to 64 there, and the weights are written
-// MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
+// (FP4 at 33 rows, 5120 x 17408: 23.7 us = 2.1 TB/s of weights; the dequantisation pass and the library GEMM that this
+// kernel took the place of, 86.6 us).  Many rows: the tensor core at its rate under load, and the last wave (FP8, 509
+// rows, 5120 x 10240: 65.6 us against 92.5; FP4, 2048 rows, 5120 x 17408: 298 us against 333).  The tcgen05 operands
+// come from shared memory rather than tensor memory because the rows of x per pass would be limited to 64 there, and the
+// weights are written MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
 //
 // Every wait is bounded; a CTA that gives up on one writes NaN and leaves.
 #include <cooperative_groups.h>
@@ -39,6 +39,7 @@
 #include <cstdlib>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "qfg_internal.h"
 
@@ -62,10 +63,15 @@ template <int MODE, int KS>
 struct RawRing {  // ring of stored, undequantised stages
   static constexpr int kRows = kBk * KS;
   static constexpr int kSlot = kRows * (MODE == kNvfp4 ? 64 + 16 : 128);
-  static constexpr int kDepth = (MODE == kNvfp4 ? 12 : 8) / KS;
+  // even: a slot then always serves the same group of dequantising warps, which has seen its previous phase complete
+  static constexpr int kDepth = KS == 1 ? (MODE == kNvfp4 ? 10 : 6) : (MODE == kNvfp4 ? 6 : 4);
   static constexpr int kBytes = MODE == kBf16 ? 0 : kSlot * kDepth;
 };
-static_assert(RawRing<kNvfp4, 1>::kDepth <= kMaxRaw && RawRing<kFp8, 2>::kDepth >= kDqGroups, "raw ring");
+static_assert(RawRing<kNvfp4, 1>::kDepth <= kMaxRaw && RawRing<kNvfp4, 1>::kDepth % kDqGroups == 0 && RawRing<kFp8, 1>::kDepth % kDqGroups == 0 &&
+                  RawRing<kNvfp4, 2>::kDepth % kDqGroups == 0 && RawRing<kFp8, 2>::kDepth % kDqGroups == 0,
+              "raw ring");
+constexpr int kOutPitch = 80;                     // bytes of a row of 32 output columns in an epilogue warp's buffer: rows 16 bytes apart in the banks
+constexpr int kOutBytes = 4 * 32 * kOutPitch;     // four warps, 32 rows of x each
 
 struct DenseSeg {
   const uint8_t* w;
@@ -82,6 +88,7 @@ struct DenseParams {
   uint16_t* out[kMaxOut];
   int col_begin[kMaxOut], width[kMaxOut];
   int nseg, M, K, ksteps, bm, m_tiles, tiles, stages, raw_tensor;
+  uint32_t out_vec;  // outputs whose rows can be written 16 bytes at a time
 };
 
 struct Ctl {
@@ -497,6 +504,11 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
     ctl.fault = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (warp == 4 && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.xmap) : "memory");
+    if (p.raw_tensor) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.wmap[0]) : "memory");
+    if (MODE == kNvfp4 && p.raw_tensor) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.smap[0]) : "memory");
+  }
   if (warp == 5) {
     if constexpr (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(Smem(&ctl.tmem)), "r"(acc_cols) : "memory");
@@ -513,46 +525,93 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   const uint32_t tmem = ctl.tmem;
 
   if (warp < 4) {
-    // ---- epilogue: lane = column 32 warp + lane of the tile, tensor memory columns = rows of x
+    // ---- epilogue
+    const uint32_t buf = smem + static_cast<uint32_t>(p.stages) * stage_bytes + RawRing<MODE, KS>::kBytes + static_cast<uint32_t>(warp * 32 * kOutPitch);
     int it = 0;
     for (int tile = first_tile; tile < p.tiles; tile += tile_step, ++it) {
       const int b = it & 1;
       const bool good = BarWait(accf0 + b * 8, static_cast<uint32_t>((it >> 1) & 1), ctl);
+      __syncwarp();
       FenceAfter();
       const TileAt t = LocateDense<PAIR>(p, tile, rank);
       const uint32_t src = tmem + (static_cast<uint32_t>(32 * warp) << 16) + static_cast<uint32_t>(b * p.bm);
-      const int n = t.n0 + 32 * warp + lane;
-      uint16_t* out = nullptr;
-      size_t width = 0;
-      if constexpr (!SPLIT) {
+      if constexpr (SPLIT) {  // lane = column 32 warp + lane of the tile
+        for (int c = 0; c < p.bm; c += 16) {
+          uint32_t v[16];
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+              : "r"(src + static_cast<uint32_t>(c)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          float* part = reinterpret_cast<float*>(smem_ptr) + c * kBn + 32 * warp + lane;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) part[i * kBn] = good ? __uint_as_float(v[i]) : __uint_as_float(0x7FFFFFFFu);
+        }
+      } else {
+        // A lane stores eight columns of a row at a time: the accumulators come as 8 x 8 fragments, columns of W down
+        // and rows of x across, and go through shared memory transposed.  One column per lane, two bytes a store, took
+        // 50 cycles a row and warp (a tile of 176 rows: 8700 cycles, a sixth of a call).
         const DenseSeg& sg = p.seg[t.seg];
+        const int chunk = lane & 3, row = lane >> 2, n = t.n0 + 32 * warp + 8 * chunk;  // widths are multiples of eight
         int j = sg.out_begin;
         for (int i = j + 1; i < sg.out_end; ++i) {
           if (n >= p.col_begin[i]) j = i;
         }
-        width = static_cast<size_t>(p.width[j]);
-        if (n < sg.n) out = p.out[j] + static_cast<size_t>(t.m0) * width + (n - p.col_begin[j]);
-      }
-      for (int c = 0; c < p.bm; c += 16) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-              "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(src + static_cast<uint32_t>(c)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!good) {
+        const size_t width = static_cast<size_t>(p.width[j]);
+        uint16_t* const out = p.out[j] + static_cast<size_t>(t.m0) * width + (n - p.col_begin[j]);
+        const bool vec = (p.out_vec >> j) & 1u;
+        const int rows = n < sg.n ? min(p.bm, p.M - t.m0) : 0;
+        const uint32_t st = buf + static_cast<uint32_t>((((lane >> 4) & 1) * 8 + (lane & 7)) * kOutPitch + ((lane >> 3) & 1) * 16);
+        const uint32_t ld = buf + static_cast<uint32_t>(row * kOutPitch + chunk * 16);
+        for (int c = 0; c < p.bm; c += 32) {
+          uint32_t v[2][2][8];  // [lower, upper 16 columns][16 rows][fragments]
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = 0x7FFFFFFFu;
-        }
-        if constexpr (SPLIT) {
-          float* part = reinterpret_cast<float*>(smem_ptr) + c * kBn + 32 * warp + lane;
+          for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) part[i * kBn] = __uint_as_float(v[i]);
-        } else if (out != nullptr) {
+            for (int k = 0; k < 2; ++k) {
+              if (k == 0 || c + 16 < p.bm) {
+                uint32_t(&f)[8] = v[h][k];
+                asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]), "=r"(f[4]), "=r"(f[5]), "=r"(f[6]), "=r"(f[7])
+                             : "r"(src + (static_cast<uint32_t>(16 * h) << 16) + static_cast<uint32_t>(c + 16 * k)));
+              }
+            }
+          }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          __syncwarp();  // the rows before have been read
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (t.m0 + c + i < p.M) out[static_cast<size_t>(c + i) * width] = __bfloat16_as_ushort(__float2bfloat16(__uint_as_float(v[i])));
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              if (k == 0 || c + 16 < p.bm) {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(v[h][k][2 * i]), __uint_as_float(v[h][k][2 * i + 1]));
+                  w[i] = good ? *reinterpret_cast<const uint32_t*>(&two) : 0x7FFF7FFFu;
+                }
+                asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(st + k * (16 * kOutPitch) + h * 32),
+                             "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                             : "memory");
+              }
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = c + 8 * i + row;
+            if (r < rows) {
+              uint32_t o[4];
+              Lds128(ld + i * (8 * kOutPitch), o);
+              uint16_t* const dst = out + static_cast<size_t>(r) * width;
+              if (vec) {
+                *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) dst[e] = static_cast<uint16_t>(o[e >> 1] >> (16 * (e & 1)));
+              }
+            }
           }
         }
       }
@@ -670,27 +729,55 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       }
       uint16_t* const out = p.out[j] + (n - p.col_begin[j]);
       const size_t width = static_cast<size_t>(p.width[j]);
-      for (int m = r0 + warp; m < r1 && t.m0 + m < p.M; m += static_cast<int>(blockDim.x) / 32) {
-        float4 v[8];
+      const bool vec = (p.out_vec >> j) & 1u;
+      const int rows = min(r1, p.M - t.m0), warps = static_cast<int>(blockDim.x) / 32;
+      // ROWS rows a warp at a time, so that the loads of all of them and of all ranks are on their way together
+      auto add_up = [&](auto rows_tag, auto ranks_tag) {
+        constexpr int ROWS = decltype(rows_tag)::value, RANKS = decltype(ranks_tag)::value;
+        for (int m0 = r0 + warp; m0 < rows; m0 += warps * ROWS) {
+          float4 v[ROWS][RANKS];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          if (r < csize) v[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, r) + m * kBn + c);
-        }
-        float4 s = v[0];
+          for (int i = 0; i < ROWS; ++i) {
 #pragma unroll
-        for (int r = 1; r < 8; ++r) {
-          if (r < csize) {
-            s.x += v[r].x;
-            s.y += v[r].y;
-            s.z += v[r].z;
-            s.w += v[r].w;
+            for (int r = 0; r < RANKS; ++r) {
+              if (r < csize && m0 + i * warps < rows)
+                v[i][r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, r) + (m0 + i * warps) * kBn + c);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) {
+            float4 s = v[i][0];
+#pragma unroll
+            for (int r = 1; r < RANKS; ++r) {
+              if (r < csize) {
+                s.x += v[i][r].x;
+                s.y += v[i][r].y;
+                s.z += v[i][r].z;
+                s.w += v[i][r].w;
+              }
+            }
+            if (m0 + i * warps < rows) {
+              uint16_t* const dst = out + static_cast<size_t>(t.m0 + m0 + i * warps) * width;
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(s.x, s.y), hi = __floats2bfloat162_rn(s.z, s.w);
+              const uint2 o = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+              if (vec) {
+                *reinterpret_cast<uint2*>(dst) = o;
+              } else {
+                dst[0] = static_cast<uint16_t>(o.x);
+                dst[1] = static_cast<uint16_t>(o.x >> 16);
+                dst[2] = static_cast<uint16_t>(o.y);
+                dst[3] = static_cast<uint16_t>(o.y >> 16);
+              }
+            }
           }
         }
-        uint16_t* const dst = out + static_cast<size_t>(t.m0 + m) * width;
-        dst[0] = __bfloat16_as_ushort(__float2bfloat16(s.x));
-        dst[1] = __bfloat16_as_ushort(__float2bfloat16(s.y));
-        dst[2] = __bfloat16_as_ushort(__float2bfloat16(s.z));
-        dst[3] = __bfloat16_as_ushort(__float2bfloat16(s.w));
+      };
+      if (csize <= 2) {
+        add_up(std::integral_constant<int, 4>(), std::integral_constant<int, 2>());
+      } else if (csize <= 4) {
+        add_up(std::integral_constant<int, 3>(), std::integral_constant<int, 4>());
+      } else {
+        add_up(std::integral_constant<int, 1>(), std::integral_constant<int, 8>());
       }
     }
   }
@@ -1070,8 +1157,12 @@ bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_
 
 constexpr int kSmemLimit = 232448 - 1024 - static_cast<int>(sizeof(Ctl)) - 64;
 
-int RawBytes(int mode) { return mode == kFp8 ? RawRing<kFp8, 1>::kBytes : mode == kNvfp4 ? RawRing<kNvfp4, 1>::kBytes : 0; }
-int BlocksFor(int mode, int xrows) { return (kSmemLimit - RawBytes(mode)) / (kABytes + xrows * kBk * 2); }
+int RawBytes(int mode, int ks) {
+  if (mode == kFp8) return ks == 2 ? RawRing<kFp8, 2>::kBytes : RawRing<kFp8, 1>::kBytes;
+  if (mode == kNvfp4) return ks == 2 ? RawRing<kNvfp4, 2>::kBytes : RawRing<kNvfp4, 1>::kBytes;
+  return 0;
+}
+int BlocksFor(int mode, int xrows, int ks) { return (kSmemLimit - kOutBytes - RawBytes(mode, ks)) / (kABytes + xrows * kBk * 2); }
 
 template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
 cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream) {
@@ -1199,7 +1290,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   p.K = g.K;
   p.bm = plan.bm;
   const int xrows = plan.pair ? p.bm / 2 : p.bm;
-  const int blocks = BlocksFor(mode, xrows), ks = plan.ks > 0 ? plan.ks : blocks >= 6 ? 2 : 1;
+  const int ks = plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1, blocks = BlocksFor(mode, xrows, ks);
   p.ksteps = (g.K + kBk * ks - 1) / (kBk * ks);
   if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
     throw std::runtime_error("SkinnyGemm(dense): cannot describe x to the copy engine");
@@ -1221,6 +1312,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
     p.out[o] = g.out[o];
     p.col_begin[o] = g.col_begin[o];
     p.width[o] = g.width[o];
+    if (reinterpret_cast<uintptr_t>(g.out[o]) % 16 == 0) p.out_vec |= 1u << o;
   }
   p.m_tiles = static_cast<int>((m + p.bm - 1) / p.bm);
   if (static_cast<int64_t>(p.m_tiles) * n_tiles > INT_MAX / 16) throw std::runtime_error("SkinnyGemm(dense): too many tiles");
@@ -1229,7 +1321,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   p.stages = std::min(kMaxStages, blocks / ks);
   // the dequantising groups take the stages in turn: fewer stages than groups would run off the ring
   if (p.stages < kDqGroups) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * (kABytes + xrows * kBk * 2) + RawBytes(mode);
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * (kABytes + xrows * kBk * 2) + RawBytes(mode, ks) + kOutBytes;
   const int slots = std::max(1, DeviceSmCount() / cluster);
   const int ctas = cluster * (cluster > 1 && !plan.pair ? p.tiles : std::min(p.tiles, slots));
   cudaError_t err;
@@ -1298,7 +1390,7 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   p.m_tiles = static_cast<int>(m_tiles);
   p.tiles = static_cast<int>(n_tiles * m_tiles);
   const int block = kABytes + p.bm * kBk * 2;
-  p.stages = std::min(kMaxStages, (kSmemLimit - 2048 - RawBytes(mode)) / block);
+  p.stages = std::min(kMaxStages, (kSmemLimit - 2048 - RawBytes(mode, 1)) / block);
   q.g = g.x;
   q.u = g.x2;
   q.gx = g.gx;
@@ -1306,7 +1398,7 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   q.routed = g.routed;
   q.gk = g.gk;
   q.cluster = C;
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode);
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode, 1);
   cudaError_t err = mode == kBf16  ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
                     : mode == kFp8 ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
                                    : LaunchShared<kNvfp4>(q, p.tiles, smem, stream);
