@@ -249,7 +249,7 @@ void LaunchDenseGemm(int mode, const GemmParams& p, int64_t m, cudaStream_t stre
 
 // dense_tc.cu: the same calls in one kernel, dequantising into shared memory.
 struct DenseTcPlan {
-  int bm = 0;     // rows of x per tile: a multiple of 16 (32 for pairs), at most 256
+  int bm = 0;     // rows of x per tile: a multiple of 16, at most 256
   int split = 1;  // CTAs (a cluster) that share the K range of a tile
   int pair = 0;   // two CTAs per tile of 256 columns
   int ks = 0;     // blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room

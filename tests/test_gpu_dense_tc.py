@@ -22,7 +22,7 @@ CASES = [
     (300, 512, [[384]]),
 ]
 # rows per tile, CTAs that split K, pair of CTAs, blocks of 64 k per stage
-PLANS = ["", "16,1,0", "48,1,0,1", "48,1,0,2", "256,1,0", "64,2,0,1", "48,3,0,2", "32,8,0", "64,1,1,1", "64,1,1,2", "256,1,1"]
+PLANS = ["", "16,1,0", "48,1,0,1", "48,1,0,2", "256,1,0", "64,2,0,1", "48,3,0,2", "32,8,0", "64,1,1,1", "64,1,1,2", "112,1,1", "256,1,1"]
 
 
 def _check(mode, M, K, seg_widths, plan, seed, x_offset=0):
@@ -104,7 +104,7 @@ def test_graph_capture_and_bad_launch_shapes(cuda):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out[0], eager)
-    for plan in ("8,1,0", "272,1,0", "48,1,1", "64,2,1", "64,9,0", "64,1,0,3"):
+    for plan in ("8,1,0", "272,1,0", "40,1,1", "64,2,1", "64,9,0", "64,1,0,3"):
         op.set_option("dense_plan", plan)
         with pytest.raises(QfgError):
             op(x, w)
