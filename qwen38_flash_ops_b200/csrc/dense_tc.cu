@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdlib>
 #include <stdexcept>
@@ -1217,6 +1218,33 @@ cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream
   return cudaLaunchKernelEx(&cfg, DenseSharedKernel<MODE>, q);
 }
 
+// Clusters of `split` CTAs, one per SM, that are resident at once: a GPC's SMs rarely divide by the size (33 clusters of
+// four, fewer than 16 of eight), and a cluster too many costs a second wave.
+int SplitSlots(int split) {
+  static std::atomic<int> known[9];
+  int n = known[split].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(split));
+  cfg.blockDim = dim3(static_cast<unsigned>(DenseThreads<kBf16>()));
+  cfg.dynamicSmemBytes = kSmemLimit;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto kernel = DenseTcKernel<kBf16, false, false, true, 1>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = std::max(1, DeviceSmCount() * 8 / (10 * split));
+  }
+  known[split].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // describes a stored weight to the copy engine
 bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int ks) {
   const uint64_t rows = static_cast<uint64_t>(K), pitch = static_cast<uint64_t>(sg.pitch), n = static_cast<uint64_t>(sg.n);
@@ -1229,8 +1257,8 @@ bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int
 
 // Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200,
 // K = 5120; us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair
-// 0.13 + 0.00098 bm (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.40 where the rows
-// are loaded in 8-byte pieces); around the blocks 4 + 0.008 bm, and 1 + 0.01 bm more where ranks add up.  More row
+// 0.13 + 0.00098 bm (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.52 and 0.41 where the
+// rows are loaded in 8-byte pieces); around the blocks 4 + 0.008 bm, and 1 + 0.01 bm more where ranks add up.  More row
 // tiles than needed are tried because they can fill the last wave better (509 rows, N = 10240: 3 x 192 56 us,
 // 2 x 256 61 us).
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count) {
@@ -1249,10 +1277,9 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
       const int bm = static_cast<int>(((m + mt - 1) / mt + 15) / 16 * 16);
       if (bm > 256 || (pair && bm < 64)) continue;
       const int64_t tiles = n_tiles * ((m + bm - 1) / bm);
-      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : pieces ? 0.40 : 0.24);
+      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : !pieces ? 0.24 : pair ? 0.41 : 0.52);
       for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
-        // clusters of more than two CTAs do not fill every GPC
-        const int64_t slots = pair || split == 2 ? sm_count / 2 : split == 1 ? sm_count : sm_count * 9 / (10 * split);
+        const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : SplitSlots(split);
         const int64_t waves = (tiles + slots - 1) / std::max<int64_t>(slots, 1);
         if (split > 1 && waves > 1) break;
         const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
