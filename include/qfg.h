@@ -100,11 +100,13 @@ QFG_API int qfg_skinny_gemm_create(const int64_t* seg_outs, int n_seg, const int
  * m-row call is computed with the arithmetic of the one-row call on that row.
  *
  * Prefill-shaped calls: with more rows than the "dense_rows" option (unless set: 8 for BF16 and FP8,
- * 16 for NVFP4 weights, where the branch starts to win on a B200; 0 switches it off) and every width a multiple of 8, the call dequantises the weights to BF16 in column
- * tiles (w_scale folded in before the rounding) and runs cublasGemmEx with FP32 accumulation, as
- * the reference does for M > 8 (fused_gemm.cu:365-428, dispatch at :578-583).  Like the
- * reference's, this branch allocates a handle and a buffer on first use, is not graph-capturable,
- * ignores `trigger`, and its accumulation order is the library's; cuBLAS is loaded at run time. */
+ * 16 for NVFP4 weights; 0 switches it off) and every width a multiple of 8, the call computes with the
+ * weights rounded to BF16, w_scale folded in before the rounding, and FP32 accumulation, as the reference
+ * does for M > 8 (fused_gemm.cu:365-428, dispatch at :578-583).  One kernel dequantises and multiplies
+ * where x and the weights have 16-byte aligned bases, k % 8 == 0 and N is a multiple of 8 (BF16), 16
+ * (FP8) or 128 (NVFP4): nothing is allocated and the call may be captured.  Other layouts dequantise to a
+ * buffer and run cublasGemmEx: that allocates a handle and a buffer on first use and is not
+ * graph-capturable, like the reference's; cuBLAS is loaded at run time.  Both ignore `trigger`. */
 QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, int64_t m, int64_t k,
                             const qfg_tensor2d* weights, int n_weights, void* const* outs, int n_outs,
                             void* stream);
@@ -113,7 +115,8 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
  * programmatic-stream-serialisation attribute and makes it wait for its predecessor
  * (griddepcontrol.wait) only after its first weight tiles are in flight.  "plan" pins the
  * launch geometry ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296"); used by the tuning sweeps.
- * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken. */
+ * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken;
+ * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape. */
 QFG_API int qfg_skinny_gemm_set_option(qfg_skinny_gemm* op, const char* key, const char* value);
 
 /* Writes a one-line description of the launch plan chosen for these shapes into buf. */
@@ -164,7 +167,9 @@ QFG_API void qfg_dequant_destroy(qfg_dequant* op);
  * g, u: BF16 [m, k]; weight [k, n] BF16 / FP8 E4M3FN, or UINT8 [k, 9n/16] NVFP4; gx: BF16 [m, gk];
  * gw: BF16 [gk]; routed: BF16 [m, n] (NULL: y is the shared term alone); out: BF16 [m, n].
  * n % 8 == 0 (NVFP4: n % 64 == 0 as for SkinnyGemm), gk even, any m >= 1 (the reference sends m > 4 to a
- * dense prefill kernel; here rows are processed eight at a time) and any k (the reference: k <= 1024).
+ * dense prefill kernel; here up to sixteen rows run eight at a time, with results that do not depend on m,
+ * and more run in one many-row kernel of the same arithmetic where g, u and the weight have the alignments
+ * SkinnyGemm's needs; "dense_rows" as there) and any k (the reference: k <= 1024).
  * The deferred-merge hook of the reference (QMoESharedExpertBridge, :34-92, :704-718) belongs to an
  * ORT-internal peer and is not reproduced. */
 QFG_API int qfg_shared_expert_down_create(const float* w_scale, size_t n_w_scale, int trigger,

@@ -75,7 +75,7 @@ struct qfg_skinny_gemm {
   int pdl_wait = 0;
   int force_slow = 0;
   int exchange_spin = qfg::kExchangeSpin;  // sharded LM head: bound of the wait for a peer's keys (iterations)
-  int dense_rows = -1;  // calls with more rows take the dequantise + library GEMM branch; -1 = qfg::DenseRowsDefault(mode), 0 = never
+  int dense_rows = -1;  // calls with more rows take the many-row kernel (or the library GEMM); -1 = qfg::DenseRowsDefault(mode), 0 = never
   qfg::DenseTcPlan dense_plan;  // bm > 0: overrides the launch shape of that branch (set_option("dense_plan", "bm,split,pair,ks"))
   unsigned long long phase_times = 0;  // device address given through set_option("phase_times", ...)
   std::string plan_spec;

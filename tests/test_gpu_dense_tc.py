@@ -108,3 +108,8 @@ def test_graph_capture_and_bad_launch_shapes(cuda):
         op.set_option("dense_plan", plan)
         with pytest.raises(QfgError):
             op(x, w)
+
+
+@pytest.mark.parametrize("mode,K", [(0, 8), (1, 8), (2, 8), (0, 24), (2, 40)])
+def test_k_shorter_than_a_block(cuda, mode, K):
+    _check(mode, 33, K, [[128], [256]], "", 5)
