@@ -351,6 +351,8 @@ void InitGemmOp(qfg_skinny_gemm* op, const int64_t* seg_outs, int n_seg, const i
   op->pdl_wait = EnvInt("QFG_PDL_WAIT", 0);
   const cudaError_t err = qfg::ConfigureSkinnyGemmKernels();
   if (err != cudaSuccess) throw std::runtime_error(std::string(name) + ": " + cudaGetErrorString(err));
+  // a node of few-row calls works without the many-row kernels: a failure is reported by the call that needs them
+  if (qfg::ConfigureDenseKernels() != cudaSuccess) cudaGetLastError();
   op->d_w_scale = UploadScales(w_scale, n_w_scale, name);
   op->w_scale_len = op->d_w_scale != nullptr ? n_w_scale : 0;
 }

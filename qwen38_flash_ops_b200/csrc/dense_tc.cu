@@ -38,6 +38,8 @@
 #include <atomic>
 #include <climits>
 #include <cstdlib>
+#include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -1173,9 +1175,6 @@ int BlocksFor(int mode, int xrows, int ks) { return (kSmemLimit - kOutBytes - Ra
 
 template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
 cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream) {
-  static const cudaError_t configured = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                             kSmemLimit + 1024);
-  if (configured != cudaSuccess) return configured;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
   cfg.blockDim = dim3(static_cast<unsigned>(DenseThreads<MODE>()));
@@ -1201,8 +1200,6 @@ cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, int ctas, int cl
 
 template <int MODE>
 cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream_t stream) {
-  static const cudaError_t configured = cudaFuncSetAttribute(DenseSharedKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - 1024);
-  if (configured != cudaSuccess) return configured;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
   cfg.blockDim = dim3(static_cast<unsigned>(SharedThreads<MODE>()));
@@ -1218,31 +1215,84 @@ cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream
   return cudaLaunchKernelEx(&cfg, DenseSharedKernel<MODE>, q);
 }
 
-// Clusters of `split` CTAs, one per SM, that are resident at once: a GPC's SMs rarely divide by the size (33 clusters of
-// four, fewer than 16 of eight), and a cluster too many costs a second wave.
-int SplitSlots(int split) {
-  static std::atomic<int> known[9];
-  int n = known[split].load(std::memory_order_relaxed);
-  if (n > 0) return n;
+// ------------------------------------------------------------------------------ set-up, once per device
+// The shared-memory limit of a kernel belongs to a device, and so do the clusters it holds at once.
+constexpr int kMaxCluster = 8;
+struct DeviceSetup {
+  int device;
+  int slots[kMaxCluster + 1];  // clusters of so many CTAs, one per SM, that are resident at once
+};
+std::mutex g_setup_mu;
+std::map<int, DeviceSetup> g_setup;  // devices that are done; an entry stays as it is
+std::atomic<const DeviceSetup*> g_setup_last{nullptr};  // the last one asked for: a process mostly drives one
+
+template <int MODE, bool SCALED, int KS>
+cudaError_t SetUpShape() {
+  cudaError_t err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  return err;
+}
+template <int MODE, bool SCALED>
+cudaError_t SetUpMode() {
+  const cudaError_t err = SetUpShape<MODE, SCALED, 1>();
+  return err == cudaSuccess ? SetUpShape<MODE, SCALED, 2>() : err;
+}
+template <int MODE>
+cudaError_t SetUpShared() {
+  return cudaFuncSetAttribute(DenseSharedKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - 1024);
+}
+
+// A GPC's SMs rarely divide by the size (33 clusters of four, fewer than 16 of eight), and a cluster too many costs a
+// second wave.
+int QuerySlots(int cluster) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(split));
+  cfg.gridDim = dim3(static_cast<unsigned>(cluster));
   cfg.blockDim = dim3(static_cast<unsigned>(DenseThreads<kBf16>()));
   cfg.dynamicSmemBytes = kSmemLimit;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const auto kernel = DenseTcKernel<kBf16, false, false, true, 1>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, DenseTcKernel<kBf16, false, false, true, 1>, &cfg) != cudaSuccess || n < 1) {
     cudaGetLastError();
-    n = std::max(1, DeviceSmCount() * 8 / (10 * split));
+    n = std::max(1, DeviceSmCount() * 8 / (10 * cluster));
   }
-  known[split].store(n, std::memory_order_relaxed);
   return n;
+}
+
+// The set-up of the current device, made on the first request.  Only a success is kept.
+cudaError_t SetUpDevice(const DeviceSetup** out) {
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  *out = g_setup_last.load(std::memory_order_acquire);
+  if (*out != nullptr && (*out)->device == dev) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(g_setup_mu);
+  auto it = g_setup.find(dev);
+  if (it == g_setup.end()) {
+    err = SetUpMode<kBf16, false>();
+    if (err == cudaSuccess) err = SetUpMode<kFp8, false>();
+    if (err == cudaSuccess) err = SetUpMode<kFp8, true>();
+    if (err == cudaSuccess) err = SetUpMode<kNvfp4, false>();
+    if (err == cudaSuccess) err = SetUpMode<kNvfp4, true>();
+    if (err == cudaSuccess) err = SetUpShared<kBf16>();
+    if (err == cudaSuccess) err = SetUpShared<kFp8>();
+    if (err == cudaSuccess) err = SetUpShared<kNvfp4>();
+    if (err != cudaSuccess) return err;
+    DeviceSetup d = {dev, {}};
+    for (int c = 1; c <= kMaxCluster; ++c) d.slots[c] = QuerySlots(c);
+    it = g_setup.emplace(dev, d).first;
+  }
+  *out = &it->second;
+  g_setup_last.store(*out, std::memory_order_release);
+  return cudaSuccess;
 }
 
 // describes a stored weight to the copy engine
@@ -1255,6 +1305,13 @@ bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int
 
 }  // namespace
 
+// Called when a node is created, so that the first call finds nothing left to do and may be captured, and again by each
+// call, which may have another device current.
+cudaError_t ConfigureDenseKernels() {
+  const DeviceSetup* setup = nullptr;
+  return SetUpDevice(&setup);
+}
+
 // Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200,
 // K = 5120; us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair
 // 0.13 + 0.00098 bm (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.52 and 0.41 where the
@@ -1262,6 +1319,8 @@ bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int
 // tiles than needed are tried because they can fill the last wave better (509 rows, N = 10240: 3 x 192 56 us,
 // 2 x 256 61 us).
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count) {
+  const DeviceSetup* setup = nullptr;
+  if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SkinnyGemm(dense): the kernels could not be set up on this device");
   DenseTcPlan best;
   double best_cost = 1e30, bytes = 0;
   bool pieces = false;
@@ -1279,7 +1338,7 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
       const int64_t tiles = n_tiles * ((m + bm - 1) / bm);
       const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : !pieces ? 0.24 : pair ? 0.41 : 0.52);
       for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
-        const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : SplitSlots(split);
+        const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : setup->slots[split];
         const int64_t waves = (tiles + slots - 1) / std::max<int64_t>(slots, 1);
         if (split > 1 && waves > 1) break;
         const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
@@ -1356,7 +1415,8 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   const size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * (kABytes + xrows * kBk * 2) + RawBytes(mode, ks) + kOutBytes;
   const int slots = std::max(1, DeviceSmCount() / cluster);
   const int ctas = cluster * (cluster > 1 && !plan.pair ? p.tiles : std::min(p.tiles, slots));
-  cudaError_t err;
+  cudaError_t err = ConfigureDenseKernels();
+  if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
   if (mode == kBf16) {
     err = LaunchMode<kBf16, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
   } else if (mode == kFp8) {
@@ -1431,9 +1491,14 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   q.gk = g.gk;
   q.cluster = C;
   const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode, 1);
-  cudaError_t err = mode == kBf16  ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
-                    : mode == kFp8 ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
-                                   : LaunchShared<kNvfp4>(q, p.tiles, smem, stream);
+  // like the streaming kernels that take the shorter calls of this op, it runs on the device they were set up for
+  cudaError_t err = CheckConfiguredDevice();
+  if (err == cudaSuccess) err = ConfigureDenseKernels();
+  if (err == cudaSuccess) {
+    err = mode == kBf16  ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
+          : mode == kFp8 ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
+                         : LaunchShared<kNvfp4>(q, p.tiles, smem, stream);
+  }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SharedExpertDown: ") + cudaGetErrorString(err));
 }

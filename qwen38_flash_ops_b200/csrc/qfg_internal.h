@@ -205,6 +205,7 @@ std::string DescribePlan(const Plan& plan, const PlanInput& in);
 cudaError_t LaunchSkinnyGemm(int mode, GemmParams& p, const Plan& plan, cudaStream_t stream);
 int DeviceSmCount();
 cudaError_t ConfigureSkinnyGemmKernels();
+cudaError_t CheckConfiguredDevice();  // cudaErrorInvalidDevice where another device than the configured one is current
 int QueryMaxActiveClusters(int mode, int direct, int threads, size_t smem, int cluster);
 
 // argmax_rows.cu
@@ -254,6 +255,7 @@ struct DenseTcPlan {
   int pair = 0;   // two CTAs per tile of 256 columns
   int ks = 0;     // blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room
 };
+cudaError_t ConfigureDenseKernels();  // on the current device
 bool DenseTcEligible(int mode, const GemmParams& p);
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count);
 void LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);  // throws std::runtime_error

@@ -2444,12 +2444,18 @@ cudaError_t ConfigureSkinnyGemmKernels() {
   return status;
 }
 
-cudaError_t LaunchSkinnyGemm(int mode, GemmParams& p, const Plan& plan, cudaStream_t stream) {
-  // The kernels' attributes (shared-memory limits, co-resident cluster counts, SM count) were set up for one
-  // device: one process drives one GPU, and a call with another device current is refused rather than launched
-  // with the wrong limits.
+// The kernels' attributes (shared-memory limits, co-resident cluster counts, SM count) were set up for one
+// device: one process drives one GPU, and a call with another device current is refused rather than launched
+// with the wrong limits.
+cudaError_t CheckConfiguredDevice() {
   int dev = -1;
   if (g_configured_device >= 0 && (cudaGetDevice(&dev) != cudaSuccess || dev != g_configured_device)) return cudaErrorInvalidDevice;
+  return cudaSuccess;
+}
+
+cudaError_t LaunchSkinnyGemm(int mode, GemmParams& p, const Plan& plan, cudaStream_t stream) {
+  const cudaError_t device = CheckConfiguredDevice();
+  if (device != cudaSuccess) return device;
   const ModeGeom geom = GeomOf(mode, plan.direct ? plan.wide : 1);
   p.wn = plan.wn;
   p.wk = plan.wk;

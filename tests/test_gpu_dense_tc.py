@@ -1,10 +1,13 @@
 """The many-row kernel of SkinnyGemm (csrc/dense_tc.cu) at the edges of its tiles: ragged rows, K that ends inside a
 block of 64, column tiles cut short, several weights and outputs, every launch shape, both ways of loading NVFP4 rows."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
-from conftest import bits, to_dev
+from conftest import ROOT, bits, to_dev
 from oracle import cpu as C
 from oracle import oracle as O
 from qwen38_flash_ops_b200 import QfgError, SkinnyGemm
@@ -113,3 +116,34 @@ def test_graph_capture_and_bad_launch_shapes(cuda):
 @pytest.mark.parametrize("mode,K", [(0, 8), (1, 8), (2, 8), (0, 24), (2, 40)])
 def test_k_shorter_than_a_block(cuda, mode, K):
     _check(mode, 33, K, [[128], [256]], "", 5)
+
+
+def test_first_call_of_a_process_may_be_captured(cuda):
+    """Nothing is left for the first call to set up: each kernel's first launch of the process is a captured one."""
+    code = """
+import torch
+from qwen38_flash_ops_b200 import SharedExpertDown, SkinnyGemm
+mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+w = mk(512, 256)
+nibbles = torch.randint(0, 256, (512, 144), device="cuda", dtype=torch.uint8)
+nibbles[:, 128:] %= 0x7F
+gx, gw, routed = mk(64, 64), mk(64, 1), mk(64, 256)
+calls = []
+for weight in (w, w.to(torch.float8_e4m3fn), nibbles):
+    for rows in (64, 700):
+        x, op, out = mk(rows, 512), SkinnyGemm([1], [256]), torch.zeros(rows, 256, device="cuda", dtype=torch.bfloat16)
+        calls.append(lambda op=op, x=x, weight=weight, out=out: op(x, weight, out=[out])[0])
+    x, op = mk(64, 512), SharedExpertDown()
+    calls.append(lambda op=op, x=x, weight=weight: op(x, x, weight, gx, gw, routed))
+torch.cuda.synchronize()
+for call in calls:
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = call()
+    graph.replay()
+    got = y.clone()
+    assert torch.equal(got, call()) and torch.isfinite(got).all() and got.abs().max() > 0
+print("ok")
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr[-2000:]
