@@ -294,8 +294,10 @@ void Run(const qfg_skinny_gemm& op, Prepared& pr, int64_t m, cudaStream_t stream
     }
     return;
   }
+  // SharedExpertDown: a pinned launch geometry or load path is one of the streaming kernels
   const int shared_rows = op.dense_rows < 0 ? qfg::kDenseSharedRows : op.dense_rows;
-  if (pr.params.fuse && shared_rows > 0 && m > shared_rows && qfg::DenseSharedEligible(pr.mode, pr.params)) {
+  if (pr.params.fuse && shared_rows > 0 && m > shared_rows && pr.params.force_slow == 0 && op.plan_spec.empty() &&
+      std::getenv("QFG_PLAN") == nullptr && qfg::DenseSharedEligible(pr.mode, pr.params)) {
     const qfg::DenseTcPlan plan =
         op.dense_plan.bm > 0 ? op.dense_plan : qfg::ChooseDenseSharedPlan(pr.params, m, pr.plan_in.sm_count);
     qfg::LaunchDenseShared(pr.mode, pr.params, m, plan, stream);

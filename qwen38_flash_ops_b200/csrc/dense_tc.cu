@@ -819,6 +819,7 @@ struct DenseShared {
   DenseParams d;
   const uint16_t *g, *u, *gx, *gw, *routed;
   int gk, cluster;
+  int trigger, pdl_wait;  // as in GemmParams
 };
 
 constexpr int kSwishWarps = 8;  // sixteen, at 64 registers a thread, measured no faster (27.0 us, and 5-10 % slower on small calls)
@@ -1023,6 +1024,9 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
   if (C > 1) cg::this_cluster().sync();  // every CTA's barriers exist
   FenceAfter();
   const uint32_t tmem = ctl.tmem;
+  // nothing of the call is read or written before this line: a predecessor may be writing any of it
+  if (q.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (q.trigger == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int kFirstSwish = kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps);
 
   // first the gates, by the warps that the sums need last
@@ -1066,6 +1070,7 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
       }
       __syncwarp();
     }
+    if (q.trigger == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   } else if (warp >= kFirstSwish) {
     SwishRole(q, ctl, warp - kFirstSwish, lane, rank, t.m0, smem, block_bytes);
   } else if (MODE != kBf16 && warp >= 6) {
@@ -1205,13 +1210,15 @@ cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream
   cfg.blockDim = dim3(static_cast<unsigned>(SharedThreads<MODE>()));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = static_cast<unsigned>(q.cluster);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = q.pdl_wait ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, DenseSharedKernel<MODE>, q);
 }
 
@@ -1490,6 +1497,8 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   q.routed = g.routed;
   q.gk = g.gk;
   q.cluster = C;
+  q.trigger = g.trigger;
+  q.pdl_wait = g.pdl_wait;
   const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode, 1);
   // like the streaming kernels that take the shorter calls of this op, it runs on the device they were set up for
   cudaError_t err = CheckConfiguredDevice();

@@ -6,7 +6,7 @@ import torch
 
 from conftest import bits, to_dev
 from oracle import oracle as O
-from qwen38_flash_ops_b200 import QfgError, SharedExpertDown
+from qwen38_flash_ops_b200 import QfgError, SharedExpertDown, SkinnyGemm
 from qwen38_flash_ops_b200 import packing as P
 
 import _util as U
@@ -95,6 +95,44 @@ def test_swish_of_every_bf16_value_is_the_streaming_kernels(cuda):
         a, b = (op(gj, u, w.bfloat16(), gx, gw, routed)[:, j] for op in (many, few))
         assert torch.equal(torch.isnan(a), torch.isnan(b))
         assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("trigger", [1, 2])
+def test_programmatic_launch_behind_an_early_trigger(cuda, mode, trigger):
+    """A predecessor that releases its dependents at once writes g; the many-row kernel must not read it before that."""
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    M, K, N = 200, 640, 1152
+    w = [mk(K, N) * 0.02, mk(K, N).to(torch.float8_e4m3fn), torch.randint(0, 0x7F, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)][mode]
+    x, wg, u, gx, gw, routed = mk(M, 2560), mk(2560, K) * 0.02, mk(M, K), mk(M, 512), mk(512, 1), mk(M, N)
+    before, op, after = SkinnyGemm([1], [K], trigger=1), SharedExpertDown(trigger=trigger), SkinnyGemm([1], [K], trigger=1)
+    for node in (before, op, after):
+        node.set_option("pdl_wait", 1)
+    for node in (before, after):
+        node.set_option("dense_rows", 0)
+    want = SharedExpertDown()(before(x, wg)[0], u, w, gx, gw, routed)
+    wn = mk(N, K) * 0.02
+    want_next = after(want, wn)[0]
+    torch.cuda.synchronize()
+
+    def chain():
+        g = before(x, wg)[0]
+        y = op(g, u, w, gx, gw, routed)
+        return y, after(y, wn)[0]
+
+    for _ in range(50):
+        y, z = chain()
+        assert torch.equal(y, want) and torch.equal(z, want_next)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y, z = chain()
+    for _ in range(20):
+        y.zero_()
+        z.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want) and torch.equal(z, want_next)
 
 
 def test_bad_launch_shapes(cuda):

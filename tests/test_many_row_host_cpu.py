@@ -122,3 +122,23 @@ def test_a_failed_set_up_is_tried_again(fake):
         print(json.dumps([bad, run_gemm(h, FP8, 64, 512, [[256]])]))
         """)
     assert out[0][0] != 0 and out[1][0] == 0
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+def test_shared_expert_options_at_any_row_count(fake, dtype):
+    """`pdl_wait` reaches the many-row kernel's launch; a pinned launch geometry or load path is the streaming kernels'."""
+    out = fake(f"""
+        r = [run_shared(shared(), {dtype}, 40, 256, 128), run_shared(shared(pdl_wait=1), {dtype}, 40, 256, 128),
+             run_shared(shared(plan="direct=0,wn=2,wk=2,cluster=1"), {dtype}, 40, 256, 128), run_shared(shared(force_slow=1), {dtype}, 40, 256, 128)]
+        os.environ["QFG_PLAN"] = "direct=0,wn=2,wk=2,cluster=1"
+        print(json.dumps(r + [run_shared(shared(), {dtype}, 40, 256, 128)]))
+        """)
+    for code, message, log in out:
+        assert code == 0, message
+    logs = [log for _, _, log in out]
+    assert _kernels(logs[0]) == _kernels(logs[1]) == ["DenseSharedKernel"]
+    assert logs[0][0].endswith("pdl=0") and logs[1][0].endswith("pdl=1")
+    for log in logs[2:]:
+        assert _kernels(log) == ["SkinnyGemm"] * 5  # eight rows a pass
+    # the three weight types' ring kernels, not whatever the planner prefers
+    assert all("SkinnyGemmRingKernel" in line and "threads=128 " in line for line in logs[2] + logs[4])
