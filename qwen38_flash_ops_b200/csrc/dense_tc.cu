@@ -27,7 +27,8 @@
 // come from shared memory rather than tensor memory because the rows of x per pass would be limited to 64 there, and the
 // weights are written MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
 //
-// Every wait is bounded; a CTA that gives up on one writes NaN and leaves.
+// Every wait is bounded.  A CTA that gives up on one writes NaN to the rest of its tiles and leaves: the call then reports
+// no error, but no output keeps what its memory held before.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -537,9 +538,10 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
     // ---- epilogue
     const uint32_t buf = smem + static_cast<uint32_t>(p.stages) * stage_bytes + RawRing<MODE, KS>::kBytes + static_cast<uint32_t>(warp * 32 * kOutPitch);
     int it = 0;
+    bool good = true;  // false from the first wait that ran out: no sums come any more, and the tiles that are left become NaN
     for (int tile = first_tile; tile < p.tiles; tile += tile_step, ++it) {
       const int b = it & 1;
-      const bool good = BarWait(accf0 + b * 8, static_cast<uint32_t>((it >> 1) & 1), ctl);
+      good = good && BarWait(accf0 + b * 8, static_cast<uint32_t>((it >> 1) & 1), ctl);
       __syncwarp();
       FenceAfter();
       const TileAt t = LocateDense<PAIR>(p, tile, rank);
@@ -626,8 +628,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       }
       FenceBefore();
       __syncwarp();
-      if (lane == 0) BarArriveLeader<PAIR>(acce0 + b * 8);
-      if (!good) break;
+      if (lane == 0 && good) BarArriveLeader<PAIR>(acce0 + b * 8);
     }
   } else if (warp == 4) {
     // ---- x (and BF16 weights)
