@@ -547,6 +547,10 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       const TileAt t = LocateDense<PAIR>(p, tile, rank);
       const uint32_t src = tmem + (static_cast<uint32_t>(32 * warp) << 16) + static_cast<uint32_t>(b * p.bm);
       if constexpr (SPLIT) {  // lane = column 32 warp + lane of the tile
+        // The sums go where the stages were.  After a wait that ran out, copies may still be landing there and other warps may
+        // not have given up yet, and would write over the NaN that the peers are to see: leave them time (a flag for the peers,
+        // read after they meet, made every call 3-5 % slower).
+        for (int i = 0; i < 16 && !good; ++i) __nanosleep(1000000);
         for (int c = 0; c < p.bm; c += 16) {
           uint32_t v[16];
           asm volatile(
