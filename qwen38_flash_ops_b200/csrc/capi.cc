@@ -285,23 +285,21 @@ qfg::Plan ComputePlan(const qfg_skinny_gemm& op, const qfg::PlanInput& in) {
 void Run(const qfg_skinny_gemm& op, Prepared& pr, int64_t m, cudaStream_t stream, const char* name) {
   const int dense_rows = op.dense_rows < 0 ? qfg::DenseRowsDefault(pr.mode) : op.dense_rows;
   if (dense_rows > 0 && m > dense_rows && qfg::DenseEligible(pr.params)) {
-    if (qfg::DenseTcEligible(pr.mode, pr.params)) {
+    if (qfg::DenseTcEligible(pr.mode, pr.params, m)) {
       const qfg::DenseTcPlan plan =
           op.dense_plan.bm > 0 ? op.dense_plan : qfg::ChooseDenseTcPlan(pr.mode, pr.params, m, pr.plan_in.sm_count);
-      qfg::LaunchDenseTc(pr.mode, pr.params, m, plan, stream);
-    } else {
-      qfg::LaunchDenseGemm(pr.mode, pr.params, m, stream);
+      if (qfg::LaunchDenseTc(pr.mode, pr.params, m, plan, stream)) return;
     }
+    qfg::LaunchDenseGemm(pr.mode, pr.params, m, stream);
     return;
   }
   // SharedExpertDown: a pinned launch geometry or load path is one of the streaming kernels
   const int shared_rows = op.dense_rows < 0 ? qfg::kDenseSharedRows : op.dense_rows;
   if (pr.params.fuse && shared_rows > 0 && m > shared_rows && pr.params.force_slow == 0 && op.plan_spec.empty() &&
-      std::getenv("QFG_PLAN") == nullptr && qfg::DenseSharedEligible(pr.mode, pr.params)) {
+      std::getenv("QFG_PLAN") == nullptr && qfg::DenseSharedEligible(pr.mode, pr.params, m)) {
     const qfg::DenseTcPlan plan =
         op.dense_plan.bm > 0 ? op.dense_plan : qfg::ChooseDenseSharedPlan(pr.params, m, pr.plan_in.sm_count);
-    qfg::LaunchDenseShared(pr.mode, pr.params, m, plan, stream);
-    return;
+    if (qfg::LaunchDenseShared(pr.mode, pr.params, m, plan, stream)) return;
   }
   const qfg::Plan plan = PlanFor(op, pr.plan_in, static_cast<int>(std::min<int64_t>(m, qfg::kMaxRows)));
   qfg::GemmParams base = pr.params;

@@ -1368,9 +1368,9 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
 }
 
 // 16-byte rows of x; weights that a tensor map describes, or NVFP4 ones in whole 128-column groups; every output a
-// multiple of eight columns.
-bool DenseTcEligible(int mode, const GemmParams& p) {
-  if (p.K % 8 != 0 || reinterpret_cast<uintptr_t>(p.x) % 16 != 0) return false;
+// multiple of eight columns; rows that fit the kernel's 32-bit counts with a tile to spare.
+bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
+  if (m > INT_MAX / 2 || p.K % 8 != 0 || reinterpret_cast<uintptr_t>(p.x) % 16 != 0) return false;
   for (int s = 0; s < p.nseg; ++s) {
     const Segment& sg = p.seg[s];
     if (reinterpret_cast<uintptr_t>(sg.w) % 16 != 0) return false;
@@ -1383,8 +1383,7 @@ bool DenseTcEligible(int mode, const GemmParams& p) {
   return Encoder() != nullptr;
 }
 
-void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
-  if (m > INT_MAX / 2) throw std::runtime_error("SkinnyGemm(dense): too many rows");
+bool LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   if (plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.split < 1 || plan.split > 8 || (plan.pair && plan.split != 1) || plan.ks < 0 || plan.ks > 2)
     throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
   DenseParams p = {};
@@ -1396,7 +1395,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   const int ks = plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1, blocks = BlocksFor(mode, xrows, ks);
   p.ksteps = (g.K + kBk * ks - 1) / (kBk * ks);
   if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
-    throw std::runtime_error("SkinnyGemm(dense): cannot describe x to the copy engine");
+    return false;
   bool scaled = false;
   p.raw_tensor = 1;
   int n_tiles = 0;
@@ -1408,7 +1407,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
     p.raw_tensor = p.raw_tensor && sg.pitch % 16 == 0;
   }
   for (int s = 0; s < g.nseg && p.raw_tensor; ++s) {
-    if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks)) throw std::runtime_error("SkinnyGemm(dense): cannot describe the weight to the copy engine");
+    if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks)) return false;
   }
   const int n_out = g.seg[g.nseg - 1].out_end;
   for (int o = 0; o < n_out; ++o) {
@@ -1418,7 +1417,7 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
     if (reinterpret_cast<uintptr_t>(g.out[o]) % 16 == 0) p.out_vec |= 1u << o;
   }
   p.m_tiles = static_cast<int>((m + p.bm - 1) / p.bm);
-  if (static_cast<int64_t>(p.m_tiles) * n_tiles > INT_MAX / 16) throw std::runtime_error("SkinnyGemm(dense): too many tiles");
+  if (static_cast<int64_t>(p.m_tiles) * n_tiles > INT_MAX / 16) return false;
   p.tiles = p.m_tiles * n_tiles;
   const int cluster = plan.pair ? 2 : std::min(plan.split, p.ksteps);
   p.stages = std::min(kMaxStages, blocks / ks);
@@ -1439,11 +1438,12 @@ void LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
+  return true;
 }
 
 // SharedExpertDown: 16-byte rows of g and u as well.
-bool DenseSharedEligible(int mode, const GemmParams& p) {
-  return p.fuse && p.nseg == 1 && DenseTcEligible(mode, p) && reinterpret_cast<uintptr_t>(p.x2) % 16 == 0;
+bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m) {
+  return p.fuse && p.nseg == 1 && DenseTcEligible(mode, p, m) && reinterpret_cast<uintptr_t>(p.x2) % 16 == 0;
 }
 
 // Rows per tile and CTAs per cluster, by a model fitted to measured launches (us): a block of 64 k costs 0.10 + 0.0125
@@ -1471,9 +1471,8 @@ DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) 
   return best;
 }
 
-void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+bool LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int C = plan.split;
-  if (m > INT_MAX / 2) throw std::runtime_error("SharedExpertDown: too many rows");
   if ((C != 1 && C != 2 && C != 4) || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm % (8 * C) != 0)
     throw std::runtime_error("SharedExpertDown: bad launch shape");
   DenseShared q = {};
@@ -1488,9 +1487,9 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   p.out[0] = g.out[0];
   p.width[0] = sg.n;
   p.raw_tensor = sg.pitch % 16 == 0;
-  if (p.raw_tensor && !EncodeWeight(p, mode, 0, sg, g.K, 1)) throw std::runtime_error("SharedExpertDown: cannot describe the weight to the copy engine");
+  if (p.raw_tensor && !EncodeWeight(p, mode, 0, sg, g.K, 1)) return false;
   const int64_t n_tiles = ((sg.n + kBn - 1) / kBn + C - 1) / C * C, m_tiles = (m + p.bm - 1) / p.bm;
-  if (n_tiles * m_tiles > INT_MAX / 16) throw std::runtime_error("SharedExpertDown: too many tiles");
+  if (n_tiles * m_tiles > INT_MAX / 16) return false;
   p.m_tiles = static_cast<int>(m_tiles);
   p.tiles = static_cast<int>(n_tiles * m_tiles);
   const int block = kABytes + p.bm * kBk * 2;
@@ -1515,6 +1514,7 @@ void LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SharedExpertDown: ") + cudaGetErrorString(err));
+  return true;
 }
 
 }  // namespace qfg

@@ -256,17 +256,19 @@ struct DenseTcPlan {
   int ks = 0;     // blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room
 };
 cudaError_t ConfigureDenseKernels();  // on the current device
-bool DenseTcEligible(int mode, const GemmParams& p);
+bool DenseTcEligible(int mode, const GemmParams& p, int64_t m);
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count);
-void LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);  // throws std::runtime_error
+// false, nothing launched: more tiles than the kernel counts, or a tensor map that could not be made.  Throws
+// std::runtime_error (a launch shape that does not exist, a launch that failed).
+bool LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);
 
 // SharedExpertDown over many rows; `split` of the plan is the cluster size (1, 2 or 4).  Calls of up to sixteen rows keep
 // the streaming kernels, whose results do not depend on the number of rows; at seventeen they take three passes, 43 us
 // (NVFP4 640 x 2560), and the many-row kernel 11.
 constexpr int kDenseSharedRows = 16;
-bool DenseSharedEligible(int mode, const GemmParams& p);
+bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m);
 DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count);
-void LaunchDenseShared(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);  // throws std::runtime_error
+bool LaunchDenseShared(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);  // as LaunchDenseTc
 
 // untile_hc.cu
 cudaError_t LaunchUntileHc(bool fp8, const void* w, void* out, const float* scale, int kind, cudaStream_t stream);

@@ -142,3 +142,20 @@ def test_shared_expert_options_at_any_row_count(fake, dtype):
         assert _kernels(log) == ["SkinnyGemm"] * 5  # eight rows a pass
     # the three weight types' ring kernels, not whatever the planner prefers
     assert all("SkinnyGemmRingKernel" in line and "threads=128 " in line for line in logs[2] + logs[4])
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+def test_what_the_many_row_kernels_cannot_take_goes_the_general_way(fake, dtype):
+    """A tensor map that cannot be made, and more rows than the kernel counts: the library branch (with its
+    dequantisation) and the streaming kernels take these calls."""
+    gemm, shared, rows = fake(f"""
+        h, s = gemm([1], [256]), shared()
+        fake.fake_refuse_encode(1)
+        r = [run_gemm(h, {dtype}, 64, 512, [[256]]), run_shared(s, {dtype}, 40, 256, 256)]
+        fake.fake_refuse_encode(0)
+        print(json.dumps(r + [run_gemm(h, {dtype}, 2 ** 30, 8, [[256]])]))
+        """)
+    library = [] if dtype == "BF16" else ["DequantKernel"]
+    assert gemm[0] == 0 and _kernels(gemm[2]) == library + ["cublas"], gemm
+    assert rows[0] == 0 and _kernels(rows[2]) == library + ["cublas"], rows
+    assert shared[0] == 0 and _kernels(shared[2]) == ["SkinnyGemm"] * 5, shared
