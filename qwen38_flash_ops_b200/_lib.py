@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import os
 from ctypes import POINTER, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_uint64, c_void_p
+from types import SimpleNamespace
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # QFG_LIBRARY names another build of the same library (a measurement build, for instance)
@@ -67,8 +68,8 @@ def load() -> ctypes.CDLL:
     lib.qfg_version.restype = c_char_p
     lib.qfg_skinny_gemm_create.argtypes = [POINTER(c_int64), c_int, POINTER(c_int64), c_int, POINTER(c_float),
                                            c_size_t, c_int, POINTER(c_void_p)]
-    # void pointers where the ops pass packed bytes for a Tensor2D or an array (structures and arrays work too)
-    lib.qfg_skinny_gemm_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int, c_void_p]
+    lib.qfg_skinny_gemm_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int,
+                                            POINTER(c_void_p), c_int, c_void_p]
     lib.qfg_skinny_gemm_set_option.argtypes = [c_void_p, c_char_p, c_char_p]
     lib.qfg_skinny_gemm_describe.argtypes = [c_void_p, c_int64, POINTER(Tensor2D), c_int, c_char_p, c_size_t]
     lib.qfg_plan_describe.argtypes = [c_int, c_int64, POINTER(c_int64), c_int, c_int, c_int, c_char_p, c_char_p,
@@ -78,18 +79,18 @@ def load() -> ctypes.CDLL:
     lib.qfg_argmax_rows.argtypes = [c_int, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p]
     lib.qfg_dequant_create.argtypes = [c_int64, c_int64, POINTER(c_int64), c_int, POINTER(c_float), c_size_t,
                                        POINTER(c_void_p)]
-    lib.qfg_dequant_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p]
+    lib.qfg_dequant_compute.argtypes = [c_void_p, POINTER(Tensor2D), POINTER(c_void_p), c_int, c_void_p]
     lib.qfg_dequant_destroy.argtypes = [c_void_p]
     lib.qfg_dequant_destroy.restype = None
     lib.qfg_lmhead_workspace_bytes.restype = c_size_t
     lib.qfg_lmhead_create.argtypes = [POINTER(c_float), c_size_t, c_int, POINTER(c_void_p)]
-    lib.qfg_lmhead_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64,
+    lib.qfg_lmhead_compute.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int64, c_int64,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.qfg_lmhead_static_max_rows.restype = c_size_t
     lib.qfg_lmhead_compute_static.argtypes = [c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_int64, c_int64,
                                               c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.qfg_shared_expert_down_create.argtypes = [POINTER(c_float), c_size_t, c_int, POINTER(c_void_p)]
-    lib.qfg_shared_expert_down_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
+    lib.qfg_shared_expert_down_compute.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, POINTER(Tensor2D), c_void_p,
                                                    c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]
     lib.qfg_shared_expert_down_set_option.argtypes = [c_void_p, c_char_p, c_char_p]
     lib.qfg_shared_expert_down_destroy.argtypes = [c_void_p]
@@ -117,6 +118,13 @@ def load() -> ctypes.CDLL:
     lib.qfg_lmhead_destroy.argtypes = [c_void_p]
     lib.qfg_lmhead_destroy.restype = None
     lib.qfg_lmhead_combine.argtypes = [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p]
+    # The same entry points for the ops, which pass packed bytes for a Tensor2D or an array of pointers: function objects of
+    # their own, so that the checks above hold for every other caller.
+    lib.packed = SimpleNamespace()
+    for name in ("qfg_skinny_gemm_compute", "qfg_dequant_compute", "qfg_lmhead_compute", "qfg_shared_expert_down_compute"):
+        fn = lib[name]
+        fn.argtypes = [c_void_p if issubclass(t, ctypes._Pointer) else t for t in getattr(lib, name).argtypes]
+        setattr(lib.packed, name, fn)
     _lib = lib
     return lib
 

@@ -113,7 +113,7 @@ class SkinnyGemm:
             lead, device = tuple(shape[:-1]), x.device
             out = [torch.empty(lead + (w,), dtype=torch.bfloat16, device=device) for w in self.widths]
         descs = b"".join([_weight(w) for w in weights])
-        code = self._lib.qfg_skinny_gemm_compute(self._h, x.data_ptr(), m, k, descs, len(weights), _pointers(out), len(out),
+        code = self._lib.packed.qfg_skinny_gemm_compute(self._h, x.data_ptr(), m, k, descs, len(weights), _pointers(out), len(out),
                                                  _stream_ptr())
         if code:
             check(code)
@@ -177,7 +177,7 @@ class DequantWeightBf16:
     def __call__(self, w: torch.Tensor, out=None):
         t = _weight(w)
         outs = out if out is not None else [torch.empty((w.shape[0], wd), dtype=torch.bfloat16, device=w.device) for wd in self.widths]
-        check(self._lib.qfg_dequant_compute(self._h, t, _pointers(outs), len(outs), _stream_ptr()))
+        check(self._lib.packed.qfg_dequant_compute(self._h, t, _pointers(outs), len(outs), _stream_ptr()))
         return outs
 
     def __del__(self):
@@ -226,7 +226,7 @@ class SharedExpertDown:
         elif w.shape[1] != n:
             raise QfgError(_lib.QFG_FAIL, "SharedExpertDown: weight N mismatch")
         out = torch.empty_like(routed)
-        check(self._lib.qfg_shared_expert_down_compute(self._h, g.data_ptr(), u.data_ptr(), m, k, t, gx.data_ptr(),
+        check(self._lib.packed.qfg_shared_expert_down_compute(self._h, g.data_ptr(), u.data_ptr(), m, k, t, gx.data_ptr(),
                                                        gk, gw.data_ptr(), routed.data_ptr(), n, out.data_ptr(), _stream_ptr()))
         return out
 
@@ -310,7 +310,7 @@ class LmHeadArgmax:
         else:
             idx, val, key = out
         lg = torch.empty((m, n), dtype=torch.bfloat16, device=x.device) if logits else None
-        check(self._lib.qfg_lmhead_compute(self._h, x.data_ptr(), m, k, t, int(n), int(col_offset),
+        check(self._lib.packed.qfg_lmhead_compute(self._h, x.data_ptr(), m, k, t, int(n), int(col_offset),
                                            self.workspace.data_ptr(), idx.data_ptr(), val.data_ptr(), key.data_ptr(),
                                            lg.data_ptr() if logits else None, _stream_ptr()))
         return (idx, val, key, lg) if logits else (idx, val, key)

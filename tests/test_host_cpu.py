@@ -139,3 +139,20 @@ def test_key_pack_orders_like_argmax():
     assert np.array_equal(np.isnan(v), np.isnan(vals))
     ok = ~np.isnan(vals)
     assert np.array_equal(v[ok], vals[ok])
+
+
+def test_entry_points_check_the_type_of_their_arguments():
+    """A weight is passed as a Tensor2D, by value or by reference; a number or a text in its place is refused."""
+    lib, w, outs = _lib.load(), _lib.Tensor2D(0, _lib.QFG_BFLOAT16, 8, 8), (ctypes.c_void_p * 1)()
+    calls = [
+        (lib.qfg_skinny_gemm_compute, lambda t: (None, None, 1, 8, t, 1, outs, 1, None)),
+        (lib.qfg_dequant_compute, lambda t: (None, t, outs, 1, None)),
+        (lib.qfg_lmhead_compute, lambda t: (None, None, 1, 8, t, 8, 0, None, None, None, None, None, None)),
+        (lib.qfg_shared_expert_down_compute, lambda t: (None, None, None, 1, 8, t, None, 8, None, None, 8, None, None)),
+    ]
+    for entry, args in calls:
+        for t in (w, ctypes.byref(w), (_lib.Tensor2D * 1)(w)):
+            assert entry(*args(t)) != _lib.QFG_OK  # no node
+        for t in (1 << 20, "weight", b"weight", outs):
+            with pytest.raises(ctypes.ArgumentError):
+                entry(*args(t))
