@@ -6,10 +6,10 @@
 //   * One cluster of up to eight CTAs per row; a CTA issues all the 16-byte loads of its share of the row at
 //     once (a scalar head and tail keep the vector body for odd vocabularies and unaligned rows), so a row
 //     costs one round trip to L2.
-//   * The value first, the index after: a thread takes the maximum of its elements two at a time with the packed
+//   * Long rows: the value first, the index after: a thread takes the maximum of its elements two at a time with the packed
 //     NaN-propagating maximum (half an instruction an element; carrying an index along cost five, and a dependent
 //     chain 48 elements long), warps meet in a redux and a shared-memory atomicMax, and only the threads that hold
-//     the CTA's maximum look through their registers for its first position.
+//     the CTA's maximum look through their registers for its first position.  Short rows carry the index along (kFewLoads).
 //   * Candidates travel as 64-bit keys whose unsigned maximum is the winner (argmax_key.cuh).
 //   * The CTAs of a cluster do not meet at a barrier at the end.  CTA 0 owns one mbarrier and one key slot
 //     per peer; a peer stores its key into CTA 0's shared memory, arrives on the barrier with release
@@ -35,6 +35,12 @@ constexpr int kMaxCluster = 8;
 // measured 0.5 us slower at one row
 template <typename T>
 constexpr int kInFlight = sizeof(T) == 4 ? 10 : 6;
+// Rows of which a thread holds no more loads than this carry the index along with the value instead: the barrier and the
+// second look that this saves cost more than the longer chain of compares (value first -> this: BF16 1 x 4099 3.17 -> 2.59
+// us, 1024 x 500 10.3 -> 5.2, 4096 x 4099 36.6 -> 19.6, FP32 1 x 32000 3.74 -> 3.14, 1 x 77777 4.45 -> 4.03).  Above it the
+// value first is the faster one (BF16 1 x 151936, five loads a thread: carried along 4.32, value first 3.78).
+template <typename T>
+constexpr int kFewLoads = sizeof(T) == 4 ? 5 : 2;
 constexpr int kPeerSpin = 1 << 24;  // bound of CTA 0's wait for its peers (iterations of about 30 ns)
 
 __device__ __forceinline__ float ToFloat(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -83,14 +89,28 @@ struct WordMax<float> {
   __device__ __forceinline__ static float Value(uint32_t w) { return __uint_as_float(w); }
 };
 
+// A thread's running best, with its index.  Candidates come in order of their index, so that a strict comparison keeps the
+// lowest index of equal values, and the first NaN stays.
+struct Best {
+  float v = 0.f;
+  long long i = -1;
+  __device__ __forceinline__ void Add(float c, long long idx) {
+    if (i < 0 || c > v || (c != c && v == v)) {
+      v = c;
+      i = idx;
+    }
+  }
+  __device__ __forceinline__ unsigned long long Key() const { return i < 0 ? 0ull : PackKey(v, i); }
+};
+
 // the value half of a key: equal for equal values, for -0 and +0 and for every NaN
 __device__ __forceinline__ uint32_t ValueKey(float v) { return static_cast<uint32_t>(PackKey(v, 0) >> 32); }
 
-template <typename T>
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict__ x, long long V,
                                                              long long* __restrict__ idx_out,
                                                              float* __restrict__ val_out) {
-  constexpr int kVecElems = 16 / sizeof(T), kLoads = kInFlight<T>;
+  constexpr int kVecElems = 16 / sizeof(T), kLoads = FEW ? kFewLoads<T> : kInFlight<T>;
   __shared__ unsigned long long s_best;               // this CTA's best key
   __shared__ uint32_t s_value;                        // its value half, before the index is known
   __shared__ unsigned long long s_slot[kMaxCluster];  // CTA 0: the peers' keys
@@ -133,67 +153,86 @@ __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict
   __syncthreads();
   if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
-  // the value first: the largest of every batch of this thread, and the first batch that holds the largest of all
-  uint32_t top = 0u;  // ValueKey; 0 is below every value's
-  long long top_v0 = v0;
-  for (;;) {
-    uint32_t m = kLow;
-#pragma unroll
-    for (int k = 0; k < kLoads; ++k) m = WordMax<T>::Max(m, WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w)));
-    const uint32_t key = v0 < vend ? ValueKey(WordMax<T>::Value(m)) : 0u;
-    if (key > top) {
-      top = key;
-      top_v0 = v0;
+  // head goes to the first CTA, tail to the last: these few elements come with their index
+  auto edge_key = [&] {
+    unsigned long long edge = 0ull;
+    if (c == 0) {
+      for (long long i = tid; i < head; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
     }
-    const long long next = v0 + static_cast<long long>(kThreads) * kLoads;
-    if (next >= vend) break;  // rows longer than one batch per thread take further round trips
-    v0 = next;
+    if (c == C - 1) {
+      for (long long i = head + nvec * kVecElems + tid; i < V; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
+    }
+    return edge;
+  };
+  if constexpr (FEW) {
+    Best best;
 #pragma unroll
     for (int k = 0; k < kLoads; ++k) {
       const long long v = v0 + static_cast<long long>(k) * kThreads;
-      q[k] = v < vend ? __ldg(xv + v) : lowest;
-    }
-  }
-  // head goes to the first CTA, tail to the last: these few elements come with their index
-  unsigned long long edge = 0ull;
-  if (c == 0) {
-    for (long long i = tid; i < head; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
-  }
-  if (c == C - 1) {
-    for (long long i = head + nvec * kVecElems + tid; i < V; i += kThreads) edge = max(edge, PackKey(ToFloat(xr[i]), i));
-  }
-  const uint32_t mine = max(top, static_cast<uint32_t>(edge >> 32));
-  const uint32_t wtop = __reduce_max_sync(0xffffffffu, mine);
-  if (lane == 0 && wtop != 0u) atomicMax(&s_value, wtop);
-  __syncthreads();
-
-  // then the index, by the threads that hold the CTA's largest value (one, but for ties): their first such element
-  const uint32_t cta_top = s_value;
-  if (mine == cta_top && cta_top != 0u) {
-    unsigned long long key = static_cast<uint32_t>(edge >> 32) == cta_top ? edge : 0ull;
-    if (top == cta_top) {
-      if (top_v0 != v0) {  // not the batch in hand
+      if (v < vend) {
+        const T* e = reinterpret_cast<const T*>(&q[k]);
 #pragma unroll
-        for (int k = 0; k < kLoads; ++k) {
-          const long long v = top_v0 + static_cast<long long>(k) * kThreads;
-          q[k] = v < vend ? __ldg(xv + v) : lowest;
-        }
+        for (int j = 0; j < kVecElems; ++j) best.Add(ToFloat(e[j]), head + v * kVecElems + j);
       }
+    }
+    const unsigned long long wkey = WarpMaxKey(max(edge_key(), best.Key()));
+    if (lane == 0 && wkey != 0ull) atomicMax(&s_best, wkey);
+  } else {
+    // the value first: the largest of every batch of this thread, and the first batch that holds the largest of all
+    uint32_t top = 0u;  // ValueKey; 0 is below every value's
+    long long top_v0 = v0;
+    for (;;) {
+      uint32_t m = kLow;
 #pragma unroll
-      for (int k = kLoads - 1; k >= 0; --k) {
-        const long long v = top_v0 + static_cast<long long>(k) * kThreads;
-        const uint32_t m = WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w));
-        if (v < vend && ValueKey(WordMax<T>::Value(m)) == cta_top) {
-          const T* e = reinterpret_cast<const T*>(&q[k]);
+      for (int k = 0; k < kLoads; ++k) m = WordMax<T>::Max(m, WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w)));
+      const uint32_t key = v0 < vend ? ValueKey(WordMax<T>::Value(m)) : 0u;
+      if (key > top) {
+        top = key;
+        top_v0 = v0;
+      }
+      const long long next = v0 + static_cast<long long>(kThreads) * kLoads;
+      if (next >= vend) break;  // rows longer than one batch per thread take further round trips
+      v0 = next;
 #pragma unroll
-          for (int j = 0; j < kVecElems; ++j) {
-            const float f = ToFloat(e[j]);
-            if (ValueKey(f) == cta_top) key = max(key, PackKey(f, head + v * kVecElems + j));  // the lower index is the larger key
+      for (int k = 0; k < kLoads; ++k) {
+        const long long v = v0 + static_cast<long long>(k) * kThreads;
+        q[k] = v < vend ? __ldg(xv + v) : lowest;
+      }
+    }
+    const unsigned long long edge = edge_key();
+    const uint32_t mine = max(top, static_cast<uint32_t>(edge >> 32));
+    const uint32_t wtop = __reduce_max_sync(0xffffffffu, mine);
+    if (lane == 0 && wtop != 0u) atomicMax(&s_value, wtop);
+    __syncthreads();
+
+    // then the index, by the threads that hold the CTA's largest value (one, but for ties): their first such element
+    const uint32_t cta_top = s_value;
+    if (mine == cta_top && cta_top != 0u) {
+      unsigned long long key = static_cast<uint32_t>(edge >> 32) == cta_top ? edge : 0ull;
+      if (top == cta_top) {
+        if (top_v0 != v0) {  // not the batch in hand
+#pragma unroll
+          for (int k = 0; k < kLoads; ++k) {
+            const long long v = top_v0 + static_cast<long long>(k) * kThreads;
+            q[k] = v < vend ? __ldg(xv + v) : lowest;
+          }
+        }
+#pragma unroll
+        for (int k = kLoads - 1; k >= 0; --k) {
+          const long long v = top_v0 + static_cast<long long>(k) * kThreads;
+          const uint32_t m = WordMax<T>::Max(WordMax<T>::Max(q[k].x, q[k].y), WordMax<T>::Max(q[k].z, q[k].w));
+          if (v < vend && ValueKey(WordMax<T>::Value(m)) == cta_top) {
+            const T* e = reinterpret_cast<const T*>(&q[k]);
+#pragma unroll
+            for (int j = 0; j < kVecElems; ++j) {
+              const float f = ToFloat(e[j]);
+              if (ValueKey(f) == cta_top) key = max(key, PackKey(f, head + v * kVecElems + j));  // the lower index is the larger key
+            }
           }
         }
       }
+      atomicMax(&s_best, key);
     }
-    atomicMax(&s_best, key);
   }
   __syncthreads();
 
@@ -259,7 +298,8 @@ cudaError_t LaunchT(const T* x, int64_t rows, int64_t V, int64_t* idx, float* va
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, ArgmaxRowsKernel<T>, x, static_cast<long long>(V),
+  const bool few = (vecs + cluster - 1) / cluster <= static_cast<long long>(kThreads) * kFewLoads<T>;
+  return cudaLaunchKernelEx(&cfg, few ? ArgmaxRowsKernel<T, true> : ArgmaxRowsKernel<T, false>, x, static_cast<long long>(V),
                             reinterpret_cast<long long*>(idx), val);
 }
 

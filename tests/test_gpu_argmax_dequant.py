@@ -222,3 +222,13 @@ def test_argmax_many_rows(cuda, dtype, rows, vocab):
             x[r].clamp_(max=0)                                # +0 and -0 tie
             x[r, p] = -0.0
     _check_argmax(x)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("vocab", [257, 4096, 8185, 8192, 8200, 20483, 65536, 65551, 81920, 81936])
+def test_argmax_rows_on_either_side_of_the_short_kernel(cuda, dtype, vocab):
+    """Up to two loads a thread (FP32: five) the index is carried along, past that the value comes first: one CTA a row and
+    eight, the same planted rows; more rows than the chip has CTAs for shrink the cluster, which moves the line."""
+    test_argmax_many_rows(cuda, dtype, 21, vocab)
+    if vocab >= 8192:
+        test_argmax_many_rows(cuda, dtype, 90, vocab)
