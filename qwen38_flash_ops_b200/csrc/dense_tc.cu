@@ -1272,7 +1272,7 @@ int QuerySlots(int cluster) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, DenseTcKernel<kBf16, false, false, true, 1>, &cfg) != cudaSuccess || n < 1) {
+  if (cudaOccupancyMaxActiveClusters(&n, DenseTcKernel<kBf16, false, false, true, 1>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     n = std::max(1, DeviceSmCount() * 8 / (10 * cluster));
   }
@@ -1351,7 +1351,8 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
       const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : !pieces ? 0.24 : pair ? 0.41 : 0.52);
       for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
         const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : setup->slots[split];
-        const int64_t waves = (tiles + slots - 1) / std::max<int64_t>(slots, 1);
+        if (slots < 1) break;  // the device holds no such cluster
+        const int64_t waves = (tiles + slots - 1) / slots;
         if (split > 1 && waves > 1) break;
         const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
         const double cost = work + 4 + 0.008 * bm + (split > 1 ? 1 + 0.01 * bm : 0);
@@ -1448,14 +1449,17 @@ bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m) {
 
 // Rows per tile and CTAs per cluster, by a model fitted to measured launches (us): a block of 64 k costs 0.10 + 0.0125
 // rows of swish_mul per CTA, or its MMAs and dequantisation where those take longer; around the blocks 6 + 0.02 bm +
-// 0.05 rows of the gate per CTA.  33 clusters of four, 74 of two are resident at once.
+// 0.05 rows of the gate per CTA.
 DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) {
+  const DeviceSetup* setup = nullptr;
+  if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SharedExpertDown: the kernels could not be set up on this device");
   DenseTcPlan best;
   double best_cost = 1e30;
   const int64_t n_tiles = (p.seg[0].n + kBn - 1) / kBn;
   const double blocks = (p.K + kBk - 1) / kBk;
   for (int c = 1; c <= 4; c *= 2) {
-    const int64_t slots = c == 4 ? sm_count * 9 / 40 : sm_count / c, groups = (n_tiles + c - 1) / c;
+    const int64_t slots = c == 1 ? sm_count : setup->slots[c], groups = (n_tiles + c - 1) / c;
+    if (slots < 1) break;
     const int unit = c == 4 ? 32 : 16;
     for (int bm = unit; bm <= 256; bm += unit) {
       const int64_t waves = (groups * ((m + bm - 1) / bm) + slots - 1) / slots;

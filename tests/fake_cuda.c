@@ -11,13 +11,14 @@
 
 static struct { const void* host; char name[256]; } g_fn[MAX];
 static struct { const void* fn; int device, value; } g_attr[MAX];
-static int n_fn, n_attr, g_device, g_setup_calls, g_refuse_setup, g_refuse_encode;
+static int n_fn, n_attr, g_device, g_setup_calls, g_refuse_setup, g_refuse_encode, g_resident = 132;
 static char g_log[1 << 20];
 static size_t g_len;
 
 API void fake_device(int d) { g_device = d; }
 API void fake_refuse_setup(int v) { g_refuse_setup = v; }
 API void fake_refuse_encode(int v) { g_refuse_encode = v; }
+API void fake_resident(int ctas) { g_resident = ctas; }  /* CTAs, one per SM, that clusters can have at once */
 API int fake_setup_calls(void) { return g_setup_calls; }
 API const char* fake_log(void) { return g_log; }
 API void fake_clear(void) { g_len = 0; g_log[0] = 0; }
@@ -54,11 +55,14 @@ API cudaError_t cudaFuncSetAttribute(const void* fn, enum cudaFuncAttribute a, i
   return cudaSuccess;
 }
 API cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes* a, const void* fn) { (void)fn; memset(a, 0, sizeof *a); a->sharedSizeBytes = 2048; return cudaSuccess; }
-API cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* fn, const cudaLaunchConfig_t* c) {
-  (void)fn;
+static int cluster_of(const cudaLaunchConfig_t* c) {
   int size = 1;
   for (unsigned i = 0; i < c->numAttrs; ++i) if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) size = c->attrs[i].val.clusterDim.x * c->attrs[i].val.clusterDim.y;
-  *n = 132 / size;
+  return size;
+}
+API cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* fn, const cudaLaunchConfig_t* c) {
+  (void)fn;
+  *n = g_resident / cluster_of(c);
   return setup();
 }
 API cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* fn, int t, size_t s) { (void)fn; (void)t; (void)s; *n = 1; return cudaSuccess; }
@@ -87,12 +91,12 @@ API cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 API const char* cudaGetErrorString(cudaError_t e) { static char b[32]; snprintf(b, sizeof b, "error %d", (int)e); return b; }
 
 /* launches */
-static cudaError_t launch(const void* fn, unsigned x, unsigned y, unsigned threads, size_t smem, int pdl) {
+static cudaError_t launch(const void* fn, unsigned x, unsigned y, unsigned threads, size_t smem, int cluster, int pdl) {
   char line[512];
   int limit = 48 * 1024;
   for (int i = 0; i < n_attr; ++i) if (g_attr[i].fn == fn && g_attr[i].device == g_device) limit = g_attr[i].value;
   if (smem > (size_t)limit) return cudaErrorInvalidValue;
-  snprintf(line, sizeof line, "launch %s device=%d grid=%u,%u threads=%u smem=%zu pdl=%d", name_of(fn), g_device, x, y, threads, smem, pdl);
+  snprintf(line, sizeof line, "launch %s device=%d grid=%u,%u threads=%u smem=%zu cluster=%d pdl=%d", name_of(fn), g_device, x, y, threads, smem, cluster, pdl);
   note(line);
   return cudaSuccess;
 }
@@ -100,14 +104,14 @@ API cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn,
   int pdl = 0;
   (void)args;
   for (unsigned i = 0; i < c->numAttrs; ++i) if (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) pdl = c->attrs[i].val.programmaticStreamSerializationAllowed;
-  return launch(fn, c->gridDim.x, c->gridDim.y, c->blockDim.x, c->dynamicSmemBytes, pdl);
+  return launch(fn, c->gridDim.x, c->gridDim.y, c->blockDim.x, c->dynamicSmemBytes, cluster_of(c), pdl);
 }
 static dim3 g_grid, g_block;
 static size_t g_smem;
 static cudaStream_t g_stream;
 API unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t s, cudaStream_t t) { g_grid = g; g_block = b; g_smem = s; g_stream = t; return 0; }
 API cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void* t) { *g = g_grid; *b = g_block; *s = g_smem; *(cudaStream_t*)t = g_stream; return cudaSuccess; }
-API cudaError_t cudaLaunchKernel(const void* fn, dim3 g, dim3 b, void** args, size_t s, cudaStream_t t) { (void)args; (void)t; return launch(fn, g.x, g.y, b.x, s, 0); }
+API cudaError_t cudaLaunchKernel(const void* fn, dim3 g, dim3 b, void** args, size_t s, cudaStream_t t) { (void)args; (void)t; return launch(fn, g.x, g.y, b.x, s, 1, 0); }
 
 /* cuBLAS */
 API int cublasCreate_v2(void** h) { static int one; *h = &one; return 0; }

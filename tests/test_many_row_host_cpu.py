@@ -159,3 +159,15 @@ def test_what_the_many_row_kernels_cannot_take_goes_the_general_way(fake, dtype)
     assert gemm[0] == 0 and _kernels(gemm[2]) == library + ["cublas"], gemm
     assert rows[0] == 0 and _kernels(rows[2]) == library + ["cublas"], rows
     assert shared[0] == 0 and _kernels(shared[2]) == ["SkinnyGemm"] * 5, shared
+
+
+@pytest.mark.parametrize("resident,clusters", [(132, True), (2, False), (1, False)])
+def test_launch_shapes_use_the_clusters_that_the_device_holds(fake, resident, clusters):
+    """Both planners ask the device: where it holds one or none at a time, neither splits K nor shares rows over clusters."""
+    out = fake(f"""
+        fake.fake_resident({resident})
+        print(json.dumps([run_gemm(gemm([1], [256]), FP8, 40, 5120, [[256]]), run_shared(shared(), FP8, 777, 640, 2560)]))
+        """)
+    for code, message, log in out:
+        assert code == 0 and len(log) == 1, message
+        assert (" cluster=1 " not in log[0]) == clusters, log
