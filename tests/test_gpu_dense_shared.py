@@ -14,7 +14,7 @@ import _util as U
 pytestmark = pytest.mark.gpu
 
 
-def _run(mode, M, K, N, gk, plan, seed, gx_offset=0, g_offset=0):
+def _run(mode, M, K, N, gk, plan, seed, gx_offset=0, g_offset=0, route=True):
     rng = np.random.default_rng(seed)
     bf = lambda a: P.f32_to_bf16_bits(a.astype(np.float32))
     arr, s = U.make_weight(rng, mode, K, N, mode != 0)
@@ -30,9 +30,16 @@ def _run(mode, M, K, N, gk, plan, seed, gx_offset=0, g_offset=0):
         return buf[offset:].view(t.shape)
 
     op = SharedExpertDown(w_scale=s if mode != 0 else None)
-    if plan:
-        op.set_option("dense_plan", plan)
-    out = op(dev(g, g_offset), dev(u), U.dev_weight(arr, mode), dev(gx, gx_offset), dev(gw), dev(routed))
+    args = dev(g, g_offset), dev(u), U.dev_weight(arr, mode), dev(gx, gx_offset), dev(gw), dev(routed)
+    # only in the many-row kernel is a launch shape that does not exist an error
+    op.set_option("dense_plan", "8,1")
+    if route:
+        with pytest.raises(QfgError, match="bad launch shape"):
+            op(*args)
+    else:
+        op(*args)
+    op.set_option("dense_plan", plan or "0")
+    out = op(*args)
     torch.cuda.synchronize()
     y, _, _, shared = O.shared_expert_down(g, u, mode, arr, N, gx, gw, routed, s if mode != 0 else None)
     got, gf, yf = bits(out), O.bf16_to_f32(bits(out)), O.bf16_to_f32(y)
@@ -52,9 +59,10 @@ def test_tile_and_cluster_edges(cuda, mode, plan):
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_layouts_on_either_side_of_the_route(cuda, mode):
-    _run(mode, 40, 256, 128, 64, "", 7, gx_offset=1)   # gate read element by element
-    _run(mode, 40, 256, 128, 64, "", 7, g_offset=2)    # rows of g the kernel cannot read: streaming passes
-    _run(mode, 40, 260, 192, 64, "", 7)                # K off 16 bytes, N an odd number of 64
+    _run(mode, 40, 256, 128, 64, "", 7, gx_offset=1)               # gate read element by element
+    _run(mode, 40, 256, 128, 64, "", 7, g_offset=2, route=False)    # rows of g the kernel cannot read: streaming passes
+    _run(mode, 40, 260, 192, 64, "", 7, route=False)                # K off 16 bytes, N an odd number of 64
+    _run(mode, 40, 256, 256, 64, "", 7)                             # NVFP4 rows on 16 bytes (at 128 columns they are not)
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
@@ -78,6 +86,29 @@ def test_repeated_calls_agree(cuda, mode, plan):
     assert torch.isfinite(first).all()
     for _ in range(40):
         assert torch.equal(op(*args), first)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_swish_times_u_is_the_streaming_kernels(cuda, seed):
+    """Every g beside random u of every size: bf16(bf16(g * bf16(sigmoid(g))) * u), through an identity weight.  A row holds 64
+    values, so g and u stay below 2^60 and sums are one term and zeros.  Products below the normal range may be rounded twice
+    (once to FP32's subnormals), so they are compared to one unit in their last place."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    g = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16)
+    g = torch.where(torch.isfinite(g) & (g.abs() < 2.0 ** 60), g, torch.zeros_like(g))[torch.randperm(65536, generator=gen, device="cuda")].view(1024, 64)
+    u = torch.randint(0, 65536, (1024, 64), generator=gen, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    u = torch.where(torch.isfinite(u) & (u.abs() < 2.0 ** 60), u, torch.ones_like(u))
+    w = torch.zeros(64, 128, device="cuda")
+    w[torch.arange(64), torch.arange(64)] = 1
+    gx, gw = torch.ones(1024, 8, device="cuda").bfloat16(), torch.full((8, 1), 10.0, device="cuda").bfloat16()
+    routed = torch.zeros(1024, 128, device="cuda").bfloat16()
+    many, few = SharedExpertDown(), SharedExpertDown()
+    few.set_option("dense_rows", 0)
+    a, b = (op(g, u, w.bfloat16(), gx, gw, routed) for op in (many, few))
+    normal = b.float().abs() >= 2.0 ** -126
+    assert torch.equal(a[normal], b[normal])
+    assert ((a.double() - b.double()).abs() <= 2.0 ** -133).logical_or(normal).all()
+    assert normal[:, :64].sum() > 30000 and torch.count_nonzero(a[:, 64:]) == 0
 
 
 def test_swish_of_every_bf16_value_is_the_streaming_kernels(cuda):

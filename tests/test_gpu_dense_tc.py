@@ -10,7 +10,7 @@ import torch
 from conftest import ROOT, bits, to_dev
 from oracle import cpu as C
 from oracle import oracle as O
-from qwen38_flash_ops_b200 import QfgError, SkinnyGemm
+from qwen38_flash_ops_b200 import DequantWeightBf16, QfgError, SkinnyGemm
 from qwen38_flash_ops_b200 import packing as P
 
 import _util as U
@@ -28,21 +28,48 @@ CASES = [
 PLANS = ["", "16,1,0", "48,1,0,1", "48,1,0,2", "256,1,0", "64,2,0,1", "48,3,0,2", "32,8,0", "64,1,1,1", "64,1,1,2", "112,1,1", "256,1,1"]
 
 
-def _check(mode, M, K, seg_widths, plan, seed, x_offset=0):
+def _takes_the_kernel(op, *args, **kw):
+    """Whether a call goes to the many-row kernel: only there is a launch shape that does not exist an error."""
+    op.set_option("dense_plan", "8,1")
+    try:
+        op(*args, **kw)
+    except QfgError as e:
+        assert "bad launch shape" in str(e)
+        return True
+    finally:
+        op.set_option("dense_plan", "0")
+    return False
+
+
+def _check(mode, M, K, seg_widths, plan, seed, x_offset=0, out_offset=0, scale_columns=None, route=True):
     rng = np.random.default_rng(seed)
     seg_outs, widths, ns = [len(w) for w in seg_widths], [w for ws in seg_widths for w in ws], [sum(w) for w in seg_widths]
     x = P.synth_x(rng, M, K)
     stored, scales = zip(*[U.make_weight(rng, mode, K, n, True) for n in ns])
-    op = SkinnyGemm(seg_outs, widths, w_scale=np.concatenate(scales) if mode != 0 else None)
-    if plan:
-        op.set_option("dense_plan", plan)
+    w_scale = np.concatenate(scales) if mode != 0 else None
+    if scale_columns is not None and mode != 0:  # a w_scale that ends early: the weights it does not cover have none
+        w_scale = w_scale[:scale_columns]
+        ends = np.cumsum(ns)
+        scales = [s if end <= scale_columns else None for s, end in zip(scales, ends)]
+    op = SkinnyGemm(seg_outs, widths, w_scale=w_scale)
     xd = to_dev(x, "bf16")
     if x_offset:
         buf = torch.empty(M * K + x_offset, dtype=torch.bfloat16, device="cuda")
         buf[x_offset:] = xd.reshape(-1)
         xd = buf[x_offset:].view(M, K)
-    outs = op(xd, *[U.dev_weight(a, mode) for a in stored])
+    wd = [U.dev_weight(a, mode) for a in stored]
+    outs = None
+    if out_offset:  # outputs inside larger buffers, the elements around them watched
+        buffers = [torch.full((M * w + 16,), 77.0, device="cuda", dtype=torch.bfloat16) for w in widths]
+        outs = [b[out_offset:out_offset + M * w].view(M, w) for b, w in zip(buffers, widths)]
+    assert _takes_the_kernel(op, xd, *wd, out=outs) == route
+    if plan:
+        op.set_option("dense_plan", plan)
+    outs = op(xd, *wd, out=outs)
     torch.cuda.synchronize()
+    if out_offset:
+        for b, w in zip(buffers, widths):
+            assert (b[:out_offset] == 77).all() and (b[out_offset + M * w:] == 77).all()
     o = 0
     for i, n in enumerate(ns):
         got = np.concatenate([bits(outs[o + j]).reshape(M, -1) for j in range(seg_outs[i])], axis=1)
@@ -61,13 +88,35 @@ def test_tile_edges(cuda, mode, plan):
         _check(mode, M, K, seg_widths, plan, 1000 * mode + i)
 
 
-@pytest.mark.parametrize("mode,K,widths,x_offset", [
-    (0, 64, [[72]], 0), (1, 64, [[144]], 0),          # the last 16-byte pieces of a row are the tile's last
-    (1, 64, [[136]], 0), (2, 64, [[192]], 0),          # rows the copies cannot address
-    (0, 68, [[128]], 0), (0, 64, [[128]], 2), (2, 128, [[256]], 4),  # K or x off 16 bytes
+@pytest.mark.parametrize("mode,K,widths,x_offset,route", [
+    (0, 64, [[72]], 0, True), (1, 64, [[144]], 0, True),          # the last 16-byte pieces of a row are the tile's last
+    (2, 64, [[128]], 0, True), (2, 64, [[256]], 0, True),          # NVFP4 rows off 16 bytes and on them
+    (1, 64, [[136]], 0, False), (2, 64, [[192]], 0, False),        # rows the copies cannot address
+    (0, 68, [[128]], 0, False), (0, 64, [[128]], 2, False), (2, 128, [[256]], 4, False),  # K or x off 16 bytes
 ])
-def test_layouts_on_either_side_of_the_route(cuda, mode, K, widths, x_offset):
-    _check(mode, 40, K, widths, "", 77, x_offset)
+def test_layouts_on_either_side_of_the_route(cuda, mode, K, widths, x_offset, route):
+    _check(mode, 40, K, widths, "", 77, x_offset, route=route)
+
+
+# Launch shapes that give a CTA, or a pair, four tiles and more: both accumulator sets come round again, and stages, rings and
+# the dequantising groups go on across tiles, with an odd number of k steps (17 blocks of 64, 9 stages' worth of two).
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("M,plan", [(300, "16,1,0,1"), (300, "16,1,0,2"), (1100, "64,1,1,1"), (1100, "64,1,1,2")])
+@pytest.mark.parametrize("K,last", [(1032, 1920), (1032, 2048), (64, 1920)])
+def test_many_tiles_a_cta(cuda, mode, M, plan, K, last):
+    bm, _, pair, _ = map(int, plan.split(","))
+    seg_widths = [[1664, 640], [last]]  # NVFP4: at 1920 columns the rows are off 16 bytes
+    tiles = sum(-(-sum(w) // (256 if pair else 128)) for w in seg_widths) * -(-M // bm)
+    assert tiles > 4 * (74 if pair else 148)
+    _check(mode, M, K, seg_widths, plan, 5000 + mode)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["", "64,1,0", "48,3,0", "64,1,1"])
+def test_outputs_off_16_bytes_and_short_scales(cuda, mode, plan):
+    """Both epilogues' two-byte stores, and weights beyond the end of w_scale."""
+    for out_offset in (1, 4):
+        _check(mode, 100, 328, [[248, 136], [128 if mode == 2 else 144]], plan, 40 + out_offset, out_offset=out_offset, scale_columns=384)
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
@@ -89,6 +138,11 @@ def test_repeated_calls_agree(cuda, mode, plan):
     op.set_option("dense_plan", plan)
     first = op(x, w)[0].clone()
     assert torch.isfinite(first).all()
+    # a fault that repeats itself: against the product of the same BF16 weights by another kernel, FP32 sums in another order
+    wide = DequantWeightBf16(N)(w)[0] if mode != 0 else w
+    want = x.float() @ wide.float()
+    bound = 2.0 ** -8 * want.abs() + 2 * K * 2.0 ** -24 * (x.float().abs() @ wide.float().abs())  # one BF16 rounding, the sums' on both sides
+    assert torch.all((first.float() - want).abs() <= bound)
     for _ in range(40):
         assert torch.equal(op(x, w)[0], first)
 

@@ -371,9 +371,9 @@ def test_register_streaming_kernel(cuda, mode, plan):
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_many_rows_take_the_dense_branch(cuda, mode):
-    """Prefill-shaped calls (more rows than the `dense_rows` option; by default 8 / 8 / 16 for BF16 / FP8 / NVFP4) dequantise the weights to
-    BF16 with w_scale folded in and run a library GEMM, as the reference does for M > 8 (fused_gemm.cu:365-428).
-    The accumulation order of that GEMM is not pinned, so the check is the tolerance against the exact sum over
+    """Prefill-shaped calls (more rows than the `dense_rows` option; by default 8 / 8 / 16 for BF16 / FP8 / NVFP4) compute with the weights
+    rounded to BF16, w_scale folded in, as the reference does for M > 8 (fused_gemm.cu:365-428), in one kernel.
+    The order of its sums is not pinned, so the check is the tolerance against the exact sum over
     the BF16-rounded weights, and agreement with the streaming passes within the rounding of those weights."""
     rng = np.random.default_rng(900 + mode)
     M, K = 80, 1024
@@ -413,8 +413,8 @@ def test_many_rows_take_the_dense_branch(cuda, mode):
 
 
 def test_dense_branch_tiles_wide_outputs_and_skips_odd_widths(cuda):
-    """An output wider than one dequantisation tile (16384 columns) is produced tile by tile; widths that are
-    not multiples of eight stay on the streaming kernels at any row count."""
+    """An output of 160 column tiles; widths that are not multiples of eight stay on the streaming kernels at any row
+    count.  (The library branch and its tiles of 16384 columns: test_library_branch_*.)"""
     rng = np.random.default_rng(77)
     M, K, n = 40, 128, 16384 + 4096
     x = P.synth_x(rng, M, K)
@@ -434,6 +434,60 @@ def test_dense_branch_tiles_wide_outputs_and_skips_odd_widths(cuda):
     one = op2(to_dev(x[17:18], "bf16"), U.dev_weight(w2, 0))
     torch.cuda.synchronize()
     assert np.array_equal(bits(one[0]).reshape(-1), bits(out2[0]).reshape(M, 100)[17])
+
+
+def _library_call(rng, mode, M, K, seg_widths, scaled, x_offset=0):
+    """A call that the many-row kernel does not take, against the oracle."""
+    ns, widths = [sum(ws) for ws in seg_widths], [w for ws in seg_widths for w in ws]
+    x = P.synth_x(rng, M, K)
+    stored, scales = zip(*[U.make_weight(rng, mode, K, n, scaled) for n in ns])
+    w_scale = np.concatenate(scales) if scaled and mode != 0 else None
+    op = SkinnyGemm([len(w) for w in seg_widths], widths, w_scale=w_scale)
+    op.set_option("dense_plan", "8,1")  # a launch shape that the many-row kernel refuses, to see that it is not asked
+    buf = torch.empty(M * K + x_offset, dtype=torch.bfloat16, device="cuda")
+    buf[x_offset:] = to_dev(x, "bf16").reshape(-1)
+    outs = op(buf[x_offset:].view(M, K), *[U.dev_weight(a, mode) for a in stored])
+    torch.cuda.synchronize()
+    o = 0
+    for i, (n, ws) in enumerate(zip(ns, seg_widths)):
+        got = np.concatenate([bits(out).reshape(M, -1) for out in outs[o:o + len(ws)]], axis=1)
+        o += len(ws)
+        w_bf16 = O.dequant_weight_bf16(mode, stored[i], n, 0, scales[i] if w_scale is not None else None)
+        _, sums, mags = C.skinny_gemm(0, x, w_bf16, n, None)
+        ok = O.gemm_within_tolerance(got, sums, mags, K)
+        assert ok.all(), f"weight {i}: {np.count_nonzero(~ok)} of {ok.size} outputs outside tolerance"
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("mode,seg_widths,K,x_offset", [
+    (1, [[16384 + 8]], 64, 0),              # FP8 rows off 16 bytes, a second tile of eight columns
+    (1, [[264], [16384, 16392]], 40, 0),    # outputs of one weight: column offsets of weight, scale and tile
+    (2, [[16384 + 192]], 64, 0),            # NVFP4, an odd number of 64 columns
+    (2, [[16512, 64], [192]], 72, 0),
+    (0, [[16384 + 40, 24]], 68, 0),         # BF16 where it lies: no dequantisation
+    (2, [[16384 + 128]], 64, 2),            # x off 16 bytes
+])
+def test_library_branch_tiles_wide_outputs(cuda, mode, seg_widths, K, x_offset, scaled):
+    _library_call(np.random.default_rng(K + mode), mode, 40, K, seg_widths, scaled, x_offset)
+
+
+def test_library_branch_buffer_grows_between_calls(cuda):
+    """The dequantisation buffer of a stream is replaced by a larger one while earlier calls may still read the old one."""
+    rng = np.random.default_rng(12)
+    small, large = U.make_weight(rng, 2, 128, 192)[0], U.make_weight(rng, 2, 512, 6 * 192)[0]
+    xs, xl = to_dev(P.synth_x(rng, 24, 128), "bf16"), to_dev(P.synth_x(rng, 24, 512), "bf16")
+    ws, wl = U.dev_weight(small, 2), U.dev_weight(large, 2)
+    a, b = SkinnyGemm([1], [192]), SkinnyGemm([1], [6 * 192])
+    want_a, want_b = a(xs, ws)[0].clone(), b(xl, wl)[0].clone()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):  # a buffer of its own, empty at first
+        got = [a(xs, ws)[0] for _ in range(20)] + [b(xl, wl)[0]] + [a(xs, ws)[0]]
+        torch.cuda.current_stream().synchronize()
+    assert all(torch.equal(g, want_a) for g in got[:20] + got[21:]) and torch.equal(got[20], want_b)
+    for op, x, w, y in ((a, xs, ws, want_a), (b, xl, wl, want_b)):
+        op.set_option("dense_rows", 0)
+        ref = op(x, w)[0].float()
+        assert torch.allclose(y.float(), ref, rtol=2.0 ** -7, atol=2.0 ** -7 * ref.abs().max().item())
 
 
 def test_trigger_attribute_and_its_environment_override(cuda, monkeypatch):
