@@ -1324,12 +1324,14 @@ cudaError_t ConfigureDenseKernels() {
   return SetUpDevice(&setup);
 }
 
-// Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200,
-// K = 5120; us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair
-// 0.13 + 0.00098 bm (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.52 and 0.41 where the
-// rows are loaded in 8-byte pieces); around the blocks 4 + 0.008 bm, and 1 + 0.01 bm more where ranks add up.  More row
-// tiles than needed are tried because they can fill the last wave better (509 rows, N = 10240: 3 x 192 56 us,
-// 2 x 256 61 us).
+// Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200;
+// us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair 0.13 + 0.00098 bm
+// (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.52 and 0.41 where the rows are loaded in
+// 8-byte pieces); around the blocks 4 + 0.008 bm, 0.9 more for a pair, and 1.8 + 0.01 bm more where ranks add up: with
+// less for those two, as K = 5120 alone had suggested, short K was split and paired where that loses (BF16 146 x 400 x
+// 3728 6.3 us in pairs of 64, 5.5 in single tiles of 48; over 150 random calls the shape chosen took 3.7 % longer than the
+// best one, and takes 1.8).  More row tiles than needed are tried because they can fill the last wave better (509 rows,
+// N = 10240: 3 x 192 56 us, 2 x 256 61 us).
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count) {
   const DeviceSetup* setup = nullptr;
   if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SkinnyGemm(dense): the kernels could not be set up on this device");
@@ -1355,7 +1357,7 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
         const int64_t waves = (tiles + slots - 1) / slots;
         if (split > 1 && waves > 1) break;
         const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
-        const double cost = work + 4 + 0.008 * bm + (split > 1 ? 1 + 0.01 * bm : 0);
+        const double cost = work + 4 + 0.008 * bm + (split > 1 ? 1.8 + 0.01 * bm : pair ? 0.9 : 0);
         if (cost < best_cost) {
           best_cost = cost;
           best.bm = bm;
