@@ -9,7 +9,7 @@
 //   0-3   epilogue: accumulators -> BF16 -> the output that owns the column
 //   4     TMA producer: the x tile of every stage, and the weight tile where the weights are BF16
 //   5     tensor memory allocation; one lane issues the MMAs
-//   6-7   FP8 / NVFP4: copy the stored weights into a ring of their own (~60 KB in flight per SM)
+//   6     FP8 / NVFP4: copies the stored weights into a ring of their own (50-60 KB in flight per SM); 7 idles
 //   8-23  FP8 / NVFP4: sixteen warps in two groups that take the stages in turn; a warp turns eight weight rows of a
 //         stage into BF16, w_scale folded in before the one rounding
 // Rows of x are what the dequantisation is shared by: at bm = 256 a stage takes the tensor core 512 cycles, at
@@ -58,22 +58,29 @@ constexpr int kABytes = kBn * kBk * 2;
 constexpr int kMaxStages = 8;
 constexpr int kDqWarps = 8;        // warps that fill one stage, eight weight rows each
 constexpr int kDqGroups = 2;       // groups of them, taking the stages in turn
-constexpr int kLoadWarps = 2;     // warps that copy the stored rows into the raw ring
+constexpr int kLoadWarps = 2;     // the first copies the stored rows into the raw ring, the second keeps the others in groups of four
 constexpr int kFirstDqWarp = 6 + kLoadWarps;
 constexpr int kMaxRaw = 12;
 constexpr int kSpin = 1 << 20;
 
+// Inside this file NVFP4 has two modes.  Where N is an odd multiple of 128 the stored rows are an odd multiple of eight bytes
+// long, and every second one starts off the 16 bytes that a tensor copy has to start on.  Two rows are then one row of the
+// tensor map, and an odd row is copied from the 16-byte boundary before it.
+constexpr int kNvfp4Odd = 3;
+template <int MODE>
+constexpr bool kFp4 = MODE == kNvfp4 || MODE == kNvfp4Odd;
+constexpr int kOddPitch = 80;  // nibble bytes copied of an odd row: 8 before the 64 of the tile, and 16-byte steps
+
 template <int MODE, int KS>
 struct RawRing {  // ring of stored, undequantised stages
   static constexpr int kRows = kBk * KS;
-  static constexpr int kSlot = kRows * (MODE == kNvfp4 ? 64 + 16 : 128);
+  static constexpr int kScales = kRows * (MODE == kNvfp4Odd ? kOddPitch : 64);  // NVFP4: where a slot's scales begin
+  static constexpr int kSlot = kFp4<MODE> ? kScales + kRows * 16 : kRows * 128;
   // even: a slot then always serves the same group of dequantising warps, which has seen its previous phase complete
-  static constexpr int kDepth = KS == 1 ? (MODE == kNvfp4 ? 10 : 6) : (MODE == kNvfp4 ? 6 : 4);
+  static constexpr int kDepth = MODE == kNvfp4 ? (KS == 1 ? 10 : 6) : MODE == kNvfp4Odd ? (KS == 1 ? 8 : 4) : (KS == 1 ? 6 : 4);
   static constexpr int kBytes = MODE == kBf16 ? 0 : kSlot * kDepth;
+  static_assert(kDepth <= kMaxRaw && kDepth % kDqGroups == 0 && kSlot % 256 == 0, "raw ring");
 };
-static_assert(RawRing<kNvfp4, 1>::kDepth <= kMaxRaw && RawRing<kNvfp4, 1>::kDepth % kDqGroups == 0 && RawRing<kFp8, 1>::kDepth % kDqGroups == 0 &&
-                  RawRing<kNvfp4, 2>::kDepth % kDqGroups == 0 && RawRing<kFp8, 2>::kDepth % kDqGroups == 0,
-              "raw ring");
 constexpr int kOutPitch = 80;                     // bytes of a row of 32 output columns in an epilogue warp's buffer: rows 16 bytes apart in the banks
 constexpr int kOutBytes = 4 * 32 * kOutPitch;     // four warps, 32 rows of x each
 
@@ -91,7 +98,7 @@ struct DenseParams {
   DenseSeg seg[kMaxSeg];
   uint16_t* out[kMaxOut];
   int col_begin[kMaxOut], width[kMaxOut];
-  int nseg, M, K, ksteps, bm, m_tiles, tiles, stages, raw_tensor;
+  int nseg, M, K, ksteps, bm, m_tiles, tiles, stages;
   uint32_t out_vec;  // outputs whose rows can be written 16 bytes at a time
 };
 
@@ -206,9 +213,6 @@ __device__ __forceinline__ unsigned long long SmemDesc(uint32_t addr, uint32_t l
   return static_cast<unsigned long long>((addr >> 4) & 0x3FFF) | (static_cast<unsigned long long>(lbo >> 4) << 16) |
          (static_cast<unsigned long long>(sbo >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void CpAsync8(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void Lds128(uint32_t a, uint32_t (&v)[4]) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
 }
@@ -271,56 +275,12 @@ __device__ __forceinline__ TileAt LocateDense(const DenseParams& p, int tile, in
   return t;
 }
 
-// ------------------------------------------------------------------------------ loading warps
-// Stored rows -> the raw ring.  A slot holds one stage: NVFP4 [rows][64 nibble bytes], then [rows][the 16 bytes that
-// hold the row's 8 block scales, at their offset in an aligned 16]; FP8 [rows][128 bytes].  One lane's tensor
-// copies where the rows are 16-byte aligned; the rest of the NVFP4 weights (N an odd multiple of 128) in 8-byte pieces
-// by all lanes of both warps, which is slower (18 copy instructions a stage) but knows no alignment beyond 8.
-template <bool PAIR, int KS>
-__device__ __forceinline__ void LoadNvfp4Pieces(const DenseParams& p, Ctl& ctl, int lane64, int rank, int kbeg, int kcount, int first_tile,
-                                                int tile_step, uint32_t ring) {
-  using R = RawRing<kNvfp4, KS>;
-  const uint32_t full0 = Smem(&ctl.raw_full[0]), empty0 = Smem(&ctl.raw_empty[0]);
-  int slot = 0;
-  uint32_t parity = 1;
-  bool first_round = true;
-  const int c = lane64 & 7, r0 = lane64 >> 3;  // nibble piece c of rows r0 + 8 j; the scales of row lane64
-  for (int tile = first_tile; tile < p.tiles; tile += tile_step) {
-    const TileAt t = LocateDense<PAIR>(p, tile, rank);
-    const DenseSeg& sg = p.seg[t.seg];
-    const bool cols = t.n0 < sg.n;
-    const int at = sg.n / 2 + t.n0 / 16;
-    const uint8_t* nib = sg.w + (static_cast<long long>(kbeg) * R::kRows + r0) * sg.pitch + t.n0 / 2 + 8 * c;
-    const uint8_t* scl = sg.w + (static_cast<long long>(kbeg) * R::kRows + lane64) * sg.pitch + at;
-    const uint32_t nib_dst = ring + static_cast<uint32_t>(r0 * 64 + c * 8);
-    const uint32_t scl_dst = ring + static_cast<uint32_t>(R::kRows * 64 + lane64 * 16 + (at & 8));
-#pragma unroll 1
-    for (int k = 0; k < kcount; ++k) {
-      if (!first_round && !BarWait(empty0 + slot * 8, parity, ctl)) return;
-      const uint32_t base = static_cast<uint32_t>(slot) * R::kSlot;
-      const int rows = cols ? p.K - (kbeg + k) * R::kRows : 0;  // rows past K read as zero
-#pragma unroll
-      for (int j = 0; j < 8 * KS; ++j) {
-        const bool ok = r0 + 8 * j < rows;
-        CpAsync8(nib_dst + base + j * 512, ok ? nib + 8 * j * sg.pitch : sg.w, ok ? 8 : 0);
-      }
-#pragma unroll
-      for (int j = 0; j < KS; ++j) {
-        const bool ok = lane64 + 64 * j < rows;
-        CpAsync8(scl_dst + base + j * 1024, ok ? scl + 64 * j * sg.pitch : sg.w, ok ? 8 : 0);
-      }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full0 + slot * 8) : "memory");
-      nib += R::kRows * sg.pitch;
-      scl += R::kRows * sg.pitch;
-      if (++slot == R::kDepth) {
-        slot = 0;
-        parity ^= 1u;
-        first_round = false;
-      }
-    }
-  }
-}
-
+// ------------------------------------------------------------------------------ loading warp
+// Stored rows -> the raw ring, by one lane's tensor copies.  A slot holds one stage: FP8 [rows][128 bytes]; NVFP4 [rows][64
+// nibble bytes], then [rows][the 16 bytes that hold the row's 8 block scales, at their offset in an aligned 16]; NVFP4 with
+// odd rows [even rows][80], [odd rows][80], [even rows][16], [odd rows][16], the 80 of a row beginning up to 8 bytes before
+// the tile.  (Such weights used to come in 8-byte cp.async pieces by two warps, 18 instructions a stage: 1024 rows of 5120 x
+// 5248 81.2 us, now 48.7, and 54.8 by dequantisation and library GEMM; 33 rows 20.0, 13.2 and 24.5.)
 template <int MODE, bool PAIR, int KS>
 __device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int rank, int kbeg, int kcount, int first_tile, int tile_step, uint32_t ring) {
   using R = RawRing<MODE, KS>;
@@ -331,7 +291,7 @@ __device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int r
   for (int tile = first_tile; tile < p.tiles; tile += tile_step) {
     const TileAt t = LocateDense<PAIR>(p, tile, rank);
     const DenseSeg& sg = p.seg[t.seg];
-    const int scl = (sg.n / 2 + t.n0 / 16) & ~15;
+    const int nib = t.n0 / 2, scl = sg.n / 2 + t.n0 / 16, odd = static_cast<int>(sg.pitch);
 #pragma unroll 1
     for (int k = 0; k < kcount; ++k) {
       if (!first_round && !BarWait(empty0 + slot * 8, parity, ctl)) return;
@@ -339,8 +299,14 @@ __device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int r
       if (ElectOne()) {
         BarExpect(bar, R::kSlot);
         if constexpr (MODE == kNvfp4) {
-          TmaLoad<false>(dst, &p.wmap[t.seg], t.n0 / 2, (kbeg + k) * R::kRows, bar);
-          TmaLoad<false>(dst + R::kRows * 64, &p.smap[t.seg], scl, (kbeg + k) * R::kRows, bar);
+          TmaLoad<false>(dst, &p.wmap[t.seg], nib, (kbeg + k) * R::kRows, bar);
+          TmaLoad<false>(dst + R::kScales, &p.smap[t.seg], scl & ~15, (kbeg + k) * R::kRows, bar);
+        } else if constexpr (MODE == kNvfp4Odd) {
+          const int pair = (kbeg + k) * (R::kRows / 2);
+          TmaLoad<false>(dst, &p.wmap[t.seg], nib, pair, bar);
+          TmaLoad<false>(dst + R::kScales / 2, &p.wmap[t.seg], (nib + odd) & ~15, pair, bar);
+          TmaLoad<false>(dst + R::kScales, &p.smap[t.seg], scl & ~15, pair, bar);
+          TmaLoad<false>(dst + R::kScales + R::kRows * 8, &p.smap[t.seg], (scl + odd) & ~15, pair, bar);
         } else {
           TmaLoad<false>(dst, &p.wmap[t.seg], t.n0, (kbeg + k) * R::kRows, bar);
         }
@@ -373,7 +339,13 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
   const int r0 = 2 * jj + par;
   const uint32_t st0 = stage0 + static_cast<uint32_t>(a * (kABytes / 2) + warp * 1024 + r0 * 128 + (((2 * q) ^ r0) * 16));
   const uint32_t row0 = static_cast<uint32_t>(warp * 8 + r0);
-  const uint32_t rd_w = ring + row0 * (MODE == kNvfp4 ? 64 : 128) + static_cast<uint32_t>(g * (MODE == kNvfp4 ? 8 : 16));
+  // where they come from: bytes of a row, of its scales, and from the first of the lane's two rows (r0, r0 + 4) to the second;
+  // the parity of its rows is par
+  constexpr bool kOdd = MODE == kNvfp4Odd;
+  constexpr uint32_t kRow = kOdd ? kOddPitch / 2 : kFp4<MODE> ? 64 : 128, kScaleRow = kOdd ? 8 : 16;
+  const uint32_t first_row = kOdd ? row0 & ~1u : row0;
+  const uint32_t rd_row = ring + first_row * kRow + static_cast<uint32_t>(g * (kFp4<MODE> ? 8 : 16)) + (kOdd ? static_cast<uint32_t>(par * (R::kScales / 2)) : 0u);
+  const uint32_t rd_scale_row = ring + R::kScales + first_row * kScaleRow + static_cast<uint32_t>(g) + (kOdd ? static_cast<uint32_t>(par * R::kRows * 8) : 0u);
   int stage = group % p.stages, slot = group % R::kDepth, tile = first_tile, k = group;
   uint32_t parity = static_cast<uint32_t>(group / p.stages) & 1u, rparity = 0;
   bool first_round = group < p.stages;
@@ -394,8 +366,9 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
 #pragma unroll
       for (int i = 0; i < 16; ++i) cs[i] = (sg.w_scale != nullptr && n + i < sg.n) ? __ldg(sg.w_scale + n + i) : 1.f;
     }
-    // the scales' offset in their 16 bytes: n0 / 16 is a multiple of eight, N / 2 of sixteen
-    const uint32_t rd_s = ring + R::kRows * 64 + row0 * 16 + static_cast<uint32_t>((t.n0 >> 4) & 8) + static_cast<uint32_t>(g);
+    // the offset in their 16 bytes: of the scales, n0 / 16 is a multiple of eight, N / 2 of sixteen; of an odd row, eight bytes
+    const uint32_t shift = kOdd && par ? static_cast<uint32_t>(sg.pitch) & 8u : 0u;
+    const uint32_t rd_w = rd_row + shift, rd_s = rd_scale_row + ((static_cast<uint32_t>(t.n0 >> 4) + shift) & 8u);
 #pragma unroll 1
     for (; k < kcount; k += GROUPS) {
       // both asked at once, the answer of the second needed after the first conversions
@@ -407,14 +380,14 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
       for (int j = 0; j < KS; ++j) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          if constexpr (MODE == kNvfp4) {
+          if constexpr (kFp4<MODE>) {
             uint32_t v[2];
-            Lds64(rd_w + at + j * (kBk * 64) + i * 256, v);
+            Lds64(rd_w + at + j * (kBk * kRow) + i * (4 * kRow), v);
             raw[j][i][0] = v[0];
             raw[j][i][1] = v[1];
-            sc[j][i] = Lds8(rd_s + at + j * (kBk * 16) + i * 64);
+            sc[j][i] = Lds8(rd_s + at + j * (kBk * kScaleRow) + i * (4 * kScaleRow));
           } else {
-            Lds128(rd_w + at + j * (kBk * 128) + i * 512, raw[j][i]);
+            Lds128(rd_w + at + j * (kBk * kRow) + i * (4 * kRow), raw[j][i]);
           }
         }
       }
@@ -425,7 +398,7 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           uint32_t h[8];
-          if constexpr (MODE == kNvfp4) {
+          if constexpr (kFp4<MODE>) {
             uint32_t lo[4], hi[4], s, unused;
             CvtE4m3x4(sc[j][i] * 0x101u, s, unused);
             CvtE2m1x8(raw[j][i][0], lo);
@@ -508,7 +481,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       BarInit(acce0 + i * 8, 4 * (PAIR ? 2 : 1));
     }
     for (int i = 0; MODE != kBf16 && i < RawRing<MODE, KS>::kDepth; ++i) {
-      BarInit(Smem(&ctl.raw_full[i]), MODE == kFp8 || p.raw_tensor ? 1 : 32 * kLoadWarps);
+      BarInit(Smem(&ctl.raw_full[i]), 1);
       BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
     }
     ctl.fault = 0;
@@ -516,8 +489,8 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   }
   if (warp == 4 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.xmap) : "memory");
-    if (p.raw_tensor) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.wmap[0]) : "memory");
-    if (MODE == kNvfp4 && p.raw_tensor) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.smap[0]) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.wmap[0]) : "memory");
+    if (kFp4<MODE>) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.smap[0]) : "memory");
   }
   if (warp == 5) {
     if constexpr (PAIR) {
@@ -714,12 +687,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   } else if constexpr (MODE != kBf16) {
     const uint32_t ring = smem + static_cast<uint32_t>(p.stages) * stage_bytes;
     if (warp < kFirstDqWarp) {
-      if (MODE == kFp8 || p.raw_tensor) {
-        if (warp == 6) LoadTensor<MODE, PAIR, KS>(p, ctl, rank, kbeg, kcount, first_tile, tile_step, ring);
-      } else if constexpr (MODE == kNvfp4) {
-        LoadNvfp4Pieces<PAIR, KS>(p, ctl, tid - 6 * 32, rank, kbeg, kcount, first_tile, tile_step, ring);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-      }
+      if (warp == 6) LoadTensor<MODE, PAIR, KS>(p, ctl, rank, kbeg, kcount, first_tile, tile_step, ring);
     } else {
       const int w = warp - kFirstDqWarp;
       DequantRole<MODE, SCALED, PAIR, KS, kDqGroups>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
@@ -1014,7 +982,7 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
     BarInit(Smem(&gate_full), 1);
     BarExpect(Smem(&gate_full), static_cast<uint32_t>(p.bm) * 4);
     for (int i = 0; MODE != kBf16 && i < RawRing<MODE, 1>::kDepth; ++i) {
-      BarInit(Smem(&ctl.raw_full[i]), MODE == kFp8 || p.raw_tensor ? 1 : 32 * kLoadWarps);
+      BarInit(Smem(&ctl.raw_full[i]), 1);
       BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
     }
     ctl.fault = 0;
@@ -1084,11 +1052,8 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
       if (warp >= kFirstDqWarp) {
         // the products are exact in BF16 without w_scale, which the epilogue applies to the sums as the streaming kernels do
         DequantRole<MODE, false, false, 1, 1>(p, ctl, warp - kFirstDqWarp, 0, lane, 0, p.ksteps, tile, p.tiles, ring, smem, block_bytes);
-      } else if (MODE == kFp8 || p.raw_tensor) {
-        if (warp == 6) LoadTensor<MODE, false, 1>(p, ctl, 0, 0, p.ksteps, tile, p.tiles, ring);
-      } else if constexpr (MODE == kNvfp4) {
-        LoadNvfp4Pieces<false, 1>(p, ctl, tid - 6 * 32, 0, 0, p.ksteps, tile, p.tiles, ring);
-        asm volatile("cp.async.wait_all;" ::: "memory");
+      } else if (warp == 6) {
+        LoadTensor<MODE, false, 1>(p, ctl, 0, 0, p.ksteps, tile, p.tiles, ring);
       }
     }
   }
@@ -1179,6 +1144,7 @@ constexpr int kSmemLimit = 232448 - 1024 - static_cast<int>(sizeof(Ctl)) - 64;
 int RawBytes(int mode, int ks) {
   if (mode == kFp8) return ks == 2 ? RawRing<kFp8, 2>::kBytes : RawRing<kFp8, 1>::kBytes;
   if (mode == kNvfp4) return ks == 2 ? RawRing<kNvfp4, 2>::kBytes : RawRing<kNvfp4, 1>::kBytes;
+  if (mode == kNvfp4Odd) return ks == 2 ? RawRing<kNvfp4Odd, 2>::kBytes : RawRing<kNvfp4Odd, 1>::kBytes;
   return 0;
 }
 int BlocksFor(int mode, int xrows, int ks) { return (kSmemLimit - kOutBytes - RawBytes(mode, ks)) / (kABytes + xrows * kBk * 2); }
@@ -1294,9 +1260,12 @@ cudaError_t SetUpDevice(const DeviceSetup** out) {
     if (err == cudaSuccess) err = SetUpMode<kFp8, true>();
     if (err == cudaSuccess) err = SetUpMode<kNvfp4, false>();
     if (err == cudaSuccess) err = SetUpMode<kNvfp4, true>();
+    if (err == cudaSuccess) err = SetUpMode<kNvfp4Odd, false>();
+    if (err == cudaSuccess) err = SetUpMode<kNvfp4Odd, true>();
     if (err == cudaSuccess) err = SetUpShared<kBf16>();
     if (err == cudaSuccess) err = SetUpShared<kFp8>();
     if (err == cudaSuccess) err = SetUpShared<kNvfp4>();
+    if (err == cudaSuccess) err = SetUpShared<kNvfp4Odd>();
     if (err != cudaSuccess) return err;
     DeviceSetup d = {dev, {}};
     for (int c = 1; c <= kMaxCluster; ++c) d.slots[c] = QuerySlots(c);
@@ -1312,7 +1281,18 @@ bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int
   const uint64_t rows = static_cast<uint64_t>(K), pitch = static_cast<uint64_t>(sg.pitch), n = static_cast<uint64_t>(sg.n);
   if (mode == kBf16) return Encode(&p.wmap[s], sg.w, 2, rows, n, pitch, kBk, 64);
   if (mode == kFp8) return Encode(&p.wmap[s], sg.w, 1, rows, n, pitch, kBk * ks, kBn);
-  return Encode(&p.wmap[s], sg.w, 1, rows, pitch, pitch, kBk * ks, kBn / 2) && Encode(&p.smap[s], sg.w, 1, rows, pitch, pitch, kBk * ks, 16);
+  const uint64_t rows_in_one = mode == kNvfp4Odd ? 2 : 1;  // K is a multiple of eight
+  const uint32_t box = static_cast<uint32_t>(kBk * ks / rows_in_one);
+  return Encode(&p.wmap[s], sg.w, 1, rows / rows_in_one, pitch * rows_in_one, pitch * rows_in_one, box, mode == kNvfp4Odd ? kOddPitch : kBn / 2) &&
+         Encode(&p.smap[s], sg.w, 1, rows / rows_in_one, pitch * rows_in_one, pitch * rows_in_one, box, 16);
+}
+
+// which of the file's modes a call is: one weight of odd rows makes all of them be read that way
+int KernelMode(int mode, const GemmParams& p) {
+  for (int s = 0; s < p.nseg && mode == kNvfp4; ++s) {
+    if (p.seg[s].pitch % 16 != 0) return kNvfp4Odd;
+  }
+  return mode;
 }
 
 }  // namespace
@@ -1326,8 +1306,7 @@ cudaError_t ConfigureDenseKernels() {
 
 // Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200;
 // us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair 0.13 + 0.00098 bm
-// (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24; 0.52 and 0.41 where the rows are loaded in
-// 8-byte pieces); around the blocks 4 + 0.008 bm, 0.9 more for a pair, and 1.8 + 0.01 bm more where ranks add up: with
+// (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24); around the blocks 4 + 0.008 bm, 0.9 more for a pair, and 1.8 + 0.01 bm more where ranks add up: with
 // less for those two, as K = 5120 alone had suggested, short K was split and paired where that loses (BF16 146 x 400 x
 // 3728 6.3 us in pairs of 64, 5.5 in single tiles of 48; over 150 random calls the shape chosen took 3.7 % longer than the
 // best one, and takes 1.8).  More row tiles than needed are tried because they can fill the last wave better (509 rows,
@@ -1337,10 +1316,8 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
   if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SkinnyGemm(dense): the kernels could not be set up on this device");
   DenseTcPlan best;
   double best_cost = 1e30, bytes = 0;
-  bool pieces = false;
   for (int s = 0; s < p.nseg; ++s) {
     bytes += static_cast<double>(p.seg[s].total_bytes);
-    pieces = pieces || (mode == kNvfp4 && p.seg[s].pitch % 16 != 0);
   }
   const int64_t blocks = (p.K + kBk - 1) / kBk, least = (m + 255) / 256;
   for (int pair = 0; pair <= 1; ++pair) {
@@ -1350,7 +1327,7 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
       const int bm = static_cast<int>(((m + mt - 1) / mt + 15) / 16 * 16);
       if (bm > 256 || (pair && bm < 64)) continue;
       const int64_t tiles = n_tiles * ((m + bm - 1) / bm);
-      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : !pieces ? 0.24 : pair ? 0.41 : 0.52);
+      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : 0.24);
       for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
         const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : setup->slots[split];
         if (slots < 1) break;  // the device holds no such cluster
@@ -1386,7 +1363,8 @@ bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
   return Encoder() != nullptr;
 }
 
-bool LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+  const int mode = KernelMode(weights, g);
   if (plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.split < 1 || plan.split > 8 || (plan.pair && plan.split != 1) || plan.ks < 0 || plan.ks > 2)
     throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
   DenseParams p = {};
@@ -1400,16 +1378,14 @@ bool LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
   if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
     return false;
   bool scaled = false;
-  p.raw_tensor = 1;
   int n_tiles = 0;
   for (int s = 0; s < g.nseg; ++s) {
     const Segment& sg = g.seg[s];
     p.seg[s] = {sg.w, sg.w_scale, sg.pitch, sg.total_bytes, sg.n, n_tiles, sg.out_begin, sg.out_end};
     n_tiles += (sg.n + (plan.pair ? 255 : 127)) / (plan.pair ? 256 : 128);
     scaled = scaled || sg.w_scale != nullptr;
-    p.raw_tensor = p.raw_tensor && sg.pitch % 16 == 0;
   }
-  for (int s = 0; s < g.nseg && p.raw_tensor; ++s) {
+  for (int s = 0; s < g.nseg; ++s) {
     if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks)) return false;
   }
   const int n_out = g.seg[g.nseg - 1].out_end;
@@ -1435,9 +1411,12 @@ bool LaunchDenseTc(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& 
     err = LaunchMode<kBf16, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
   } else if (mode == kFp8) {
     err = scaled ? LaunchMode<kFp8, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream) : LaunchMode<kFp8, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
-  } else {
+  } else if (mode == kNvfp4) {
     err = scaled ? LaunchMode<kNvfp4, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream)
                  : LaunchMode<kNvfp4, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+  } else {
+    err = scaled ? LaunchMode<kNvfp4Odd, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream)
+                 : LaunchMode<kNvfp4Odd, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
@@ -1477,7 +1456,8 @@ DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) 
   return best;
 }
 
-bool LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
+  const int mode = KernelMode(weights, g);
   const int C = plan.split;
   if ((C != 1 && C != 2 && C != 4) || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm % (8 * C) != 0)
     throw std::runtime_error("SharedExpertDown: bad launch shape");
@@ -1492,8 +1472,7 @@ bool LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   p.seg[0] = {sg.w, sg.w_scale, sg.pitch, sg.total_bytes, sg.n, 0, 0, 1};
   p.out[0] = g.out[0];
   p.width[0] = sg.n;
-  p.raw_tensor = sg.pitch % 16 == 0;
-  if (p.raw_tensor && !EncodeWeight(p, mode, 0, sg, g.K, 1)) return false;
+  if (!EncodeWeight(p, mode, 0, sg, g.K, 1)) return false;
   const int64_t n_tiles = ((sg.n + kBn - 1) / kBn + C - 1) / C * C, m_tiles = (m + p.bm - 1) / p.bm;
   if (n_tiles * m_tiles > INT_MAX / 16) return false;
   p.m_tiles = static_cast<int>(m_tiles);
@@ -1514,9 +1493,10 @@ bool LaunchDenseShared(int mode, const GemmParams& g, int64_t m, const DenseTcPl
   cudaError_t err = CheckConfiguredDevice();
   if (err == cudaSuccess) err = ConfigureDenseKernels();
   if (err == cudaSuccess) {
-    err = mode == kBf16  ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
-          : mode == kFp8 ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
-                         : LaunchShared<kNvfp4>(q, p.tiles, smem, stream);
+    err = mode == kBf16    ? LaunchShared<kBf16>(q, p.tiles, smem, stream)
+          : mode == kFp8   ? LaunchShared<kFp8>(q, p.tiles, smem, stream)
+          : mode == kNvfp4 ? LaunchShared<kNvfp4>(q, p.tiles, smem, stream)
+                           : LaunchShared<kNvfp4Odd>(q, p.tiles, smem, stream);
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SharedExpertDown: ") + cudaGetErrorString(err));
