@@ -23,7 +23,7 @@
 // What bounds it.  Few rows: the dequantising warps and the barriers between the roles, about 400 cycles a block of 64 k
 // (FP4 at 33 rows, 5120 x 17408: 23.7 us = 2.1 TB/s of weights; the dequantisation pass and the library GEMM that this
 // kernel took the place of, 86.6 us).  Many rows: the tensor core at its rate under load, and the last wave (FP8, 509
-// rows, 5120 x 10240: 65.6 us against 92.5; FP4, 2048 rows, 5120 x 17408: 298 us against 333).  The tcgen05 operands
+// rows, 5120 x 10240: 65.6 us against 92.5; FP4, 2048 rows, 5120 x 17408: 291 to 302 us against 333).  The tcgen05 operands
 // come from shared memory rather than tensor memory because the rows of x per pass would be limited to 64 there, and the
 // weights are written MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
 //
@@ -786,8 +786,8 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
 // trips to memory deep and little else, so every phase spreads over as many warps as it can: all of them finish the
 // sums (the four epilogue warps alone, 16 rows at a time, took half of a call).
 //
-// The streaming kernels that served these calls eight rows at a time took 1256 us for 777 rows of FP8 640 x 2560; this
-// one 27.  It is bound by swish_mul and latency: 0.6 us per block of 64 k at 160 rows against 0.17 us of MMAs.
+// The streaming kernels that served these calls eight rows at a time took 1403 us for 777 rows of FP8 640 x 2560; this
+// one 25.5.  It is bound by swish_mul and latency: 0.6 us per block of 64 k at 160 rows against 0.17 us of MMAs.
 struct DenseShared {
   DenseParams d;
   const uint16_t *g, *u, *gx, *gw, *routed;

@@ -241,9 +241,10 @@ cudaError_t LaunchDequant(const DequantParams& p, cudaStream_t stream);
 
 // Calls with more than `dense_rows` rows (an option of the node; 0 disables it) leave the streaming kernels: dense_tc.cu,
 // or dense_gemm.cc for the layouts that does not take.
-// The defaults are where the branch starts to win on a B200 (K = 5120): BF16 weights need no dequantisation
-// pass, so two streaming passes already lose (N = 2048: 37.7 us against 16.3); FP8 pays 48.5 us at N = 10240
-// against 35 us per eight rows; NVFP4 pays 89 us at N = 17408, which three passes (105 us) exceed.
+// At and below the defaults a row's result does not depend on the number of rows in the call: the streaming kernels compute
+// it as a one-row call does.  Speed alone would put the lines lower.  5120 x 17408, streaming / many-row kernel, us: eight
+// rows BF16 66 / 32, FP8 31 / 25, NVFP4 25 / 23; nine rows (two passes) 98 / 32, 55 / 25, 44 / 23; sixteen rows NVFP4 49 / 23.
+// NVFP4's 16 was the break-even of a dequantisation pass and a library GEMM (89 us at any number of rows).
 constexpr int DenseRowsDefault(int mode) { return mode == kNvfp4 ? 16 : 8; }
 bool DenseEligible(const GemmParams& p);
 void LaunchDenseGemm(int mode, const GemmParams& p, int64_t m, cudaStream_t stream);  // throws std::runtime_error
@@ -263,8 +264,8 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
 bool LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);
 
 // SharedExpertDown over many rows; `split` of the plan is the cluster size (1, 2 or 4).  Calls of up to sixteen rows keep
-// the streaming kernels, whose results do not depend on the number of rows; at seventeen they take three passes, 43 us
-// (NVFP4 640 x 2560), and the many-row kernel 11.
+// the streaming kernels, whose results do not depend on the number of rows.  NVFP4 640 x 2560, streaming / many-row kernel,
+// us: nine rows 30 / 12, sixteen 33 / 12, seventeen (three passes) 46 / 12.
 constexpr int kDenseSharedRows = 16;
 bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m);
 DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count);
