@@ -79,6 +79,7 @@ struct qfg_skinny_gemm {
   qfg::DenseTcPlan dense_plan;  // bm > 0: overrides the launch shape of that branch (set_option("dense_plan", "bm,split,pair,ks"))
   unsigned long long phase_times = 0;  // device address given through set_option("phase_times", ...)
   std::string plan_spec;
+  std::string stream_spec;  // set_option("stream_plan", "width,wk,teams,cluster,tail"): overrides that kernel's launch shape; "0": not that kernel
   // plans already computed for this node, keyed by the shape of the call
   mutable std::mutex plan_mu;
   mutable std::map<std::string, qfg::Plan> plans;
@@ -92,7 +93,7 @@ struct qfg_skinny_gemm {
   qfg_skinny_gemm(const qfg_skinny_gemm& o)
       : seg_outs(o.seg_outs), widths(o.widths), trigger(o.trigger), d_w_scale(o.d_w_scale), w_scale_len(o.w_scale_len),
         pdl_wait(o.pdl_wait), force_slow(o.force_slow), exchange_spin(o.exchange_spin), dense_rows(o.dense_rows),
-        dense_plan(o.dense_plan), phase_times(o.phase_times), plan_spec(o.plan_spec) {}
+        dense_plan(o.dense_plan), phase_times(o.phase_times), plan_spec(o.plan_spec), stream_spec(o.stream_spec) {}
 };
 
 struct qfg_dequant {
@@ -229,7 +230,7 @@ qfg::Plan ComputePlan(const qfg_skinny_gemm& op, const qfg::PlanInput& in);
 
 bool SamePlanInput(const qfg::PlanInput& a, const qfg::PlanInput& b) {
   if (a.K != b.K || a.nseg != b.nseg || a.mode != b.mode || a.row_align != b.row_align || a.sm_count != b.sm_count ||
-      a.max_rows != b.max_rows || a.max_clusters != b.max_clusters || a.allow_tail != b.allow_tail) {
+      a.max_rows != b.max_rows || a.max_clusters != b.max_clusters || a.allow_tail != b.allow_tail || a.fuse != b.fuse) {
     return false;
   }
   for (int s = 0; s < a.nseg; ++s) {
@@ -277,6 +278,16 @@ qfg::Plan ComputePlan(const qfg_skinny_gemm& op, const qfg::PlanInput& in) {
   }
   if (!spec.empty() && !qfg::ApplyPlanOverrides(spec, in, &plan)) throw InvalidArgument("SkinnyGemm: bad plan override");
   qfg::FinishPlan(in, spec, &plan);
+  // a pinned launch geometry is one of the other kernels'
+  if (spec.empty()) {
+    if (op.stream_spec.empty()) {
+      plan.stream = qfg::ChooseStreamPlan(in);
+    } else if (op.stream_spec != "0") {
+      qfg::StreamPlan& s = plan.stream;
+      if (std::sscanf(op.stream_spec.c_str(), "%d,%d,%d,%d,%d", &s.width, &s.wk, &s.teams, &s.cluster, &s.tail) < 3 || !qfg::CompleteStreamPlan(in, &s))
+        throw InvalidArgument("SkinnyGemm: bad stream_plan override");
+    }
+  }
   return plan;
 }
 
@@ -322,7 +333,8 @@ void Run(const qfg_skinny_gemm& op, Prepared& pr, int64_t m, cudaStream_t stream
     if (q.lm) {
       if (m > qfg::kMaxRows) throw InvalidArgument(std::string(name) + ": at most 8 rows per call");
     }
-    cudaError_t err = qfg::LaunchSkinnyGemm(pr.mode, q, plan, stream);
+    cudaError_t err = cudaSuccess;
+    if (plan.stream.width == 0 || !qfg::LaunchSkinnyStream(pr.mode, q, plan.stream, stream, &err)) err = qfg::LaunchSkinnyGemm(pr.mode, q, plan, stream);
     if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess) throw std::runtime_error(std::string(name) + ": " + cudaGetErrorString(err));
     done += chunk;
@@ -374,6 +386,12 @@ int SetGemmOption(qfg_skinny_gemm* op, const char* key, const char* value) {
   else if (k == "phase_times") op->phase_times = std::strtoull(value, nullptr, 10);  // measurement builds only
 #endif
   else if (k == "plan") op->plan_spec = value;
+  else if (k == "stream_plan") {
+    std::lock_guard<std::mutex> lock(op->plan_mu);
+    op->stream_spec = value;
+    op->plans.clear();
+    op->last_valid = false;
+  }
   else if (k == "trigger") op->trigger = std::atoi(value);
   else return Fail(QFG_INVALID_ARGUMENT, "set_option: unknown key " + k);
   return QFG_OK;
@@ -515,7 +533,7 @@ int qfg_skinny_gemm_describe(const qfg_skinny_gemm* op, int64_t k, const qfg_ten
   try {
     Prepared pr = Prepare(*op, nullptr, 1, k, weights, n_weights, nullptr, 0, false);
     const qfg::Plan plan = PlanFor(*op, pr.plan_in, qfg::kMaxRows);
-    const std::string d = qfg::DescribePlan(plan, pr.plan_in) + ",trigger=" + std::to_string(op->trigger);
+    const std::string d = qfg::DescribePlan(plan, pr.plan_in) + "," + qfg::DescribeStreamPlan(plan.stream) + ",trigger=" + std::to_string(op->trigger);
     std::snprintf(buf, buf_len, "%s", d.c_str());
     return QFG_OK;
   } catch (const std::exception& e) {
@@ -616,6 +634,7 @@ int qfg_shared_expert_down_compute(const qfg_shared_expert_down* op, const void*
     void* outs[1] = {out};
     Prepared pr = Prepare(op->gemm, g, m, k, weight, 1, outs, 1, true, n);
     pr.params.fuse = 1;
+    pr.plan_in.fuse = true;
     pr.params.x2 = static_cast<const uint16_t*>(u);
     pr.params.gx = static_cast<const uint16_t*>(gx);
     pr.params.gw = static_cast<const uint16_t*>(gw);

@@ -46,6 +46,8 @@
 #include <type_traits>
 
 #include "qfg_internal.h"
+#include "swish.cuh"
+#include "tensor_map.h"
 
 namespace qfg {
 namespace {
@@ -806,35 +808,6 @@ __device__ __forceinline__ float SigmoidBf16(float a) {
   const float e = expf(-fabsf(a));
   return RoundBf16(a > 0.0f ? 1.0f / (1.0f + e) : e / (1.0f + e));
 }
-// sigmoid(a) before its rounding, for a BF16 a: exp(-|a|) as 2^y with y = -|a| h exact (h: the upper 16 bits of log2 e,
-// against the eight of a) and the rest of the exponent to first order, then a reciprocal; next to zero, where a / 4 can
-// lie on a rounding boundary to within less than an ulp, the Taylor polynomial.  Fifteen instructions where expf and an
-// IEEE division take over forty; after rounding the same for each of the 65536 inputs.
-__device__ __forceinline__ float SigmoidOfBf16(float a) {
-  const float x = fminf(fabsf(a), 256.f);  // 2^-369 is zero
-  constexpr float h = 47274.f / 32768.f, rest = 4.888495e-06f;  // log2 e = h + 7.052608e-6; that times ln 2
-  float e, r;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(x * -h));
-  e = fmaf(e, x * -rest, e);
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  const float far = (a > 0.0f ? 1.0f : e) * r, near = fmaf(a, fmaf(a * a, -1.f / 48.f, 0.25f), 0.5f);
-  return x < 0.03125f ? near : far;
-}
-__device__ __forceinline__ uint32_t PackBf16(float lo, float hi) {
-  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&b);
-}
-__device__ __forceinline__ uint32_t MulBf16x2(uint32_t a, uint32_t b) {  // one rounding, like the FP32 product rounded
-  uint32_t r;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ float Lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float Hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-__device__ __forceinline__ uint32_t SwishMul2(uint32_t g2, uint32_t u2) {  // two BF16 per word
-  return MulBf16x2(MulBf16x2(g2, PackBf16(SigmoidOfBf16(Lo(g2)), SigmoidOfBf16(Hi(g2)))), u2);
-}
-
 // Warps that share a block.  A barrier's parity tells a phase from the next only, so a warp must have seen a stage's
 // previous block consumed (or a later one) before it waits for the stage again: no more blocks in hand than stages.
 __device__ __forceinline__ int SwishWarpsPerBlock(int stages) { return kSwishWarps / (stages >= 8 ? 8 : stages >= 4 ? 4 : stages >= 2 ? 2 : 1); }
@@ -1114,25 +1087,11 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
 }
 
 // ------------------------------------------------------------------------------ host
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn Encoder() {
-  static const EncodeFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<EncodeFn>(f);
-  }();
-  return fn;
-}
-
 // rows x cols elements of `elem` bytes (2: BF16, boxes swizzled in 128 bytes; 1: bytes, plain), row-major
 bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols) {
   const cuuint64_t dims[2] = {cols, rows}, strides[1] = {pitch_bytes};
   const cuuint32_t box[2] = {box_cols, box_rows}, step[2] = {1, 1};
-  const EncodeFn fn = Encoder();
+  const TensorMapEncodeFn fn = TensorMapEncoder();
   return fn != nullptr &&
          fn(map, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, step,
             CU_TENSOR_MAP_INTERLEAVE_NONE, elem == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1360,7 +1319,7 @@ bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
   for (int o = 0; o < n_out; ++o) {
     if (p.out[o] == nullptr || p.width[o] % 8 != 0) return false;
   }
-  return Encoder() != nullptr;
+  return TensorMapEncoder() != nullptr;
 }
 
 bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {

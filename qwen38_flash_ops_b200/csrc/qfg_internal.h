@@ -57,6 +57,17 @@ inline int DirectSlotBytes(int mode, int wide) {
 
 // Launch geometry.  It depends on (K, segment widths, weight type) only - never on the
 // number of rows - so that a row's reduction order is the same in every call.
+// Launch shape of the kernel that streams the weights by tensor copies (skinny_stream.cu).
+struct StreamPlan {
+  int width = 0;    // granules (16 bytes of a row; NVFP4: 128 columns) per column tile; 0: the call goes to the other kernels
+  int wk = 0;       // warps sharing a stage along K, two k-steps each
+  int teams = 1;    // sets of warps that take the stages in turn
+  int cluster = 1;  // CTAs splitting K
+  int tail = 0;     // fused LM head: as Plan::tail
+  int tail_split = 1;
+  int tiles[kMaxSeg] = {0, 0, 0, 0};
+};
+
 struct Plan {
   int wn = 4;       // warps side by side along N
   int wk = 2;       // warps splitting each stage along K
@@ -74,6 +85,7 @@ struct Plan {
   int warps() const { return tc ? wn * wk + 1 + wk : wn * wk; }
   int threads() const { return 32 * warps(); }
   int rows_per_stage() const { return 16 * wk * ks; }
+  StreamPlan stream;
 };
 
 // Columns a CTA of this plan can hold.
@@ -187,6 +199,7 @@ struct PlanInput {
   // Co-resident clusters (CTAs for cluster == 1) of a launch shape on the current device, or null
   // when planning without a device (then a B200-like packing loss is assumed for clusters).
   int (*max_clusters)(int mode, int direct, int threads, size_t smem, int cluster) = nullptr;
+  bool fuse = false;        // SharedExpertDown
   bool allow_tail = false;  // the call is a fused LM head whose workspace can hold the shared-tail partial sums
 };
 Plan ChoosePlan(const PlanInput& in);
@@ -207,6 +220,15 @@ int DeviceSmCount();
 cudaError_t ConfigureSkinnyGemmKernels();
 cudaError_t CheckConfiguredDevice();  // cudaErrorInvalidDevice where another device than the configured one is current
 int QueryMaxActiveClusters(int mode, int direct, int threads, size_t smem, int cluster);
+
+// skinny_stream.cu
+cudaError_t ConfigureStreamKernels();  // for the device of the other streaming kernels
+StreamPlan ChooseStreamPlan(const PlanInput& in);
+// Fills in what follows from width, wk, teams, cluster and tail; false: no such launch shape for these weights.
+bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan);
+std::string DescribeStreamPlan(const StreamPlan& plan);
+// false, nothing launched: x off 16 bytes, or a tensor map that could not be made.
+bool LaunchSkinnyStream(int mode, GemmParams& p, const StreamPlan& plan, cudaStream_t stream, cudaError_t* err);
 
 // argmax_rows.cu
 cudaError_t LaunchArgmaxRows(int dtype, const void* x, int64_t rows, int64_t vocab, int64_t* idx, float* val,

@@ -1,0 +1,1059 @@
+// SkinnyGemm for up to eight rows, the weights streamed by tensor copies.
+//
+// One CTA per SM owns a column tile of one weight and one of `cluster` slices of K.  One lane of a producer warp copies
+// boxes of R weight rows by the tile's width into a ring that fills the SM's shared memory; teams of wn x wk consumer
+// warps take the stages in turn, warp (i, j) of a team the columns of its 128 bytes (64 for NVFP4) and k-steps j and j + wk
+// of a stage, with the arithmetic of skinny_common.cuh.  The producer waits for nobody until the ring is full, so x is staged and converted
+// while the first 200 KB per SM are on their way, and what is left of the call is the stream and the epilogue.
+//
+// Why tensor copies: one instruction fetches a whole box.  A copy-only kernel of this shape streams 52 MB in 10.4 us and
+// the 437 MB LM head in 69 us, launch included, against 96 us for the rings of 16-byte cp.async copies that each warp
+// issued for itself; they need 8 KB or more per copy instruction (boxes of 16 rows by 64 bytes reach 0.9 TB/s).
+//
+// Layout of a stage: R rows of `pitch` bytes, then (NVFP4) R rows of `spitch` bytes that hold the rows' block scales.
+// A lane (g, t) reads rows 2t, 2t + 1, 2t + 8 and 2t + 9 of a k-step, 16 bytes (NVFP4: 8) at g: the rows of a quarter
+// (half) warp have to lie 32 (64) bytes apart in the banks, which an odd number of 16-byte pieces per row gives, so boxes
+// of an even number are copied one piece wider (swizzling would need boxes of exactly 128 bytes).
+// NVFP4 weights whose N is an odd multiple of 128 have rows an odd multiple of eight bytes long: two rows are then one row
+// of the tensor map, a stage holds R / 2 even rows and R / 2 odd rows, the latter copied from the 16-byte boundary before
+// them, and `pitch` is 32 or 96 modulo 128.
+//
+// Every wait is bounded; a CTA that gives up on one writes NaN.
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+#include <climits>
+#include <cstdio>
+#include <mutex>
+#include <type_traits>
+
+#include "skinny_common.cuh"
+#include "swish.cuh"
+#include "tensor_map.h"
+
+namespace qfg {
+namespace {
+
+constexpr int kStreamWarps = 18;                             // consumers, at most
+constexpr int kStreamThreads = 32 * (kStreamWarps + 2);      // and the producer, and the LM head's tail warp
+constexpr int kStreamStages = 24;
+constexpr int kStreamSpin = 1 << 20;
+
+struct StreamParams {
+  GemmParams g;
+  CUtensorMap wmap[kMaxSeg];  // stored rows (nibbles of NVFP4) in elements of eight bytes
+  CUtensorMap smap[kMaxSeg];  // NVFP4 block scales
+  CUtensorMap tail_wmap, tail_smap;
+  int warps;                  // consumers: teams * wk * wn
+  int teams, team_warps, team_wk, team_inv;  // team t takes stages t, t + teams, ...; 65536 / team_warps, rounded up
+  int wn_inv;                 // 65536 / wn, rounded up
+  int rows;                   // R = 32 team_wk
+  int nstages;                // stages of the whole K range
+  int odd;                    // rows in pairs (see above)
+  int boxes, col_boxes;       // per stage (and half): boxes of box_rows rows, side by side the boxes of a swizzled tile
+  int swizzle;                // 0, or the bytes of a swizzled box's rows
+  uint32_t box_rows, pitch, spitch, half, shalf, scale_off, tx;
+  int row_warps, row_pass, row_inv;  // how the consumer warps share the rows of x (ShareOf)
+  int rank_cols;              // cluster: columns of the tile that a rank finishes
+  uint32_t x_off;             // staged x in shared memory
+  uint32_t tail_off, tail_pitch, tail_tx, tail_rows;
+};
+
+struct StreamCtl {
+  unsigned long long full[kStreamStages], empty[kStreamStages], tail_full;
+  volatile uint32_t fault;
+};
+
+__device__ __forceinline__ void BarInit(uint32_t a, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(n) : "memory"); }
+__device__ __forceinline__ void BarArrive(uint32_t a) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(a) : "memory");
+}
+__device__ __forceinline__ void BarExpect(uint32_t a, uint32_t bytes) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes) : "memory");
+}
+// false once a wait of this CTA ran out
+__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& c) {
+  for (int i = 0; i < kStreamSpin; ++i) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 255) == 255 && c.fault) return false;
+  }
+  c.fault = 1;
+  return false;
+}
+// x in elements of eight bytes, an even number: a copy starts on 16 bytes
+__device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
+               "r"(bar), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ bool ElectOne() {
+  uint32_t yes;
+  asm volatile("{ .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(yes)::"memory");
+  return yes != 0;
+}
+// the B fragments of two k-steps: k-step a in v[0], v[1], k-step b in v[2], v[3]
+__device__ __forceinline__ void LoadX2(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
+}
+
+// Where a lane finds its rows: `w` the first of them in a k-step at the start of a region, d1 and d2 from row 2t to 2t + 1 and
+// to 2t + 8, `step` from a k-step to the next; s, e1, e2, sstep the same of the scales.
+struct LaneRows {
+  uint32_t w, d1, d2, step, s, e1, e2, sstep;
+};
+template <int MODE>
+__device__ __forceinline__ LaneRows RowsOf(const Segment& sg, int n0, int col_warp, int lane, int odd, uint32_t pitch, uint32_t spitch, uint32_t half,
+                                           uint32_t shalf, int swizzle = 0, uint32_t rows = 0) {
+  const int g = lane >> 2, t = lane & 3;
+  LaneRows r;
+  const uint32_t row = static_cast<uint32_t>(odd ? t : 2 * t), per = odd ? 4u : 8u;
+  r.w = row * pitch + static_cast<uint32_t>(MODE == kNvfp4 ? col_warp * 64 + g * 8 : col_warp * 128 + g * 16);
+  r.d1 = odd ? half + (static_cast<uint32_t>(sg.pitch) & 8u) : pitch;
+  r.d2 = per * pitch;
+  r.step = 2 * per * pitch;
+  if (swizzle == 128) {  // pieces of 16 bytes exclusive-or the row, modulo eight
+    const int piece = MODE == kNvfp4 ? (col_warp & 1) * 4 + (g >> 1) : g, at = piece ^ (2 * t);
+    r.w = static_cast<uint32_t>(MODE == kNvfp4 ? col_warp >> 1 : col_warp) * rows * 128u + row * 128u + static_cast<uint32_t>(at * 16 + (MODE == kNvfp4 ? (g & 1) * 8 : 0));
+    r.d1 = 128u + static_cast<uint32_t>(((at ^ 1) - at) * 16);
+  } else if (swizzle == 64) {  // pieces exclusive-or half the row, modulo four (NVFP4, one group)
+    r.w = row * 64u + static_cast<uint32_t>(((g >> 1) ^ t) * 16 + (g & 1) * 8);
+  }
+  const uint32_t scl = static_cast<uint32_t>(sg.n >> 1) + static_cast<uint32_t>(n0 >> 4), shift = scl & 8u;
+  r.s = row * spitch + static_cast<uint32_t>(col_warp * 8 + g) + shift;
+  r.e1 = odd ? shalf + ((scl + static_cast<uint32_t>(sg.pitch)) & 8u) - shift : spitch;
+  r.e2 = per * spitch;
+  r.sstep = 2 * per * spitch;
+  return r;
+}
+template <int MODE>
+__device__ __forceinline__ void LoadRows(Raw<MODE>& raw, const LaneRows& r, uint32_t w, uint32_t s) {
+  if constexpr (MODE == kNvfp4) {
+    raw.r[0][0] = Lds64(w);
+    raw.r[0][1] = Lds64(w + r.d1);
+    raw.r[0][2] = Lds64(w + r.d2);
+    raw.r[0][3] = Lds64(w + r.d1 + r.d2);
+    raw.s[0][0] = Lds8(s);
+    raw.s[0][1] = Lds8(s + r.e1);
+    raw.s[0][2] = Lds8(s + r.e2);
+    raw.s[0][3] = Lds8(s + r.e1 + r.e2);
+  } else {
+    raw.r[0] = Lds128(w);
+    raw.r[1] = Lds128(w + r.d1);
+    raw.r[2] = Lds128(w + r.d2);
+    raw.r[3] = Lds128(w + r.d1 + r.d2);
+  }
+}
+
+// max and min of the non-zero of eight packed BF16 magnitudes, two at a time (min is kept less one, so that zero is never it)
+__device__ __forceinline__ void TrackPair(uint32_t w, uint32_t& mx, uint32_t& mn) {
+  w &= 0x7FFF7FFFu;
+  mx = __vmaxu2(mx, w);
+  mn = __vminu2(mn, __vsub2(w, 0x00010001u));
+}
+__device__ __forceinline__ uint4 ScaleToHalf8(uint4 v, float sc) {
+  return make_uint4(ScaleToHalf2(v.x, sc), ScaleToHalf2(v.y, sc), ScaleToHalf2(v.z, sc), ScaleToHalf2(v.w, sc));
+}
+
+struct StreamScratch {
+  uint32_t xmax[kMaxRows][kStreamWarps], xmin[kMaxRows][kStreamWarps];
+  float gate[kMaxRows][2], inv[kMaxRows];  // SharedExpertDown: the two halves of the gate's sum; 1 / scale of a row
+};
+
+// The consumer warps side by side on the rows of the call: `wpr` of them per row, `rpp` rows at a time.
+struct RowShare {
+  int row, part, wpr, rpp;
+  bool any;
+};
+__device__ __forceinline__ RowShare ShareOf(const StreamParams& q, int warp) {
+  RowShare r;
+  r.wpr = q.row_warps;
+  r.rpp = q.row_pass;
+  r.row = (warp * q.row_inv) >> 16;  // warp / wpr
+  r.part = warp - r.row * r.wpr;
+  r.any = r.row < r.rpp && warp < q.warps;
+  return r;
+}
+
+// x of the slice to shared memory, rows padded with zeros to whole stages (so that the K loop needs no end), for the
+// quantised modes scaled by a power of two and converted to FP16 (skinny_common.cuh).  A thread converts what it stored
+// itself, so that the whole takes two barriers and one trip to L2.  Returns true if the CTA must take the BF16 path.
+template <int MODE>
+__device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, int padded,
+                                             const RowShare& rs, int lane) {
+  const GemmParams& p = q.g;
+  constexpr int kBatch = 4;
+  const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // K is a multiple of eight
+  auto copy = [&](int m, uint32_t& mx, uint32_t& mn) {
+    const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + tl.kbeg);
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 1
+    for (int c = c_first; c < chunks; c += kBatch * step) {
+      uint4 v[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) v[i] = c + i * step < valid ? __ldg(src + c + i * step) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        if (c + i * step < chunks) dst[c + i * step] = v[i];
+        if constexpr (MODE != kBf16) {
+          TrackPair(v[i].x, mx, mn);
+          TrackPair(v[i].y, mx, mn);
+          TrackPair(v[i].z, mx, mn);
+          TrackPair(v[i].w, mx, mn);
+        }
+      }
+    }
+  };
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    uint32_t mx = 0, mn = 0xFFFFFFFFu;
+    copy(m, mx, mn);
+    if constexpr (MODE != kBf16) {
+      mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
+      mn = __reduce_min_sync(0xffffffffu, min(mn & 0xFFFFu, mn >> 16));
+      if (lane == 0) {
+        sx.xmax[m][rs.part] = mx;
+        sx.xmin[m][rs.part] = mn;
+      }
+    }
+  }
+  __syncthreads();  // every warp also sees the mbarriers
+  if constexpr (MODE == kBf16) {
+    if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = 1.f;  // for the epilogue, behind further barriers
+    return false;
+  } else {
+    // Power-of-two scale per row that puts the slice maximum in [2^14, 2^15).  Every non-zero element must land in the
+    // normal FP16 range: exponent no more than 28 below the maximum's.
+    bool bad = p.force_slow != 0;
+#pragma unroll 1
+    for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+      const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < rs.wpr ? sx.xmax[m][lane] : 0u);
+      const uint32_t mn = __reduce_min_sync(0xffffffffu, lane < rs.wpr ? sx.xmin[m][lane] : 0xFFFFu);
+      const int e = static_cast<int>(mx >> 7);  // BF16 exponent field of the row maximum
+      const bool out = mx != 0 && (e < 32 || e >= 255 || static_cast<int>((mn + 1) >> 7) < e - 28);
+      bad = bad || out;
+      const float sc = mx != 0 && !out ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
+      if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f / sc;
+      uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 2
+      for (int c = c_first; c < chunks; c += step) dst[c] = ScaleToHalf8(dst[c], sc);
+    }
+    if (__syncthreads_or(bad)) {  // rare: the rows as they are
+#pragma unroll 1
+      for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+        uint32_t mx = 0, mn = 0;
+        copy(m, mx, mn);
+        if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f;
+      }
+      __syncthreads();
+      return true;
+    }
+    return false;
+  }
+}
+
+// SharedExpertDown's: x = swish_mul(g, u), and the gate of every row.  Everything a thread needs first is asked for before
+// anything is computed, so that the phase is one trip to memory.  The gate's sum is made in an order of its own, whatever
+// the number of rows: chunk c of eight elements to lane c mod 64, lanes by shuffles, the two halves in order.
+template <int MODE>
+__device__ __forceinline__ bool StageXShared(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, int padded,
+                                             const RowShare& rs, int lane) {
+  const GemmParams& p = q.g;
+  const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane, gate_chunks = p.gk >> 3;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  constexpr int kGate = 5;  // chunks of the gate a lane asks for at once: 2560 elements
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    const uint4* g = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + tl.kbeg);
+    const uint4* u = reinterpret_cast<const uint4*>(p.x2 + static_cast<size_t>(m) * p.K + tl.kbeg);
+    const uint4* gx = reinterpret_cast<const uint4*>(p.gx + static_cast<size_t>(m) * p.gk);
+    const uint4* gw = reinterpret_cast<const uint4*>(p.gw);
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+    uint4 gv = c_first < valid ? __ldg(g + c_first) : zero, uv = c_first < valid ? __ldg(u + c_first) : zero;
+    for (int half = rs.part; half < 2; half += rs.wpr) {
+      float sum = 0.f;
+#pragma unroll 1
+      for (int c = half * 32 + lane; c < gate_chunks; c += 64 * kGate) {
+        uint4 a[kGate], b[kGate];
+#pragma unroll
+        for (int i = 0; i < kGate; ++i) {
+          const bool in = c + 64 * i < gate_chunks;
+          a[i] = in ? __ldg(gx + c + 64 * i) : zero;
+          b[i] = in ? __ldg(gw + c + 64 * i) : zero;
+        }
+#pragma unroll
+        for (int i = 0; i < kGate; ++i) {
+          const uint32_t av[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, bv[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+          if (c + 64 * i < gate_chunks) {  // what lies past the end adds nothing, not even to an infinity
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              sum += __uint_as_float(av[e] << 16) * __uint_as_float(bv[e] << 16);
+              sum += __uint_as_float(av[e] & 0xFFFF0000u) * __uint_as_float(bv[e] & 0xFFFF0000u);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      if (lane == 0) sx.gate[m][half] = sum;
+    }
+    uint32_t mx = 0, mn = 0xFFFFFFFFu;
+#pragma unroll 1
+    for (int c = c_first; c < chunks;) {
+      const int next = c + step;
+      const uint4 gn = next < valid ? __ldg(g + next) : zero, un = next < valid ? __ldg(u + next) : zero;
+      const uint4 v = make_uint4(SwishMul2(gv.x, uv.x), SwishMul2(gv.y, uv.y), SwishMul2(gv.z, uv.z), SwishMul2(gv.w, uv.w));
+      dst[c] = v;
+      if constexpr (MODE != kBf16) {
+        TrackPair(v.x, mx, mn);
+        TrackPair(v.y, mx, mn);
+        TrackPair(v.z, mx, mn);
+        TrackPair(v.w, mx, mn);
+      }
+      gv = gn;
+      uv = un;
+      c = next;
+    }
+    if constexpr (MODE != kBf16) {
+      mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
+      mn = __reduce_min_sync(0xffffffffu, min(mn & 0xFFFFu, mn >> 16));
+      if (lane == 0) {
+        sx.xmax[m][rs.part] = mx;
+        sx.xmin[m][rs.part] = mn;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < p.M) {  // for the epilogue, behind further barriers
+    sh.gate[threadIdx.x] = SigmoidBf16(RoundBf16(sx.gate[threadIdx.x][0] + sx.gate[threadIdx.x][1]));
+    sh.inv_scale[threadIdx.x] = 1.f;
+  }
+  if constexpr (MODE == kBf16) return false;
+  // as in StageXStream, except that the rows are not read again: all scales are known before anything is converted
+  bool bad = p.force_slow != 0;
+#pragma unroll 1
+  for (int m = 0; m < p.M; ++m) {
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < rs.wpr ? sx.xmax[m][lane] : 0u);
+    const uint32_t mn = __reduce_min_sync(0xffffffffu, lane < rs.wpr ? sx.xmin[m][lane] : 0xFFFFu);
+    const int e = static_cast<int>(mx >> 7);
+    bad = bad || (mx != 0 && (e < 32 || e >= 255 || static_cast<int>((mn + 1) >> 7) < e - 28));
+  }
+  if (bad) {
+    __syncthreads();
+    return true;
+  }
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < rs.wpr ? sx.xmax[m][lane] : 0u);
+    const float sc = mx != 0 ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
+    if (rs.part == 0 && lane == 0) sx.inv[m] = 1.f / sc;
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 1
+    for (int c = c_first; c < chunks; c += step) dst[c] = ScaleToHalf8(dst[c], sc);
+  }
+  __syncthreads();
+  if (threadIdx.x < p.M) sh.inv_scale[threadIdx.x] = sx.inv[threadIdx.x];
+  return false;
+}
+
+// The warps' partial sums in `smem` ([wk][M][TNc], see StorePartials) to the outputs, across the cluster where K is split:
+// added in warp order, then in rank order.  `first_scale`, `first_routed`: what the thread's first column needs from global
+// memory, read before the K loop.
+template <int MODE, bool FUSE>
+__device__ __forceinline__ void FinishStream(const StreamParams& q, const Tile& tl, uint8_t* smem, SharedScratch& sh, const RowShare& rs, int lane, int cb,
+                                             int share, float first_scale, uint32_t first_routed) {
+  const GemmParams& p = q.g;
+  const Segment& sg = p.seg[tl.seg];
+  const int M = p.M, C = tl.C, TNc = p.wn * 8 * Geom<MODE>::kColsPerThread;
+  const float* red = reinterpret_cast<const float*>(smem);
+  float* part = reinterpret_cast<float*>(smem) + p.wk * M * TNc;
+  const int j_first = rs.part * 32 + lane, step = rs.wpr * 32;
+  auto local = [&](int m, int c) {
+    const float* at = red + m * TNc + RedCol(c, m);
+    float sum = 0.f;
+#pragma unroll 1
+    for (int w = 0; w < p.wk; w += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = w + i < p.wk ? at[(w + i) * M * TNc] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (w + i < p.wk) sum += v[i];
+      }
+    }
+    return sum * sh.inv_scale[m];
+  };
+  cg::cluster_group cluster = cg::this_cluster();
+  if (C > 1) {
+    for (int m = rs.row; rs.any && m < M; m += rs.rpp) {
+      for (int c = j_first; c < TNc; c += step) part[m * TNc + c] = local(m, c);
+    }
+    cluster.sync();
+  }
+  for (int m = rs.row; rs.any && m < M; m += rs.rpp) {
+    for (int j = j_first; j < share; j += step) {
+      const int c = cb + j, n = tl.n0 + c;
+      float v;
+      if (C > 1) {
+        // all ranks' sums are asked for before the first is added
+        float r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = i < C ? cluster.map_shared_rank(part, i)[m * TNc + c] : 0.f;
+        v = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i < C) v += r[i];
+        }
+      } else {
+        v = local(m, c);
+      }
+      const bool first = j == j_first && m == rs.row;
+      if (MODE != kBf16 && sg.w_scale != nullptr) v *= j == j_first ? first_scale : sg.w_scale[n];
+      if constexpr (FUSE) {
+        // SharedExpertDown: routed + bf16(bf16(sum) * gate), every step rounded to BF16 (skinny_gemm.cuh:226-240)
+        v = RoundBf16(RoundBf16(v) * sh.gate[m]);
+        if (p.routed != nullptr) {
+          const uint32_t r = first ? first_routed : p.routed[static_cast<size_t>(m) * sg.n + n];
+          v = __uint_as_float(r << 16) + v;
+        }
+      }
+      int o = sg.out_begin;
+      for (int i = o + 1; i < sg.out_end; ++i) {
+        if (n >= p.col_begin[i]) o = i;
+      }
+      p.out[o][static_cast<size_t>(m) * p.width[o] + (n - p.col_begin[o])] = __bfloat16_as_ushort(__float2bfloat16(v));
+    }
+  }
+  if (C > 1) cluster.sync();  // no CTA leaves while a peer still reads its sums
+}
+
+enum StreamKind : int { kPlain = 0, kShared = 1, kHead = 2 };
+
+#ifdef QFG_PHASE_TIMES
+#define QFG_CLOCK(v) const long long v = clock64()
+#define QFG_WAITED(v) waited += (v)
+#else
+#define QFG_CLOCK(v)
+#define QFG_WAITED(v)
+#endif
+
+// KIND: plain, SharedExpertDown, fused LM head.
+template <int MODE, int KIND>
+__global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(const __grid_constant__ StreamParams q) {
+  using G = Geom<MODE>;
+  constexpr int NM = G::kMmas;
+  constexpr bool kTail = MODE == kNvfp4 && KIND == kHead;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ SharedScratch sh;
+  __shared__ StreamScratch sx;
+  __shared__ StreamCtl ctl;
+  const GemmParams& p = q.g;
+  if (p.trigger == 1) GridLaunchDependents();
+  Stamp(p, 0);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  Tile tl = LocateTile(p);
+  const Segment& sg = p.seg[tl.seg];
+  // K in whole stages, so that no copy reaches into the next slice
+  const int st0 = tl.crank * q.nstages / tl.C, nst = (tl.crank + 1) * q.nstages / tl.C - st0;
+  tl.kbeg = st0 * q.rows;
+  tl.kend = min(p.K, (st0 + nst) * q.rows);
+  tl.kslice = max(0, tl.kend - tl.kbeg);
+  const uint32_t ring = (SmemAddr(smem_raw) + 1023u) & ~1023u;  // swizzled boxes begin on 1024 bytes
+  uint8_t* const smem = smem_raw + (ring - SmemAddr(smem_raw));
+  const uint32_t full0 = SmemAddr(&ctl.full[0]), empty0 = SmemAddr(&ctl.empty[0]);
+
+  // Shared tail of the fused LM head (see GemmParams::tail_groups): one K slice of a left-over column group per hosting CTA
+  int tail_index = -1, tail_first = 0, tail_count = 0, tail_col = 0;
+  if constexpr (kTail) {
+    if (p.tail_groups > 0 && static_cast<int>(blockIdx.x) % p.tail_stride == 0) {
+      const int i = static_cast<int>(blockIdx.x) / p.tail_stride;
+      if (i < p.tail_groups * p.tail_split) {
+        const int ksteps = (tl.kslice + 15) >> 4;
+        tail_index = i;
+        const int tg = i / p.tail_split, slice = i - tg * p.tail_split;
+        tail_first = slice * ksteps / p.tail_split;
+        tail_count = (slice + 1) * ksteps / p.tail_split - tail_first;
+        tail_col = sg.n - p.tail_groups * 128 + tg * 128;
+      }
+    }
+  }
+
+  // ---- producer: where this CTA's boxes begin, in elements of eight bytes
+  const int wpitch8 = static_cast<int>(sg.pitch >> 3);
+  const int x0 = MODE == kBf16 ? tl.n0 >> 2 : MODE == kFp8 ? tl.n0 >> 3 : tl.n0 >> 4;
+  const int sc0 = MODE == kNvfp4 ? ((sg.n >> 1) + (tl.n0 >> 4)) >> 3 : 0;
+  auto issue = [&](int s, int slot) {  // one lane
+    const uint32_t bar = full0 + static_cast<uint32_t>(slot) * 8u;
+    uint32_t dst = ring + static_cast<uint32_t>(slot) * static_cast<uint32_t>(p.stage_bytes), sdst = dst + q.scale_off;
+    int row = (tl.kbeg + s * q.rows) >> q.odd;
+    BarExpect(bar, q.tx);
+#pragma unroll 1
+    for (int b = 0; b < q.boxes; ++b) {
+      TmaLoad(dst, &q.wmap[tl.seg], x0, row, bar);
+#pragma unroll 1
+      for (int c = 1; c < q.col_boxes; ++c) TmaLoad(dst + c * q.rows * 128, &q.wmap[tl.seg], x0 + c * 16, row, bar);
+      if constexpr (MODE == kNvfp4) {
+        if (q.odd) TmaLoad(dst + q.half, &q.wmap[tl.seg], (x0 + wpitch8) & ~1, row, bar);
+        TmaLoad(sdst, &q.smap[tl.seg], sc0 & ~1, row, bar);
+        if (q.odd) TmaLoad(sdst + q.shalf, &q.smap[tl.seg], (sc0 + wpitch8) & ~1, row, bar);
+        sdst += q.box_rows * q.spitch;
+      }
+      dst += q.box_rows * q.pitch;
+      row += static_cast<int>(q.box_rows);
+    }
+  };
+  if (warp == q.warps) {
+    if (ElectOne()) {
+      for (int i = 0; i < p.stages; ++i) {
+        BarInit(full0 + i * 8, 1);
+        BarInit(empty0 + i * 8, q.team_warps);
+      }
+      BarInit(SmemAddr(&ctl.tail_full), 1);
+      ctl.fault = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      for (int s = 0; s < p.stages && s < nst; ++s) issue(s, s);
+      if constexpr (kTail) {
+        if (tail_index >= 0) {
+          const uint32_t bar = SmemAddr(&ctl.tail_full), dst = ring + q.tail_off, sdst = dst + q.tail_rows * q.tail_pitch;
+          const uint32_t hw = q.tail_rows / 2 * q.tail_pitch, hs = q.tail_rows / 2 * 16;
+          const int tx0 = tail_col >> 4, tsx = ((sg.n >> 1) + (tail_col >> 4)) >> 3, row = tail_first * 16;
+          BarExpect(bar, q.tail_tx);
+          if (q.odd) {  // even rows, odd rows
+            TmaLoad(dst, &q.tail_wmap, tx0, row >> 1, bar);
+            TmaLoad(dst + hw, &q.tail_wmap, (tx0 + wpitch8) & ~1, row >> 1, bar);
+            TmaLoad(sdst, &q.tail_smap, tsx & ~1, row >> 1, bar);
+            TmaLoad(sdst + hs, &q.tail_smap, (tsx + wpitch8) & ~1, row >> 1, bar);
+          } else {      // upper half, lower half
+            const int below = row + static_cast<int>(q.tail_rows / 2);
+            TmaLoad(dst, &q.tail_wmap, tx0, row, bar);
+            TmaLoad(dst + hw, &q.tail_wmap, tx0, below, bar);
+            TmaLoad(sdst, &q.tail_smap, tsx & ~1, row, bar);
+            TmaLoad(sdst + hs, &q.tail_smap, tsx & ~1, below, bar);
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+  const RowShare rs = ShareOf(q, warp);
+  // this thread's outputs: columns cb + 32 part + lane, ... of the tile
+  const int cper = tl.C > 1 ? q.rank_cols : p.wn * 8 * G::kColsPerThread, cb = tl.crank * cper;
+  const int share = min(cper, tl.n1 - tl.n0 - cb), first_n = tl.n0 + cb + rs.part * 32 + lane;
+  float first_scale = 1.f;
+  uint32_t first_routed = 0;
+  if constexpr (KIND != kHead) {
+    if (MODE != kBf16 && sg.w_scale != nullptr && first_n < tl.n1) first_scale = __ldg(sg.w_scale + first_n);
+  }
+  // weights do not depend on the predecessor kernel, x may be its output
+  if (p.pdl_wait) GridDependencyWait();
+  if constexpr (KIND == kShared) {
+    if (p.routed != nullptr && first_n < tl.n1 && rs.any && rs.row < p.M) first_routed = p.routed[static_cast<size_t>(rs.row) * sg.n + first_n];
+  }
+  uint16_t* const xs = reinterpret_cast<uint16_t*>(smem + q.x_off);
+  const int padded = nst * q.rows;
+  Stamp(p, 1);
+  bool slow;
+  if constexpr (KIND == kShared) {
+    slow = StageXShared<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
+  } else {
+    slow = StageXStream<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
+  }
+  Stamp(p, 2);
+
+  float acc[NM][4];
+#pragma unroll
+  for (int j = 0; j < NM; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+  const int team = (warp * q.team_inv) >> 16, part_k = (warp * q.wn_inv) >> 16, wn = warp - part_k * p.wn, wk = part_k - team * q.team_wk;
+  const bool consumer = warp < q.warps;
+  constexpr int kWarpCols = 8 * G::kColsPerThread;
+  // rows of x that do not exist read row 0; their sums are never stored
+  const uint32_t x_row = ring + q.x_off + static_cast<uint32_t>(((lane & 7) < p.M ? (lane & 7) : 0) * p.xpitch * 2 + ((lane >> 3) & 1) * 16);
+#ifdef QFG_PHASE_TIMES
+  long long waited = 0;
+#endif
+  QFG_CLOCK(loop_begin);
+
+  if (warp == q.warps) {
+    int slot = 0;
+    uint32_t parity = 0;
+    for (int s = p.stages; s < nst; ++s) {
+      if (!BarWait(empty0 + slot * 8, parity, ctl)) break;
+      if (ElectOne()) issue(s, slot);
+      __syncwarp();
+      if (++slot == p.stages) {
+        slot = 0;
+        parity ^= 1u;
+      }
+    }
+  } else if (consumer) {
+    // A warp without columns of its own (the last tile's) works on whatever its places hold; those sums are never stored.
+    const LaneRows r = RowsOf<MODE>(sg, tl.n0, wn, lane, q.odd, q.pitch, q.spitch, q.half, q.shalf, q.swizzle, static_cast<uint32_t>(q.rows));
+    // two k-steps of every stage, wk and wk + p.wk; ldmatrix takes x of the first for the lower half warp, of the second for the upper
+    const uint32_t w0 = r.w + static_cast<uint32_t>(wk) * r.step, w1 = w0 + r.d1, w2 = w0 + r.d2, w3 = w1 + r.d2;
+    const uint32_t s0 = q.scale_off + r.s + static_cast<uint32_t>(wk) * r.sstep, s1 = s0 + r.e1, s2 = s0 + r.e2, s3 = s1 + r.e2;
+    const uint32_t wstep = static_cast<uint32_t>(q.team_wk) * r.step, sstep = static_cast<uint32_t>(q.team_wk) * r.sstep;
+    const uint32_t first = static_cast<uint32_t>(team), teams = static_cast<uint32_t>(q.teams), stage_bytes = static_cast<uint32_t>(p.stage_bytes);
+    const uint32_t at_step = teams * stage_bytes, bar_step = teams * 8u, xstep = teams * static_cast<uint32_t>(q.team_wk) * 64u;
+    const uint32_t full_end = full0 + static_cast<uint32_t>(p.stages) * 8u;
+    uint32_t x_at = x_row + static_cast<uint32_t>(wk + (lane >> 4) * q.team_wk + team * 2 * q.team_wk) * 32u;
+    bool good = true;
+    auto load = [&](Raw<MODE>& raw, uint32_t w, uint32_t s) {
+      if constexpr (MODE == kNvfp4) {
+        raw.r[0][0] = Lds64(w0 + w);
+        raw.r[0][1] = Lds64(w1 + w);
+        raw.r[0][2] = Lds64(w2 + w);
+        raw.r[0][3] = Lds64(w3 + w);
+        raw.s[0][0] = Lds8(s0 + s);
+        raw.s[0][1] = Lds8(s1 + s);
+        raw.s[0][2] = Lds8(s2 + s);
+        raw.s[0][3] = Lds8(s3 + s);
+      } else {
+        raw.r[0] = Lds128(w0 + w);
+        raw.r[1] = Lds128(w1 + w);
+        raw.r[2] = Lds128(w2 + w);
+        raw.r[3] = Lds128(w3 + w);
+      }
+    };
+    auto k_loop = [&](auto slow_tag) {
+      constexpr bool kSlow = decltype(slow_tag)::value;
+      uint32_t parity = 0, at = ring + first * stage_bytes, bar = full0 + first * 8u;
+#pragma unroll 1
+      for (int left = nst - team; left > 0; left -= q.teams) {
+        QFG_CLOCK(c0);
+        if (!BarWait(bar, parity, ctl)) {
+          good = false;
+          break;
+        }
+        QFG_CLOCK(c1);
+        QFG_WAITED(c1 - c0);
+        Raw<MODE> ra, rb;
+        uint32_t xv[4];
+        load(ra, at, at);
+        LoadX2(x_at, xv);
+        load(rb, at + wstep, at + sstep);
+        __syncwarp();
+        if (lane == 0) BarArrive(bar + (empty0 - full0));  // the stage is read
+        ComputeStep<MODE, kSlow>(acc, ra, xv[0], xv[1]);
+        ComputeStep<MODE, kSlow>(acc, rb, xv[2], xv[3]);
+        x_at += xstep;
+        at += at_step;
+        bar += bar_step;
+        if (bar >= full_end) {  // the stages are a multiple of the teams: a slot always serves the same one, which sees its every phase
+          bar = full0 + first * 8u;
+          at = ring + first * stage_bytes;
+          parity ^= 1u;
+        }
+      }
+    };
+    if constexpr (MODE == kBf16) {
+      k_loop(std::false_type{});
+    } else {
+      if (slow) {
+        k_loop(std::true_type{});
+      } else {
+        k_loop(std::false_type{});
+      }
+    }
+    if (!good) {
+#pragma unroll
+      for (int j = 0; j < NM; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = __uint_as_float(0x7FFFFFFFu);
+    }
+  } else if constexpr (kTail) {
+    if (tail_index >= 0) {
+      const uint32_t hw = q.odd ? q.tail_rows / 2 * q.tail_pitch : 0, hs = q.odd ? q.tail_rows / 2 * 16 : 0;
+      const LaneRows r = RowsOf<MODE>(sg, tail_col, 0, lane, q.odd, q.tail_pitch, 16, hw, hs);
+      uint32_t w = ring + q.tail_off + r.w, sc = ring + q.tail_off + q.tail_rows * q.tail_pitch + r.s;
+      uint32_t x_at = x_row + static_cast<uint32_t>(tail_first + (lane >> 4)) * 32u;
+      const bool good = BarWait(SmemAddr(&ctl.tail_full), 0, ctl);
+#pragma unroll 1
+      for (int i = 0; i < tail_count && good; ++i) {
+        Raw<MODE> ra;
+        uint32_t xv[4];
+        LoadRows<MODE>(ra, r, w, sc);
+        LoadX2(x_at, xv);
+        if (slow) {
+          ComputeStep<MODE, true>(acc, ra, xv[0], xv[1]);
+        } else {
+          ComputeStep<MODE, false>(acc, ra, xv[0], xv[1]);
+        }
+        w += r.step;
+        sc += r.sstep;
+        x_at += 32;
+      }
+      float* const dst = p.lm_tail + static_cast<size_t>(tail_index) * kMaxRows * 128;
+      const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+      for (int j = 0; j < NM; ++j) {
+        const int cl = g * 16 + 2 * j, m0 = 2 * t, m1 = 2 * t + 1;
+        if (!good) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = __uint_as_float(0x7FFFFFFFu);
+        if (m0 < p.M) *reinterpret_cast<float2*>(&dst[m0 * 128 + cl]) = make_float2(acc[j][0], acc[j][2]);
+        if (m1 < p.M) *reinterpret_cast<float2*>(&dst[m1 * 128 + cl]) = make_float2(acc[j][1], acc[j][3]);
+      }
+      __threadfence();
+    }
+  }
+#ifdef QFG_PHASE_TIMES
+  if (p.phase_times != nullptr && tid == 0) {
+    unsigned long long* o = p.phase_times + (static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 16;
+    o[8] = waited;
+    o[9] = clock64() - loop_begin;
+  }
+#endif
+  Stamp(p, 3);
+  if (p.trigger == 2) GridLaunchDependents();
+  if (ctl.fault) __nanosleep(1000000);  // copies of a CTA that gave up may still be landing where the sums go now
+  __syncthreads();
+  if (consumer) StorePartials<MODE, 1>(p, tl, acc, smem, tl.n0 + wn * kWarpCols < tl.n1);
+  __syncthreads();
+  Stamp(p, 4);
+  if constexpr (KIND == kHead) {
+    EpilogueTail<MODE, false>(p, tl, smem, sh, p.wk, p.wn * kWarpCols);
+  } else {
+    FinishStream<MODE, KIND == kShared>(q, tl, smem, sh, rs, lane, cb, share, first_scale, first_routed);
+  }
+  Stamp(p, 5);
+}
+
+// ------------------------------------------------------------------------------ host
+constexpr int kStreamSmem = 232448 - static_cast<int>(sizeof(SharedScratch) + sizeof(StreamScratch) + sizeof(StreamCtl)) - 256;
+constexpr int kStreamPad = 1024;  // past the staged x: the tail warp's ldmatrix reads a k-step ahead
+
+struct StreamSetup {
+  cudaError_t status = cudaErrorNotReady;
+  int slots[9] = {};  // clusters of so many CTAs, one per SM, that are resident at once
+};
+StreamSetup g_stream;
+
+template <int MODE, int KIND>
+cudaError_t SetUpStream() {
+  return cudaFuncSetAttribute(SkinnyGemmStreamKernel<MODE, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+}
+
+template <int MODE>
+cudaError_t SetUpMode() {
+  cudaError_t err = SetUpStream<MODE, kPlain>();
+  if (err == cudaSuccess) err = SetUpStream<MODE, kShared>();
+  return err == cudaSuccess ? SetUpStream<MODE, kHead>() : err;
+}
+
+int StreamSlots(int cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, static_cast<unsigned>(cluster));
+  cfg.blockDim = dim3(static_cast<unsigned>(kStreamThreads));
+  cfg.dynamicSmemBytes = kStreamSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, SkinnyGemmStreamKernel<kBf16, kPlain>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = std::max(1, DeviceSmCount() * 8 / (10 * cluster));
+  }
+  return n;
+}
+
+// rows x row_bytes, in elements of eight bytes
+bool Encode8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, uint32_t box_bytes, int swizzle = 0) {
+  const cuuint64_t dims[2] = {row_bytes / 8, rows}, strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {box_bytes / 8, box_rows}, step[2] = {1, 1};
+  const TensorMapEncodeFn fn = TensorMapEncoder();
+  return fn != nullptr && fn(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int StreamGran(int mode) { return mode == kBf16 ? 8 : mode == kFp8 ? 16 : 128; }
+int StreamGranBytes(int mode) { return mode == kNvfp4 ? 64 : 16; }
+
+// The shared memory of a launch: a function of the plan and the rows of the call.
+struct StreamLayout {
+  int wn, pitch, spitch, swizzle, row_bytes, rows, stage, nstages, xpitch, red, tail_rows, tail_bytes, stages, ring;
+  size_t smem;
+};
+StreamLayout LayOut(int mode, bool odd, int K, const StreamPlan& plan, int m) {
+  StreamLayout l = {};
+  const int tile_bytes = plan.width * StreamGranBytes(mode);
+  l.wn = mode == kNvfp4 ? plan.width : (tile_bytes + 127) / 128;
+  l.swizzle = mode != kNvfp4 || odd ? 0 : tile_bytes % 128 == 0 ? 128 : tile_bytes == 64 ? 64 : 0;
+  l.pitch = l.swizzle > 0 ? l.swizzle : odd ? tile_bytes + 32 : (tile_bytes / 16 | 1) * 16;
+  l.row_bytes = l.swizzle > 0 ? tile_bytes : l.pitch;
+  if (mode == kNvfp4) l.spitch = (plan.width * 8 + 8 + 15) / 16 * 16;
+  l.rows = 32 * plan.wk;
+  l.stage = (l.rows * (l.row_bytes + l.spitch) + 1023) / 1024 * 1024;
+  const int ksteps = (K + 15) / 16;
+  l.nstages = (ksteps * 16 + l.rows - 1) / l.rows;
+  const int slice = (l.nstages + plan.cluster - 1) / plan.cluster * l.rows;
+  l.xpitch = (slice + 63) / 64 * 64 + 8;  // rows 16 bytes apart in the banks
+  const int cols = l.wn * GeomOf(mode).cols_per_warp;
+  l.red = (plan.wk * plan.teams + (plan.cluster > 1 ? 1 : 0)) * m * cols * 4;
+  if (plan.tail > 0) {
+    l.tail_rows = (ksteps + plan.tail_split - 1) / plan.tail_split * 16;
+    l.tail_bytes = (l.tail_rows * ((odd ? 96 : 80) + 16) + 127) / 128 * 128;
+  }
+  const int fixed = m * l.xpitch * 2 + kStreamPad + l.tail_bytes;
+  l.stages = std::min({kStreamStages, (kStreamSmem - 1024 - fixed) / l.stage, (l.nstages + plan.cluster - 1) / plan.cluster + plan.teams - 1});
+  // whole rounds of the teams; where the slice has fewer stages than that, the last teams have none
+  l.stages = std::max(l.stages / plan.teams, 1) * plan.teams;
+  l.ring = (std::max(l.stages * l.stage, l.red) + 127) / 128 * 128;
+  l.smem = static_cast<size_t>(l.ring) + fixed + 1024;
+  return l;
+}
+
+template <int MODE, int KIND>
+cudaError_t Launch(const StreamParams& q, int tiles, int threads, size_t smem, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(q.g.cluster), 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n_attr = 0;
+  if (q.g.cluster > 1) {
+    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attr].val.clusterDim.x = 1;
+    attr[n_attr].val.clusterDim.y = static_cast<unsigned>(q.g.cluster);
+    attr[n_attr].val.clusterDim.z = 1;
+    ++n_attr;
+  }
+  if (q.g.pdl_wait) {
+    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+    ++n_attr;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n_attr;
+  return cudaLaunchKernelEx(&cfg, SkinnyGemmStreamKernel<MODE, KIND>, q);
+}
+
+template <int MODE>
+cudaError_t LaunchMode(const StreamParams& q, int tiles, int threads, size_t smem, cudaStream_t stream) {
+  if (q.g.fuse) return Launch<MODE, kShared>(q, tiles, threads, smem, stream);
+  return q.g.lm ? Launch<MODE, kHead>(q, tiles, threads, smem, stream) : Launch<MODE, kPlain>(q, tiles, threads, smem, stream);
+}
+
+bool OddRows(int mode, const PlanInput& in) {
+  for (int s = 0; mode == kNvfp4 && s < in.nseg; ++s) {
+    if (in.n[s] % 256 != 0) return true;
+  }
+  return false;
+}
+
+}  // namespace
+
+cudaError_t ConfigureStreamKernels() {
+  cudaError_t err = SetUpMode<kBf16>();
+  if (err == cudaSuccess) err = SetUpMode<kFp8>();
+  if (err == cudaSuccess) err = SetUpMode<kNvfp4>();
+  for (int c = 1; err == cudaSuccess && c <= 8; ++c) g_stream.slots[c] = StreamSlots(c);
+  g_stream.status = err;
+  return err;
+}
+
+bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan) {
+  if (g_stream.status != cudaSuccess || plan->width < 1 || plan->wk < 1 || plan->teams < 1 || plan->cluster < 1 || plan->cluster > 8) return false;
+  if (in.K % 8 != 0 || in.K > (1 << 20) || in.row_align < (in.mode == kNvfp4 ? 8 : 16)) return false;
+  const int gran = StreamGran(in.mode);
+  const bool odd = OddRows(in.mode, in);
+  int tiles = 0;
+  if (plan->tail > 0) {
+    // every left-over group's K range in up to sixteen slices, one per CTA
+    if (!in.allow_tail || in.nseg != 1 || in.mode != kNvfp4 || plan->cluster != 1 || plan->tail > kMaxTailGroups || plan->tail >= in.n[0] / gran) return false;
+  }
+  for (int s = 0; s < in.nseg; ++s) {
+    if (in.n[s] % gran != 0) return false;
+    const int granules = in.n[s] / gran - plan->tail;
+    plan->tiles[s] = (granules + plan->width - 1) / plan->width;
+    tiles += plan->tiles[s];
+  }
+  if (plan->tail > 0) {
+    if (tiles < 2 * plan->tail) return false;
+    plan->tail_split = std::min(kMaxTailSplit, tiles / plan->tail);
+  }
+  const StreamLayout l = LayOut(in.mode, odd, in.K, *plan, kMaxRows);
+  if (l.wn * plan->wk * plan->teams > kStreamWarps || l.pitch > 2048 || l.smem > kStreamSmem || l.tail_rows > 512) return false;
+  // eight rows of x leave the ring room for the stages in use and as much on its way
+  return l.stages >= std::min(plan->teams + (l.stage < 40960 ? 2 : 1), (l.nstages + plan->cluster - 1) / plan->cluster);
+}
+
+// The cheapest launch shape by a model fitted to measured launches (one B200, one to eight rows, microseconds):
+//   the stream: all bytes at 6.0 TB/s, a ninth to a third more where tiles begin inside lines of 128 bytes; or a CTA's share
+//   at 14 ns per KB, or slower where its ring (at four rows) is less than two microseconds of that; a row and 128 columns
+//   of NVFP4 1.75 ns, its arithmetic (more where a tile is one group wide: two copied rows for 72 bytes, and few warps);
+//   around it: 2.2 (BF16) or 3.4 for launch, first copies, x and the epilogue; 1.9 more where ranks of a cluster add up;
+//   SharedExpertDown: swish_mul of the slice, which every CTA computes for itself.
+// Against other shapes: BF16 5120 x 5120 8 pieces wide, two teams of four warps, no cluster 11.1 (16 wide in clusters of three
+// 12.7, 5 wide 12.8); FP8 6144 x 2560 in clusters of four to six 8.1 (of two 10.1); NVFP4 17408 x 5120 two groups wide in
+// clusters of six 16.6 (one group, clusters of three 18.3); NVFP4 640 x 2560 in clusters of five 5.4 (none 6.4).
+StreamPlan ChooseStreamPlan(const PlanInput& in) {
+  StreamPlan best;
+  if (g_stream.status != cudaSuccess) return best;
+  const int gran = StreamGran(in.mode), ksteps = (in.K + 15) / 16;
+  const bool odd = OddRows(in.mode, in), fp4 = in.mode == kNvfp4;
+  // A vocabulary of at least four groups of 128 columns per SM and a few more: the head gives the few away in slices of K
+  // (GemmParams::tail_groups), the plain product takes a group more per CTA and adds up K in the same order.
+  if (in.nseg == 1 && fp4 && in.n[0] % gran == 0 && !in.fuse) {
+    const int slots = g_stream.slots[1], groups = in.n[0] / gran, per = groups / slots, rest = groups % slots;
+    if (per >= 4 && rest >= 1 && rest <= kMaxTailGroups && per < kStreamWarps) {
+      PlanInput head = in;
+      head.allow_tail = true;
+      StreamPlan with, without;
+      with.width = per;
+      without.width = per + 1;
+      with.wk = without.wk = 1;
+      with.teams = without.teams = std::min(3, kStreamWarps / (per + 1));
+      with.tail = rest;
+      if (CompleteStreamPlan(head, &with) && CompleteStreamPlan(in, &without)) return in.allow_tail ? with : without;
+    }
+  }
+  double best_cost = 1e30, total = 0;
+  for (int s = 0; s < in.nseg; ++s) total += static_cast<double>(in.K) * in.n[s] * (in.mode == kBf16 ? 2.0 : in.mode == kFp8 ? 1.0 : 0.5625);
+  for (int cluster = 1; cluster <= 8; ++cluster) {
+    const int slots = g_stream.slots[cluster], slice = (ksteps + cluster - 1) / cluster * 16;
+    const double around = (in.mode == kBf16 ? 2.2 : 3.4) + (cluster > 1 ? 1.7 + 0.1 * cluster : 0.0);
+    if (cluster > 1 && (ksteps < 8 * cluster || total / 6.0e6 + around >= best_cost)) break;
+    for (int width = fp4 ? 1 : 3; slots > 0 && width <= (fp4 ? kStreamWarps : 32); ++width) {
+      const double extra = fp4 || width % 8 == 0 ? 1.0 : 1.0 + 1.0 / width, all = total * extra / 6.0e6;
+      if (all + around >= best_cost) continue;
+      int tiles = 0;
+      for (int s = 0; s < in.nseg; ++s) tiles += (in.n[s] / gran + width - 1) / width;
+      const int waves = (tiles + slots - 1) / slots;
+      if (all + waves * around >= best_cost) continue;
+      StreamPlan p;
+      p.width = width;
+      p.cluster = cluster;
+      // eight warps along K (as two teams where the arithmetic of a stage is short), fewer where columns take them or K is short
+      const int wn = fp4 ? width : (width + 7) / 8;
+      if (wn == 1) {
+        p.wk = in.mode == kBf16 || in.fuse || slice < 1024 ? 4 : 8;
+        p.teams = in.fuse || (in.mode == kBf16 && slice >= 1024) || (fp4 && slice >= 2048) ? 2 : 1;
+      } else if (wn == 2) {
+        p.wk = 4;
+        p.teams = slice < 512 && !in.fuse ? 1 : 2;
+      } else {
+        p.wk = std::min(4, kStreamWarps / wn);
+      }
+      if (!CompleteStreamPlan(in, &p)) continue;
+      const StreamLayout l = LayOut(in.mode, odd, in.K, p, 4);
+      const double rows = static_cast<double>((l.nstages + cluster - 1) / cluster) * l.rows;
+      const double ring_kb = l.stages * l.stage / 1024.0;
+      double row_ns;
+      if (fp4) {
+        row_ns = wn > 1 ? 1.75 * wn : p.wk * p.teams >= 16 ? 2.05 : p.wk * p.teams >= 8 ? 2.3 : 4.5;
+      } else {
+        row_ns = std::max(1.5, width / 64.0 * (l.stages * cluster >= l.nstages ? 14.0 : std::max(14.0, 2000.0 / ring_kb)));
+      }
+      const double stream = std::max(all, waves * rows * row_ns * 1e-3);
+      const double cost = stream + waves * around + std::max(0.0, rows - 5120) * 4e-4 + (fp4 && wn > 1 && slice < 1024 ? 2.0 : 0.0) +
+                          (in.fuse ? rows * (in.mode == kBf16 ? 0.5e-3 : 3e-3) : 0);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = p;
+      }
+    }
+  }
+  return best;
+}
+
+std::string DescribeStreamPlan(const StreamPlan& p) {
+  char buf[96];
+  std::snprintf(buf, sizeof(buf), "stream=%d/%d/%d/%d/%d", p.width, p.wk, p.teams, p.cluster, p.tail);
+  return buf;
+}
+
+bool LaunchSkinnyStream(int mode, GemmParams& p, const StreamPlan& plan, cudaStream_t stream, cudaError_t* err) {
+  *err = CheckConfiguredDevice();
+  if (*err != cudaSuccess) return true;
+  if (reinterpret_cast<uintptr_t>(p.x) % 16 != 0) return false;
+  if (p.fuse && (p.gk % 8 != 0 || reinterpret_cast<uintptr_t>(p.x2) % 16 != 0 || reinterpret_cast<uintptr_t>(p.gx) % 16 != 0 || reinterpret_cast<uintptr_t>(p.gw) % 16 != 0))
+    return false;
+  StreamParams q;
+  bool odd = false;
+  for (int s = 0; s < p.nseg; ++s) odd = odd || (mode == kNvfp4 && p.seg[s].pitch % 16 != 0);
+  const StreamLayout l = LayOut(mode, odd, p.K, plan, p.M);
+  p.wn = l.wn;
+  p.wk = plan.wk * plan.teams;
+  p.cluster = plan.cluster;
+  p.gran = StreamGran(mode);
+  p.stages = l.stages;
+  p.stage_bytes = l.stage;
+  p.ring_bytes = l.ring;
+  p.xpitch = l.xpitch;
+  p.tail_groups = plan.tail;
+  p.tail_split = plan.tail_split;
+  int tiles = 0;
+  for (int s = 0; s < p.nseg; ++s) {
+    p.seg[s].tile_begin = tiles;
+    p.seg[s].tiles = plan.tiles[s];
+    p.seg[s].tail_cols = plan.tail * 128;
+    p.seg[s].granules = (p.seg[s].n - p.seg[s].tail_cols) / p.gran;
+    if (plan.tiles[s] < 1 || plan.tiles[s] > 65535) {
+      *err = cudaErrorInvalidValue;
+      return true;
+    }
+    p.seg[s].gran_quot = p.seg[s].granules / plan.tiles[s];
+    p.seg[s].gran_rem = p.seg[s].granules % plan.tiles[s];
+    tiles += plan.tiles[s];
+  }
+  p.tail_stride = plan.tail > 0 ? tiles / (plan.tail * plan.tail_split) : 0;
+  if (plan.tail > 0 && (!p.lm || p.lm_tail == nullptr || p.tail_stride < 1)) {
+    *err = cudaErrorInvalidValue;
+    return true;
+  }
+  const uint32_t div = odd ? 2 : 1;
+  q.boxes = (l.rows / static_cast<int>(div) + 255) / 256;
+  q.box_rows = static_cast<uint32_t>(l.rows / static_cast<int>(div) / q.boxes);  // rows are a multiple of 32, at most 512
+  for (int s = 0; s < p.nseg; ++s) {
+    const Segment& sg = p.seg[s];
+    const uint64_t rows = static_cast<uint64_t>(p.K) / div, row_bytes = static_cast<uint64_t>(sg.pitch) * div;
+    if (!Encode8(&q.wmap[s], sg.w, rows, row_bytes, q.box_rows, static_cast<uint32_t>(l.pitch), l.swizzle)) return false;
+    if (mode == kNvfp4 && !Encode8(&q.smap[s], sg.w, rows, row_bytes, q.box_rows, static_cast<uint32_t>(l.spitch))) return false;
+    if (plan.tail > 0) {
+      q.tail_pitch = odd ? 96 : 80;
+      if (!Encode8(&q.tail_wmap, sg.w, rows, row_bytes, static_cast<uint32_t>(l.tail_rows) / 2, q.tail_pitch) ||
+          !Encode8(&q.tail_smap, sg.w, rows, row_bytes, static_cast<uint32_t>(l.tail_rows) / 2, 16))
+        return false;
+      q.tail_rows = static_cast<uint32_t>(l.tail_rows);
+      q.tail_tx = q.tail_rows * (q.tail_pitch + 16);
+    }
+  }
+  q.g = p;
+  q.teams = plan.teams;
+  q.team_wk = plan.wk;
+  q.team_warps = l.wn * plan.wk;
+  q.team_inv = 65535 / q.team_warps + 1;
+  q.warps = q.team_warps * plan.teams;
+  q.rows = l.rows;
+  q.nstages = l.nstages;
+  q.odd = odd ? 1 : 0;
+  q.pitch = static_cast<uint32_t>(l.pitch);
+  q.spitch = static_cast<uint32_t>(l.spitch);
+  q.half = static_cast<uint32_t>(l.rows / 2 * l.pitch);
+  q.shalf = static_cast<uint32_t>(l.rows / 2 * l.spitch);
+  q.swizzle = l.swizzle;
+  q.col_boxes = l.swizzle > 0 ? l.row_bytes / l.swizzle : 1;
+  q.scale_off = static_cast<uint32_t>(l.rows * l.row_bytes);
+  q.tx = static_cast<uint32_t>(l.rows * (l.row_bytes + l.spitch));
+  q.x_off = static_cast<uint32_t>(l.ring + l.tail_bytes);
+  q.tail_off = static_cast<uint32_t>(l.ring);
+  q.wn_inv = 65535 / l.wn + 1;
+  q.row_warps = std::max(1, q.warps / p.M);
+  q.row_pass = q.warps / q.row_warps;
+  q.row_inv = 65535 / q.row_warps + 1;
+  q.rank_cols = (l.wn * GeomOf(mode).cols_per_warp + plan.cluster - 1) / plan.cluster;
+  const int threads = 32 * (q.warps + 1 + (plan.tail > 0 ? 1 : 0));
+  *err = mode == kBf16 ? LaunchMode<kBf16>(q, tiles, threads, l.smem, stream)
+         : mode == kFp8 ? LaunchMode<kFp8>(q, tiles, threads, l.smem, stream)
+                        : LaunchMode<kNvfp4>(q, tiles, threads, l.smem, stream);
+  return true;
+}
+
+}  // namespace qfg

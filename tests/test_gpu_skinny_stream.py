@@ -1,0 +1,136 @@
+"""The kernel that streams the weights by tensor copies (csrc/skinny_stream.cu) at the edges of its launch shapes, against
+the CPU oracle with the tolerances of test_gpu_skinny_gemm.py and test_gpu_shared_expert_down.py."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import bits, to_dev
+from oracle import oracle as O
+from qwen38_flash_ops_b200 import ArgmaxRows, LmHeadArgmax, QfgError, SharedExpertDown, SkinnyGemm
+from qwen38_flash_ops_b200 import packing as P
+
+import _util as U
+from test_gpu_shared_expert_down import _check, _inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _gemm(rng, mode, M, K, seg_widths, plan, x=None, force_slow=False):
+    """One call in the launch shape `plan`; the row-independent check of every output against the oracle."""
+    ns = [sum(w) for w in seg_widths]
+    x = P.synth_x(rng, M, K) if x is None else x
+    made = [U.make_weight(rng, mode, K, n, True) for n in ns]
+    scales = [s for _, s in made]
+    w_scale = np.concatenate(scales) if mode != 0 else None
+    op = SkinnyGemm([len(w) for w in seg_widths], [v for w in seg_widths for v in w], w_scale=w_scale)
+    weights = [U.dev_weight(a, mode) for a, _ in made]
+    xd = to_dev(x, "bf16")
+    op.set_option("stream_plan", plan)
+    if force_slow:
+        op.set_option("force_slow", 1)
+    outs = op(xd, *weights)
+    assert f"stream={plan.replace(',', '/')}/0" in op.describe(K, *weights)
+    torch.cuda.synchronize()
+    o = 0
+    for (arr, s), widths, n in zip(made, seg_widths, ns):
+        got = np.concatenate([bits(outs[o + j]).reshape(M, -1) for j in range(len(widths))], axis=1)
+        U.check_against_oracle(mode, x, arr, n, s if mode != 0 else None, got, K, f"mode{mode} M{M} K{K} {plan}")
+        o += len(widths)
+    return op, xd, weights, outs
+
+
+# width,wk,teams,cluster: one and many tiles, a last tile of one granule, warps without columns, more teams or ranks than
+# stages, a ring that wraps many times, stages of two boxes
+@pytest.mark.parametrize("mode,plan", [
+    (0, "3,4,1,1"), (0, "8,4,2,1"), (0, "9,2,2,3"), (0, "24,1,2,2"), (0, "8,8,2,1"), (0, "31,4,1,8"),
+    (1, "3,4,1,1"), (1, "8,8,1,1"), (1, "9,2,2,3"), (1, "24,1,2,2"), (1, "8,1,4,5"), (1, "17,4,1,8"),
+    (2, "1,4,1,1"), (2, "1,8,2,1"), (2, "2,4,2,3"), (2, "3,2,2,2"), (2, "9,1,2,1"), (2, "1,1,4,8"), (2, "1,9,1,1")])
+def test_launch_shapes(cuda, mode, plan):
+    rng = np.random.default_rng(1000 * mode + sum(map(ord, plan)))
+    # NVFP4 rows of a multiple of 16 bytes, and of an odd multiple of 8
+    cases = [(1, 2312, [[1280, 384]]), (5, 1000, [[512], [256, 256]]), (8, 72, [[256]])]
+    if mode == 2:
+        cases += [(3, 2312, [[640, 384], [896]]), (8, 136, [[384]]), (2, 8, [[128]])]
+    else:
+        cases += [(3, 2312, [[16 * 37]]), (8, 8, [[16], [48]])]
+    for M, K, segs in cases:
+        _gemm(rng, mode, M, K, segs, plan)
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_values_outside_the_fp16_range(cuda, mode):
+    """Rows whose magnitudes spread too far for FP16, and the forced BF16 path."""
+    rng = np.random.default_rng(mode)
+    x = P.synth_x(rng, 4, 520)
+    x[1, 3] = 0x7180   # 2^100: times 448, the largest E4M3 value, and a few thousand N(0, 1) terms still an FP32 number
+    x[2, 7] = 0x0080   # the smallest normal number
+    _gemm(rng, mode, 4, 520, [[256]], "1,4,2,1" if mode == 2 else "8,4,2,1", x=x)
+    _gemm(rng, mode, 4, 520, [[384]], "1,4,1,2" if mode == 2 else "8,4,1,2", force_slow=True)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("M", [1, 3, 8])
+def test_rows_are_independent_and_calls_agree(cuda, mode, M):
+    """The same bits in any company, and in every one of many calls (a ring slot read after it was written again would not
+    give them)."""
+    rng = np.random.default_rng(7 * mode + M)
+    plan = "2,2,2,2" if mode == 2 else "16,2,2,2"
+    op, x, weights, outs = _gemm(rng, mode, M, 5120, [[512, 256]], plan)
+    for m in range(M):
+        for one, all_rows in zip(op(x[m:m + 1].contiguous(), *weights), outs):
+            assert torch.equal(one[0], all_rows[m])
+    for _ in range(50):
+        for again, first in zip(op(x, *weights), outs):
+            assert torch.equal(again, first)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["1,4,2,1", "1,4,1,3", "2,1,4,1"])
+def test_shared_expert(cuda, mode, plan):
+    width, rest = plan.split(",", 1)
+    plan = plan if mode == 2 else f"{8 * int(width) - 1},{rest}"
+    rng = np.random.default_rng(mode + sum(map(ord, plan)))
+    for M, K, N, gk in [(1, 640, 256, 2560), (5, 296, 384, 8), (8, 1032, 128, 1000)]:
+        arr, s = U.make_weight(rng, mode, K, N, mode != 0)
+        g, u, gx, gw, routed = _inputs(rng, M, K, N, gk)
+        op = SharedExpertDown(w_scale=s if mode != 0 else None)
+        op.set_option("stream_plan", plan)
+        args = [to_dev(g, "bf16"), to_dev(u, "bf16"), U.dev_weight(arr, mode), to_dev(gx, "bf16"), to_dev(gw, "bf16"), to_dev(routed, "bf16")]
+        out = op(*args)
+        y, _, _, shared = O.shared_expert_down(g, u, mode, arr, N, gx, gw, routed, s if mode != 0 else None)
+        _check(bits(out), y, shared, O.bf16_to_f32(routed), f"mode {mode} M {M} {plan}")
+        for m in range(M):
+            row = [a[m:m + 1].contiguous() if a.shape[0] == M and i not in (2, 4) else a for i, a in enumerate(args)]
+            assert torch.equal(op(*row)[0], out[m])
+
+
+@pytest.mark.parametrize("groups", [33, 34])  # rows of 8 modulo 16 bytes, and of 0
+@pytest.mark.parametrize("tail", [1, 3])
+def test_head_tail(cuda, groups, tail):
+    """Left-over column groups in slices of K: the argmax of the kernel's own logits, which are the plain product's."""
+    rng = np.random.default_rng(groups + tail)
+    N, K, M = 128 * groups, 1032, 5
+    w = U.dev_weight(U.make_weight(rng, 2, K, N, False)[0], 2)
+    x = to_dev(P.synth_x(rng, M, K), "bf16")
+    head, plain = LmHeadArgmax(), SkinnyGemm([1], [N])
+    head.set_option("stream_plan", f"2,1,2,1,{tail}")
+    plain.set_option("stream_plan", "3,1,2,1")
+    for _ in range(3):
+        idx, val, _, logits = head(x, w, N, logits=True)
+        i, v = ArgmaxRows()(logits)
+        assert torch.equal(idx, i) and torch.equal(val, v)
+        ref = plain(x, w)[0]
+        main = N - 128 * tail
+        assert torch.equal(logits[:, :main], ref[:, :main])
+        # the tail's sums are FP32 in another order: one BF16 ULP, and K * 2^-24 of the magnitudes where they cancel
+        assert torch.allclose(logits.float(), ref.float(), rtol=2.0 ** -7, atol=K * 2.0 ** -24 * float(x.float().abs().sum(1).max()) * 0.2)
+
+
+def test_shapes_that_do_not_exist_are_refused(cuda):
+    w = U.dev_weight(U.make_weight(np.random.default_rng(0), 2, 64, 256, False)[0], 2)
+    x = to_dev(np.zeros((1, 64), np.uint16), "bf16")
+    for plan in ("1,19,1,1", "19,1,1,1", "0,1,1,1", "1,1,1,9", "1,1,0,1", "1,4", "1,4,1,1,1"):
+        op = SkinnyGemm([1], [256])
+        op.set_option("stream_plan", plan)
+        with pytest.raises(QfgError):
+            op(x, w)
