@@ -15,7 +15,7 @@ from ctypes import c_void_p
 
 import torch
 
-from . import _lib
+from . import _calls, _lib
 from ._lib import QfgError, Tensor2D, check
 
 _DTYPES = {
@@ -27,10 +27,26 @@ _DTYPES = {
 }
 
 
-# The host's part of a call is about as long as the smallest kernels (15.4 us for one SkinnyGemm before the lines below
-# were written with its time in mind, 10.6 after; 4.5 of them are the launch), so the per-call plumbing avoids what costs
-# microseconds: torch.cuda.current_stream() builds a Stream object (3.5 us; the raw handle 0.15), ctypes structures and
-# arrays are built field by field (1.6 us; one struct.pack 0.3).
+# The host's part of a call is longer than the smallest kernels, so a call of the ordinary form goes through csrc/calls.cc,
+# which does all of it in C++.  What that does not take (it returns None: a tensor subclass, a wrapped tensor, an argument
+# that is wrong) and the calls with outputs given take the Python code below, written with its time in mind as well:
+# torch.cuda.current_stream() builds a Stream object (3.5 us; the raw handle 0.15), ctypes structures and arrays are built
+# field by field (1.6 us; one struct.pack 0.3).
+_bound = False
+
+
+def _load():
+    """The library, its entry points handed to csrc/calls.cc."""
+    global _bound
+    lib = _lib.load()
+    if not _bound:
+        _calls.bind(*[ctypes.cast(getattr(lib, name), c_void_p).value
+                      for name in ("qfg_skinny_gemm_compute", "qfg_argmax_rows", "qfg_dequant_compute", "qfg_lmhead_compute",
+                                   "qfg_shared_expert_down_compute")])
+        _bound = True
+    return lib
+
+
 if hasattr(torch._C, "_cuda_getCurrentRawStream") and hasattr(torch._C, "_cuda_getDevice"):
     def _stream_ptr() -> int:
         return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
@@ -79,7 +95,7 @@ class SkinnyGemm:
     """
 
     def __init__(self, seg_outs, widths, w_scale=None, trigger: int = 0):
-        lib = _lib.load()
+        lib = _load()
         self._lib = lib
         self._h = c_void_p()
         so, wi = _lib.i64_array(seg_outs), _lib.i64_array(widths)
@@ -90,6 +106,7 @@ class SkinnyGemm:
             keep, ptr, n = None, None, 0
         check(lib.qfg_skinny_gemm_create(so, len(seg_outs), wi, len(widths), ptr, n, int(trigger),
                                          ctypes.byref(self._h)))
+        self._p = self._h.value
         self.seg_outs = [int(v) for v in seg_outs]
         self.widths = [int(v) for v in widths]
 
@@ -103,6 +120,10 @@ class SkinnyGemm:
         return buf.value.decode()
 
     def __call__(self, x: torch.Tensor, *weights: torch.Tensor, out=None):
+        if out is None:
+            r = _calls.skinny_gemm(self._p, x, weights, self.widths)
+            if r is not None:
+                return r if r.__class__ is list else check(r)
         _require_cuda(x, "x")
         if x.dtype != torch.bfloat16:
             raise QfgError(_lib.QFG_INVALID_ARGUMENT, "SkinnyGemm: x must be BF16")
@@ -131,10 +152,14 @@ class ArgmaxRows:
     optionally also the maximum as FP32.  The output rank is the input rank minus one."""
 
     def __init__(self):
-        self._lib = _lib.load()
+        self._lib = _load()
 
     def __call__(self, x: torch.Tensor, with_val: bool = True, out=None):
         """`out`: optional (idx, val) tensors to write into (val may be None)."""
+        if out is None:
+            r = _calls.argmax_rows(x, with_val)
+            if r is not None:
+                return r if r.__class__ is not int else check(r)
         _require_cuda(x, "x")
         if x.dtype not in (torch.bfloat16, torch.float16, torch.float32):
             raise QfgError(_lib.QFG_INVALID_ARGUMENT, "ArgmaxRows: logits must be BF16/FP16/FP32")
@@ -161,7 +186,7 @@ class DequantWeightBf16:
     The optional second input of the reference op is unused there and omitted here."""
 
     def __init__(self, n_cols: int, col_offset: int = 0, widths=None, w_scale=None):
-        lib = _lib.load()
+        lib = _load()
         self._lib = lib
         self._h = c_void_p()
         widths = list(widths) if widths else []
@@ -172,9 +197,14 @@ class DequantWeightBf16:
         else:
             keep, ptr, n = None, None, 0
         check(lib.qfg_dequant_create(int(n_cols), int(col_offset), wi, len(widths), ptr, n, ctypes.byref(self._h)))
+        self._p = self._h.value
         self.widths = widths if widths else [int(n_cols)]
 
     def __call__(self, w: torch.Tensor, out=None):
+        if out is None:
+            r = _calls.dequant(self._p, w, self.widths)
+            if r is not None:
+                return r if r.__class__ is list else check(r)
         t = _weight(w)
         outs = out if out is not None else [torch.empty((w.shape[0], wd), dtype=torch.bfloat16, device=w.device) for wd in self.widths]
         check(self._lib.packed.qfg_dequant_compute(self._h, t, _pointers(outs), len(outs), _stream_ptr()))
@@ -193,7 +223,7 @@ class SharedExpertDown:
     gx BF16 [..., gk]; gw BF16 [gk, 1]; routed BF16 [..., N].  Attributes: optional `w_scale`, `trigger`."""
 
     def __init__(self, w_scale=None, trigger: int = 0):
-        lib = _lib.load()
+        lib = _load()
         self._lib = lib
         self._h = c_void_p()
         if w_scale is not None and len(w_scale) > 0:
@@ -202,11 +232,15 @@ class SharedExpertDown:
         else:
             keep, ptr, n = None, None, 0
         check(lib.qfg_shared_expert_down_create(ptr, n, int(trigger), ctypes.byref(self._h)))
+        self._p = self._h.value
 
     def set_option(self, key: str, value) -> None:
         check(self._lib.qfg_shared_expert_down_set_option(self._h, key.encode(), str(value).encode()))
 
     def __call__(self, g, u, w, gx, gw, routed):
+        r = _calls.shared_expert_down(self._p, g, u, w, gx, gw, routed)
+        if r is not None:
+            return r if r.__class__ is not int else check(r)
         for name, t in (("g", g), ("u", u), ("gx", gx), ("gw", gw), ("routed", routed)):
             if not t.is_cuda or not t.is_contiguous():
                 _require_cuda(t, name)
@@ -243,7 +277,7 @@ class UntileHcBf16:
     input of the reference op only ties buffer lifetimes and is omitted here."""
 
     def __init__(self, kind: int, w_scale=None):
-        lib = _lib.load()
+        lib = _load()
         self._lib = lib
         self._h = c_void_p()
         self.kind = int(kind)
@@ -281,7 +315,7 @@ class LmHeadArgmax:
     """
 
     def __init__(self, w_scale=None, trigger: int = 0, device="cuda"):
-        lib = _lib.load()
+        lib = _load()
         self._lib = lib
         self._h = c_void_p()
         if w_scale is not None and len(w_scale) > 0:
@@ -290,6 +324,7 @@ class LmHeadArgmax:
         else:
             keep, ptr, n = None, None, 0
         check(lib.qfg_lmhead_create(ptr, n, int(trigger), ctypes.byref(self._h)))
+        self._p = self._h.value
         self.workspace = torch.zeros(lib.qfg_lmhead_workspace_bytes(), dtype=torch.uint8, device=device)
 
     def set_option(self, key: str, value) -> None:
@@ -297,6 +332,10 @@ class LmHeadArgmax:
 
     def __call__(self, x: torch.Tensor, w: torch.Tensor, n: int, col_offset: int = 0, logits: bool = False,
                  out=None):
+        if out is None and not logits:
+            r = _calls.lmhead(self._p, self.workspace, x, w, n, col_offset)
+            if r is not None:
+                return r if r.__class__ is not int else check(r)
         _require_cuda(x, "x")
         if x.dtype != torch.bfloat16:
             raise QfgError(_lib.QFG_INVALID_ARGUMENT, "LmHead: x must be BF16")
