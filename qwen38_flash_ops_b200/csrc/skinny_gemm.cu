@@ -7,7 +7,9 @@
 // scales) and issues m16n8k16 MMAs with the weights as the 16-row operand and x (padded to 8 rows)
 // as the 8-column operand.  Every weight and every product is exact; accumulation is FP32.
 //
-// Two kernels share that arithmetic and differ in how the weight bytes reach the registers:
+// Calls whose rows tensor copies can fetch go to skinny_stream.cu; these kernels take the rest (K not a multiple of eight, x
+// off 16 bytes, rows off 16 bytes or NVFP4 widths off 128) and launch shapes pinned with the `plan` option.  Two of them share
+// that arithmetic and differ in how the weight bytes reach the registers:
 //   * SkinnyGemmDirectKernel (the fast path): every warp streams its own rows from HBM into a
 //     warp-private shared-memory ring with lane-private cp.async copies, `depth` k-steps ahead of
 //     the MMAs.  No CTA barrier in the K loop; the bytes in flight per SM are warps x depth x
