@@ -1,0 +1,60 @@
+"""Which kernel a call of few rows goes to (csrc/capi.cc, csrc/skinny_stream.cu), against the CUDA runtime that runs nothing
+and records every launch (fake_cuda.c)."""
+import pytest
+
+from test_many_row_host_cpu import fake  # noqa: F401  (a fixture)
+
+
+def _kernel(log):
+    return [next((k for k in ("SkinnyGemmStreamKernel", "SkinnyGemm") if k in line), line.split()[0]) for line in log]
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+def test_routes(fake, dtype):  # noqa: F811
+    """Copies need rows of 16 bytes (NVFP4: 8) and K in eights; a pinned geometry, and a map that cannot be made, are the
+    general kernels'."""
+    narrow = 192 if dtype == "U8" else 264 if dtype == "FP8" else 260
+    out = fake(f"""
+        h = gemm([1], [256])
+        r = [run_gemm(h, {dtype}, m, 512, [[256]]) for m in (1, 8)]
+        r += [run_gemm(h, {dtype}, 2, 516, [[256]]), run_gemm(gemm([1], [{narrow}]), {dtype}, 2, 512, [[{narrow}]]),
+              run_gemm(gemm([1], [256], plan="wn=1,wk=2,cluster=1"), {dtype}, 2, 512, [[256]]),
+              run_gemm(gemm([1], [256], stream_plan="0"), {dtype}, 2, 512, [[256]])]
+        fake.fake_refuse_encode(1)
+        r.append(run_gemm(h, {dtype}, 2, 512, [[256]]))
+        fake.fake_refuse_encode(0)
+        os.environ["QFG_PLAN"] = "wn=1,wk=2,cluster=1"
+        r.append(run_gemm(gemm([1], [256]), {dtype}, 2, 512, [[256]]))
+        print(json.dumps(r))
+        """)
+    for code, message, _ in out:
+        assert code == 0, message
+    assert [_kernel(log) for _, _, log in out] == [["SkinnyGemmStreamKernel"]] * 2 + [["SkinnyGemm"]] * 6
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+def test_shared_expert_in_passes_of_eight(fake, dtype):  # noqa: F811
+    out = fake(f"""
+        s = shared(pdl_wait=1)
+        calls = fake.fake_setup_calls()
+        fake.fake_refuse_setup(1)
+        r = [run_shared(s, {dtype}, m, 256, 128) for m in (3, 16)]
+        fake.fake_device(1)
+        print(json.dumps([r, run_shared(s, {dtype}, 3, 256, 128), calls == fake.fake_setup_calls()]))
+        """)
+    (few, two_passes), other_device, no_setup = out
+    assert few[0] == two_passes[0] == 0 and no_setup
+    assert _kernel(few[2]) == ["SkinnyGemmStreamKernel"] and _kernel(two_passes[2]) == ["SkinnyGemmStreamKernel"] * 2
+    assert all(line.endswith("pdl=1") for line in few[2] + two_passes[2])
+    assert other_device[0] != 0
+
+
+@pytest.mark.parametrize("resident,clusters", [(132, True), (1, False)])
+def test_clusters_that_the_device_holds(fake, resident, clusters):  # noqa: F811
+    # K short enough for eight rows of x in one CTA (16384 would take 256 KB): without clusters the kernel is still the one
+    out = fake(f"""
+        fake.fake_resident({resident})
+        print(json.dumps(run_gemm(gemm([1], [256]), FP8, 4, 8192, [[256]])))
+        """)
+    assert out[0] == 0 and _kernel(out[2]) == ["SkinnyGemmStreamKernel"]
+    assert (" cluster=1 " not in out[2][0]) == clusters, out[2]
