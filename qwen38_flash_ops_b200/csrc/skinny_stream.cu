@@ -61,7 +61,7 @@ struct StreamParams {
 };
 
 struct StreamCtl {
-  unsigned long long full[kStreamStages], empty[kStreamStages], tail_full;
+  unsigned long long full[kStreamStages], empty[kStreamStages], tail_full, x_full;
   volatile uint32_t fault;
 };
 
@@ -88,6 +88,10 @@ __device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, in
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
                "r"(bar), "r"(x), "r"(y)
                : "memory");
+}
+// `bytes` contiguous bytes, a multiple of sixteen, from and to sixteen-byte boundaries
+__device__ __forceinline__ void BulkLoad(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ bool ElectOne() {
   uint32_t yes;
@@ -179,13 +183,23 @@ __device__ __forceinline__ RowShare ShareOf(const StreamParams& q, int warp) {
 
 // x of the slice to shared memory, rows padded with zeros to whole stages (so that the K loop needs no end), for the
 // quantised modes scaled by a power of two and converted to FP16 (skinny_common.cuh).  A thread converts what it stored
-// itself, so that the whole takes two barriers and one trip to L2.  Returns true if the CTA must take the BF16 path.
-template <int MODE>
-__device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, int padded,
-                                             const RowShare& rs, int lane) {
+// or looked at itself, so that the whole takes two barriers and one trip to L2.  BULK: the producer has the rows copied, and
+// they are only waited for; that gave the LM head 3 us of 85 at four rows and cost calls of 5 to 17 us 0.3 us, so only the
+// head does it.  Returns true if the CTA must take the BF16 path.
+template <int MODE, bool BULK>
+__device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, StreamCtl& ctl,
+                                             int padded, const RowShare& rs, int lane) {
   const GemmParams& p = q.g;
   constexpr int kBatch = 4;
   const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // K is a multiple of eight
+  auto track = [&](const uint4& v, uint32_t& mx, uint32_t& mn) {
+    if constexpr (MODE != kBf16) {
+      TrackPair(v.x, mx, mn);
+      TrackPair(v.y, mx, mn);
+      TrackPair(v.z, mx, mn);
+      TrackPair(v.w, mx, mn);
+    }
+  };
   auto copy = [&](int m, uint32_t& mx, uint32_t& mn) {
     const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + tl.kbeg);
     uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
@@ -197,19 +211,28 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
 #pragma unroll
       for (int i = 0; i < kBatch; ++i) {
         if (c + i * step < chunks) dst[c + i * step] = v[i];
-        if constexpr (MODE != kBf16) {
-          TrackPair(v[i].x, mx, mn);
-          TrackPair(v[i].y, mx, mn);
-          TrackPair(v[i].z, mx, mn);
-          TrackPair(v[i].w, mx, mn);
-        }
+        track(v[i], mx, mn);
       }
     }
   };
+  // (copies that never came: the K loop gives up like this wait, and its sums become NaN)
+  if constexpr (BULK) BarWait(SmemAddr(&ctl.x_full), 0, ctl);
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
     uint32_t mx = 0, mn = 0xFFFFFFFFu;
-    copy(m, mx, mn);
+    if constexpr (BULK) {
+      uint4* row = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 4
+      for (int c = c_first; c < chunks; c += step) {
+        if (c >= valid) {
+          row[c] = make_uint4(0, 0, 0, 0);
+        } else {
+          track(row[c], mx, mn);
+        }
+      }
+    } else {
+      copy(m, mx, mn);
+    }
     if constexpr (MODE != kBf16) {
       mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
       mn = __reduce_min_sync(0xffffffffu, min(mn & 0xFFFFu, mn >> 16));
@@ -219,7 +242,7 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       }
     }
   }
-  __syncthreads();  // every warp also sees the mbarriers
+  __syncthreads();  // without BULK: every warp also sees the mbarriers
   if constexpr (MODE == kBf16) {
     if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = 1.f;  // for the epilogue, behind further barriers
     return false;
@@ -444,7 +467,7 @@ template <int MODE, int KIND>
 __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(const __grid_constant__ StreamParams q) {
   using G = Geom<MODE>;
   constexpr int NM = G::kMmas;
-  constexpr bool kTail = MODE == kNvfp4 && KIND == kHead;
+  constexpr bool kTail = MODE == kNvfp4 && KIND == kHead, kBulkX = KIND == kHead;
   extern __shared__ uint8_t smem_raw[];
   __shared__ SharedScratch sh;
   __shared__ StreamScratch sx;
@@ -504,8 +527,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
       row += static_cast<int>(q.box_rows);
     }
   };
+  const uint32_t x_smem = ring + q.x_off, x_full = SmemAddr(&ctl.x_full);
+  auto issue_x = [&]() {  // one lane
+    const uint32_t bytes = static_cast<uint32_t>(tl.kslice) * 2u;
+    BarExpect(x_full, bytes * static_cast<uint32_t>(p.M));
+#pragma unroll 1
+    for (int m = 0; m < p.M && bytes > 0; ++m)
+      BulkLoad(x_smem + static_cast<uint32_t>(m * p.xpitch) * 2u, p.x + static_cast<size_t>(m) * p.K + tl.kbeg, bytes, x_full);
+  };
   if (warp == q.warps) {
     if (ElectOne()) {
+      if (kBulkX) BarInit(x_full, 1);
       for (int i = 0; i < p.stages; ++i) {
         BarInit(full0 + i * 8, 1);
         BarInit(empty0 + i * 8, q.team_warps);
@@ -513,6 +545,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
       BarInit(SmemAddr(&ctl.tail_full), 1);
       ctl.fault = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (kBulkX) asm volatile("bar.arrive 1, %0;" ::"r"(static_cast<int>(blockDim.x)) : "memory");  // the others may wait on the barriers
+    if (ElectOne()) {
+      // x before the weights, so that it does not queue behind them - unless it is still the predecessor kernel's to write
+      if (kBulkX && !p.pdl_wait) issue_x();
       for (int s = 0; s < p.stages && s < nst; ++s) issue(s, s);
       if constexpr (kTail) {
         if (tail_index >= 0) {
@@ -547,7 +585,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
     if (MODE != kBf16 && sg.w_scale != nullptr && first_n < tl.n1) first_scale = __ldg(sg.w_scale + first_n);
   }
   // weights do not depend on the predecessor kernel, x may be its output
-  if (p.pdl_wait) GridDependencyWait();
+  if (p.pdl_wait) {
+    GridDependencyWait();
+    if (kBulkX && warp == q.warps) {
+      if (ElectOne()) issue_x();
+      __syncwarp();
+    }
+  }
   if constexpr (KIND == kShared) {
     if (p.routed != nullptr && first_n < tl.n1 && rs.any && rs.row < p.M) first_routed = p.routed[static_cast<size_t>(rs.row) * sg.n + first_n];
   }
@@ -558,7 +602,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   if constexpr (KIND == kShared) {
     slow = StageXShared<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
   } else {
-    slow = StageXStream<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
+    if (kBulkX && warp != q.warps) asm volatile("bar.sync 1, %0;" ::"r"(static_cast<int>(blockDim.x)) : "memory");
+    slow = StageXStream<MODE, kBulkX>(q, tl, xs, sh, sx, ctl, padded, rs, lane);
   }
   Stamp(p, 2);
 
