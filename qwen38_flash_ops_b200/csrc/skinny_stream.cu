@@ -821,7 +821,7 @@ int StreamGranBytes(int mode) { return mode == kNvfp4 ? 64 : 16; }
 
 // The shared memory of a launch: a function of the plan and the rows of the call.
 struct StreamLayout {
-  int wn, pitch, spitch, swizzle, row_bytes, rows, stage, nstages, xpitch, red, tail_rows, tail_bytes, stages, ring;
+  int wn, pitch, spitch, swizzle, row_bytes, rows, boxes, box_rows, stage, nstages, xpitch, red, tail_rows, tail_bytes, stages, ring;
   size_t smem;
 };
 StreamLayout LayOut(int mode, bool odd, int K, const StreamPlan& plan, int m) {
@@ -833,6 +833,9 @@ StreamLayout LayOut(int mode, bool odd, int K, const StreamPlan& plan, int m) {
   l.row_bytes = l.swizzle > 0 ? tile_bytes : l.pitch;
   if (mode == kNvfp4) l.spitch = (plan.width * 8 + 8 + 15) / 16 * 16;
   l.rows = 32 * plan.wk;
+  const int box_all = odd ? l.rows / 2 : l.rows;
+  l.boxes = (box_all + 255) / 256;
+  l.box_rows = box_all / l.boxes;
   l.stage = (l.rows * (l.row_bytes + l.spitch) + 1023) / 1024 * 1024;
   const int ksteps = (K + 15) / 16;
   l.nstages = (ksteps * 16 + l.rows - 1) / l.rows;
@@ -925,6 +928,8 @@ bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan) {
   }
   const StreamLayout l = LayOut(in.mode, odd, in.K, *plan, kMaxRows);
   if (l.wn * plan->wk * plan->teams > kStreamWarps || l.pitch > 2048 || l.smem > kStreamSmem || l.tail_rows > 512) return false;
+  // the boxes make up the stage (17 warps along K: 544 rows are not three boxes), each on the 128 bytes that a copy begins on
+  if (l.boxes * l.box_rows != (odd ? l.rows / 2 : l.rows) || l.box_rows % 8 != 0) return false;
   // eight rows of x leave the ring room for the stages in use and as much on its way
   return l.stages >= std::min(plan->teams + (l.stage < 40960 ? 2 : 1), (l.nstages + plan->cluster - 1) / plan->cluster);
 }
@@ -1054,8 +1059,8 @@ bool LaunchSkinnyStream(int mode, GemmParams& p, const StreamPlan& plan, cudaStr
     return true;
   }
   const uint32_t div = odd ? 2 : 1;
-  q.boxes = (l.rows / static_cast<int>(div) + 255) / 256;
-  q.box_rows = static_cast<uint32_t>(l.rows / static_cast<int>(div) / q.boxes);  // rows are a multiple of 32, at most 512
+  q.boxes = l.boxes;
+  q.box_rows = static_cast<uint32_t>(l.box_rows);
   for (int s = 0; s < p.nseg; ++s) {
     const Segment& sg = p.seg[s];
     const uint64_t rows = static_cast<uint64_t>(p.K) / div, row_bytes = static_cast<uint64_t>(sg.pitch) * div;

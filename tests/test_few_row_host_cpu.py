@@ -58,3 +58,18 @@ def test_clusters_that_the_device_holds(fake, resident, clusters):  # noqa: F811
         """)
     assert out[0] == 0 and _kernel(out[2]) == ["SkinnyGemmStreamKernel"]
     assert (" cluster=1 " not in out[2][0]) == clusters, out[2]
+
+
+@pytest.mark.parametrize("dtype,n", [("BF16", 256), ("FP8", 256), ("U8", 256), ("U8", 128)])
+def test_a_stage_is_made_of_whole_boxes(fake, dtype, n):  # noqa: F811
+    """A box has at most 256 rows and begins on 128 bytes.  17 warps along K make 544 rows, which three boxes are not; where rows
+    are copied in pairs (NVFP4, N an odd multiple of 128) they are two boxes of 136 of either kind."""
+    width = 1 if dtype == "U8" else 3
+    out = fake(f"""
+        print(json.dumps([run_gemm(gemm([1], [{n}], stream_plan="{width},%d,1,1" % wk), {dtype}, 1, 4096, [[{n}]]) for wk in range(1, 19)]))
+        """)
+    for wk, (code, message, log) in enumerate(out, 1):
+        if wk == 17 and n == 256:
+            assert code != 0 and "stream_plan" in message and log == []
+        else:
+            assert code == 0 and _kernel(log) == ["SkinnyGemmStreamKernel"], (wk, message)
