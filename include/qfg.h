@@ -224,6 +224,9 @@ QFG_API size_t qfg_lmhead_static_max_rows(void);
 QFG_API int qfg_lmhead_compute_static(const qfg_lmhead* op, const void* x, int64_t m, int64_t k,
                                       const qfg_tensor2d* weight, int64_t n, int64_t col_offset, int64_t* idx,
                                       float* val, uint64_t* key, void* logits, void* stream);
+/* The launch options of qfg_skinny_gemm_set_option for this node, "exchange_spin" (below), and "x_spin": the tries after which
+ * a CTA stops waiting for its copy of x (default 1048576, each suspended by the hardware for a while).  A CTA that stops
+ * waiting writes NaN for its columns, so the row's winner is a NaN; the call itself succeeds and the next one is whole. */
 QFG_API int qfg_lmhead_set_option(qfg_lmhead* op, const char* key, const char* value);
 QFG_API void qfg_lmhead_destroy(qfg_lmhead* op);
 

@@ -112,6 +112,7 @@ struct Segment {
   int svec = 4;   // cp.async width for the NVFP4 scale bytes of a row
 };
 
+constexpr int kStreamSpin = 1 << 20;  // skinny_stream.cu: bound of a wait (tries that the hardware suspends for a while)
 constexpr int kExchangeSpin = 1 << 22;  // default bound of the wait for a peer's words (iterations of about 50 ns)
 
 struct GemmParams {
@@ -155,6 +156,7 @@ struct GemmParams {
   int tail_split = 1;
   int tail_stride = 0;
   float* lm_tail = nullptr;
+  int x_spin = kStreamSpin;  // skinny_stream.cu: bound of the wait for the copies of x
 
   // SharedExpertDown (fuse != 0): x is replaced by swish_mul(x, x2) while it is staged, and the output is
   // routed + bf16(bf16(sum) * gate[m]) with gate[m] = bf16(sigmoid(bf16(dot(gx[m], gw)))).

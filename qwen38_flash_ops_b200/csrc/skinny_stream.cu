@@ -18,7 +18,7 @@
 // of the tensor map, a stage holds R / 2 even rows and R / 2 odd rows, the latter copied from the 16-byte boundary before
 // them, and `pitch` is 32 or 96 modulo 128.
 //
-// Every wait is bounded; a CTA that gives up on one writes NaN.
+// Every wait is bounded; a CTA that gives up on one writes NaN, once its copies in flight have landed.
 #include <cuda.h>
 
 #include <algorithm>
@@ -38,7 +38,6 @@ namespace {
 constexpr int kStreamWarps = 18;                             // consumers, at most
 constexpr int kStreamThreads = 32 * (kStreamWarps + 2);      // and the producer, and the LM head's tail warp
 constexpr int kStreamStages = 24;
-constexpr int kStreamSpin = 1 << 20;
 
 struct StreamParams {
   GemmParams g;
@@ -72,16 +71,25 @@ __device__ __forceinline__ void BarArrive(uint32_t a) {
 __device__ __forceinline__ void BarExpect(uint32_t a, uint32_t bytes) {
   asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes) : "memory");
 }
-// false once a wait of this CTA ran out
-__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& c) {
-  for (int i = 0; i < kStreamSpin; ++i) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-    if (ok) return true;
+__device__ __forceinline__ bool BarTry(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+  return ok != 0;
+}
+// False if the wait ran out, or spun while another wait of this CTA had.  True says nothing of the other waits: a copy that has
+// landed is taken whatever became of the rest.
+__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& c, int spin = kStreamSpin) {
+  for (int i = 0; i < spin; ++i) {
+    if (BarTry(a, parity)) return true;
     if ((i & 255) == 255 && c.fault) return false;
   }
   c.fault = 1;
   return false;
+}
+// The last thing a CTA that gave up waits for: what it asked for must not arrive in shared memory that is used again.
+__device__ __noinline__ void BarDrain(uint32_t a, uint32_t parity) {
+  for (int i = 0; i < kStreamSpin && !BarTry(a, parity); ++i) {
+  }
 }
 // x in elements of eight bytes, an even number: a copy starts on 16 bytes
 __device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -215,8 +223,8 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       }
     }
   };
-  // (copies that never came: the K loop gives up like this wait, and its sums become NaN)
-  if constexpr (BULK) BarWait(SmemAddr(&ctl.x_full), 0, ctl);
+  // (copies that never came: ctl.fault makes NaN of the sums, wherever the weights have come)
+  if constexpr (BULK) BarWait(SmemAddr(&ctl.x_full), 0, ctl, p.x_spin);
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
     uint32_t mx = 0, mn = 0xFFFFFFFFu;
@@ -622,12 +630,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
 #endif
   QFG_CLOCK(loop_begin);
 
+  int issued = min(p.stages, nst);  // by the producer
   if (warp == q.warps) {
     int slot = 0;
     uint32_t parity = 0;
-    for (int s = p.stages; s < nst; ++s) {
+    for (; issued < nst; ++issued) {
       if (!BarWait(empty0 + slot * 8, parity, ctl)) break;
-      if (ElectOne()) issue(s, slot);
+      if (ElectOne()) issue(issued, slot);
       __syncwarp();
       if (++slot == p.stages) {
         slot = 0;
@@ -703,7 +712,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         k_loop(std::false_type{});
       }
     }
-    if (!good) {
+    if (!good || (kBulkX && ctl.fault)) {  // a wait for x that ran out came before the barriers of the staging
 #pragma unroll
       for (int j = 0; j < NM; ++j)
 #pragma unroll
@@ -731,12 +740,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         sc += r.sstep;
         x_at += 32;
       }
+      const bool sound = good && !ctl.fault;
       float* const dst = p.lm_tail + static_cast<size_t>(tail_index) * kMaxRows * 128;
       const int g = lane >> 2, t = lane & 3;
 #pragma unroll
       for (int j = 0; j < NM; ++j) {
         const int cl = g * 16 + 2 * j, m0 = 2 * t, m1 = 2 * t + 1;
-        if (!good) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = __uint_as_float(0x7FFFFFFFu);
+        if (!sound) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = __uint_as_float(0x7FFFFFFFu);
         if (m0 < p.M) *reinterpret_cast<float2*>(&dst[m0 * 128 + cl]) = make_float2(acc[j][0], acc[j][2]);
         if (m1 < p.M) *reinterpret_cast<float2*>(&dst[m1 * 128 + cl]) = make_float2(acc[j][1], acc[j][3]);
       }
@@ -752,8 +762,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
 #endif
   Stamp(p, 3);
   if (p.trigger == 2) GridLaunchDependents();
-  if (ctl.fault) __nanosleep(1000000);  // copies of a CTA that gave up may still be landing where the sums go now
   __syncthreads();
+  if (ctl.fault) {  // behind the barrier: the same for every thread
+    if (warp == q.warps) {
+      for (int s = max(0, issued - p.stages); s < issued; ++s) BarDrain(full0 + (s % p.stages) * 8, (s / p.stages) & 1);
+      if (kBulkX) BarDrain(x_full, 0);
+      if (kTail && tail_index >= 0) BarDrain(SmemAddr(&ctl.tail_full), 0);
+    }
+    __syncthreads();
+  }
   if (consumer) StorePartials<MODE, 1>(p, tl, acc, smem, tl.n0 + wn * kWarpCols < tl.n1);
   __syncthreads();
   Stamp(p, 4);
