@@ -1417,7 +1417,8 @@ cudaError_t ConfigureSkinnyGemmKernels() {
     if (status == cudaSuccess) status = ConfigureKernel(SkinnyGemmRingKernel<kBf16>);
     if (status == cudaSuccess) status = ConfigureKernel(SkinnyGemmRingKernel<kFp8>);
     if (status == cudaSuccess) status = ConfigureKernel(SkinnyGemmRingKernel<kNvfp4>);
-    if (status == cudaSuccess) status = ConfigureStreamKernels();
+    // without the kernel of skinny_stream.cu every call is these kernels'
+    if (status == cudaSuccess && ConfigureStreamKernels() != cudaSuccess) cudaGetLastError();
   });
   return status;
 }

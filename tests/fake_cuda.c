@@ -17,6 +17,8 @@ static size_t g_len;
 
 API void fake_device(int d) { g_device = d; }
 API void fake_refuse_setup(int v) { g_refuse_setup = v; }
+static char g_refuse_kernel[64];
+API void fake_refuse_setup_of(const char* part) { snprintf(g_refuse_kernel, sizeof g_refuse_kernel, "%s", part); }  /* kernels named so */
 API void fake_refuse_encode(int v) { g_refuse_encode = v; }
 API void fake_resident(int ctas) { g_resident = ctas; }  /* CTAs, one per SM, that clusters can have at once */
 API int fake_setup_calls(void) { return g_setup_calls; }
@@ -49,6 +51,7 @@ API void __cudaRegisterFunction(void** h, const char* host, char* dev, const cha
 static cudaError_t setup(void) { ++g_setup_calls; return g_refuse_setup ? cudaErrorStreamCaptureUnsupported : cudaSuccess; }
 API cudaError_t cudaFuncSetAttribute(const void* fn, enum cudaFuncAttribute a, int v) {
   if (setup() != cudaSuccess) return cudaErrorStreamCaptureUnsupported;
+  if (g_refuse_kernel[0] && strstr(name_of(fn), g_refuse_kernel)) return cudaErrorInvalidValue;
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize && n_attr < MAX) {
     g_attr[n_attr].fn = fn; g_attr[n_attr].device = g_device; g_attr[n_attr++].value = v;
   }

@@ -73,3 +73,16 @@ def test_a_stage_is_made_of_whole_boxes(fake, dtype, n):  # noqa: F811
             assert code != 0 and "stream_plan" in message and log == []
         else:
             assert code == 0 and _kernel(log) == ["SkinnyGemmStreamKernel"], (wk, message)
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+def test_a_device_that_refuses_the_kernel(fake, dtype):  # noqa: F811
+    """Its shared-memory limit could not be raised: nodes are made, and their calls are the general kernels'."""
+    out = fake(f"""
+        fake.fake_refuse_setup_of(b"SkinnyGemmStreamKernel")
+        r = [run_gemm(gemm([1], [256]), {dtype}, 2, 512, [[256]]), run_shared(shared(), {dtype}, 3, 256, 128)]
+        print(json.dumps(r + [run_gemm(gemm([1], [256], stream_plan="1,4,1,1"), {dtype}, 2, 512, [[256]])]))
+        """)
+    for code, message, log in out[:2]:
+        assert code == 0 and _kernel(log) == ["SkinnyGemm"], message
+    assert out[2][0] != 0 and out[2][2] == []  # a pinned shape of that kernel is an error
