@@ -967,7 +967,7 @@ StreamPlan ChooseStreamPlan(const PlanInput& in) {
   const bool odd = OddRows(in.mode, in), fp4 = in.mode == kNvfp4;
   // A vocabulary of at least four groups of 128 columns per SM and a few more: the head gives the few away in slices of K
   // (GemmParams::tail_groups), the plain product takes a group more per CTA and adds up K in the same order.
-  if (in.nseg == 1 && fp4 && in.n[0] % gran == 0 && !in.fuse) {
+  if (in.nseg == 1 && fp4 && in.n[0] % gran == 0 && !in.fuse && g_stream.slots[1] > 0) {
     const int slots = g_stream.slots[1], groups = in.n[0] / gran, per = groups / slots, rest = groups % slots;
     if (per >= 4 && rest >= 1 && rest <= kMaxTailGroups && per < kStreamWarps) {
       PlanInput head = in;

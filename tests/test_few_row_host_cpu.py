@@ -86,3 +86,12 @@ def test_a_device_that_refuses_the_kernel(fake, dtype):  # noqa: F811
     for code, message, log in out[:2]:
         assert code == 0 and _kernel(log) == ["SkinnyGemm"], message
     assert out[2][0] != 0 and out[2][2] == []  # a pinned shape of that kernel is an error
+
+
+def test_a_device_that_reports_no_resident_block(fake):  # noqa: F811
+    """A few more groups of 128 columns than SMs hold: the rule for that shape divides by the resident CTAs."""
+    out = fake("""
+        fake.fake_resident(0)
+        print(json.dumps(run_gemm(gemm([1], [128 * 600]), U8, 2, 512, [[128 * 600]])))
+        """)
+    assert out[0] == 0 and _kernel(out[2]) == ["SkinnyGemm"], out[1]
