@@ -277,4 +277,12 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, g_methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__calls(void) { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__calls(void) {
+  PyObject* m = PyModule_Create(&g_module);
+  // the torch whose headers this was compiled against: ops.py uses the module with no other
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", QFG_TORCH_VERSION) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

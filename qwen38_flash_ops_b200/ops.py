@@ -10,12 +10,15 @@ libqfg_b200.so on the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import os
 import struct
+import warnings
 from ctypes import c_void_p
+from types import SimpleNamespace
 
 import torch
 
-from . import _calls, _lib
+from . import _lib
 from ._lib import QfgError, Tensor2D, check
 
 _DTYPES = {
@@ -31,7 +34,19 @@ _DTYPES = {
 # which does all of it in C++.  What that does not take (it returns None: a tensor subclass, a wrapped tensor, an argument
 # that is wrong) and the calls with outputs given take the Python code below, written with its time in mind as well:
 # torch.cuda.current_stream() builds a Stream object (3.5 us; the raw handle 0.15), ctypes structures and arrays are built
-# field by field (1.6 us; one struct.pack 0.3).
+# field by field (1.6 us; one struct.pack 0.3).  Without the extension, or with one that was built for another torch, the
+# Python code serves every call: the same kernels, some microseconds later.
+try:
+    from . import _calls
+    _built_for = getattr(_calls, "torch_version", "another version")
+    if _built_for != torch.__version__:
+        raise ImportError(f"it was built for torch {_built_for}, this is {torch.__version__}")
+except ImportError as e:
+    warnings.warn(f"{__package__}._calls cannot be used ({e}): calls take longer on the host; "
+                  f"`make -C {os.path.join(os.path.dirname(os.path.abspath(__file__)), 'csrc')}` builds it", RuntimeWarning)
+    _handed_back = lambda *args: None
+    _calls = SimpleNamespace(bind=_handed_back, skinny_gemm=_handed_back, argmax_rows=_handed_back, dequant=_handed_back,
+                             lmhead=_handed_back, shared_expert_down=_handed_back)
 _bound = False
 
 

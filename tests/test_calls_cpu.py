@@ -1,8 +1,14 @@
 """csrc/calls.cc without a GPU: what is not a plain dense CUDA tensor is handed back to the Python code, with no error left
 behind."""
+import os
+import shutil
+import subprocess
+import sys
+
 import pytest
 import torch
 
+import qwen38_flash_ops_b200 as package
 from qwen38_flash_ops_b200 import ArgmaxRows, QfgError, _calls
 from qwen38_flash_ops_b200 import ops
 
@@ -52,3 +58,57 @@ def test_errors_are_the_python_codes(monkeypatch):
     ops._load()
     with pytest.raises(QfgError, match="contiguous CUDA tensor"):
         ArgmaxRows()(torch.zeros(2, 8))
+
+
+@pytest.mark.parametrize("extension", ["absent", "damaged", "for another torch", "without a version"])
+def test_ops_without_the_extension(tmp_path, extension):
+    """The package with the library alone, or beside an extension that this torch cannot load: the Python code serves the calls."""
+    src = os.path.dirname(package.__file__)
+    pkg = tmp_path / os.path.basename(src)
+    pkg.mkdir()
+    for name in os.listdir(src):
+        if name.endswith(".py"):
+            shutil.copy(os.path.join(src, name), pkg)
+    if extension == "damaged":
+        (pkg / "_calls.so").write_bytes(b"not a library")
+    elif extension != "absent":
+        (pkg / "_calls.py").write_text("torch_version = '1.0'\n" if extension == "for another torch" else "")
+    code = """
+import warnings, torch
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    from qwen38_flash_ops_b200 import ArgmaxRows, QfgError
+assert any("_calls" in str(w.message) for w in seen)
+try:
+    ArgmaxRows()(torch.zeros(2, 8))
+except QfgError as e:
+    assert "contiguous CUDA tensor" in str(e)
+else:
+    raise AssertionError("accepted")
+"""
+    env = {**os.environ, "PYTHONPATH": str(tmp_path), "QFG_LIBRARY": os.path.join(src, "libqfg_b200.so")}
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_the_extension_serves_this_torch():
+    assert _calls.torch_version == torch.__version__ and ops._calls is _calls
+
+
+@pytest.mark.gpu
+def test_calls_handed_back_give_the_same(cuda, monkeypatch):
+    from qwen38_flash_ops_b200 import DequantWeightBf16, LmHeadArgmax, SharedExpertDown, SkinnyGemm
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    x, w, g, u, gx, gw, routed = mk(2, 3, 64), mk(64, 256), mk(3, 64), mk(3, 64), mk(3, 32), mk(32, 1), mk(3, 256)
+
+    def every():
+        return [*SkinnyGemm([2], [64, 192])(x, w), *ArgmaxRows()(x), ArgmaxRows()(x, with_val=False), *DequantWeightBf16(256, widths=[128, 128])(w),
+                *LmHeadArgmax()(x, w, 256), SharedExpertDown()(g, u, w, gx, gw, routed)]
+
+    direct = every()
+    for name in ("skinny_gemm", "argmax_rows", "dequant", "lmhead", "shared_expert_down"):
+        monkeypatch.setattr(ops._calls, name, lambda *args: None)
+    for a, b in zip(direct, every(), strict=True):
+        assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride() and torch.equal(a, b)
