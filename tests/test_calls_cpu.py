@@ -112,3 +112,25 @@ def test_calls_handed_back_give_the_same(cuda, monkeypatch):
         monkeypatch.setattr(ops._calls, name, lambda *args: None)
     for a, b in zip(direct, every(), strict=True):
         assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride() and torch.equal(a, b)
+
+
+def _make(*args):
+    src = os.path.join(os.path.dirname(package.__file__), "csrc")
+    return subprocess.run(["make", "-C", src, *args], capture_output=True, text=True, timeout=300)
+
+
+def test_make_without_torch_builds_the_rest():
+    """Hosts of the C ABI need neither Python nor torch."""
+    r = _make("-n", "PYTHON=false", "CALLS=/nonexistent/_calls.so", "LIB=/nonexistent/libqfg.so")
+    assert r.returncode == 0 and "libqfg.so" in r.stdout and "calls.cc" not in r.stdout, r.stderr
+
+
+def test_make_builds_the_extension_anew_for_another_torch(tmp_path):
+    python = tmp_path / "python"
+    calls = tmp_path / "_calls.so"
+    for version, expected in (("1", True), ("1", False), ("2", True)):
+        python.write_text(f"#!/bin/sh\necho -DQFG_TORCH_VERSION={version}\n")
+        python.chmod(0o755)
+        r = _make(f"PYTHON={python}", f"CALLS={calls}", f"OBJ={tmp_path}", "HOSTCXX=true", str(calls))  # compiles nothing
+        assert r.returncode == 0 and ("calls.cc" in r.stdout) == expected, (version, r.stdout, r.stderr)
+        calls.touch()
