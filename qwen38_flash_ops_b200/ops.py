@@ -159,7 +159,7 @@ class SkinnyGemm:
         h = getattr(self, "_h", None)
         if h:
             self._lib.qfg_skinny_gemm_destroy(h)
-            self._h = None
+            self._h = self._p = None
 
 
 class ArgmaxRows:
@@ -229,7 +229,7 @@ class DequantWeightBf16:
         h = getattr(self, "_h", None)
         if h:
             self._lib.qfg_dequant_destroy(h)
-            self._h = None
+            self._h = self._p = None
 
 
 class SharedExpertDown:
@@ -283,7 +283,7 @@ class SharedExpertDown:
         h = getattr(self, "_h", None)
         if h:
             self._lib.qfg_shared_expert_down_destroy(h)
-            self._h = None
+            self._h = self._p = None
 
 
 class UntileHcBf16:
@@ -405,7 +405,7 @@ class LmHeadArgmax:
         h = getattr(self, "_h", None)
         if h:
             self._lib.qfg_lmhead_destroy(h)
-            self._h = None
+            self._h = self._p = None
 
 
 def lmhead_combine(keys: torch.Tensor, ranks: int, m: int):

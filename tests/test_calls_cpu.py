@@ -134,3 +134,19 @@ def test_make_builds_the_extension_anew_for_another_torch(tmp_path):
         r = _make(f"PYTHON={python}", f"CALLS={calls}", f"OBJ={tmp_path}", "HOSTCXX=true", str(calls))  # compiles nothing
         assert r.returncode == 0 and ("calls.cc" in r.stdout) == expected, (version, r.stdout, r.stderr)
         calls.touch()
+
+
+@pytest.mark.parametrize("name", ["SkinnyGemm", "DequantWeightBf16", "SharedExpertDown", "LmHeadArgmax"])
+def test_a_destroyed_node_is_not_called(name):
+    """Its address goes with the handle: the C++ calls hand None back, and the library refuses a null node."""
+    freed = []
+
+    class Lib:
+        def __getattr__(self, entry):
+            return freed.append
+
+    op = object.__new__(getattr(ops, name))
+    op._lib, op._h, op._p = Lib(), 1, 1
+    op.__del__()
+    op.__del__()
+    assert freed == [1] and op._h is None and op._p is None
