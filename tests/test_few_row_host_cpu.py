@@ -39,10 +39,13 @@ def test_shared_expert_in_passes_of_eight(fake, dtype):  # noqa: F811
         calls = fake.fake_setup_calls()
         fake.fake_refuse_setup(1)
         r = [run_shared(s, {dtype}, m, 256, 128) for m in (3, 16)]
+        general = shared(stream_plan="0", dense_rows=0, pdl_wait=1)
+        r.append(run_shared(general, {dtype}, 20, 256, 128))
         fake.fake_device(1)
         print(json.dumps([r, run_shared(s, {dtype}, 3, 256, 128), calls == fake.fake_setup_calls()]))
         """)
-    (few, two_passes), other_device, no_setup = out
+    (few, two_passes, general), other_device, no_setup = out
+    assert general[0] == 0 and _kernel(general[2]) == ["SkinnyGemm"] * 3
     assert few[0] == two_passes[0] == 0 and no_setup
     assert _kernel(few[2]) == ["SkinnyGemmStreamKernel"] and _kernel(two_passes[2]) == ["SkinnyGemmStreamKernel"] * 2
     assert all(line.endswith("pdl=1") for line in few[2] + two_passes[2])

@@ -88,9 +88,19 @@ def test_repeated_calls_agree(cuda, mode, plan):
         assert torch.equal(op(*args), first)
 
 
+def _three_kernels():
+    """The many-row kernel, the few-row kernel in passes, the general kernels in passes."""
+    many, few, general = SharedExpertDown(), SharedExpertDown(), SharedExpertDown()
+    for op in (few, general):
+        op.set_option("dense_rows", 0)
+    general.set_option("stream_plan", "0")
+    return many, few, general
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_swish_times_u_is_the_streaming_kernels(cuda, seed):
-    """Every g beside random u of every size: bf16(bf16(g * bf16(sigmoid(g))) * u), through an identity weight.  A row holds 64
+    """Every g beside random u of every size: bf16(bf16(g * bf16(sigmoid(g))) * u), through an identity weight, in the many-row
+    and the few-row kernel, which share swish.cuh, against the general kernels, whose sigmoid is expf and a division.  A row holds 64
     values, so g and u stay below 2^60 and sums are one term and zeros.  Products below the normal range may be rounded twice
     (once to FP32's subnormals), so they are compared to one unit in their last place."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
@@ -102,13 +112,12 @@ def test_swish_times_u_is_the_streaming_kernels(cuda, seed):
     w[torch.arange(64), torch.arange(64)] = 1
     gx, gw = torch.ones(1024, 8, device="cuda").bfloat16(), torch.full((8, 1), 10.0, device="cuda").bfloat16()
     routed = torch.zeros(1024, 128, device="cuda").bfloat16()
-    many, few = SharedExpertDown(), SharedExpertDown()
-    few.set_option("dense_rows", 0)
-    a, b = (op(g, u, w.bfloat16(), gx, gw, routed) for op in (many, few))
+    many, few, b = (op(g, u, w.bfloat16(), gx, gw, routed) for op in _three_kernels())
     normal = b.float().abs() >= 2.0 ** -126
-    assert torch.equal(a[normal], b[normal])
-    assert ((a.double() - b.double()).abs() <= 2.0 ** -133).logical_or(normal).all()
-    assert normal[:, :64].sum() > 30000 and torch.count_nonzero(a[:, 64:]) == 0
+    for a in (many, few):
+        assert torch.equal(a[normal], b[normal])
+        assert ((a.double() - b.double()).abs() <= 2.0 ** -133).logical_or(normal).all()
+        assert normal[:, :64].sum() > 30000 and torch.count_nonzero(a[:, 64:]) == 0
 
 
 def test_swish_of_every_bf16_value_is_the_streaming_kernels(cuda):
@@ -118,14 +127,14 @@ def test_swish_of_every_bf16_value_is_the_streaming_kernels(cuda):
     w[torch.arange(64), torch.arange(64)] = 1
     gx, gw = torch.ones(1024, 8, device="cuda").bfloat16(), torch.full((8, 1), 10.0, device="cuda").bfloat16()
     u, routed = torch.ones_like(g), torch.zeros(1024, 128, device="cuda").bfloat16()
-    many, few = SharedExpertDown(), SharedExpertDown()
-    few.set_option("dense_rows", 0)
+    kernels = _three_kernels()
     for j in range(64):
         gj = torch.zeros_like(g)
         gj[:, j] = g[:, j]
-        a, b = (op(gj, u, w.bfloat16(), gx, gw, routed)[:, j] for op in (many, few))
-        assert torch.equal(torch.isnan(a), torch.isnan(b))
-        assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+        many, few, b = (op(gj, u, w.bfloat16(), gx, gw, routed)[:, j] for op in kernels)
+        for a in (many, few):
+            assert torch.equal(torch.isnan(a), torch.isnan(b))
+            assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
