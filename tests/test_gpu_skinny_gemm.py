@@ -137,8 +137,10 @@ def test_row_independence_and_determinism(cuda, mode):
     U.check_against_oracle(mode, x, arr, N, s if mode != 0 else None, full, K, "row-scaled")
 
 
-@pytest.mark.parametrize("mode", [1, 2])
-def test_wide_dynamic_range_takes_bf16_path(cuda, mode):
+@pytest.mark.parametrize("mode,option", [(m, o) for m in (1, 2) for o in (
+    "", "stream_plan=0", "plan=direct=0,wn=2,wk=4,cluster=2", "plan=direct=1,wn=2,wk=4,cluster=2", "plan=direct=2,wn=2,wk=4,cluster=2")
+    if m == 1 or "direct=2" not in o])  # every kernel has a BF16 path of its own
+def test_wide_dynamic_range_takes_bf16_path(cuda, mode, option):
     """x whose K slice spans more than 2^28 is not exactly representable in FP16 after the
     power-of-two prescale; the CTA then runs the BF16 MMA on exact BF16 operands.  Both paths
     must satisfy the tolerance; on ordinary inputs they must agree bit for bit."""
@@ -151,6 +153,8 @@ def test_wide_dynamic_range_takes_bf16_path(cuda, mode):
     x[1, 100] = np.float32(2.0 ** -120)
     xb = P.f32_to_bf16_bits(x)
     op = SkinnyGemm([1], [N], w_scale=s)
+    if option:
+        op.set_option(*option.split("=", 1))
     w = U.dev_weight(arr, mode)
     got = bits(op(to_dev(xb, "bf16"), w)[0])
     U.check_against_oracle(mode, xb, arr, N, s, got, K, "wide range")

@@ -104,6 +104,31 @@ def test_shared_expert(cuda, mode, plan):
             assert torch.equal(op(*row)[0], out[m])
 
 
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("plan", ["1,4,2,1", "1,4,1,2"])
+def test_shared_expert_outside_the_fp16_range(cuda, mode, plan):
+    """swish_mul that spreads too far for FP16, in the last row and the last slice of K alone, and the forced BF16 path, whose
+    sums are those of the FP16 one."""
+    plan = plan if mode == 2 else f"8{plan[1:]}"
+    rng = np.random.default_rng(mode)
+    M, K, N, gk = 5, 1032, 128, 64
+    arr, s = U.make_weight(rng, mode, K, N, True)
+    g, u, gx, gw, routed = _inputs(rng, M, K, N, gk)
+    op = SharedExpertDown(w_scale=s)
+    op.set_option("stream_plan", plan)
+    run = lambda u: bits(op(*[to_dev(a, "bf16") if a is not arr else U.dev_weight(arr, mode) for a in (g, u, arr, gx, gw, routed)]))
+    plain = run(u)
+    for value in (0x7180, 0x0D00):  # 2^100, 2^-101
+        wide = u.copy()
+        wide[M - 1, K - 1] = value
+        y, _, _, shared = O.shared_expert_down(g, wide, mode, arr, N, gx, gw, routed, s)
+        got = run(wide)
+        _check(got, y, shared, O.bf16_to_f32(routed), f"mode {mode} {plan} {value:x}")
+        assert np.array_equal(got[:M - 1], plain[:M - 1])
+    op.set_option("force_slow", 1)
+    assert np.array_equal(run(u), plain)
+
+
 @pytest.mark.parametrize("groups", [33, 34])  # rows of 8 modulo 16 bytes, and of 0
 @pytest.mark.parametrize("tail", [1, 3])
 def test_head_tail(cuda, groups, tail):
