@@ -38,8 +38,8 @@ HEAD = "C5_nvfp4_lmhead_5120x151936"
 
 
 # DRAM sectors per launch of the fused LM-head kernel, from an ncu capture of this workload:
-# (439.54 MB read + 4.58 MB written) / 437.58 MB of packed weights
-NCU_DRAM_BYTES_PER_WEIGHT_BYTE = 1.0150
+# (439.93 MB read + 3.92 MB written) / 437.58 MB of packed weights
+NCU_DRAM_BYTES_PER_WEIGHT_BYTE = 1.0143
 
 
 def peaks():
@@ -596,6 +596,8 @@ def run_ours(args):
     # DRAM bytes per launch from the ncu capture of this kernel on this workload (read + write sectors
     # over the packed weight bytes), scaled to the shard
     traffic = round(NCU_DRAM_BYTES_PER_WEIGHT_BYTE * shard_bytes)
+    plan = describe_plan(head, k, shard)
+    kernel = "SkinnyGemmStreamKernel" if plan.startswith("stream_") else "SkinnyGemmDirectKernel"
     line = {
         "metric": METRIC, "value": round(value, 4), "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(us_step / 1000.0, 6), "higher_is_better": True,
@@ -605,12 +607,12 @@ def run_ours(args):
                    "parallelism": f"vocab-sharded x{world}" if world > 1 else "single GPU",
                    "l2": "inputs larger than L2 (437.6 MB of weights per step" +
                          (f", {shard_bytes / 1e6:.1f} MB per rank)" if world > 1 else ")"),
-                   "plan": describe_plan(head, k, shard)},
+                   "plan": plan},
         "us_per_call": round(us_step, 2),
         "frac_of_8TBps": round(value / 8.0 / world, 4),
         "roofline": {"bound": "hbm", "achieved": round(shard_bytes / us_kernel / 1e3, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(shard_bytes / us_kernel / 1e3 / peak, 4), "traffic": traffic,
-                     "peak_source": f"{peak_kind} copy bandwidth", "kernel": "SkinnyGemmKernel<NVFP4> (fused argmax)",
+                     "peak_source": f"{peak_kind} copy bandwidth", "kernel": f"{kernel}<NVFP4> (fused argmax)",
                      "kernel_us": round(us_kernel, 2), "algorithmic_bytes": shard_bytes},
         "e2e": {"value": round(total_bytes / us_e2e / 1e6, 4), "unit": UNIT, "h2d_bytes_per_step": x.numel() * 2,
                 "d2h_bytes_per_step": m * 12, "us_per_step": round(us_e2e, 2)},
@@ -724,7 +726,9 @@ def describe_plan(head, k, shard):
     n = shard.shape[1] * 16 // 9
     align = 16 if (shard.data_ptr() % 16 == 0 and shard.shape[1] % 16 == 0) else 8 if shard.shape[1] % 8 == 0 else 4
     p = _lib.plan_describe(_lib.QFG_UINT8, k, [n], align, spec="lmhead")
-    return ",".join(f"{a}={b}" for a, b in p.items() if a != "seg_tiles")
+    # the kernel of the tensor copies, or the general ones (whose plan has no such prefix)
+    stream = p["stream_width"] > 0
+    return ",".join(f"{a}={b}" for a, b in p.items() if a != "seg_tiles" and a.startswith("stream_") == stream)
 
 
 def run_profile_case(args):

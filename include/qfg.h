@@ -114,19 +114,25 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
 /* Launch options that are not node attributes.  "pdl_wait" = 1 launches the kernel with the
  * programmatic-stream-serialisation attribute and makes it wait for its predecessor
  * (griddepcontrol.wait) only after its first weight tiles are in flight.  "plan" pins the
- * launch geometry ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296"); used by the tuning sweeps.
+ * geometry of the general kernels ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296") and sends the call to them; "stream_plan"
+ * = "width,wk,teams,cluster,tail" pins that of the kernel that streams the weights by tensor copies, "0" sends no call
+ * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.
  * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken;
  * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape. */
 QFG_API int qfg_skinny_gemm_set_option(qfg_skinny_gemm* op, const char* key, const char* value);
 
-/* Writes a one-line description of the launch plan chosen for these shapes into buf. */
+/* Writes a one-line description of the launch plan chosen for these shapes into buf: the general kernels' geometry, then
+ * "stream=width/wk/teams/cluster/tail", by which the call goes instead unless width is 0 (or x is off sixteen bytes). */
 QFG_API int qfg_skinny_gemm_describe(const qfg_skinny_gemm* op, int64_t k, const qfg_tensor2d* weights, int n_weights,
                              char* buf, size_t buf_len);
 
 /* Diagnostic, needs no device: the launch plan for `nseg` weights of `n[i]` columns, element
  * type `dtype`, K rows, rows aligned to `row_align` (16, 8 or 4) bytes, on a GPU with `sm_count`
- * SMs; `spec` (may be NULL) is a "plan" override as above.  No counterpart in the reference, whose
- * planner is the table at src/fused_gemm/fused_gemm.cu:125-175. */
+ * SMs; `spec` (may be NULL) is a "plan" override as above, or "lmhead" (then ",key=value...") for the fused
+ * LM head.  "key=value" items: the general kernels' geometry, then as "stream_*" that of "stream_plan", by which
+ * the call goes instead unless stream_width is 0.  Resident clusters are the device's where a node was made on one with
+ * `sm_count` SMs, else assumed.  No counterpart in the reference, whose planner is the table at
+ * src/fused_gemm/fused_gemm.cu:125-175. */
 QFG_API int qfg_plan_describe(int dtype, int64_t k, const int64_t* n, int nseg, int row_align, int sm_count,
                               const char* spec, char* buf, size_t buf_len);
 

@@ -576,6 +576,10 @@ int qfg_plan_describe(int dtype, int64_t k, const int64_t* n, int nseg, int row_
   std::string d = qfg::DescribePlan(plan, in);
   d += ",seg_tiles=";
   for (int s = 0; s < nseg; ++s) d += (s ? "/" : "") + std::to_string(plan.tiles[s]);
+  // a pinned launch geometry is one of the general kernels'
+  const qfg::StreamPlan stream = overrides.empty() ? qfg::ChooseStreamPlan(in) : qfg::StreamPlan();
+  d += ",stream_width=" + std::to_string(stream.width) + ",stream_wk=" + std::to_string(stream.wk) + ",stream_teams=" + std::to_string(stream.teams) +
+       ",stream_cluster=" + std::to_string(stream.cluster) + ",stream_tail=" + std::to_string(stream.tail);
   std::snprintf(buf, buf_len, "%s", d.c_str());
   return QFG_OK;
 }

@@ -792,6 +792,13 @@ struct StreamSetup {
 };
 StreamSetup g_stream;
 
+// Of a launch on the device that was set up; for a description without it, the loss in packing that planner.cc assumes.
+int Resident(const PlanInput& in, int cluster) {
+  if (g_stream.status == cudaSuccess && in.sm_count == DeviceSmCount()) return g_stream.slots[cluster];
+  return cluster == 1 ? in.sm_count : std::max(1, in.sm_count * 8 / (10 * cluster));
+}
+bool Refused() { return g_stream.status != cudaSuccess && g_stream.status != cudaErrorNotReady; }
+
 template <int MODE, int KIND>
 cudaError_t SetUpStream() {
   return cudaFuncSetAttribute(SkinnyGemmStreamKernel<MODE, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
@@ -924,7 +931,7 @@ cudaError_t ConfigureStreamKernels() {
 }
 
 bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan) {
-  if (g_stream.status != cudaSuccess || plan->width < 1 || plan->wk < 1 || plan->teams < 1 || plan->cluster < 1 || plan->cluster > 8) return false;
+  if (Refused() || plan->width < 1 || plan->wk < 1 || plan->teams < 1 || plan->cluster < 1 || plan->cluster > 8) return false;
   if (in.K % 8 != 0 || in.K > (1 << 20) || in.row_align < (in.mode == kNvfp4 ? 8 : 16)) return false;
   const int gran = StreamGran(in.mode);
   const bool odd = OddRows(in.mode, in);
@@ -962,13 +969,13 @@ bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan) {
 // clusters of six 16.6 (one group, clusters of three 18.3); NVFP4 640 x 2560 in clusters of five 5.4 (none 6.4).
 StreamPlan ChooseStreamPlan(const PlanInput& in) {
   StreamPlan best;
-  if (g_stream.status != cudaSuccess) return best;
+  if (Refused()) return best;
   const int gran = StreamGran(in.mode), ksteps = (in.K + 15) / 16;
   const bool odd = OddRows(in.mode, in), fp4 = in.mode == kNvfp4;
   // A vocabulary of at least four groups of 128 columns per SM and a few more: the head gives the few away in slices of K
   // (GemmParams::tail_groups), the plain product takes a group more per CTA and adds up K in the same order.
-  if (in.nseg == 1 && fp4 && in.n[0] % gran == 0 && !in.fuse && g_stream.slots[1] > 0) {
-    const int slots = g_stream.slots[1], groups = in.n[0] / gran, per = groups / slots, rest = groups % slots;
+  if (in.nseg == 1 && fp4 && in.n[0] % gran == 0 && !in.fuse && Resident(in, 1) > 0) {
+    const int slots = Resident(in, 1), groups = in.n[0] / gran, per = groups / slots, rest = groups % slots;
     if (per >= 4 && rest >= 1 && rest <= kMaxTailGroups && per < kStreamWarps) {
       PlanInput head = in;
       head.allow_tail = true;
@@ -984,7 +991,7 @@ StreamPlan ChooseStreamPlan(const PlanInput& in) {
   double best_cost = 1e30, total = 0;
   for (int s = 0; s < in.nseg; ++s) total += static_cast<double>(in.K) * in.n[s] * (in.mode == kBf16 ? 2.0 : in.mode == kFp8 ? 1.0 : 0.5625);
   for (int cluster = 1; cluster <= 8; ++cluster) {
-    const int slots = g_stream.slots[cluster], slice = (ksteps + cluster - 1) / cluster * 16;
+    const int slots = Resident(in, cluster), slice = (ksteps + cluster - 1) / cluster * 16;
     const double around = (in.mode == kBf16 ? 2.2 : 3.4) + (cluster > 1 ? 1.7 + 0.1 * cluster : 0.0);
     if (cluster > 1 && (ksteps < 8 * cluster || total / 6.0e6 + around >= best_cost)) break;
     for (int width = fp4 ? 1 : 3; slots > 0 && width <= (fp4 ? kStreamWarps : 32); ++width) {

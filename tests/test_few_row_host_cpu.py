@@ -52,6 +52,33 @@ def test_shared_expert_in_passes_of_eight(fake, dtype):  # noqa: F811
     assert other_device[0] != 0
 
 
+@pytest.mark.parametrize("dtype,k,widths", [("BF16", 5120, [5120]), ("FP8", 6144, [2560]), ("U8", 5120, [17408, 17408]), ("U8", 17408, [5120]), ("BF16", 516, [256])])
+def test_the_described_plan_is_the_launched_one(fake, dtype, k, widths):  # noqa: F811
+    out = fake(f"""
+        fake.fake_resident(148)
+        h = gemm([1] * {len(widths)}, {widths})
+        buf = ctypes.create_string_buffer(512)
+        w = (L.Tensor2D * {len(widths)})(*[L.Tensor2D(P, {dtype}, {k}, cols({dtype}, n)) for n in {widths}])
+        assert lib.qfg_skinny_gemm_describe(h, {k}, w, {len(widths)}, buf, 512) == 0
+        pinned = L.plan_describe({dtype}, {k}, {widths}, spec="wn=1,wk=2,cluster=1")
+        print(json.dumps([run_gemm(h, {dtype}, 1, {k}, [[n] for n in {widths}]), L.plan_describe({dtype}, {k}, {widths}), pinned, buf.value.decode()]))
+        """)
+    (code, message, log), plan, pinned, described = out
+    assert code == 0, message
+    keys = ("width", "wk", "teams", "cluster", "tail")
+    assert "stream=" + "/".join(str(plan[f"stream_{key}"]) for key in keys) in described
+    assert pinned["stream_width"] == 0
+    if k % 8:
+        assert plan["stream_width"] == 0 and _kernel(log) == ["SkinnyGemm"]
+        return
+    assert _kernel(log) == ["SkinnyGemmStreamKernel"]
+    columns = {"BF16": 8, "FP8": 16, "U8": 128}[dtype] * plan["stream_width"]
+    tiles = sum(-(-n // columns) for n in widths)
+    wide = -(-columns // {"BF16": 64, "FP8": 128, "U8": 128}[dtype])
+    threads = 32 * (plan["stream_wk"] * plan["stream_teams"] * wide + 1)
+    assert f"grid={tiles},{plan['stream_cluster']} threads={threads} " in log[0], (plan, log)
+
+
 @pytest.mark.parametrize("resident,clusters", [(132, True), (1, False)])
 def test_clusters_that_the_device_holds(fake, resident, clusters):  # noqa: F811
     # K short enough for eight rows of x in one CTA (16384 would take 256 KB): without clusters the kernel is still the one
