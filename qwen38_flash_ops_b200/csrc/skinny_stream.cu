@@ -962,8 +962,16 @@ bool CompleteStreamPlan(const PlanInput& in, StreamPlan* plan) {
 //   the stream: all bytes at 6.0 TB/s, a ninth to a third more where tiles begin inside lines of 128 bytes; or a CTA's share
 //   at 14 ns per KB, or slower where its ring (at four rows) is less than two microseconds of that; a row and 128 columns
 //   of NVFP4 1.75 ns, its arithmetic (more where a tile is one group wide: two copied rows for 72 bytes, and few warps);
-//   around it: 2.2 (BF16) or 3.4 for launch, first copies, x and the epilogue; 1.9 more where ranks of a cluster add up;
+//   around it: 2.2 (BF16) or 3.4 for launch, first copies, x and the epilogue; 1.8 (a pair) to 2.5 (eight) more where ranks of a
+//   cluster add up; 0.4 ns for each row of a slice past 5120, whose x is staged in further rounds; 2 for NVFP4 of several groups
+//   per CTA over fewer than 1024 rows, whose few stages do not hide the first;
 //   SharedExpertDown: swish_mul of the slice, which every CTA computes for itself.
+// What a term decides, on 2000 random shapes (K 256 to 17408, N 256 to 23170, one to three weights, one to eight rows) with the
+// model's choice 4.7 % behind the best launch tried.  Without it: lines of 128 bytes: 772 of 1339 BF16 / FP8 shapes get another
+// launch, 1 % slower on average; least 1.5 ns a row: 361 of 1339, 20 % slower; ring of two microseconds: 8, 3 % slower; x past 5120
+// rows: 71, 4 % slower; few stages of NVFP4: 347 of 661, 8 % slower; eight NVFP4 warps taken for sixteen (2.05): 46 of 661, 19 %
+// slower; four taken for eight (2.3): 138, no difference on average; sixteen taken for eight (2.3): 26, 6 % faster, not
+// followed up; swish_mul: 72 of 400 shared experts, 10 % (NVFP4 22 %) slower.
 // Against other shapes: BF16 5120 x 5120 8 pieces wide, two teams of four warps, no cluster 11.1 (16 wide in clusters of three
 // 12.7, 5 wide 12.8); FP8 6144 x 2560 in clusters of four to six 8.1 (of two 10.1); NVFP4 17408 x 5120 two groups wide in
 // clusters of six 16.6 (one group, clusters of three 18.3); NVFP4 640 x 2560 in clusters of five 5.4 (none 6.4).
@@ -1004,7 +1012,12 @@ StreamPlan ChooseStreamPlan(const PlanInput& in) {
       StreamPlan p;
       p.width = width;
       p.cluster = cluster;
-      // eight warps along K (as two teams where the arithmetic of a stage is short), fewer where columns take them or K is short
+      // Eight warps along K (as two teams where the arithmetic of a stage is short), fewer where columns take them or K is short.
+      // The same 2000 shapes, time over that of the line taken: one column warp, BF16, slices below 512 rows 4 x 1, 4 x 2 1.03,
+      // 8 x 1 1.04, from 1024 4 x 2, 8 x 1 1.00, 4 x 1 1.01 to 1.03; FP8 below 512 4 x 1, 8 x 1 and 4 x 2 1.00, to 1024 8 x 1 0.97,
+      // beyond 8 x 1, 4 x 2 1.00 to 1.04, 4 x 1 1.10; NVFP4 below 1024 4 x 1, 8 x 1 0.93 to 0.96, to 2048 8 x 1, 8 x 2 1.05, 4 x 1
+      // 1.11, beyond 8 x 2, 8 x 1 1.00, 4 x 2 1.06.  Two column warps: 4 x 2, BF16 / FP8 2 x 2 0.95 to 0.99, NVFP4 to 1024 4 x 1 0.98,
+      // beyond 3 x 2 1.02 to 1.05.  Three and more: 4 x 1, 2 x 2 0.96 to 1.07.  One or two warps and one team: 1.1 to 3.
       const int wn = fp4 ? width : (width + 7) / 8;
       if (wn == 1) {
         p.wk = in.mode == kBf16 || in.fuse || slice < 1024 ? 4 : 8;
