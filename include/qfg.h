@@ -113,7 +113,8 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
 
 /* Launch options that are not node attributes.  "pdl_wait" = 1 launches the kernel with the
  * programmatic-stream-serialisation attribute and makes it wait for its predecessor
- * (griddepcontrol.wait) only after its first weight tiles are in flight.  "plan" pins the
+ * (griddepcontrol.wait) only after its first weight tiles are in flight; trigger 1 then releases the dependents behind
+ * that wait.  "plan" pins the
  * geometry of the general kernels ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296") and sends the call to them; "stream_plan"
  * = "width,wk,teams,cluster,tail" pins that of the kernel that streams the weights by tensor copies, "0" sends no call
  * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.
