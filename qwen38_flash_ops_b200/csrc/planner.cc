@@ -1,4 +1,6 @@
-// Launch planning for the streaming kernel: how many column tiles per weight, how many warps
+// Launch planning for the general few-row kernels (skinny_gemm.cu), which take what skinny_stream.cu does not: x or weight rows
+// off 16 bytes, K off eights, NVFP4 widths off 128, refused tensor maps, pinned geometries.  The figures below are from when they
+// took every call.  How many column tiles per weight, how many warps
 // side by side, how deep the ring, how many CTAs split K.  The plan is a function of
 // (K, segment widths, weight type, row alignment, SM count) only - the number of rows never
 // enters, so a row is reduced in the same order whatever the batch (the property the reference
@@ -157,8 +159,8 @@ void DistributeTiles(const PlanInput& in, int total_tiles, Plan* plan) {
 //   balance          - CTAs versus the resident CTA slots of whole waves (16 warps per SM);
 //   pipeline length  - k-steps per warp, so that fill and drain of the load pipeline amortise;
 //   row width        - contiguous bytes a CTA reads per weight row.
-// Launch shapes measured best on B200 (148 SMs) for the decode GEMMs of the model this library
-// serves; the counterpart of the reference's H200 table (src/fused_gemm/fused_gemm.cu:132-156).
+// Launch shapes measured best for these kernels on B200 (148 SMs), for the decode GEMMs of the model this library
+// serves (with x off 16 bytes, say; as skinny_stream.cu takes them otherwise); the counterpart of the reference's H200 table (src/fused_gemm/fused_gemm.cu:132-156).
 // Every other shape, and these shapes on a different SM count, go through the scoring rule below.
 struct TunedShape {
   int mode, K, nseg;

@@ -266,10 +266,9 @@ cudaError_t LaunchDequant(const DequantParams& p, cudaStream_t stream);
 // Calls with more than `dense_rows` rows (an option of the node; 0 disables it) leave the streaming kernels: dense_tc.cu,
 // or dense_gemm.cc for the layouts that does not take.
 // At and below the defaults a row's result does not depend on the number of rows in the call: the streaming kernels compute
-// it as a one-row call does.  Speed alone would put the lines lower for BF16: 5120 x 17408, eight rows of BF16 / FP8 / NVFP4 in
-// the many-row kernel 32 / 25 / 23 us; in one pass of skinny_stream.cu NVFP4 takes 15 to 16, so nine rows (two passes) cost
-// a third more than the many-row kernel.
-// NVFP4's 16 was the break-even of a dequantisation pass and a library GEMM (89 us at any number of rows).
+// it as a one-row call does.  5120 x 17408 in a graph, passes of skinny_stream.cu / many-row kernel, us: eight rows BF16 32 / 31,
+// FP8 23 / 24, NVFP4 18 / 22; nine (two passes) 61 / 31, 36 / 24, 32 / 22.  So speed puts the line at eight for every type; NVFP4
+// keeps sixteen because its rows up to there were always independent of the row count, which the tests hold it to.
 constexpr int DenseRowsDefault(int mode) { return mode == kNvfp4 ? 16 : 8; }
 bool DenseEligible(const GemmParams& p);
 void LaunchDenseGemm(int mode, const GemmParams& p, int64_t m, cudaStream_t stream);  // throws std::runtime_error
@@ -289,8 +288,8 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
 bool LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);
 
 // SharedExpertDown over many rows; `split` of the plan is the cluster size (1, 2 or 4).  Calls of up to sixteen rows keep
-// the streaming kernels, whose results do not depend on the number of rows: 640 x 2560 NVFP4, eight rows 7 to 8 us a pass,
-// seventeen rows in the many-row kernel 11.
+// the streaming kernels, whose results do not depend on the number of rows: 640 x 2560 NVFP4 in a graph, eight rows 8.7 us,
+// nine in two passes 15 against 10.5 in the many-row kernel, sixteen 17 against 11.
 constexpr int kDenseSharedRows = 16;
 bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m);
 DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count);
