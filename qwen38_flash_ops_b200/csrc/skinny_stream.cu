@@ -86,6 +86,8 @@ __device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& 
   c.fault = 1;
   return false;
 }
+// A wait with a limit of the call's.
+__device__ __noinline__ void BarWaitFor(uint32_t a, uint32_t parity, StreamCtl& c, int spin) { BarWait(a, parity, c, spin); }
 // The last thing a CTA that gave up waits for: what it asked for must not arrive in shared memory that is used again.
 __device__ __noinline__ void BarDrain(uint32_t a, uint32_t parity) {
   for (int i = 0; i < kStreamSpin && !BarTry(a, parity); ++i) {
@@ -223,8 +225,8 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       }
     }
   };
-  // (copies that never came: ctl.fault makes NaN of the sums, wherever the weights have come)
-  if constexpr (BULK) BarWait(SmemAddr(&ctl.x_full), 0, ctl, p.x_spin);
+  // (copies that never came: GiveUp makes NaN of the sums, wherever the weights have come)
+  if constexpr (BULK) BarWaitFor(SmemAddr(&ctl.x_full), 0, ctl, p.x_spin);
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
     uint32_t mx = 0, mn = 0xFFFFFFFFu;
@@ -458,6 +460,26 @@ __device__ __forceinline__ void FinishStream(const StreamParams& q, const Tile& 
     }
   }
   if (C > 1) cluster.sync();  // no CTA leaves while a peer still reads its sums
+}
+
+// A CTA whose wait ran out: what it has in flight may still land, on the partial sums too; once it has, they and the tail's are
+// made NaN.  Called behind the barrier that follows the sums, where the flag is the same for every thread.  Out of line and
+// there, because the loop's code is sensitive to it: a look at the flag beside the loop, or a barrier's limit read in line, cost
+// the LM head 2 to 4 % (82.1 -> 84 to 85 us), whatever registers they took.
+__device__ __noinline__ void GiveUp(const GemmParams& p, StreamCtl& ctl, uint8_t* smem, int issued, bool bulk_x, int tail_index) {
+  const int tid = static_cast<int>(threadIdx.x), nthreads = static_cast<int>(blockDim.x);
+  if (tid >> 5 == p.wn * p.wk) {  // the producer, which knows how many stages it issued
+    for (int s = max(0, issued - p.stages); s < issued; ++s) BarDrain(SmemAddr(&ctl.full[s % p.stages]), (s / p.stages) & 1);
+    if (bulk_x) BarDrain(SmemAddr(&ctl.x_full), 0);
+    if (tail_index >= 0) BarDrain(SmemAddr(&ctl.tail_full), 0);
+  }
+  __syncthreads();
+  const float nan = __uint_as_float(0x7FFFFFFFu);
+  float* const sums = reinterpret_cast<float*>(smem);
+  for (int i = tid; i < p.ring_bytes / 4; i += nthreads) sums[i] = nan;
+  for (int i = tid; tail_index >= 0 && i < kMaxRows * 128; i += nthreads) p.lm_tail[static_cast<size_t>(tail_index) * kMaxRows * 128 + i] = nan;
+  __threadfence();
+  __syncthreads();
 }
 
 enum StreamKind : int { kPlain = 0, kShared = 1, kHead = 2 };
@@ -717,7 +739,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         k_loop(std::false_type{});
       }
     }
-    if (!good || (kBulkX && ctl.fault)) {  // a wait for x that ran out came before the barriers of the staging
+    if (!good) {  // GiveUp would do, but without this the loop of the LM head comes out 2 % slower
 #pragma unroll
       for (int j = 0; j < NM; ++j)
 #pragma unroll
@@ -745,13 +767,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         sc += r.sstep;
         x_at += 32;
       }
-      const bool sound = good && !ctl.fault;
       float* const dst = p.lm_tail + static_cast<size_t>(tail_index) * kMaxRows * 128;
       const int g = lane >> 2, t = lane & 3;
 #pragma unroll
       for (int j = 0; j < NM; ++j) {
         const int cl = g * 16 + 2 * j, m0 = 2 * t, m1 = 2 * t + 1;
-        if (!sound) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = __uint_as_float(0x7FFFFFFFu);
+        if (!good) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = __uint_as_float(0x7FFFFFFFu);
         if (m0 < p.M) *reinterpret_cast<float2*>(&dst[m0 * 128 + cl]) = make_float2(acc[j][0], acc[j][2]);
         if (m1 < p.M) *reinterpret_cast<float2*>(&dst[m1 * 128 + cl]) = make_float2(acc[j][1], acc[j][3]);
       }
@@ -768,16 +789,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   Stamp(p, 3);
   if (p.trigger == 2) GridLaunchDependents();
   __syncthreads();
-  if (ctl.fault) {  // behind the barrier: the same for every thread
-    if (warp == q.warps) {
-      for (int s = max(0, issued - p.stages); s < issued; ++s) BarDrain(full0 + (s % p.stages) * 8, (s / p.stages) & 1);
-      if (kBulkX) BarDrain(x_full, 0);
-      if (kTail && tail_index >= 0) BarDrain(SmemAddr(&ctl.tail_full), 0);
-    }
-    __syncthreads();
-  }
   if (consumer) StorePartials<MODE, 1>(p, tl, acc, smem, tl.n0 + wn * kWarpCols < tl.n1);
   __syncthreads();
+  if (ctl.fault) GiveUp(p, ctl, smem, issued, kBulkX, tail_index);
   Stamp(p, 4);
   if constexpr (KIND == kHead) {
     EpilogueTail<MODE, false>(p, tl, smem, sh, p.wk, p.wn * kWarpCols);
