@@ -118,6 +118,9 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
  * geometry of the general kernels ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296") and sends the call to them; "stream_plan"
  * = "width,wk,teams,cluster,tail" pins that of the kernel that streams the weights by tensor copies, "0" sends no call
  * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.
+ * Every wait of that kernel is bounded; a block whose wait ran out writes NaN for its columns (the winner of such a row
+ * of the LM head is a NaN), the call succeeds and the next one is whole.  "give_up" = 1, for tests, makes every block of
+ * an LM head act as if its wait for x had run out.
  * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken;
  * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape. */
 QFG_API int qfg_skinny_gemm_set_option(qfg_skinny_gemm* op, const char* key, const char* value);
@@ -231,9 +234,7 @@ QFG_API size_t qfg_lmhead_static_max_rows(void);
 QFG_API int qfg_lmhead_compute_static(const qfg_lmhead* op, const void* x, int64_t m, int64_t k,
                                       const qfg_tensor2d* weight, int64_t n, int64_t col_offset, int64_t* idx,
                                       float* val, uint64_t* key, void* logits, void* stream);
-/* The launch options of qfg_skinny_gemm_set_option for this node, "exchange_spin" (below), and "x_spin": the tries after which
- * a CTA stops waiting for its copy of x (default 1048576, each suspended by the hardware for a while).  A CTA that stops
- * waiting writes NaN for its columns, so the row's winner is a NaN; the call itself succeeds and the next one is whole. */
+/* The launch options of qfg_skinny_gemm_set_option for this node, and "exchange_spin" (below). */
 QFG_API int qfg_lmhead_set_option(qfg_lmhead* op, const char* key, const char* value);
 QFG_API void qfg_lmhead_destroy(qfg_lmhead* op);
 

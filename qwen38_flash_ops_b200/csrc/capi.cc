@@ -74,8 +74,8 @@ struct qfg_skinny_gemm {
   size_t w_scale_len = 0;
   int pdl_wait = 0;
   int force_slow = 0;
+  int give_up = 0;
   int exchange_spin = qfg::kExchangeSpin;  // sharded LM head: bound of the wait for a peer's keys (iterations)
-  int x_spin = qfg::kStreamSpin;           // LM head: bound of the wait for the copies of x (tries)
   int dense_rows = -1;  // calls with more rows take the many-row kernel (or the library GEMM); -1 = qfg::DenseRowsDefault(mode), 0 = never
   qfg::DenseTcPlan dense_plan;  // bm > 0: overrides the launch shape of that branch (set_option("dense_plan", "bm,split,pair,ks"))
   unsigned long long phase_times = 0;  // device address given through set_option("phase_times", ...)
@@ -93,7 +93,7 @@ struct qfg_skinny_gemm {
   qfg_skinny_gemm() = default;
   qfg_skinny_gemm(const qfg_skinny_gemm& o)
       : seg_outs(o.seg_outs), widths(o.widths), trigger(o.trigger), d_w_scale(o.d_w_scale), w_scale_len(o.w_scale_len),
-        pdl_wait(o.pdl_wait), force_slow(o.force_slow), exchange_spin(o.exchange_spin), x_spin(o.x_spin), dense_rows(o.dense_rows),
+        pdl_wait(o.pdl_wait), force_slow(o.force_slow), give_up(o.give_up), exchange_spin(o.exchange_spin), dense_rows(o.dense_rows),
         dense_plan(o.dense_plan), phase_times(o.phase_times), plan_spec(o.plan_spec), stream_spec(o.stream_spec) {}
 };
 
@@ -148,6 +148,7 @@ Prepared Prepare(const qfg_skinny_gemm& op, const void* x, int64_t m, int64_t k,
   p.trigger = op.trigger;
   p.pdl_wait = op.pdl_wait;
   p.force_slow = op.force_slow;
+  p.give_up = op.give_up;
   p.phase_times = reinterpret_cast<unsigned long long*>(static_cast<uintptr_t>(op.phase_times));
   int o = 0;
   size_t scale_off = 0;
@@ -383,7 +384,7 @@ int SetGemmOption(qfg_skinny_gemm* op, const char* key, const char* value) {
     op->dense_plan = plan;
   }
   else if (k == "exchange_spin") op->exchange_spin = std::max(0, std::atoi(value));
-  else if (k == "x_spin") op->x_spin = std::max(0, std::atoi(value));
+  else if (k == "give_up") op->give_up = std::atoi(value) != 0;
 #ifdef QFG_PHASE_TIMES
   else if (k == "phase_times") op->phase_times = std::strtoull(value, nullptr, 10);  // measurement builds only
 #endif
@@ -438,7 +439,6 @@ int LmheadComputeWithWorkspace(const qfg_lmhead* op, const void* x, int64_t m, i
     pr.params.lm_val = val;
     pr.params.lm_key_out = reinterpret_cast<unsigned long long*>(key);
     pr.params.lm_col_offset = col_offset;
-    pr.params.x_spin = call.x_spin;
     if (exchange != nullptr && exchange->world > 1) {
       if (exchange->world > QFG_MAX_RANKS || exchange->rank < 0 || exchange->rank >= exchange->world)
         throw InvalidArgument("LmHead: bad exchange (1 <= world <= 8, 0 <= rank < world)");

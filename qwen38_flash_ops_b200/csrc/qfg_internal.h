@@ -112,7 +112,6 @@ struct Segment {
   int svec = 4;   // cp.async width for the NVFP4 scale bytes of a row
 };
 
-constexpr int kStreamSpin = 1 << 20;  // skinny_stream.cu: bound of a wait (tries that the hardware suspends for a while)
 constexpr int kExchangeSpin = 1 << 22;  // default bound of the wait for a peer's words (iterations of about 50 ns)
 
 struct GemmParams {
@@ -126,6 +125,7 @@ struct GemmParams {
   int width[kMaxOut] = {};
   int trigger = 0;
   int pdl_wait = 0;
+  int give_up = 0;     // testing (skinny_stream.cu): 1: every CTA goes on as if its first wait had run out, the LM head's for x
   int force_slow = 0;  // testing: always take the BF16-MMA path of the quantised modes
   unsigned long long* phase_times = nullptr;  // [CTA][16] timer stamps; written only by builds with -DQFG_PHASE_TIMES
   // plan
@@ -156,7 +156,6 @@ struct GemmParams {
   int tail_split = 1;
   int tail_stride = 0;
   float* lm_tail = nullptr;
-  int x_spin = kStreamSpin;  // skinny_stream.cu: bound of the wait for the copies of x
 
   // SharedExpertDown (fuse != 0): x is replaced by swish_mul(x, x2) while it is staged, and the output is
   // routed + bf16(bf16(sum) * gate[m]) with gate[m] = bf16(sigmoid(bf16(dot(gx[m], gw)))).

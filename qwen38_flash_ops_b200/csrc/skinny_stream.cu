@@ -18,7 +18,7 @@
 // of the tensor map, a stage holds R / 2 even rows and R / 2 odd rows, the latter copied from the 16-byte boundary before
 // them, and `pitch` is 32 or 96 modulo 128.
 //
-// Every wait is bounded; a CTA that gives up on one writes NaN, once its copies in flight have landed.
+// Every wait is bounded; a CTA that gives up on one writes NaN.
 #include <cuda.h>
 
 #include <algorithm>
@@ -38,6 +38,8 @@ namespace {
 constexpr int kStreamWarps = 18;                             // consumers, at most
 constexpr int kStreamThreads = 32 * (kStreamWarps + 2);      // and the producer, and the LM head's tail warp
 constexpr int kStreamStages = 24;
+constexpr int kTriggerBehindWait = 3;                        // GemmParams::trigger of this kernel: 1 where the kernel itself waits
+constexpr int kStreamSpin = 1 << 20;  // tries of a wait, each suspended by the hardware for a while
 
 struct StreamParams {
   GemmParams g;
@@ -71,27 +73,17 @@ __device__ __forceinline__ void BarArrive(uint32_t a) {
 __device__ __forceinline__ void BarExpect(uint32_t a, uint32_t bytes) {
   asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool BarTry(uint32_t a, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-  return ok != 0;
-}
 // False if the wait ran out, or spun while another wait of this CTA had.  True says nothing of the other waits: a copy that has
 // landed is taken whatever became of the rest.
-__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& c, int spin = kStreamSpin) {
-  for (int i = 0; i < spin; ++i) {
-    if (BarTry(a, parity)) return true;
+__device__ __forceinline__ bool BarWait(uint32_t a, uint32_t parity, StreamCtl& c) {
+  for (int i = 0; i < kStreamSpin; ++i) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+    if (ok) return true;
     if ((i & 255) == 255 && c.fault) return false;
   }
   c.fault = 1;
   return false;
-}
-// A wait with a limit of the call's.
-__device__ __noinline__ void BarWaitFor(uint32_t a, uint32_t parity, StreamCtl& c, int spin) { BarWait(a, parity, c, spin); }
-// The last thing a CTA that gave up waits for: what it asked for must not arrive in shared memory that is used again.
-__device__ __noinline__ void BarDrain(uint32_t a, uint32_t parity) {
-  for (int i = 0; i < kStreamSpin && !BarTry(a, parity); ++i) {
-  }
 }
 // x in elements of eight bytes, an even number: a copy starts on 16 bytes
 __device__ __forceinline__ void TmaLoad(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -195,11 +187,15 @@ __device__ __forceinline__ RowShare ShareOf(const StreamParams& q, int warp) {
 // quantised modes scaled by a power of two and converted to FP16 (skinny_common.cuh).  A thread converts what it stored
 // or looked at itself, so that the whole takes two barriers and one trip to L2.  BULK: the producer has the rows copied, and
 // they are only waited for; that gave the LM head 3 us of 85 at four rows and cost calls of 5 to 17 us 0.3 us, so only the
-// head does it.  Returns true if the CTA must take the BF16 path.
+// head does it.  Returns true if the CTA must take the BF16 path (which reads x itself, copies or not).
+// Where the copies did not come, the rows are scaled by NaN and so are the sums: the stages of the weights come all the same, and
+// the loop would take them.  The look at the flag stands here because the loop's code is sensitive to what surrounds it: one beside
+// the loop or behind the sums, or a limit of the wait that is not a constant, cost heads 1 to 4 % (82.1 -> 84 to 85 us).
 template <int MODE, bool BULK>
 __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, StreamCtl& ctl,
                                              int padded, const RowShare& rs, int lane) {
   const GemmParams& p = q.g;
+  const float kNaN = __uint_as_float(0x7FFFFFFFu);
   constexpr int kBatch = 4;
   const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // K is a multiple of eight
   auto track = [&](const uint4& v, uint32_t& mx, uint32_t& mn) {
@@ -225,8 +221,7 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       }
     }
   };
-  // (copies that never came: GiveUp makes NaN of the sums, wherever the weights have come)
-  if constexpr (BULK) BarWaitFor(SmemAddr(&ctl.x_full), 0, ctl, p.x_spin);
+  if constexpr (BULK) BarWait(SmemAddr(&ctl.x_full), 0, ctl);
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
     uint32_t mx = 0, mn = 0xFFFFFFFFu;
@@ -254,7 +249,7 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
   }
   __syncthreads();  // without BULK: every warp also sees the mbarriers
   if constexpr (MODE == kBf16) {
-    if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = 1.f;  // for the epilogue, behind further barriers
+    if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = BULK && ctl.fault ? kNaN : 1.f;  // for the epilogue, behind further barriers
     return false;
   } else {
     // Power-of-two scale per row that puts the slice maximum in [2^14, 2^15).  Every non-zero element must land in the
@@ -267,7 +262,7 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       const int e = static_cast<int>(mx >> 7);  // BF16 exponent field of the row maximum
       const bool out = mx != 0 && (e < 32 || e >= 255 || static_cast<int>((mn + 1) >> 7) < e - 28);
       bad = bad || out;
-      const float sc = mx != 0 && !out ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
+      const float sc = BULK && ctl.fault ? kNaN : mx != 0 && !out ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
       if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f / sc;
       uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
 #pragma unroll 2
@@ -462,26 +457,6 @@ __device__ __forceinline__ void FinishStream(const StreamParams& q, const Tile& 
   if (C > 1) cluster.sync();  // no CTA leaves while a peer still reads its sums
 }
 
-// A CTA whose wait ran out: what it has in flight may still land, on the partial sums too; once it has, they and the tail's are
-// made NaN.  Called behind the barrier that follows the sums, where the flag is the same for every thread.  Out of line and
-// there, because the loop's code is sensitive to it: a look at the flag beside the loop, or a barrier's limit read in line, cost
-// the LM head 2 to 4 % (82.1 -> 84 to 85 us), whatever registers they took.
-__device__ __noinline__ void GiveUp(const GemmParams& p, StreamCtl& ctl, uint8_t* smem, int issued, bool bulk_x, int tail_index) {
-  const int tid = static_cast<int>(threadIdx.x), nthreads = static_cast<int>(blockDim.x);
-  if (tid >> 5 == p.wn * p.wk) {  // the producer, which knows how many stages it issued
-    for (int s = max(0, issued - p.stages); s < issued; ++s) BarDrain(SmemAddr(&ctl.full[s % p.stages]), (s / p.stages) & 1);
-    if (bulk_x) BarDrain(SmemAddr(&ctl.x_full), 0);
-    if (tail_index >= 0) BarDrain(SmemAddr(&ctl.tail_full), 0);
-  }
-  __syncthreads();
-  const float nan = __uint_as_float(0x7FFFFFFFu);
-  float* const sums = reinterpret_cast<float*>(smem);
-  for (int i = tid; i < p.ring_bytes / 4; i += nthreads) sums[i] = nan;
-  for (int i = tid; tail_index >= 0 && i < kMaxRows * 128; i += nthreads) p.lm_tail[static_cast<size_t>(tail_index) * kMaxRows * 128 + i] = nan;
-  __threadfence();
-  __syncthreads();
-}
-
 enum StreamKind : int { kPlain = 0, kShared = 1, kHead = 2 };
 
 #ifdef QFG_PHASE_TIMES
@@ -503,7 +478,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   __shared__ StreamScratch sx;
   __shared__ StreamCtl ctl;
   const GemmParams& p = q.g;
-  if (p.trigger == 1 && !p.pdl_wait) GridLaunchDependents();
+  if (p.trigger == 1) GridLaunchDependents();
   Stamp(p, 0);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   Tile tl = LocateTile(p);
@@ -573,7 +548,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         BarInit(empty0 + i * 8, q.team_warps);
       }
       BarInit(SmemAddr(&ctl.tail_full), 1);
-      ctl.fault = 0;
+      ctl.fault = kBulkX ? static_cast<uint32_t>(p.give_up) : 0u;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -621,7 +596,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
     // calls would pile up, CTAs of later calls in the places beside the running one's.  NVFP4 2560 x 2560 after itself, eight
     // rows, 12.2 -> 8.2 us a call (8.9 without programmatic launch); 1024 x 4096 and back, one row, 7.0 -> 6.3; 640 x 640 4.5 ->
     // 4.6; calls whose CTAs have their SMs to themselves the same.
-    if (p.trigger == 1) GridLaunchDependents();
+    if (p.trigger == kTriggerBehindWait) GridLaunchDependents();
     if (kBulkX && warp == q.warps) {
       if (ElectOne()) issue_x();
       __syncwarp();
@@ -657,13 +632,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
 #endif
   QFG_CLOCK(loop_begin);
 
-  int issued = min(p.stages, nst);  // by the producer
   if (warp == q.warps) {
     int slot = 0;
     uint32_t parity = 0;
-    for (; issued < nst; ++issued) {
+    for (int s = p.stages; s < nst; ++s) {
       if (!BarWait(empty0 + slot * 8, parity, ctl)) break;
-      if (ElectOne()) issue(issued, slot);
+      if (ElectOne()) issue(s, slot);
       __syncwarp();
       if (++slot == p.stages) {
         slot = 0;
@@ -739,7 +713,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
         k_loop(std::false_type{});
       }
     }
-    if (!good) {  // GiveUp would do, but without this the loop of the LM head comes out 2 % slower
+    if (!good) {
 #pragma unroll
       for (int j = 0; j < NM; ++j)
 #pragma unroll
@@ -788,10 +762,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
 #endif
   Stamp(p, 3);
   if (p.trigger == 2) GridLaunchDependents();
+  if (ctl.fault) __nanosleep(1000000);  // copies of a CTA that gave up may still be landing where the sums go now
   __syncthreads();
   if (consumer) StorePartials<MODE, 1>(p, tl, acc, smem, tl.n0 + wn * kWarpCols < tl.n1);
   __syncthreads();
-  if (ctl.fault) GiveUp(p, ctl, smem, issued, kBulkX, tail_index);
   Stamp(p, 4);
   if constexpr (KIND == kHead) {
     EpilogueTail<MODE, false>(p, tl, smem, sh, p.wk, p.wn * kWarpCols);
@@ -1132,6 +1106,7 @@ bool LaunchSkinnyStream(int mode, GemmParams& p, const StreamPlan& plan, cudaStr
     }
   }
   q.g = p;
+  if (p.pdl_wait && p.trigger == 1) q.g.trigger = kTriggerBehindWait;
   q.teams = plan.teams;
   q.team_wk = plan.wk;
   q.team_warps = l.wn * plan.wk;

@@ -163,9 +163,9 @@ def test_shapes_that_do_not_exist_are_refused(cuda):
 
 @pytest.mark.parametrize("mode,N,plan", [(0, 1040, ""), (1, 1040, "9,2,2,2"), (2, 4224, "2,1,2,1,3"), (2, 4352, "2,1,2,1,1"), (2, 384, "1,4,2,1")])
 @pytest.mark.parametrize("pdl_wait", [0, 1])
-def test_a_head_that_gave_up_on_x_says_so(cuda, mode, N, plan, pdl_wait):
-    """The limit of the wait for x is set to nothing: every logit is NaN although the weights are there, and the next call's are
-    the ones before."""
+def test_a_head_that_gave_up_says_so(cuda, mode, N, plan, pdl_wait):
+    """As if the wait for x had run out: every logit is NaN although the weights are there, and the next call's are the ones
+    before."""
     rng = np.random.default_rng(N + mode)
     K, M = 1032, 5
     x, w = to_dev(P.synth_x(rng, M, K), "bf16"), U.dev_weight(U.make_weight(rng, mode, K, N, False)[0], mode)
@@ -174,9 +174,9 @@ def test_a_head_that_gave_up_on_x_says_so(cuda, mode, N, plan, pdl_wait):
     head.set_option("pdl_wait", pdl_wait)
     first = head(x, w, N, logits=True)
     for _ in range(3):
-        head.set_option("x_spin", 0)
+        head.set_option("give_up", 1)
         _, val, _, logits = head(x, w, N, logits=True)
         assert torch.isnan(val).all() and torch.isnan(logits).all()
-        head.set_option("x_spin", 1 << 20)
+        head.set_option("give_up", 0)
         for a, b in zip(head(x, w, N, logits=True), first):
             assert torch.equal(a, b)
