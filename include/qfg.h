@@ -82,8 +82,8 @@ QFG_API const char* qfg_version(void);
  * op schema is SkinnyGemmOp, :818-840).  Attributes: `seg_outs` (number of outputs slicing
  * each weight), `widths` (output widths in order), optional `w_scale` (host floats, the
  * concatenated per-column scales of the quantised weights, uploaded once here), optional
- * `trigger` (0 off, 1 = release programmatic-dependent-launch dependents at kernel start,
- * 2 = after the K loop; a non-zero value is overridden by the environment variable
+ * `trigger` (0 off, 1 = release programmatic-dependent-launch dependents at kernel start, behind the
+ * kernel's own wait for its predecessor, 2 = after the K loop; a non-zero value is overridden by the environment variable
  * SKINNY_TRIGGER_FORCE as in the reference, :105-113).  Fails with QFG_INVALID_ARGUMENT
  * unless 1 <= n_seg <= 4 and sum(seg_outs) == n_widths <= 8. */
 QFG_API int qfg_skinny_gemm_create(const int64_t* seg_outs, int n_seg, const int64_t* widths, int n_widths,
@@ -111,10 +111,11 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
                             const qfg_tensor2d* weights, int n_weights, void* const* outs, int n_outs,
                             void* stream);
 
-/* Launch options that are not node attributes.  "pdl_wait" = 1 launches the kernel with the
- * programmatic-stream-serialisation attribute and makes it wait for its predecessor
- * (griddepcontrol.wait) only after its first weight tiles are in flight; trigger 1 then releases the dependents behind
- * that wait.  "plan" pins the
+/* Launch options that are not node attributes.  Outside a stream capture the kernels of the ordinary layouts are launched
+ * with the programmatic-stream-serialisation attribute and wait for their predecessor (griddepcontrol.wait) before they
+ * touch memory, so they see what stream order shows them.  That holds for a predecessor that was itself launched with
+ * the attribute as long as it executes that wait too, as such kernels have to.  "pdl_wait" = 1 launches the kernel so in
+ * captures too and makes it wait only after its first weight tiles are in flight.  "plan" pins the
  * geometry of the general kernels ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296") and sends the call to them; "stream_plan"
  * = "width,wk,teams,cluster,tail" pins that of the kernel that streams the weights by tensor copies, "0" sends no call
  * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.

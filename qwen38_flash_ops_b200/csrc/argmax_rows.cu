@@ -25,6 +25,7 @@
 
 #include "argmax_key.cuh"
 #include "qfg_internal.h"
+#include "stream_order.cuh"
 
 namespace qfg {
 namespace {
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(kThreads) ArgmaxRowsKernel(const T* __restrict
   const int C = static_cast<int>(gridDim.x);  // the cluster spans the grid's x extent
   const int c = static_cast<int>(blockIdx.x);
   const long long row = blockIdx.y;
-  const T* xr = x + row * V;
+  GridDependencyWait();
+  const T* xr = BehindWait(x) + row * V;
   const int tid = threadIdx.x, lane = tid & 31;
 
   // Row layout: `head` scalar elements up to the first 16-byte boundary, `nvec` vectors, a scalar tail;
@@ -291,13 +293,14 @@ cudaError_t LaunchT(const T* x, int64_t rows, int64_t V, int64_t* idx, float* va
   cfg.gridDim = dim3(static_cast<unsigned>(cluster), static_cast<unsigned>(rows), 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1] = OverlapAttribute();
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = MayOverlapPredecessor(s) ? 2 : 1;
   const bool few = (vecs + cluster - 1) / cluster <= static_cast<long long>(kThreads) * kFewLoads<T>;
   return cudaLaunchKernelEx(&cfg, few ? ArgmaxRowsKernel<T, true> : ArgmaxRowsKernel<T, false>, x, static_cast<long long>(V),
                             reinterpret_cast<long long*>(idx), val);

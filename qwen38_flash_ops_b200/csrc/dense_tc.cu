@@ -46,6 +46,7 @@
 #include <type_traits>
 
 #include "qfg_internal.h"
+#include "stream_order.cuh"
 #include "swish.cuh"
 #include "tensor_map.h"
 
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
     }
   }
   FenceBefore();
+  GridDependencyWait();
   __syncthreads();
   if constexpr (PAIR) cg::this_cluster().sync();  // the leader's barriers exist before the peer arrives on them
   FenceAfter();
@@ -814,6 +816,7 @@ __device__ __forceinline__ int SwishWarpsPerBlock(int stages) { return kSwishWar
 
 __device__ __forceinline__ void SwishRole(const DenseShared& q, Ctl& ctl, int warp, int lane, int rank, int m0, uint32_t smem, uint32_t block_bytes) {
   const DenseParams& p = q.d;
+  const uint16_t *const g_in = BehindWait(q.g), *const u_in = BehindWait(q.u);
   const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]);
   const int per_block = SwishWarpsPerBlock(p.stages), blocks = kSwishWarps / per_block, sub = warp / blocks;
   const int part = p.bm / q.cluster, chunk = lane & 7, rsub = lane >> 3;
@@ -832,8 +835,8 @@ __device__ __forceinline__ void SwishRole(const DenseShared& q, Ctl& ctl, int wa
         const int r = r0 + 4 * j + rsub, m = m0 + r;
         gv[j] = uv[j] = make_uint4(0, 0, 0, 0);
         if (r < last && m < p.M && col < p.K) {  // K is a multiple of eight
-          gv[j] = __ldg(reinterpret_cast<const uint4*>(q.g + static_cast<size_t>(m) * p.K + col));
-          uv[j] = __ldg(reinterpret_cast<const uint4*>(q.u + static_cast<size_t>(m) * p.K + col));
+          gv[j] = __ldg(reinterpret_cast<const uint4*>(g_in + static_cast<size_t>(m) * p.K + col));
+          uv[j] = __ldg(reinterpret_cast<const uint4*>(u_in + static_cast<size_t>(m) * p.K + col));
         }
       }
       if (!free && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
@@ -868,6 +871,7 @@ __device__ __forceinline__ void SwishRole(const DenseShared& q, Ctl& ctl, int wa
 // This CTA's share of the gates, by `warps` warps, to every CTA of the cluster: asynchronous stores that count their
 // bytes in on the receiver's barrier.
 __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, uint32_t bar, int warp, int warps, int lane, int rank, int m0) {
+  const uint16_t *const gx_in = BehindWait(q.gx), *const gw_in = BehindWait(q.gw);
   const int part = q.d.bm / q.cluster, p0 = rank * part;
   const bool vec = reinterpret_cast<uintptr_t>(q.gx) % 16 == 0 && reinterpret_cast<uintptr_t>(q.gw) % 16 == 0 && q.gk % 8 == 0;
   constexpr int kRows = 2, kAhead = 5;
@@ -876,7 +880,7 @@ __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, uint
     const int m = m0 + p0 + r0;
     if (vec) {
       const int chunks = q.gk >> 3;
-      const uint4* gw = reinterpret_cast<const uint4*>(q.gw);
+      const uint4* gw = reinterpret_cast<const uint4*>(gw_in);
       for (int c0 = lane; c0 < chunks; c0 += 32 * kAhead) {
         uint4 w[kAhead], x[kRows][kAhead];
 #pragma unroll
@@ -885,7 +889,7 @@ __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, uint
           w[i] = c < chunks ? __ldg(gw + c) : make_uint4(0, 0, 0, 0);
 #pragma unroll
           for (int j = 0; j < kRows; ++j) {
-            x[j][i] = c < chunks && m + j < q.d.M ? __ldg(reinterpret_cast<const uint4*>(q.gx + static_cast<size_t>(m + j) * q.gk) + c)
+            x[j][i] = c < chunks && m + j < q.d.M ? __ldg(reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m + j) * q.gk) + c)
                                                   : make_uint4(0, 0, 0, 0);
           }
         }
@@ -971,8 +975,8 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
   FenceAfter();
   const uint32_t tmem = ctl.tmem;
   // nothing of the call is read or written before this line: a predecessor may be writing any of it
-  if (q.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (q.trigger == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  GridDependencyWait();
+  if (q.trigger == 1) GridLaunchDependents();
   constexpr int kFirstSwish = kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps);
 
   // first the gates, by the warps that the sums need last
@@ -1016,7 +1020,7 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
       }
       __syncwarp();
     }
-    if (q.trigger == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (q.trigger == 2) GridLaunchDependents();
   } else if (warp >= kFirstSwish) {
     SwishRole(q, ctl, warp - kFirstSwish, lane, rank, t.m0, smem, block_bytes);
   } else if (MODE != kBf16 && warp >= 6) {
@@ -1115,13 +1119,16 @@ cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, 
   cfg.blockDim = dim3(static_cast<unsigned>(DenseThreads<MODE>()));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  if (cluster > 1) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  }
+  if (MayOverlapPredecessor(stream)) attr[cfg.numAttrs++] = OverlapAttribute();
   return cudaLaunchKernelEx(&cfg, DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS>, p);
 }
 
@@ -1145,10 +1152,9 @@ cudaError_t LaunchShared(const DenseShared& q, int ctas, size_t smem, cudaStream
   attr[0].val.clusterDim.x = static_cast<unsigned>(q.cluster);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1] = OverlapAttribute();
   cfg.attrs = attr;
-  cfg.numAttrs = q.pdl_wait ? 2 : 1;
+  cfg.numAttrs = q.pdl_wait || MayOverlapPredecessor(stream) ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, DenseSharedKernel<MODE>, q);
 }
 

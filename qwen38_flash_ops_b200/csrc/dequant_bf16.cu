@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "qfg_internal.h"
+#include "stream_order.cuh"
 
 namespace qfg {
 namespace {
@@ -44,12 +45,12 @@ struct RawChunk {
 };
 
 template <int MODE, bool ALIGNED>
-__device__ __forceinline__ RawChunk LoadChunk(const DequantParams& p, int r, int src_col) {
+__device__ __forceinline__ RawChunk LoadChunk(const DequantParams& p, const uint8_t* w, int r, int src_col) {
   RawChunk raw;
   raw.v = make_uint4(0, 0, 0, 0);
   raw.s = 0;
   if constexpr (MODE == kBf16) {
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(p.w) + static_cast<size_t>(r) * p.row_stride + src_col;
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(w) + static_cast<size_t>(r) * p.row_stride + src_col;
     if constexpr (ALIGNED) {
       raw.v = __ldg(reinterpret_cast<const uint4*>(src));
     } else {
@@ -59,7 +60,7 @@ __device__ __forceinline__ RawChunk LoadChunk(const DequantParams& p, int r, int
       raw.v = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
     }
   } else if constexpr (MODE == kFp8) {
-    const uint8_t* src = p.w + static_cast<size_t>(r) * p.row_stride + src_col;
+    const uint8_t* src = w + static_cast<size_t>(r) * p.row_stride + src_col;
     if constexpr (ALIGNED) {
       const uint2 q = __ldg(reinterpret_cast<const uint2*>(src));
       raw.v.x = q.x;
@@ -73,7 +74,7 @@ __device__ __forceinline__ RawChunk LoadChunk(const DequantParams& p, int r, int
     }
   } else {
     const size_t row_bytes = static_cast<size_t>(p.row_stride) * 9 / 16;
-    const uint8_t* row_p = p.w + static_cast<size_t>(r) * row_bytes;
+    const uint8_t* row_p = w + static_cast<size_t>(r) * row_bytes;
     const uint8_t* q = row_p + (src_col >> 1);
     if constexpr (ALIGNED) {
       raw.v.x = __ldg(reinterpret_cast<const uint32_t*>(q));
@@ -122,6 +123,8 @@ constexpr int kDequantRows = 4;
 
 template <int MODE, bool ALIGNED>
 __global__ void __launch_bounds__(256) DequantKernel(const DequantParams p) {
+  GridDependencyWait();
+  const uint8_t* const w = BehindWait(p.w);
   const int chunks_per_row = p.N / 8;
   const int row_groups = (p.K + kDequantRows - 1) / kDequantRows;
   const long long total = static_cast<long long>(row_groups) * chunks_per_row;
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(256) DequantKernel(const DequantParams p) {
     RawChunk raw[kDequantRows];
 #pragma unroll
     for (int i = 0; i < kDequantRows; ++i) {
-      if (r0 + i < p.K) raw[i] = LoadChunk<MODE, ALIGNED>(p, r0 + i, src_col);
+      if (r0 + i < p.K) raw[i] = LoadChunk<MODE, ALIGNED>(p, w, r0 + i, src_col);
     }
     float sc[8];
 #pragma unroll
@@ -165,12 +168,15 @@ __global__ void __launch_bounds__(256) DequantKernel(const DequantParams p) {
 }
 
 template <int MODE>
-void LaunchMode(const DequantParams& p, int blocks, cudaStream_t stream) {
-  if (p.aligned) {
-    DequantKernel<MODE, true><<<blocks, 256, 0, stream>>>(p);
-  } else {
-    DequantKernel<MODE, false><<<blocks, 256, 0, stream>>>(p);
-  }
+cudaError_t LaunchMode(const DequantParams& p, int blocks, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1] = {OverlapAttribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = MayOverlapPredecessor(stream) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, p.aligned ? DequantKernel<MODE, true> : DequantKernel<MODE, false>, p);
 }
 
 }  // namespace
@@ -183,13 +189,15 @@ cudaError_t LaunchDequant(const DequantParams& params, cudaStream_t stream) {
   const int sms = DeviceSmCount();
   const long long want = (total + 255) / 256;
   const int blocks = static_cast<int>(std::min<long long>(want, static_cast<long long>(sms) * 32));
+  cudaError_t err;
   switch (p.mode) {
-    case kBf16: LaunchMode<kBf16>(p, blocks, stream); break;
-    case kFp8: LaunchMode<kFp8>(p, blocks, stream); break;
-    case kNvfp4: LaunchMode<kNvfp4>(p, blocks, stream); break;
+    case kBf16: err = LaunchMode<kBf16>(p, blocks, stream); break;
+    case kFp8: err = LaunchMode<kFp8>(p, blocks, stream); break;
+    case kNvfp4: err = LaunchMode<kNvfp4>(p, blocks, stream); break;
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+  const cudaError_t last = cudaGetLastError();
+  return err == cudaSuccess ? last : err;
 }
 
 }  // namespace qfg

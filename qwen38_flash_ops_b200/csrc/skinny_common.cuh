@@ -9,6 +9,7 @@
 
 #include "argmax_key.cuh"
 #include "qfg_internal.h"
+#include "stream_order.cuh"
 
 namespace qfg {
 namespace {
@@ -170,10 +171,6 @@ __device__ __forceinline__ void Mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
   }
 }
-__device__ __forceinline__ void GridLaunchDependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void GridDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ int CeilLog2(int v) { return v <= 1 ? 0 : 32 - __clz(v - 1); }
 

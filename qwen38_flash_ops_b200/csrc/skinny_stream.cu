@@ -38,7 +38,6 @@ namespace {
 constexpr int kStreamWarps = 18;                             // consumers, at most
 constexpr int kStreamThreads = 32 * (kStreamWarps + 2);      // and the producer, and the LM head's tail warp
 constexpr int kStreamStages = 24;
-constexpr int kTriggerBehindWait = 3;                        // GemmParams::trigger of this kernel: 1 where the kernel itself waits
 constexpr int kStreamSpin = 1 << 20;  // tries of a wait, each suspended by the hardware for a while
 
 struct StreamParams {
@@ -195,6 +194,7 @@ template <int MODE, bool BULK>
 __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, StreamCtl& ctl,
                                              int padded, const RowShare& rs, int lane) {
   const GemmParams& p = q.g;
+  const uint16_t* const x = BehindWait(p.x);
   const float kNaN = __uint_as_float(0x7FFFFFFFu);
   constexpr int kBatch = 4;
   const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // K is a multiple of eight
@@ -207,7 +207,7 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
     }
   };
   auto copy = [&](int m, uint32_t& mx, uint32_t& mn) {
-    const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + tl.kbeg);
+    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * p.K + tl.kbeg);
     uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
 #pragma unroll 1
     for (int c = c_first; c < chunks; c += kBatch * step) {
@@ -291,13 +291,14 @@ __device__ __forceinline__ bool StageXShared(const StreamParams& q, const Tile& 
   const GemmParams& p = q.g;
   const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane, gate_chunks = p.gk >> 3;
   const uint4 zero = make_uint4(0, 0, 0, 0);
+  const uint16_t *const g_in = BehindWait(p.x), *const u_in = BehindWait(p.x2), *const gx_in = BehindWait(p.gx), *const gw_in = BehindWait(p.gw);
   constexpr int kGate = 5;  // chunks of the gate a lane asks for at once: 2560 elements
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
-    const uint4* g = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + tl.kbeg);
-    const uint4* u = reinterpret_cast<const uint4*>(p.x2 + static_cast<size_t>(m) * p.K + tl.kbeg);
-    const uint4* gx = reinterpret_cast<const uint4*>(p.gx + static_cast<size_t>(m) * p.gk);
-    const uint4* gw = reinterpret_cast<const uint4*>(p.gw);
+    const uint4* g = reinterpret_cast<const uint4*>(g_in + static_cast<size_t>(m) * p.K + tl.kbeg);
+    const uint4* u = reinterpret_cast<const uint4*>(u_in + static_cast<size_t>(m) * p.K + tl.kbeg);
+    const uint4* gx = reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m) * p.gk);
+    const uint4* gw = reinterpret_cast<const uint4*>(gw_in);
     uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
     uint4 gv = c_first < valid ? __ldg(g + c_first) : zero, uv = c_first < valid ? __ldg(u + c_first) : zero;
     for (int half = rs.part; half < 2; half += rs.wpr) {
@@ -478,7 +479,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   __shared__ StreamScratch sx;
   __shared__ StreamCtl ctl;
   const GemmParams& p = q.g;
-  if (p.trigger == 1) GridLaunchDependents();
   Stamp(p, 0);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   Tile tl = LocateTile(p);
@@ -552,9 +552,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
+    if (!p.pdl_wait) GridDependencyWait();  // without the option the weights are the predecessor's to write too
     if (kBulkX) asm volatile("bar.arrive 1, %0;" ::"r"(static_cast<int>(blockDim.x)) : "memory");  // the others may wait on the barriers
     if (ElectOne()) {
-      // x before the weights, so that it does not queue behind them - unless it is still the predecessor kernel's to write
+      // x before the weights, so that it does not queue behind them - unless it may still be the predecessor kernel's to write
       if (kBulkX && !p.pdl_wait) issue_x();
       for (int s = 0; s < p.stages && s < nst; ++s) issue(s, s);
       if constexpr (kTail) {
@@ -589,18 +590,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   if constexpr (KIND != kHead) {
     if (MODE != kBf16 && sg.w_scale != nullptr && first_n < tl.n1) first_scale = __ldg(sg.w_scale + first_n);
   }
-  // weights do not depend on the predecessor kernel, x may be its output
-  if (p.pdl_wait) {
-    GridDependencyWait();
-    // Not at the start: a kernel that itself still waits would let the next ones in, and where several CTAs fit an SM a chain of
-    // calls would pile up, CTAs of later calls in the places beside the running one's.  NVFP4 2560 x 2560 after itself, eight
-    // rows, 12.2 -> 8.2 us a call (8.9 without programmatic launch); 1024 x 4096 and back, one row, 7.0 -> 6.3; 640 x 640 4.5 ->
-    // 4.6; calls whose CTAs have their SMs to themselves the same.
-    if (p.trigger == kTriggerBehindWait) GridLaunchDependents();
-    if (kBulkX && warp == q.warps) {
-      if (ElectOne()) issue_x();
-      __syncwarp();
-    }
+  // with pdl_wait the weights do not depend on the predecessor kernel, x may be its output
+  GridDependencyWait();
+  // Not at the start: a kernel that itself still waits would let the next ones in, and where several CTAs fit an SM a chain of
+  // calls would pile up, CTAs of later calls in the places beside the running one's.  NVFP4 2560 x 2560 after itself, eight
+  // rows, 12.2 -> 8.2 us a call (8.9 without programmatic launch); 1024 x 4096 and back, one row, 7.0 -> 6.3; 640 x 640 4.5 ->
+  // 4.6; calls whose CTAs have their SMs to themselves the same.
+  if (p.trigger == 1) GridLaunchDependents();
+  if (kBulkX && p.pdl_wait && warp == q.warps) {
+    if (ElectOne()) issue_x();
+    __syncwarp();
   }
   if constexpr (KIND == kShared) {
     if (p.routed != nullptr && first_n < tl.n1 && rs.any && rs.row < p.M) first_routed = p.routed[static_cast<size_t>(rs.row) * sg.n + first_n];
@@ -889,11 +888,7 @@ cudaError_t Launch(const StreamParams& q, int tiles, int threads, size_t smem, c
     attr[n_attr].val.clusterDim.z = 1;
     ++n_attr;
   }
-  if (q.g.pdl_wait) {
-    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-    ++n_attr;
-  }
+  if (q.g.pdl_wait || MayOverlapPredecessor(stream)) attr[n_attr++] = OverlapAttribute();
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
   return cudaLaunchKernelEx(&cfg, SkinnyGemmStreamKernel<MODE, KIND>, q);
@@ -1106,7 +1101,6 @@ bool LaunchSkinnyStream(int mode, GemmParams& p, const StreamPlan& plan, cudaStr
     }
   }
   q.g = p;
-  if (p.pdl_wait && p.trigger == 1) q.g.trigger = kTriggerBehindWait;
   q.teams = plan.teams;
   q.team_wk = plan.wk;
   q.team_warps = l.wn * plan.wk;

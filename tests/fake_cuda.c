@@ -21,6 +21,8 @@ static char g_refuse_kernel[64];
 API void fake_refuse_setup_of(const char* part) { snprintf(g_refuse_kernel, sizeof g_refuse_kernel, "%s", part); }  /* kernels named so */
 API void fake_refuse_encode(int v) { g_refuse_encode = v; }
 API void fake_resident(int ctas) { g_resident = ctas; }  /* CTAs, one per SM, that clusters can have at once */
+static int g_capturing = -1;
+API void fake_capturing(int status) { g_capturing = status; }  /* of every stream: a cudaStreamCaptureStatus, or -1: cannot be asked for */
 API int fake_setup_calls(void) { return g_setup_calls; }
 API const char* fake_log(void) { return g_log; }
 API void fake_clear(void) { g_len = 0; g_log[0] = 0; }
@@ -90,6 +92,12 @@ API cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind
 API cudaError_t cudaMemset(void* p, int v, size_t n) { (void)p; (void)v; (void)n; return cudaSuccess; }
 API cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
 API cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
+API cudaError_t cudaStreamIsCapturing(cudaStream_t s, enum cudaStreamCaptureStatus* status) {
+  (void)s;
+  if (g_capturing < 0) return cudaErrorStreamCaptureImplicit;
+  *status = (enum cudaStreamCaptureStatus)g_capturing;
+  return cudaSuccess;
+}
 API cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 API const char* cudaGetErrorString(cudaError_t e) { static char b[32]; snprintf(b, sizeof b, "error %d", (int)e); return b; }
 

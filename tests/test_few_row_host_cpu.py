@@ -125,3 +125,25 @@ def test_a_device_that_reports_no_resident_block(fake):  # noqa: F811
         print(json.dumps(run_gemm(gemm([1], [128 * 600]), U8, 2, 512, [[128 * 600]])))
         """)
     assert out[0] == 0 and _kernel(out[2]) == ["SkinnyGemm"], out[1]
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP8", "U8"])
+@pytest.mark.parametrize("status,overlaps", [(0, True), (1, False), (2, False), (-1, False)])
+def test_launches_overlap_their_predecessor_outside_captures(fake, dtype, status, overlaps):  # noqa: F811
+    """Programmatic launches where the stream is known not to be captured, plain ones otherwise; `pdl_wait` asks for the former."""
+    logs = fake(f"""
+        fake.fake_capturing({status})
+        r = [run_gemm(gemm([1], [256]), {dtype}, m, 512, [[256]])[2] for m in (4, 40)]
+        r += [run_shared(shared(), {dtype}, m, 256, 128)[2] for m in (4, 40)]
+        fake.fake_clear()
+        assert lib.qfg_argmax_rows(BF16, P, 4, 4096, P, P, None) == 0
+        h = ctypes.c_void_p()
+        assert lib.qfg_dequant_create(256, 0, None, 0, None, 0, ctypes.byref(h)) == 0
+        w = L.Tensor2D(P, {dtype}, 512, cols({dtype}, 256))
+        assert lib.qfg_dequant_compute(h, ctypes.byref(w), (ctypes.c_void_p * 1)(P), 1, None) == 0
+        r.append(fake.fake_log().decode().split("\\n")[:-1])
+        print(json.dumps(r + [run_gemm(gemm([1], [256], pdl_wait=1), {dtype}, 4, 512, [[256]])[2]]))
+        """)
+    assert [len(log) for log in logs] == [1, 1, 1, 1, 2, 1]
+    assert all(line.endswith(f"pdl={int(overlaps)}") for log in logs[:5] for line in log)
+    assert logs[5][0].endswith("pdl=1")
