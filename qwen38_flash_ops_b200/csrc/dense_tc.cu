@@ -783,15 +783,19 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
 // ------------------------------------------------------------------------------ SharedExpertDown over many rows
 // out = routed + bf16(bf16(swish_mul(g, u) @ W) * gate), gate = bf16(sigmoid(bf16(gx . gw))), in the same tiles and
 // roles.  A tile of 128 columns is one of N / 128 that need the same rows of swish_mul, so the C CTAs of a cluster
-// (neighbouring column tiles, the same rows) each evaluate 1 / C of them: a warp or two per block of 64 k compute their
-// CTA's share, store it into this CTA's stage and send it to the others' with bulk copies between shared memories,
+// (neighbouring column tiles, the same rows) each evaluate a share of them: a warp or two per block of 64 k compute their
+// CTA's rows, store them into this CTA's stage and send them to the others' with bulk copies between shared memories,
 // which count themselves in on the receivers' barriers.  A stage is free when the MMAs of all C CTAs have read it
-// (multicast commits).  The gates are shared the same way, by the warps that have nothing to do yet.  A call is a few
-// trips to memory deep and little else, so every phase spreads over as many warps as it can: all of them finish the
-// sums (the four epilogue warps alone, 16 rows at a time, took half of a call).
+// (multicast commits).  The gates are shared the same way, by the warps that have nothing to do until the sums are complete,
+// which all warps finish.
 //
 // The streaming kernels that served these calls eight rows at a time took 1403 us for 777 rows of FP8 640 x 2560; this
-// one 25.5.  It is bound by swish_mul and latency: 0.6 us per block of 64 k at 160 rows against 0.17 us of MMAs.
+// one 16.8 in clusters of seven (25.5 with the dot products of the gates multiplied out ahead of the dequantisation and the outputs
+// written a column per lane, 23.4 of them on the device).  What bounds it there is the exchange: 67 KB leave and reach an SM in
+// 4500 cycles, 15 bytes a cycle, and a CTA needs 175 KB; `clock64` stamps, cycles: blocks evaluated 3500 to 7500 for the first,
+// first MMA 12 000, last 24 000, written 28 000.  With few rows it is set-up (3500 cycles until the CTAs have met), the gates'
+// trips to memory and 500 cycles a block of dequantisation (60 rows 9.8 us).
+// Joining the gates' warps as theirs ends, items taken in turn: no faster at 777 rows, 4 % slower at 60.
 struct DenseShared {
   DenseParams d;
   const uint16_t *g, *u, *gx, *gw, *routed;
@@ -800,6 +804,7 @@ struct DenseShared {
 };
 
 constexpr int kSwishWarps = 8;  // sixteen, at 64 registers a thread, measured no faster (27.0 us, and 5-10 % slower on small calls)
+constexpr int kGateWarps = 4;   // the first four, which have nothing else to do until the sums are complete
 template <int MODE>
 constexpr int SharedThreads() {
   return 32 * (kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps) + kSwishWarps);
@@ -813,121 +818,173 @@ __device__ __forceinline__ float SigmoidBf16(float a) {
 // Warps that share a block.  A barrier's parity tells a phase from the next only, so a warp must have seen a stage's
 // previous block consumed (or a later one) before it waits for the stage again: no more blocks in hand than stages.
 __device__ __forceinline__ int SwishWarpsPerBlock(int stages) { return kSwishWarps / (stages >= 8 ? 8 : stages >= 4 ? 4 : stages >= 2 ? 2 : 1); }
+// The rows of a tile that a rank evaluates: its share of the groups of eight.
+__device__ __forceinline__ int FirstRow(const DenseShared& q, int rank) { return rank * (q.d.bm >> 3) / q.cluster * 8; }
 
-__device__ __forceinline__ void SwishRole(const DenseShared& q, Ctl& ctl, int warp, int lane, int rank, int m0, uint32_t smem, uint32_t block_bytes) {
-  const DenseParams& p = q.d;
-  const uint16_t *const g_in = BehindWait(q.g), *const u_in = BehindWait(q.u);
-  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]);
-  const int per_block = SwishWarpsPerBlock(p.stages), blocks = kSwishWarps / per_block, sub = warp / blocks;
-  const int part = p.bm / q.cluster, chunk = lane & 7, rsub = lane >> 3;
-  // this warp's rows of the tile, in groups of eight: [first, last)
-  const int first = rank * part + sub * (part >> 3) / per_block * 8, last = rank * part + (sub + 1) * (part >> 3) / per_block * 8;
-  for (int k = warp % blocks; k < p.ksteps; k += blocks) {
-    const int stage = k % p.stages, round = k / p.stages;
-    const int col = k * kBk + chunk * 8;
-    const uint32_t dst = smem + static_cast<uint32_t>(stage) * block_bytes + kABytes;
-    bool free = round == 0;
-    constexpr int kBatch = 4;
-    for (int r0 = first; r0 < last; r0 += 4 * kBatch) {
-      uint4 gv[kBatch], uv[kBatch];
+// swish_mul by one warp: eight rows by 64 k at a time, the next eight asked for before these are computed.
+struct SwishRole {
+  const DenseShared& q;
+  const uint16_t *g, *u;
+  int lane, rank, m0, blocks, sub, first, last, k, r0;
+  uint4 gv[2], uv[2];
+
+  __device__ __forceinline__ SwishRole(const DenseShared& call, int warp, int lane_, int rank_, int m0_) : q(call), lane(lane_), rank(rank_), m0(m0_) {
+    if (warp < 0) return;  // another role's
+    const int per_block = SwishWarpsPerBlock(q.d.stages), begin = FirstRow(q, rank), groups = (FirstRow(q, rank + 1) - begin) >> 3;
+    blocks = kSwishWarps / per_block;
+    sub = warp / blocks;
+    first = begin + sub * groups / per_block * 8;
+    last = begin + (sub + 1) * groups / per_block * 8;
+    k = warp % blocks;
+    r0 = first;
+    g = BehindWait(q.g);
+    u = BehindWait(q.u);
+    Load(k, r0, gv, uv);
+  }
+  __device__ __forceinline__ void Load(int kk, int rr, uint4 (&a)[2], uint4 (&b)[2]) const {
+    const int col = kk * kBk + (lane & 7) * 8;
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int r = r0 + 4 * j + rsub, m = m0 + r;
-        gv[j] = uv[j] = make_uint4(0, 0, 0, 0);
-        if (r < last && m < p.M && col < p.K) {  // K is a multiple of eight
-          gv[j] = __ldg(reinterpret_cast<const uint4*>(g_in + static_cast<size_t>(m) * p.K + col));
-          uv[j] = __ldg(reinterpret_cast<const uint4*>(u_in + static_cast<size_t>(m) * p.K + col));
-        }
+    for (int j = 0; j < 2; ++j) {
+      const int r = rr + 4 * j + (lane >> 3), m = m0 + r;
+      a[j] = b[j] = make_uint4(0, 0, 0, 0);
+      if (r < last && m < q.d.M && col < q.d.K) {  // K is a multiple of eight
+        a[j] = __ldg(reinterpret_cast<const uint4*>(g + static_cast<size_t>(m) * q.d.K + col));
+        b[j] = __ldg(reinterpret_cast<const uint4*>(u + static_cast<size_t>(m) * q.d.K + col));
       }
-      if (!free && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
-      free = true;
+    }
+  }
+  __device__ __forceinline__ void Run(Ctl& ctl, uint32_t smem, uint32_t block_bytes) {
+    const DenseParams& p = q.d;
+    const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]);
+    const int chunk = lane & 7;
+    while (k < p.ksteps) {
+      const int stage = k % p.stages, round = k / p.stages;
+      const uint32_t dst = smem + static_cast<uint32_t>(stage) * block_bytes + kABytes;
+      int kn = k, rn = r0 + 8;
+      if (rn >= last) {
+        rn = first;
+        kn += blocks;
+      }
+      uint4 gn[2], un[2];
+      if (kn < p.ksteps) Load(kn, rn, gn, un);
+      // a warp without rows of its own still may not count itself in on a stage that is in use
+      if (r0 == first && round > 0 && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int r = r0 + 4 * j + rsub;
+      for (int j = 0; j < 2; ++j) {
+        const int r = r0 + 4 * j + (lane >> 3);
         if (r < last) {
           const uint32_t v[4] = {SwishMul2(gv[j].x, uv[j].x), SwishMul2(gv[j].y, uv[j].y), SwishMul2(gv[j].z, uv[j].z), SwishMul2(gv[j].w, uv[j].w)};
           Sts128(dst + static_cast<uint32_t>(r * 128 + ((chunk ^ (r & 7)) * 16)), v);
         }
       }
-    }
-    // a warp without rows of its own still may not count itself in on a stage that is in use
-    if (!free && !BarWait(empty0 + stage * 8, static_cast<uint32_t>((round - 1) & 1), ctl)) return;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (ElectOne()) {
-      const uint32_t bytes = static_cast<uint32_t>((last - first) * 128), bar = full0 + stage * 8, src = dst + static_cast<uint32_t>(first * 128);
-      BarExpect(bar, bytes * static_cast<uint32_t>(q.cluster - 1));  // what this warp's counterparts in the other CTAs send
-      for (int i = 1; i < q.cluster && bytes > 0; ++i) {
-        const uint32_t peer = static_cast<uint32_t>((rank + i) % q.cluster);
-        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(MapRank(src, peer)), "r"(src),
-                     "r"(bytes), "r"(MapRank(bar, peer))
-                     : "memory");
+      if (kn != k) {  // the warp's rows of this block are complete
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (ElectOne()) {
+          const uint32_t bytes = static_cast<uint32_t>((last - first) * 128), bar = full0 + stage * 8, src = dst + static_cast<uint32_t>(first * 128);
+          // one warp of the block counts in what the other CTAs send
+          const int mine = FirstRow(q, rank + 1) - FirstRow(q, rank);
+          if (sub == 0) {
+            BarExpect(bar, static_cast<uint32_t>((p.bm - mine) * 128));
+          } else {
+            BarArrive(bar);
+          }
+          int peer = rank;
+          for (int i = 1; i < q.cluster && bytes > 0; ++i) {
+            if (++peer == q.cluster) peer = 0;
+            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             MapRank(src, static_cast<uint32_t>(peer))),
+                         "r"(src), "r"(bytes), "r"(MapRank(bar, static_cast<uint32_t>(peer)))
+                         : "memory");
+          }
+        }
+        __syncwarp();
+      }
+      k = kn;
+      r0 = rn;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        gv[j] = gn[j];
+        uv[j] = un[j];
       }
     }
-    __syncwarp();
   }
-}
+};
 
-// This CTA's share of the gates, by `warps` warps, to every CTA of the cluster: asynchronous stores that count their
-// bytes in on the receiver's barrier.
-__device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, uint32_t bar, int warp, int warps, int lane, int rank, int m0) {
+// This CTA's share of the gates, to every CTA of the cluster: asynchronous stores that count their bytes in on the
+// receiver's barrier.  The dot products are MMAs of sixteen rows of gx with gw in every column: a lane reads 16 bytes of two
+// rows, eight k of its own, and the same eight of gw, so that the order of k within an MMA is free (multiplied out they were
+// 24 instructions per 16 bytes, a third of the call).  A warp takes a quarter of k; the quarters are added in order.
+__device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, float (*quarter)[256], uint32_t bar, int warp, int lane, int rank, int m0) {
   const uint16_t *const gx_in = BehindWait(q.gx), *const gw_in = BehindWait(q.gw);
-  const int part = q.d.bm / q.cluster, p0 = rank * part;
+  const int p0 = FirstRow(q, rank), part = FirstRow(q, rank + 1) - p0;
   const bool vec = reinterpret_cast<uintptr_t>(q.gx) % 16 == 0 && reinterpret_cast<uintptr_t>(q.gw) % 16 == 0 && q.gk % 8 == 0;
-  constexpr int kRows = 2, kAhead = 5;
-  for (int r0 = warp * kRows; r0 < part; r0 += warps * kRows) {
-    float acc[kRows] = {0.f, 0.f};
-    const int m = m0 + p0 + r0;
-    if (vec) {
-      const int chunks = q.gk >> 3;
+  if (vec) {
+    const int g = lane >> 2, t = lane & 3, chunks = q.gk >> 3, steps = (chunks + 3) >> 2, s1 = (warp + 1) * steps / kGateWarps;
+    constexpr int kAhead = 5;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int r0 = 0; r0 < part; r0 += 16) {
+      const int m = m0 + p0 + r0 + g;
+      const bool lo_in = m < q.d.M, hi_in = m + 8 < q.d.M && r0 + 8 < part;
+      const uint4* lo_row = reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m) * q.gk);
+      const uint4* hi_row = reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m + 8) * q.gk);
       const uint4* gw = reinterpret_cast<const uint4*>(gw_in);
-      for (int c0 = lane; c0 < chunks; c0 += 32 * kAhead) {
-        uint4 w[kAhead], x[kRows][kAhead];
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int s = warp * steps / kGateWarps; s < s1; s += kAhead) {
+        uint4 lo[kAhead], hi[kAhead], w[kAhead];
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-          const int c = c0 + 32 * i;
-          w[i] = c < chunks ? __ldg(gw + c) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-          for (int j = 0; j < kRows; ++j) {
-            x[j][i] = c < chunks && m + j < q.d.M ? __ldg(reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m + j) * q.gk) + c)
-                                                  : make_uint4(0, 0, 0, 0);
-          }
+          const int at = (s + i) * 4 + t;
+          const bool in = s + i < s1 && at < chunks;  // nothing past the end is added, not even to an infinity
+          lo[i] = in && lo_in ? __ldg(lo_row + at) : zero;
+          hi[i] = in && hi_in ? __ldg(hi_row + at) : zero;
+          w[i] = in ? __ldg(gw + at) : zero;
         }
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-          const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
-#pragma unroll
-          for (int j = 0; j < kRows; ++j) {
-            const uint32_t xx[4] = {x[j][i].x, x[j][i].y, x[j][i].z, x[j][i].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              acc[j] += Lo(xx[e]) * Lo(ww[e]);
-              acc[j] += Hi(xx[e]) * Hi(ww[e]);
-            }
-          }
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo[i].x), "r"(hi[i].x), "r"(lo[i].y), "r"(hi[i].y), "r"(w[i].x), "r"(w[i].y));
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo[i].z), "r"(hi[i].z), "r"(lo[i].w), "r"(hi[i].w), "r"(w[i].z), "r"(w[i].w));
         }
       }
-    } else {
+      if (t == 0) {
+        quarter[warp][r0 + g] = c[0];
+        if (r0 + 8 < part) quarter[warp][r0 + 8 + g] = c[2];
+      }
+    }
+  } else {
+    // element by element, four rows at a time
+    for (int r0 = warp * 4; r0 < part; r0 += kGateWarps * 4) {
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      const int m = m0 + p0 + r0;
+#pragma unroll 2
       for (int c = lane; c < q.gk; c += 32) {
-        const float w = __uint_as_float(static_cast<uint32_t>(q.gw[c]) << 16);
+        const float w = __uint_as_float(static_cast<uint32_t>(gw_in[c]) << 16);
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) {
-          if (m + j < q.d.M) acc[j] += __uint_as_float(static_cast<uint32_t>(q.gx[static_cast<size_t>(m + j) * q.gk + c]) << 16) * w;
+        for (int j = 0; j < 4; ++j) {
+          if (m + j < q.d.M) acc[j] += __uint_as_float(static_cast<uint32_t>(gx_in[static_cast<size_t>(m + j) * q.gk + c]) << 16) * w;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
+        if (lane == 0) {
+          quarter[0][r0 + j] = acc[j];
+          quarter[1][r0 + j] = quarter[2][r0 + j] = quarter[3][r0 + j] = 0.f;
         }
       }
     }
-#pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
-    }
-    // lane = (peer, row): part is even, so both rows exist
-    const float logit = (lane & 1) ? acc[1] : acc[0];
-    const int peer = lane >> 1;
-    if (peer < q.cluster) {
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
-                       MapRank(Smem(gate + p0 + r0 + (lane & 1)), static_cast<uint32_t>(peer))),
-                   "r"(__float_as_uint(SigmoidBf16(RoundBf16(logit)))), "r"(MapRank(bar, static_cast<uint32_t>(peer)))
+  }
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * kGateWarps) : "memory");
+  for (int r = warp * 32 + lane; r < part; r += 32 * kGateWarps) {
+    const float logit = ((quarter[0][r] + quarter[1][r]) + quarter[2][r]) + quarter[3][r];
+    const uint32_t value = __float_as_uint(SigmoidBf16(RoundBf16(logit))), at = Smem(gate + p0 + r);
+    for (int peer = 0; peer < q.cluster; ++peer) {
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(MapRank(at, static_cast<uint32_t>(peer))), "r"(value),
+                   "r"(MapRank(bar, static_cast<uint32_t>(peer)))
                    : "memory");
     }
   }
@@ -937,7 +994,7 @@ template <int MODE>
 __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(const __grid_constant__ DenseShared q) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Ctl ctl;
-  __shared__ float gate[256];
+  __shared__ float gate[256], quarter[kGateWarps][256];
   __shared__ unsigned long long gate_full;
   const DenseParams& p = q.d;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -969,22 +1026,20 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(Smem(&ctl.tmem)), "r"(acc_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // nothing of the call is read or written before this line: a predecessor may be writing any of it
+  GridDependencyWait();
+  if (q.trigger == 1) GridLaunchDependents();
+  constexpr int kFirstSwish = kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps), kSumGroups = (kFirstSwish + kSwishWarps) / 4;
+  SwishRole swish(q, warp - kFirstSwish, lane, rank, t.m0);  // its first rows are on their way while the CTAs meet
   FenceBefore();
   __syncthreads();
   if (C > 1) cg::this_cluster().sync();  // every CTA's barriers exist
   FenceAfter();
   const uint32_t tmem = ctl.tmem;
-  // nothing of the call is read or written before this line: a predecessor may be writing any of it
-  GridDependencyWait();
-  if (q.trigger == 1) GridLaunchDependents();
-  constexpr int kFirstSwish = kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps);
 
-  // first the gates, by the warps that the sums need last
-  constexpr int kGateWarps = MODE == kBf16 ? 6 : 4 + kDqWarps, kSumGroups = (kFirstSwish + kSwishWarps) / 4;
-  const int gate_warp = warp < 4 ? warp : MODE == kBf16 ? (warp == 6 || warp == 7 ? warp - 2 : -1) : warp >= kFirstDqWarp && warp < kFirstSwish ? warp - 4 : -1;
-  if (gate_warp >= 0) GateRole(q, gate, Smem(&gate_full), gate_warp, kGateWarps, lane, rank, t.m0);
-
-  if (warp == 4) {
+  if (warp < kGateWarps) {
+    GateRole(q, gate, quarter, Smem(&gate_full), warp, lane, rank, t.m0);
+  } else if (warp == 4) {
     if constexpr (MODE == kBf16) {
       for (int k = 0; k < p.ksteps; ++k) {
         const int stage = k % p.stages, round = k / p.stages;
@@ -1022,7 +1077,7 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
     }
     if (q.trigger == 2) GridLaunchDependents();
   } else if (warp >= kFirstSwish) {
-    SwishRole(q, ctl, warp - kFirstSwish, lane, rank, t.m0, smem, block_bytes);
+    swish.Run(ctl, smem, block_bytes);
   } else if (MODE != kBf16 && warp >= 6) {
     const uint32_t ring = smem + static_cast<uint32_t>(p.stages) * block_bytes;
     if constexpr (MODE != kBf16) {
@@ -1035,43 +1090,90 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
     }
   }
 
-  // the sums, by every warp: lane = column 32 (warp % 4) + lane of the tile, sixteen rows at a time
+  // The sums, by every warp: columns 32 (warp % 4) ... of the tile, sixteen rows at a time.  They come as fragments, columns
+  // of W down and rows of x across, are scaled and rounded as such, and go through shared memory (where the stored
+  // weights were, which nobody else writes or reads) transposed, so that routed is read and the output written
+  // 16 bytes at a time.  A column per lane, two bytes an access, took a fifth of the call: 9500 of 42 100 cycles for 160 rows.
   __syncwarp();
   {
     const DenseSeg& sg = p.seg[0];
-    const int quad = warp & 3, n = t.n0 + 32 * quad + lane;
-    const bool mine = n < sg.n;
-    const float scale = mine && sg.w_scale != nullptr ? __ldg(sg.w_scale + n) : 1.f;
-    const uint32_t src = tmem + (static_cast<uint32_t>(32 * quad) << 16);
+    const int quad = warp & 3, n0 = t.n0 + 32 * quad, chunk = lane & 3, row = lane >> 2, n = n0 + 8 * chunk;  // widths are multiples of eight
+    float scale[2][2];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int at = n0 + 8 * h + row;
+      scale[h >> 1][h & 1] = at < sg.n && sg.w_scale != nullptr ? __ldg(sg.w_scale + at) : 1.f;
+    }
+    const uint32_t src = tmem + (static_cast<uint32_t>(32 * quad) << 16), buf = smem + static_cast<uint32_t>(p.stages) * block_bytes + static_cast<uint32_t>(warp * 16 * kOutPitch);
+    const uint32_t st = buf + static_cast<uint32_t>((((lane >> 4) & 1) * 8 + (lane & 7)) * kOutPitch + ((lane >> 3) & 1) * 16);
+    const uint32_t ld = buf + static_cast<uint32_t>(row * kOutPitch + chunk * 16);
     const size_t at0 = static_cast<size_t>(t.m0) * sg.n + n;
     uint16_t* const out = p.out[0] + at0;
     const uint16_t* const routed = q.routed != nullptr ? q.routed + at0 : nullptr;
+    const bool vec_out = reinterpret_cast<uintptr_t>(p.out[0]) % 16 == 0, vec_in = reinterpret_cast<uintptr_t>(q.routed) % 16 == 0;
     bool good = true, waited = false;
     for (int c = 16 * (warp >> 2); c < p.bm && t.m0 + c < p.M; c += 16 * kSumGroups) {
-      uint32_t v[16], rt[16];
+      uint32_t rt[2][4];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) rt[i] = mine && routed != nullptr && t.m0 + c + i < p.M ? routed[static_cast<size_t>(c + i) * sg.n] : 0;
+      for (int i = 0; i < 2; ++i) {
+        const int r = c + 8 * i + row;
+        rt[i][0] = rt[i][1] = rt[i][2] = rt[i][3] = 0;
+        if (n < sg.n && routed != nullptr && t.m0 + r < p.M) {
+          const uint16_t* const from = routed + static_cast<size_t>(r) * sg.n;
+          if (vec_in) {
+            const uint4 v = *reinterpret_cast<const uint4*>(from);
+            rt[i][0] = v.x, rt[i][1] = v.y, rt[i][2] = v.z, rt[i][3] = v.w;
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) rt[i][e >> 1] |= static_cast<uint32_t>(from[e]) << (16 * (e & 1));
+          }
+        }
+      }
       if (!waited) {
         good = BarWaitCluster(Smem(&gate_full), 0, ctl) && BarWait(accf0, 0, ctl);
         waited = true;
         __syncwarp();
         FenceAfter();
       }
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-            "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(src + static_cast<uint32_t>(c)));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (mine) {
+      uint32_t v[2][8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          if (t.m0 + c + i < p.M) {
+      for (int h = 0; h < 2; ++h) {
+        uint32_t(&f)[8] = v[h];
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]), "=r"(f[4]), "=r"(f[5]), "=r"(f[6]), "=r"(f[7])
+                     : "r"(src + (static_cast<uint32_t>(16 * h) << 16) + static_cast<uint32_t>(c)));
+      }
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      __syncwarp();  // the rows before have been read
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = PackBf16(__uint_as_float(v[h][2 * i]) * scale[h][i & 1], __uint_as_float(v[h][2 * i + 1]) * scale[h][i & 1]);
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(st + h * 32), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                     : "memory");
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = c + 8 * i + row;
+        if (n < sg.n && t.m0 + r < p.M) {
+          const float gt = gate[r];
+          uint32_t o[4];
+          Lds128(ld + i * (8 * kOutPitch), o);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
             // every step rounded to BF16 (the reference's skinny_gemm.cuh:226-240)
-            float y = RoundBf16(RoundBf16(__uint_as_float(v[i]) * scale) * gate[c + i]);
-            if (routed != nullptr) y += __uint_as_float(rt[i] << 16);
-            if (!good) y = __uint_as_float(0x7FFFFFFFu);
-            out[static_cast<size_t>(c + i) * sg.n] = __bfloat16_as_ushort(__float2bfloat16(y));
+            float lo = RoundBf16(Lo(o[e]) * gt), hi = RoundBf16(Hi(o[e]) * gt);
+            if (routed != nullptr) lo += Lo(rt[i][e]), hi += Hi(rt[i][e]);
+            o[e] = good ? PackBf16(lo, hi) : 0x7FFF7FFFu;
+          }
+          uint16_t* const dst = out + static_cast<size_t>(r) * sg.n;
+          if (vec_out) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) dst[e] = static_cast<uint16_t>(o[e >> 1] >> (16 * (e & 1)));
           }
         }
       }
@@ -1103,6 +1205,9 @@ bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_
 }
 
 constexpr int kSmemLimit = 232448 - 1024 - static_cast<int>(sizeof(Ctl)) - 64;
+
+// DenseSharedKernel has the gates and their quarters besides
+constexpr int kSharedSmemLimit = kSmemLimit - 1024 * (1 + kGateWarps) - 64;
 
 int RawBytes(int mode, int ks) {
   if (mode == kFp8) return ks == 2 ? RawRing<kFp8, 2>::kBytes : RawRing<kFp8, 1>::kBytes;
@@ -1185,7 +1290,7 @@ cudaError_t SetUpMode() {
 }
 template <int MODE>
 cudaError_t SetUpShared() {
-  return cudaFuncSetAttribute(DenseSharedKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - 1024);
+  return cudaFuncSetAttribute(DenseSharedKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedSmemLimit);
 }
 
 // A GPC's SMs rarely divide by the size (33 clusters of four, fewer than 16 of eight), and a cluster too many costs a
@@ -1393,9 +1498,12 @@ bool DenseSharedEligible(int mode, const GemmParams& p, int64_t m) {
   return p.fuse && p.nseg == 1 && DenseTcEligible(mode, p, m) && reinterpret_cast<uintptr_t>(p.x2) % 16 == 0;
 }
 
-// Rows per tile and CTAs per cluster, by a model fitted to measured launches (us): a block of 64 k costs 0.10 + 0.0125
-// rows of swish_mul per CTA, or its MMAs and dequantisation where those take longer; around the blocks 6 + 0.02 bm +
-// 0.05 rows of the gate per CTA.
+// Rows per tile and CTAs per cluster, by a model fitted to measured launches (us).  `own`: the rows that a CTA evaluates.  A
+// block of 64 k costs 0.027 for each of them, and no less than 0.4 (dequantisation, MMAs, the waits between the roles); around the
+// blocks 1.6 + 0.0064 bm, 0.14 for each gate of 2560 elements, 1.4 + 0.19 c where CTAs share.  On 52 shapes (17 to 2048
+// rows, K 256 to 2560, N 1024 to 5120, the three types) the shape chosen takes 0.4 % longer than the best of the 100 tried, 8 %
+// at worst (BF16 2048 rows 2560 x 1024 43.5 us, 40.4 in tiles of 128 and clusters of four); the model before this
+// one, made for clusters of up to four with even shares, 3 % and 22 % (FP8 621 rows 2256 x 2400 34.4, 28.3).
 DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) {
   const DeviceSetup* setup = nullptr;
   if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SharedExpertDown: the kernels could not be set up on this device");
@@ -1403,18 +1511,19 @@ DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) 
   double best_cost = 1e30;
   const int64_t n_tiles = (p.seg[0].n + kBn - 1) / kBn;
   const double blocks = (p.K + kBk - 1) / kBk;
-  for (int c = 1; c <= 4; c *= 2) {
+  for (int c = 1; c <= kMaxCluster; ++c) {
     const int64_t slots = c == 1 ? sm_count : setup->slots[c], groups = (n_tiles + c - 1) / c;
     if (slots < 1) break;
-    const int unit = c == 4 ? 32 : 16;
-    for (int bm = unit; bm <= 256; bm += unit) {
+    for (int bm = (8 * c + 15) / 16 * 16; bm <= 256; bm += 16) {
       const int64_t waves = (groups * ((m + bm - 1) / bm) + slots - 1) / slots;
-      const double block = std::max(0.10 + 0.0125 * bm / c, 0.30 + 0.0011 * bm);
-      const double cost = waves * (blocks * block + 6 + 0.02 * bm + 0.05 * bm / c);
+      const int own = (bm / 8 + c - 1) / c * 8;
+      const double block = std::max(0.004 + 0.027 * own + 0.00024 * (bm - own), 0.40 + 0.00014 * bm);
+      const double cost = waves * (blocks * block + 1.6 + 0.0064 * bm + 0.14 / 2560 * own * p.gk + (c > 1 ? 1.4 + 0.19 * c : 0.0));
       if (cost < best_cost) {
         best_cost = cost;
         best.bm = bm;
         best.split = c;
+        best.ks = 1;
       }
     }
   }
@@ -1424,7 +1533,9 @@ DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) 
 bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int mode = KernelMode(weights, g);
   const int C = plan.split;
-  if ((C != 1 && C != 2 && C != 4) || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm % (8 * C) != 0)
+  // a pinned shape has even shares in a cluster of up to four, unless it names the blocks per stage, of which there is one
+  const bool even = (C == 1 || C == 2 || C == 4) && plan.bm % (8 * C) == 0;
+  if (C < 1 || C > kMaxCluster || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm < 8 * C || (!even && plan.ks != 1))
     throw std::runtime_error("SharedExpertDown: bad launch shape");
   DenseShared q = {};
   DenseParams& p = q.d;
@@ -1443,7 +1554,9 @@ bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseT
   p.m_tiles = static_cast<int>(m_tiles);
   p.tiles = static_cast<int>(n_tiles * m_tiles);
   const int block = kABytes + p.bm * kBk * 2;
-  p.stages = std::min(kMaxStages, (kSmemLimit - 2048 - RawBytes(mode, 1)) / block);
+  // behind the stages the stored weights, and in their place each warp's buffer for the outputs
+  const int behind = std::max(RawBytes(mode, 1), (mode == kBf16 ? SharedThreads<kBf16>() : SharedThreads<kFp8>()) / 32 * 16 * kOutPitch);
+  p.stages = std::min(kMaxStages, (kSharedSmemLimit - 1024 - behind) / block);
   q.g = g.x;
   q.u = g.x2;
   q.gx = g.gx;
@@ -1453,7 +1566,7 @@ bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseT
   q.cluster = C;
   q.trigger = g.trigger;
   q.pdl_wait = g.pdl_wait;
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + RawBytes(mode, 1);
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * block + behind;
   // like the streaming kernels that take the shorter calls of this op, it runs on the device they were set up for
   cudaError_t err = CheckConfiguredDevice();
   if (err == cudaSuccess) err = ConfigureDenseKernels();

@@ -286,7 +286,7 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
 // std::runtime_error (a launch shape that does not exist, a launch that failed).
 bool LaunchDenseTc(int mode, const GemmParams& p, int64_t m, const DenseTcPlan& plan, cudaStream_t stream);
 
-// SharedExpertDown over many rows; `split` of the plan is the cluster size (1, 2 or 4).  Calls of up to sixteen rows keep
+// SharedExpertDown over many rows; `split` of the plan is the cluster size (1 to 8).  Calls of up to sixteen rows keep
 // the streaming kernels, whose results do not depend on the number of rows: 640 x 2560 NVFP4 in a graph, eight rows 8.7 us,
 // nine in two passes 15 against 10.5 in the many-row kernel, sixteen 17 against 11.
 constexpr int kDenseSharedRows = 16;

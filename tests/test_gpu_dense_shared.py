@@ -1,5 +1,7 @@
 """The many-row kernel of SharedExpertDown (csrc/dense_tc.cu) at the edges of its tiles and clusters, and its sigmoid on
 every BF16 value."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -7,6 +9,7 @@ import torch
 from conftest import bits, to_dev
 from oracle import oracle as O
 from qwen38_flash_ops_b200 import QfgError, SharedExpertDown, SkinnyGemm
+from qwen38_flash_ops_b200 import _lib as L
 from qwen38_flash_ops_b200 import packing as P
 
 import _util as U
@@ -57,6 +60,44 @@ def test_tile_and_cluster_edges(cuda, mode, plan):
         _run(mode, M, K, N, gk, plan, 100 * mode + i)
 
 
+# clusters whose CTAs have unequal shares of the rows, or columns past the end
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["32,3,0,1", "48,5,0,1", "64,7,0,1", "80,8,0,1", "160,7,0,1", "256,6,0,1"])
+def test_uneven_shares(cuda, mode, plan):
+    """Whoever evaluates a row, sums and gates are added in one order: the bits of the launch without clusters."""
+    gen = torch.Generator(device="cuda").manual_seed(mode)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    for M, K, N, gk in ((17, 256, 128, 256), (170, 648, 1152, 1000), (35, 1096, 640, 26)):
+        w = [mk(K, N), mk(K, N).to(torch.float8_e4m3fn), torch.randint(0, 0x70, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)][mode]
+        args = mk(M, K), mk(M, K), w, mk(M, gk) * 0.2, mk(gk, 1) * 0.2, mk(M, N)
+        op = SharedExpertDown()
+        op.set_option("dense_plan", "32,1")
+        want = op(*args)
+        op.set_option("dense_plan", plan)
+        assert torch.equal(op(*args), want)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_outputs_off_sixteen_bytes(cuda, mode):
+    """routed, and the output that is made beside it, at an odd element: the same values, two bytes at a time."""
+    gen = torch.Generator(device="cuda").manual_seed(mode)
+    M, K, N = 70, 256, 384
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    w = [mk(K, N), mk(K, N).to(torch.float8_e4m3fn), torch.randint(0, 0x70, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)][mode]
+    g, u, gx, gw, routed = mk(M, K), mk(M, K), mk(M, 64), mk(64, 1), mk(M, N)
+    op = SharedExpertDown()
+    want = op(g, u, w, gx, gw, routed)
+    for shift_in, shift_out in ((1, 0), (0, 1), (3, 5)):
+        src, dst = torch.zeros(M * N + 8, dtype=torch.bfloat16, device="cuda"), torch.zeros(M * N + 8, dtype=torch.bfloat16, device="cuda")
+        src[shift_in:shift_in + M * N] = routed.reshape(-1)
+        t = L.Tensor2D(w.data_ptr(), [L.QFG_BFLOAT16, L.QFG_FLOAT8E4M3FN, L.QFG_UINT8][mode], *w.shape)
+        code = L.load().qfg_shared_expert_down_compute(op._h, g.data_ptr(), u.data_ptr(), M, K, ctypes.byref(t), gx.data_ptr(), 64, gw.data_ptr(),
+                                                       src.data_ptr() + 2 * shift_in, N, dst.data_ptr() + 2 * shift_out, torch.cuda.current_stream().cuda_stream)
+        assert code == 0
+        assert torch.equal(dst[shift_out:shift_out + M * N].view(M, N), want)
+        assert not dst[:shift_out].any() and not dst[shift_out + M * N:].any()
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_layouts_on_either_side_of_the_route(cuda, mode):
     _run(mode, 40, 256, 128, 64, "", 7, gx_offset=1)               # gate read element by element
@@ -66,7 +107,7 @@ def test_layouts_on_either_side_of_the_route(cuda, mode):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
-@pytest.mark.parametrize("plan", ["160,4", "256,4", "64,2", "32,1"])
+@pytest.mark.parametrize("plan", ["160,4", "256,4", "64,2", "32,1", "160,7,0,1", "80,8,0,1"])
 def test_repeated_calls_agree(cuda, mode, plan):
     """A stage reused before every CTA of the cluster has read it shows as a run that differs."""
     gen = torch.Generator(device="cuda").manual_seed(3)
