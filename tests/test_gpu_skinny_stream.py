@@ -180,3 +180,44 @@ def test_a_head_that_gave_up_says_so(cuda, mode, N, plan, pdl_wait):
         head.set_option("give_up", 0)
         for a, b in zip(head(x, w, N, logits=True), first):
             assert torch.equal(a, b)
+
+
+# what stands among ordinary values of x: [2^-22, 2^11) is scaled in one look, the rest row by row or not at all
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("kind", ["plain", "cluster", "shared", "head"])
+@pytest.mark.parametrize("least,most", [(2.0 ** -22, 1.9921875 * 2.0 ** 10), (1.9921875 * 2.0 ** -23, 1.0), (2.0 ** -10, 2.0 ** 11), (2.0 ** -30, 2.0 ** -4),
+                                        (2.0 ** 10, 2.0 ** 36), (2.0 ** -40, 2.0 ** 20), (2.0 ** -130, 1.0), (0.0, float("inf")), (0.0, float("nan"))])
+def test_scalings_of_x_agree(cuda, mode, kind, least, most):
+    """Scaled or not, the products are exact and so are the powers of two: the bits of the BF16 path, which scales nothing."""
+    gen = torch.Generator(device="cuda").manual_seed(mode)
+    M, K, N = 3, 1160, 512
+    x = (torch.rand(M, K, generator=gen, device="cuda") + 0.5) * torch.where(torch.rand(M, K, generator=gen, device="cuda") < 0.5, 1.0, -1.0)
+    if least >= 2.0 ** 10:
+        x *= 2.0 ** 12
+    if 0 < least < 2.0 ** -22 and most < 1:
+        x *= 2.0 ** -5
+    x[0, 5], x[0, 1159], x[1, 700], x[2, :64] = least, -most, -least, 0.0
+    x = x.bfloat16()
+    w = torch.randn(K, N, generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    if mode == 2:
+        w = torch.randint(0, 256, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)
+        w[:, N // 2:] = w[:, N // 2:] % 0x60  # block scales: finite, not negative
+    outs = []
+    for slow in (0, 1):
+        if kind == "head":
+            op = LmHeadArgmax()
+            op.set_option("force_slow", slow)
+            outs.append(op(x, w, N, logits=True)[3])
+        elif kind == "shared":
+            op = SharedExpertDown()
+            op.set_option("force_slow", slow)
+            g, one = torch.full_like(x, 16.0), torch.ones(64, 1, dtype=torch.bfloat16, device="cuda")  # bf16(sigmoid(16)) is 1
+            outs.append(op(g, (x.float() / 16).bfloat16(), w, torch.ones(M, 64, dtype=torch.bfloat16, device="cuda"), one, torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")))
+        else:
+            op = SkinnyGemm([1], [N])
+            op.set_option("force_slow", slow)
+            op.set_option("stream_plan", ("1,4,1,3" if mode == 2 else "8,4,1,3") if kind == "cluster" else "")
+            outs.append(op(x, w)[0])
+    a, b = outs
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+    assert torch.isfinite(a).any()
