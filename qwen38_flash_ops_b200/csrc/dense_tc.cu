@@ -84,6 +84,8 @@ struct RawRing {  // ring of stored, undequantised stages
   static constexpr int kBytes = MODE == kBf16 ? 0 : kSlot * kDepth;
   static_assert(kDepth <= kMaxRaw && kDepth % kDqGroups == 0 && kSlot % 256 == 0, "raw ring");
 };
+// Kernels that hand the weights over in tensor memory (TM, see DequantTmRole): at most 128 rows a tile, four stages of two blocks
+constexpr int kTmBm = 128, kTmKs = 2, kTmStages = 4, kTmGroups = 4, kTmColumns = 512, kTmFirst = 256, kTmWarps = 4;
 constexpr int kOutPitch = 80;                     // bytes of a row of 32 output columns in an epilogue warp's buffer: rows 16 bytes apart in the banks
 constexpr int kOutBytes = 4 * 32 * kOutPitch;     // four warps, 32 rows of x each
 
@@ -102,6 +104,7 @@ struct DenseParams {
   uint16_t* out[kMaxOut];
   int col_begin[kMaxOut], width[kMaxOut];
   int nseg, M, K, ksteps, bm, m_tiles, tiles, stages;
+  int raw_depth;  // TM: slots of the raw ring
   uint32_t out_vec;  // outputs whose rows can be written 16 bytes at a time
 };
 
@@ -197,6 +200,11 @@ __device__ __forceinline__ void MmaSs(uint32_t d, unsigned long long a, unsigned
                  : "memory");
   }
 }
+__device__ __forceinline__ void MmaTs(uint32_t d, uint32_t a, unsigned long long b, uint32_t idesc, bool add) {
+  asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(b),
+               "r"(idesc), "r"(add ? 1 : 0)
+               : "memory");
+}
 // arrives on the barrier (of both CTAs of a pair) when the MMAs issued so far have completed
 template <bool PAIR>
 __device__ __forceinline__ void MmaCommit(uint32_t bar) {
@@ -226,6 +234,16 @@ __device__ __forceinline__ uint32_t Lds8(uint32_t a) {
   uint32_t v;
   asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
+}
+__device__ __forceinline__ void LdsmTrans(uint32_t a, uint32_t (&v)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+}
+// sixteen lanes of tensor memory by 32 columns: register 2 i + h of lane (g, t) is lane 8 h + g, column 4 i + t
+__device__ __forceinline__ void StoreTmem(uint32_t a, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(a), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+               "r"(v[14]), "r"(v[15])
+               : "memory");
 }
 __device__ __forceinline__ void Sts128(uint32_t a, const uint32_t* v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
@@ -285,7 +303,8 @@ __device__ __forceinline__ TileAt LocateDense(const DenseParams& p, int tile, in
 // the tile.  (Such weights used to come in 8-byte cp.async pieces by two warps, 18 instructions a stage: 1024 rows of 5120 x
 // 5248 81.2 us, now 48.7, and 54.8 by dequantisation and library GEMM; 33 rows 20.0, 13.2 and 24.5.)
 template <int MODE, bool PAIR, int KS>
-__device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int rank, int kbeg, int kcount, int first_tile, int tile_step, uint32_t ring) {
+__device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int rank, int kbeg, int kcount, int first_tile, int tile_step, uint32_t ring,
+                                           int depth = RawRing<MODE, KS>::kDepth) {
   using R = RawRing<MODE, KS>;
   const uint32_t full0 = Smem(&ctl.raw_full[0]), empty0 = Smem(&ctl.raw_empty[0]);
   int slot = 0;
@@ -315,7 +334,7 @@ __device__ __forceinline__ void LoadTensor(const DenseParams& p, Ctl& ctl, int r
         }
       }
       __syncwarp();
-      if (++slot == R::kDepth) {
+      if (++slot == depth) {
         slot = 0;
         parity ^= 1u;
         first_round = false;
@@ -450,13 +469,137 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
   }
 }
 
+// The same for tiles of up to 128 rows, with the weights in tensor memory instead of shared memory: there the tensor core's
+// operand does not compete for the 128 bytes a cycle of shared memory, which a block of 64 k and few rows fills (16 KB
+// written and 16 KB read of 54 KB at 33 rows: 400 cycles a block, an MMA every 85).  5120 x 17408, NVFP4, 17 / 33 / 64 rows 20.8 / 21.5 / 23.5
+// -> 16.5 / 18.4 / 20.3 us, FP8 5120 x 10240 22.0 / 22.6 / 23.4 -> 17.1 / 17.9 / 18.6.  Four warps, one for each 32 lanes of tensor memory, take a stage; four such groups take the stages in
+// turn.  Lane (g, t) loads two stored bytes of rows 2t and 2t + 1 of every eight by transposing loads (the ring is swizzled, so
+// they are free of bank conflicts), turns them into FP32, by one mixed FMA each with the block scale of its row (NVFP4),
+// and packs rows 2t and 2t + 1 of a column into the word that the operand wants: pairs along k, though the bytes hold pairs along N.
+// Lane 16 s + 8 h + g of the 32 then is column 16 s + 2 g + h (FP8), or 4 g + 2 s + h (NVFP4) of the warp's, see TmColumn.
+template <int MODE>
+__device__ __forceinline__ int TmColumn(int s, int h, int g) {
+  return MODE == kFp8 ? 16 * s + 2 * g + h : 4 * g + 2 * s + h;
+}
+template <int MODE, bool SCALED>
+__device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, int warp, int lane, int kcount, int first_tile, int tile_step, uint32_t ring,
+                                              uint32_t tmem) {
+  using R = RawRing<MODE, kTmKs>;
+  constexpr bool kNib = kFp4<MODE>;
+  const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), rfull0 = Smem(&ctl.raw_full[0]), rempty0 = Smem(&ctl.raw_empty[0]);
+  const int quad = warp & 3, group = warp >> 2, g = lane >> 2, t = lane & 3;
+  // this lane's row address of a transposing load.  NVFP4: four times eight rows of the warp's 16 bytes; FP8: twice eight rows of
+  // its two times 16 bytes.  Swizzled: 16-byte pieces exclusive-or bits 7 to 8 (9) of the address.
+  const int row = kNib ? lane : (lane & 15), piece = kNib ? quad ^ ((lane >> 1) & 3) : (2 * quad + (lane >> 4)) ^ (lane & 7);
+  const uint32_t rd = ring + static_cast<uint32_t>(row * (kNib ? 64 : 128) + piece * 16);
+  const uint32_t rd_s = ring + R::kScales + static_cast<uint32_t>(2 * t * 16 + 2 * quad + (g >> 2));
+  const uint32_t a0 = tmem + kTmFirst + (static_cast<uint32_t>(32 * quad) << 16);
+  const float zero = -0.f;  // the addend that leaves the sign of a zero as it is
+  int stage = group % kTmStages, slot = group % p.raw_depth, tile = first_tile, k = group;
+  uint32_t parity = 0, rparity = 0;
+  bool first_round = true;
+  auto next_tile = [&]() {  // the stages go from group to group across tile boundaries too
+    while (k >= kcount && tile < p.tiles) {
+      k -= kcount;
+      tile += tile_step;
+    }
+  };
+  next_tile();
+  while (tile < p.tiles) {
+    const TileAt at_tile = LocateDense<false>(p, tile, 0);
+    const DenseSeg& sg = p.seg[at_tile.seg];
+    float cs[2][2] = {{1.f, 1.f}, {1.f, 1.f}};
+    if constexpr (SCALED) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = at_tile.n0 + 32 * quad + TmColumn<MODE>(i >> 1, i & 1, g);
+        cs[i >> 1][i & 1] = (sg.w_scale != nullptr && n < sg.n) ? __ldg(sg.w_scale + n) : 1.f;
+      }
+    }
+    const uint32_t shift = static_cast<uint32_t>(at_tile.n0 >> 4) & 8u;  // of the scales in their 16 bytes
+#pragma unroll 1
+    for (; k < kcount; k += kTmGroups) {
+      const bool room = first_round || BarTest(empty0 + stage * 8, parity ^ 1u);
+      if (!BarWait(rfull0 + slot * 8, rparity, ctl)) return;
+      const uint32_t at = static_cast<uint32_t>(slot) * R::kSlot;
+      bool free = room;
+#pragma unroll
+      for (int j = 0; j < kTmKs; ++j) {
+        uint32_t v[2][16];
+#pragma unroll
+        for (int q = 0; q < (kNib ? 2 : 4); ++q) {
+          uint32_t raw[4];
+          LdsmTrans(rd + at + static_cast<uint32_t>((j * kBk + q * (kNib ? 32 : 16)) * (kNib ? 64 : 128)), raw);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float lo[2][2], hi[2][2];  // [set][half]: rows 2t and 2t + 1 of the lane's columns
+            if constexpr (kNib) {
+              const uint32_t rs = rd_s + at + shift + static_cast<uint32_t>((j * kBk + q * 32 + i * 8) * 16);
+              uint32_t h[4], s, unused;
+              CvtE4m3x4(Lds8(rs) | (Lds8(rs + 16) << 8), s, unused);
+              CvtE2m1x8(raw[i], h);
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                asm("{ .reg .f16 a, b, s, t;\n mov.b32 {a, b}, %2;\n mov.b32 {s, t}, %3;\n fma.rn.f32.f16 %0, a, s, %4;\n fma.rn.f32.f16 %1, b, s, %4;\n}"
+                    : "=f"(lo[u][0]), "=f"(lo[u][1]) : "r"(h[u]), "r"(s), "f"(zero));
+                asm("{ .reg .f16 a, b, s, t;\n mov.b32 {a, b}, %2;\n mov.b32 {s, t}, %3;\n fma.rn.f32.f16 %0, a, t, %4;\n fma.rn.f32.f16 %1, b, t, %4;\n}"
+                    : "=f"(hi[u][0]), "=f"(hi[u][1]) : "r"(h[2 + u]), "r"(s), "f"(zero));
+              }
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) v[u][2 * (4 * q + i) + e] = PackBf16(SCALED ? lo[u][e] * cs[u][e] : lo[u][e], SCALED ? hi[u][e] * cs[u][e] : hi[u][e]);
+              }
+            } else {
+              uint32_t ha, hb;
+              CvtE4m3x4(raw[i], ha, hb);
+              constexpr int u0 = 0;
+              asm("{ .reg .f16 a, b;\n mov.b32 {a, b}, %2;\n add.f32.f16 %0, a, %3;\n add.f32.f16 %1, b, %3;\n}" : "=f"(lo[u0][0]), "=f"(lo[u0][1]) : "r"(ha), "f"(zero));
+              asm("{ .reg .f16 a, b;\n mov.b32 {a, b}, %2;\n add.f32.f16 %0, a, %3;\n add.f32.f16 %1, b, %3;\n}" : "=f"(hi[u0][0]), "=f"(hi[u0][1]) : "r"(hb), "f"(zero));
+              const int u = i >> 1, i8 = 2 * q + (i & 1);  // raw: rows 0 to 7, 8 to 15 of the first 16 bytes, then of the second
+#pragma unroll
+              for (int e = 0; e < 2; ++e) v[u][2 * i8 + e] = PackBf16(SCALED ? lo[u0][e] * cs[u][e] : lo[u0][e], SCALED ? hi[u0][e] * cs[u][e] : hi[u0][e]);
+            }
+          }
+        }
+        if (!free && !BarWait(empty0 + stage * 8, parity ^ 1u, ctl)) return;
+        if (j == 0) {
+          free = true;
+          __syncwarp();
+          FenceAfter();
+        }
+        const uint32_t a = a0 + static_cast<uint32_t>((stage * kTmKs + j) * 32);
+        StoreTmem(a, v[0]);
+        StoreTmem(a + (16u << 16), v[1]);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      FenceBefore();
+      __syncwarp();
+      if (lane == 0) {  // behind stores that depend on the ring's loads, as in DequantRole
+        BarArrive(rempty0 + slot * 8);
+        BarArrive(full0 + stage * 8);
+      }
+      slot += kTmGroups;
+      if (slot >= p.raw_depth) {
+        slot -= p.raw_depth;
+        rparity ^= 1u;
+      }
+      // as many stages as groups: a group always fills the same one
+      parity ^= 1u;
+      first_round = false;
+    }
+    next_tile();
+  }
+}
+
 template <int MODE>
 constexpr int DenseThreads() {
   return 32 * (kFirstDqWarp + (MODE == kBf16 ? 0 : kDqWarps * kDqGroups));
 }
 
-// SPLIT: K is split over the CTAs of the cluster, one tile per cluster.  PAIR: see above.  Never both.
-template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
+// SPLIT: K is split over the CTAs of the cluster, one tile per cluster.  PAIR: see above.  Never both.  TM: the weights go through
+// tensor memory; not in pairs.
+template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS, bool TM>
 __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const __grid_constant__ DenseParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Ctl ctl;
@@ -469,23 +612,26 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   const int kbeg = SPLIT ? rank * p.ksteps / csize : 0;
   const int kcount = SPLIT ? (rank + 1) * p.ksteps / csize - kbeg : p.ksteps;
   const int xrows = PAIR ? p.bm / 2 : p.bm;
-  const uint32_t block_bytes = static_cast<uint32_t>(kABytes + xrows * kBk * 2), stage_bytes = block_bytes * KS;
+  static_assert(!TM || (KS == kTmKs && !PAIR && (MODE == kFp8 || MODE == kNvfp4)), "");
+  constexpr int kX = TM ? 0 : kABytes;  // where x begins in a block
+  const uint32_t block_bytes = static_cast<uint32_t>(kX + xrows * kBk * 2), stage_bytes = block_bytes * KS;
   const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), accf0 = Smem(&ctl.acc_full[0]), acce0 = Smem(&ctl.acc_empty[0]);
-  int acc_cols = 32;
+  int acc_cols = TM ? kTmColumns : 32;
   while (acc_cols < 2 * p.bm) acc_cols *= 2;
+  const int raw_depth = TM ? p.raw_depth : RawRing<MODE, KS>::kDepth;
 
   if (tid == 0) {
     for (int i = 0; i < p.stages; ++i) {
-      BarInit(full0 + i * 8, 1 + (MODE == kBf16 ? 0 : kDqWarps * (PAIR ? 2 : 1)));
+      BarInit(full0 + i * 8, 1 + (MODE == kBf16 ? 0 : TM ? kTmWarps : kDqWarps * (PAIR ? 2 : 1)));
       BarInit(empty0 + i * 8, 1);
     }
     for (int i = 0; i < 2; ++i) {
       BarInit(accf0 + i * 8, 1);
       BarInit(acce0 + i * 8, 4 * (PAIR ? 2 : 1));
     }
-    for (int i = 0; MODE != kBf16 && i < RawRing<MODE, KS>::kDepth; ++i) {
+    for (int i = 0; MODE != kBf16 && i < raw_depth; ++i) {
       BarInit(Smem(&ctl.raw_full[i]), 1);
-      BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
+      BarInit(Smem(&ctl.raw_empty[i]), TM ? kTmWarps : kDqWarps);
     }
     ctl.fault = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -513,7 +659,8 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
 
   if (warp < 4) {
     // ---- epilogue
-    const uint32_t buf = smem + static_cast<uint32_t>(p.stages) * stage_bytes + RawRing<MODE, KS>::kBytes + static_cast<uint32_t>(warp * 32 * kOutPitch);
+    const uint32_t raw_bytes = TM ? static_cast<uint32_t>(RawRing<MODE, KS>::kSlot * raw_depth) : static_cast<uint32_t>(RawRing<MODE, KS>::kBytes);
+    const uint32_t buf = smem + static_cast<uint32_t>(p.stages) * stage_bytes + raw_bytes + static_cast<uint32_t>(warp * 32 * kOutPitch);
     int it = 0;
     bool good = true;  // false from the first wait that ran out: no sums come any more, and the tiles that are left become NaN
     for (int tile = first_tile; tile < p.tiles; tile += tile_step, ++it) {
@@ -536,7 +683,8 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
               : "r"(src + static_cast<uint32_t>(c)));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float* part = reinterpret_cast<float*>(smem_ptr) + c * kBn + 32 * warp + lane;
+          const int col = TM ? TmColumn<MODE>(lane >> 4, (lane >> 3) & 1, lane & 7) : lane;
+          float* part = reinterpret_cast<float*>(smem_ptr) + c * kBn + 32 * warp + col;
 #pragma unroll
           for (int i = 0; i < 16; ++i) part[i * kBn] = good ? __uint_as_float(v[i]) : __uint_as_float(0x7FFFFFFFu);
         }
@@ -576,7 +724,20 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
           for (int h = 0; h < 2; ++h) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-              if (k == 0 || c + 16 < p.bm) {
+              if constexpr (TM) {
+                if (k == 0 || c + 16 < p.bm) {
+                  // lanes g and g + 8 are neighbouring columns: their words lie beside one another, rows 2t, 2t + 1 and eight on
+                  const int lane_t = lane & 3, word = TmColumn<MODE>(h, 0, lane >> 2) / 2;
+                  const uint32_t to = buf + static_cast<uint32_t>((16 * k + 2 * lane_t) * kOutPitch + word * 4);
+                  const uint32_t(&f)[8] = v[h][k];
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    const int lo = 4 * (i >> 1) + (i & 1);
+                    const uint32_t w = good ? PackBf16(__uint_as_float(f[lo]), __uint_as_float(f[lo + 2])) : 0x7FFF7FFFu;
+                    asm volatile("st.shared.b32 [%0], %1;" ::"r"(to + static_cast<uint32_t>((8 * (i >> 1) + (i & 1)) * kOutPitch)), "r"(w) : "memory");
+                  }
+                }
+              } else if (k == 0 || c + 16 < p.bm) {
                 uint32_t w[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -635,7 +796,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
               TmaLoad<PAIR>(at, &p.wmap[t.seg], t.n0, k0, bar);
               TmaLoad<PAIR>(at + kABytes / 2, &p.wmap[t.seg], t.n0 + 64, k0, bar);
             }
-            TmaLoad<PAIR>(at + kABytes, &p.xmap, k0, t.m0 + (PAIR ? rank * xrows : 0), bar);
+            TmaLoad<PAIR>(at + kX, &p.xmap, k0, t.m0 + (PAIR ? rank * xrows : 0), bar);
           }
         }
         __syncwarp();
@@ -649,9 +810,9 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
     // ---- MMAs (the leader's, for both CTAs of a pair)
     if (!PAIR || rank == 0) {
       // FP32 accumulators, BF16 operands, A MN-major, N = bm, M = 128 (256 across a pair)
-      const uint32_t idesc = 0x10u | (1u << 7) | (1u << 10) | (1u << 15) | (static_cast<uint32_t>(p.bm >> 3) << 17) |
+      const uint32_t idesc = 0x10u | (1u << 7) | (1u << 10) | (TM ? 0u : 1u << 15) | (static_cast<uint32_t>(p.bm >> 3) << 17) |
                              (static_cast<uint32_t>(PAIR ? 16 : 8) << 24);
-      const unsigned long long a0 = SmemDesc(smem, kABytes / 2, 1024), b0 = SmemDesc(smem + kABytes, 16, 1024);
+      const unsigned long long a0 = SmemDesc(smem, kABytes / 2, 1024), b0 = SmemDesc(smem + kX, 16, 1024);
       int stage = 0, it = 0;
       uint32_t parity = 0;
       bool good = true, ready = false;
@@ -666,7 +827,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
             break;
           }
           FenceAfter();
-          const uint32_t off = static_cast<uint32_t>(stage) * stage_bytes >> 4, done = empty0 + stage * 8;
+          const uint32_t off = static_cast<uint32_t>(stage) * stage_bytes >> 4, done = empty0 + stage * 8, a_tm = tmem + kTmFirst + static_cast<uint32_t>(stage * KS * 32);
           if (++stage == p.stages) {
             stage = 0;
             parity ^= 1u;
@@ -678,7 +839,11 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
 #pragma unroll
               for (int i = 0; i < kBk / 16; ++i) {
                 const uint32_t at = off + j * (block_bytes >> 4);
-                MmaSs<PAIR>(d, a0 + at + i * (2048 >> 4), b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
+                if constexpr (TM) {
+                  MmaTs(d, a_tm + j * 32 + i * 8, b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
+                } else {
+                  MmaSs<PAIR>(d, a0 + at + i * (2048 >> 4), b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
+                }
               }
             }
             MmaCommit<PAIR>(done);
@@ -691,10 +856,14 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   } else if constexpr (MODE != kBf16) {
     const uint32_t ring = smem + static_cast<uint32_t>(p.stages) * stage_bytes;
     if (warp < kFirstDqWarp) {
-      if (warp == 6) LoadTensor<MODE, PAIR, KS>(p, ctl, rank, kbeg, kcount, first_tile, tile_step, ring);
+      if (warp == 6) LoadTensor<MODE, PAIR, KS>(p, ctl, rank, kbeg, kcount, first_tile, tile_step, ring, raw_depth);
     } else {
       const int w = warp - kFirstDqWarp;
-      DequantRole<MODE, SCALED, PAIR, KS, kDqGroups>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
+      if constexpr (TM) {
+        DequantTmRole<MODE, SCALED>(p, ctl, w, lane, kcount, first_tile, tile_step, ring, tmem);
+      } else {
+        DequantRole<MODE, SCALED, PAIR, KS, kDqGroups>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
+      }
     }
   }
 
@@ -1193,14 +1362,16 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
 }
 
 // ------------------------------------------------------------------------------ host
-// rows x cols elements of `elem` bytes (2: BF16, boxes swizzled in 128 bytes; 1: bytes, plain), row-major
-bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols) {
+// rows x cols elements of `elem` bytes (2: BF16, boxes swizzled in 128 bytes; 1: bytes, plain or swizzled as given), row-major
+bool Encode(CUtensorMap* map, const void* base, int elem, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols,
+            int swizzle = 0) {
   const cuuint64_t dims[2] = {cols, rows}, strides[1] = {pitch_bytes};
   const cuuint32_t box[2] = {box_cols, box_rows}, step[2] = {1, 1};
   const TensorMapEncodeFn fn = TensorMapEncoder();
   return fn != nullptr &&
          fn(map, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, step,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, elem == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, elem == 2 || swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1217,7 +1388,7 @@ int RawBytes(int mode, int ks) {
 }
 int BlocksFor(int mode, int xrows, int ks) { return (kSmemLimit - kOutBytes - RawBytes(mode, ks)) / (kABytes + xrows * kBk * 2); }
 
-template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS>
+template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS, bool TM = false>
 cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
@@ -1234,11 +1405,16 @@ cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, 
     cfg.numAttrs = 1;
   }
   if (MayOverlapPredecessor(stream)) attr[cfg.numAttrs++] = OverlapAttribute();
-  return cudaLaunchKernelEx(&cfg, DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS>, p);
+  return cudaLaunchKernelEx(&cfg, DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS, TM>, p);
 }
 
 template <int MODE, bool SCALED>
-cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, int ctas, int cluster, size_t smem, cudaStream_t stream) {
+cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, bool tm, int ctas, int cluster, size_t smem, cudaStream_t stream) {
+  if constexpr (MODE == kFp8 || MODE == kNvfp4) {
+    if (tm)
+      return cluster > 1 ? LaunchOne<MODE, SCALED, false, true, kTmKs, true>(p, ctas, cluster, smem, stream)
+                         : LaunchOne<MODE, SCALED, false, false, kTmKs, true>(p, ctas, 1, smem, stream);
+  }
   if (pair) return ks == 2 ? LaunchOne<MODE, SCALED, true, false, 2>(p, ctas, 2, smem, stream) : LaunchOne<MODE, SCALED, true, false, 1>(p, ctas, 2, smem, stream);
   if (cluster > 1)
     return ks == 2 ? LaunchOne<MODE, SCALED, false, true, 2>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, true, 1>(p, ctas, cluster, smem, stream);
@@ -1276,11 +1452,17 @@ std::atomic<const DeviceSetup*> g_setup_last{nullptr};  // the last one asked fo
 
 template <int MODE, bool SCALED, int KS>
 cudaError_t SetUpShape() {
-  cudaError_t err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  cudaError_t err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  if constexpr (KS == kTmKs && (MODE == kFp8 || MODE == kNvfp4)) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  }
   return err;
 }
 template <int MODE, bool SCALED>
@@ -1308,7 +1490,7 @@ int QuerySlots(int cluster) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, DenseTcKernel<kBf16, false, false, true, 1>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, DenseTcKernel<kBf16, false, false, true, 1, false>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     n = std::max(1, DeviceSmCount() * 8 / (10 * cluster));
   }
@@ -1347,13 +1529,13 @@ cudaError_t SetUpDevice(const DeviceSetup** out) {
 }
 
 // describes a stored weight to the copy engine
-bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int ks) {
+bool EncodeWeight(DenseParams& p, int mode, int s, const Segment& sg, int K, int ks, bool tm = false) {
   const uint64_t rows = static_cast<uint64_t>(K), pitch = static_cast<uint64_t>(sg.pitch), n = static_cast<uint64_t>(sg.n);
   if (mode == kBf16) return Encode(&p.wmap[s], sg.w, 2, rows, n, pitch, kBk, 64);
-  if (mode == kFp8) return Encode(&p.wmap[s], sg.w, 1, rows, n, pitch, kBk * ks, kBn);
+  if (mode == kFp8) return Encode(&p.wmap[s], sg.w, 1, rows, n, pitch, kBk * ks, kBn, tm ? 128 : 0);
   const uint64_t rows_in_one = mode == kNvfp4Odd ? 2 : 1;  // K is a multiple of eight
   const uint32_t box = static_cast<uint32_t>(kBk * ks / rows_in_one);
-  return Encode(&p.wmap[s], sg.w, 1, rows / rows_in_one, pitch * rows_in_one, pitch * rows_in_one, box, mode == kNvfp4Odd ? kOddPitch : kBn / 2) &&
+  return Encode(&p.wmap[s], sg.w, 1, rows / rows_in_one, pitch * rows_in_one, pitch * rows_in_one, box, mode == kNvfp4Odd ? kOddPitch : kBn / 2, tm ? 64 : 0) &&
          Encode(&p.smap[s], sg.w, 1, rows / rows_in_one, pitch * rows_in_one, pitch * rows_in_one, box, 16);
 }
 
@@ -1433,6 +1615,9 @@ bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
   return TensorMapEncoder() != nullptr;
 }
 
+// Whether a launch shape that does not name its stages hands the weights over in tensor memory.
+bool TakesTm(int mode, const DenseTcPlan& plan) { return (mode == kFp8 || mode == kNvfp4) && !plan.pair && plan.bm <= kTmBm; }
+
 bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int mode = KernelMode(weights, g);
   if (plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.split < 1 || plan.split > 8 || (plan.pair && plan.split != 1) || plan.ks < 0 || plan.ks > 2)
@@ -1443,7 +1628,8 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   p.K = g.K;
   p.bm = plan.bm;
   const int xrows = plan.pair ? p.bm / 2 : p.bm;
-  const int ks = plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1, blocks = BlocksFor(mode, xrows, ks);
+  const bool tm = plan.ks == 0 && TakesTm(mode, plan);
+  const int ks = tm ? kTmKs : plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1, blocks = BlocksFor(mode, xrows, ks);
   p.ksteps = (g.K + kBk * ks - 1) / (kBk * ks);
   if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
     return false;
@@ -1456,7 +1642,7 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
     scaled = scaled || sg.w_scale != nullptr;
   }
   for (int s = 0; s < g.nseg; ++s) {
-    if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks)) return false;
+    if (!EncodeWeight(p, mode, s, g.seg[s], g.K, ks, tm)) return false;
   }
   const int n_out = g.seg[g.nseg - 1].out_end;
   for (int o = 0; o < n_out; ++o) {
@@ -1469,24 +1655,31 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   if (static_cast<int64_t>(p.m_tiles) * n_tiles > INT_MAX / 16) return false;
   p.tiles = p.m_tiles * n_tiles;
   const int cluster = plan.pair ? 2 : std::min(plan.split, p.ksteps);
-  p.stages = std::min(kMaxStages, blocks / ks);
+  p.stages = tm ? kTmStages : std::min(kMaxStages, blocks / ks);
   // the dequantising groups take the stages in turn: fewer stages than groups would run off the ring
   if (p.stages < kDqGroups) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * (kABytes + xrows * kBk * 2) + RawBytes(mode, ks) + kOutBytes;
+  size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * ((tm ? 0 : kABytes) + xrows * kBk * 2) + kOutBytes;
+  if (tm) {
+    const int slot = mode == kFp8 ? RawRing<kFp8, kTmKs>::kSlot : RawRing<kNvfp4, kTmKs>::kSlot;
+    p.raw_depth = smem + 2 * kTmGroups * slot <= static_cast<size_t>(kSmemLimit) ? 2 * kTmGroups : kTmGroups;
+    smem += static_cast<size_t>(p.raw_depth) * slot;
+  } else {
+    smem += static_cast<size_t>(RawBytes(mode, ks));
+  }
   const int slots = std::max(1, DeviceSmCount() / cluster);
   const int ctas = cluster * (cluster > 1 && !plan.pair ? p.tiles : std::min(p.tiles, slots));
   cudaError_t err = ConfigureDenseKernels();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
   if (mode == kBf16) {
-    err = LaunchMode<kBf16, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+    err = LaunchMode<kBf16, false>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream);
   } else if (mode == kFp8) {
-    err = scaled ? LaunchMode<kFp8, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream) : LaunchMode<kFp8, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+    err = scaled ? LaunchMode<kFp8, true>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream) : LaunchMode<kFp8, false>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream);
   } else if (mode == kNvfp4) {
-    err = scaled ? LaunchMode<kNvfp4, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream)
-                 : LaunchMode<kNvfp4, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+    err = scaled ? LaunchMode<kNvfp4, true>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream)
+                 : LaunchMode<kNvfp4, false>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream);
   } else {
-    err = scaled ? LaunchMode<kNvfp4Odd, true>(p, plan.pair != 0, ks, ctas, cluster, smem, stream)
-                 : LaunchMode<kNvfp4Odd, false>(p, plan.pair != 0, ks, ctas, cluster, smem, stream);
+    err = scaled ? LaunchMode<kNvfp4Odd, true>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream)
+                 : LaunchMode<kNvfp4Odd, false>(p, plan.pair != 0, ks, tm, ctas, cluster, smem, stream);
   }
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("SkinnyGemm(dense): ") + cudaGetErrorString(err));
