@@ -84,8 +84,9 @@ struct RawRing {  // ring of stored, undequantised stages
   static constexpr int kBytes = MODE == kBf16 ? 0 : kSlot * kDepth;
   static_assert(kDepth <= kMaxRaw && kDepth % kDqGroups == 0 && kSlot % 256 == 0, "raw ring");
 };
-// Kernels that hand the weights over in tensor memory (TM, see DequantTmRole): at most 128 rows a tile, four stages of two blocks
-constexpr int kTmBm = 128, kTmKs = 2, kTmStages = 4, kTmGroups = 4, kTmColumns = 512, kTmFirst = 256, kTmWarps = 4;
+// Kernels that hand the weights over in tensor memory (TM, see DequantTmRole): four stages of two blocks, behind the two sets of
+// accumulators of at most 128 rows
+constexpr int kTmKs = 2, kTmStages = 4, kTmGroups = 4, kTmWarps = 4, kTmColumns = 512, kTmFirst = kTmColumns - kTmStages * kTmKs * 32, kTmBm = kTmFirst / 2;
 constexpr int kOutPitch = 80;                     // bytes of a row of 32 output columns in an epilogue warp's buffer: rows 16 bytes apart in the banks
 constexpr int kOutBytes = 4 * 32 * kOutPitch;     // four warps, 32 rows of x each
 
@@ -200,10 +201,17 @@ __device__ __forceinline__ void MmaSs(uint32_t d, unsigned long long a, unsigned
                  : "memory");
   }
 }
+template <bool PAIR>
 __device__ __forceinline__ void MmaTs(uint32_t d, uint32_t a, unsigned long long b, uint32_t idesc, bool add) {
-  asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(b),
-               "r"(idesc), "r"(add ? 1 : 0)
-               : "memory");
+  if constexpr (PAIR) {
+    asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(b),
+                 "r"(idesc), "r"(add ? 1 : 0)
+                 : "memory");
+  } else {
+    asm volatile("{ .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(b),
+                 "r"(idesc), "r"(add ? 1 : 0)
+                 : "memory");
+  }
 }
 // arrives on the barrier (of both CTAs of a pair) when the MMAs issued so far have completed
 template <bool PAIR>
@@ -469,6 +477,19 @@ __device__ __forceinline__ void DequantRole(const DenseParams& p, Ctl& ctl, int 
   }
 }
 
+// Two values times the scales of their columns, in one instruction where the warps that do it set the pace (FP8, 33 rows of 5120 x 10240:
+// 21.1 -> 20.2 us; in pairs, where they wait for room, 509 rows 59.5 -> 60.9).
+template <bool PAIR>
+__device__ __forceinline__ void ScalePair(float (&v)[2], const float (&s)[2]) {
+  if constexpr (PAIR) {
+    v[0] *= s[0];
+    v[1] *= s[1];
+  } else {
+    asm("{ .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n mul.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}"
+        : "+f"(v[0]), "+f"(v[1])
+        : "f"(s[0]), "f"(s[1]));
+  }
+}
 // The same for tiles of up to 128 rows, with the weights in tensor memory instead of shared memory: there the tensor core's
 // operand does not compete for the 128 bytes a cycle of shared memory, which a block of 64 k and few rows fills (16 KB
 // written and 16 KB read of 54 KB at 33 rows: 400 cycles a block, an MMA every 85).  5120 x 17408, NVFP4, 17 / 33 / 64 rows 20.8 / 21.5 / 23.5
@@ -481,8 +502,8 @@ template <int MODE>
 __device__ __forceinline__ int TmColumn(int s, int h, int g) {
   return MODE == kFp8 ? 16 * s + 2 * g + h : 4 * g + 2 * s + h;
 }
-template <int MODE, bool SCALED>
-__device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, int warp, int lane, int kcount, int first_tile, int tile_step, uint32_t ring,
+template <int MODE, bool SCALED, bool PAIR>
+__device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, int warp, int lane, int rank, int kcount, int first_tile, int tile_step, uint32_t ring,
                                               uint32_t tmem) {
   using R = RawRing<MODE, kTmKs>;
   constexpr bool kNib = kFp4<MODE>;
@@ -506,7 +527,7 @@ __device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, in
   };
   next_tile();
   while (tile < p.tiles) {
-    const TileAt at_tile = LocateDense<false>(p, tile, 0);
+    const TileAt at_tile = LocateDense<PAIR>(p, tile, rank);
     const DenseSeg& sg = p.seg[at_tile.seg];
     float cs[2][2] = {{1.f, 1.f}, {1.f, 1.f}};
     if constexpr (SCALED) {
@@ -548,7 +569,10 @@ __device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, in
 #pragma unroll
               for (int u = 0; u < 2; ++u) {
 #pragma unroll
-                for (int e = 0; e < 2; ++e) v[u][2 * (4 * q + i) + e] = PackBf16(SCALED ? lo[u][e] * cs[u][e] : lo[u][e], SCALED ? hi[u][e] * cs[u][e] : hi[u][e]);
+                for (int e = 0; e < 2; ++e) {
+                  if (SCALED && e == 0) ScalePair<PAIR>(lo[u], cs[u]), ScalePair<PAIR>(hi[u], cs[u]);
+                  v[u][2 * (4 * q + i) + e] = PackBf16(lo[u][e], hi[u][e]);
+                }
               }
             } else {
               uint32_t ha, hb;
@@ -558,7 +582,10 @@ __device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, in
               asm("{ .reg .f16 a, b;\n mov.b32 {a, b}, %2;\n add.f32.f16 %0, a, %3;\n add.f32.f16 %1, b, %3;\n}" : "=f"(hi[u0][0]), "=f"(hi[u0][1]) : "r"(hb), "f"(zero));
               const int u = i >> 1, i8 = 2 * q + (i & 1);  // raw: rows 0 to 7, 8 to 15 of the first 16 bytes, then of the second
 #pragma unroll
-              for (int e = 0; e < 2; ++e) v[u][2 * i8 + e] = PackBf16(SCALED ? lo[u0][e] * cs[u][e] : lo[u0][e], SCALED ? hi[u0][e] * cs[u][e] : hi[u0][e]);
+              for (int e = 0; e < 2; ++e) {
+                if (SCALED && e == 0) ScalePair<PAIR>(lo[u0], cs[u]), ScalePair<PAIR>(hi[u0], cs[u]);
+                v[u][2 * i8 + e] = PackBf16(lo[u0][e], hi[u0][e]);
+              }
             }
           }
         }
@@ -577,7 +604,7 @@ __device__ __forceinline__ void DequantTmRole(const DenseParams& p, Ctl& ctl, in
       __syncwarp();
       if (lane == 0) {  // behind stores that depend on the ring's loads, as in DequantRole
         BarArrive(rempty0 + slot * 8);
-        BarArrive(full0 + stage * 8);
+        BarArriveLeader<PAIR>(full0 + stage * 8);
       }
       slot += kTmGroups;
       if (slot >= p.raw_depth) {
@@ -598,7 +625,7 @@ constexpr int DenseThreads() {
 }
 
 // SPLIT: K is split over the CTAs of the cluster, one tile per cluster.  PAIR: see above.  Never both.  TM: the weights go through
-// tensor memory; not in pairs.
+// tensor memory.
 template <int MODE, bool SCALED, bool PAIR, bool SPLIT, int KS, bool TM>
 __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const __grid_constant__ DenseParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -612,7 +639,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   const int kbeg = SPLIT ? rank * p.ksteps / csize : 0;
   const int kcount = SPLIT ? (rank + 1) * p.ksteps / csize - kbeg : p.ksteps;
   const int xrows = PAIR ? p.bm / 2 : p.bm;
-  static_assert(!TM || (KS == kTmKs && !PAIR && (MODE == kFp8 || MODE == kNvfp4)), "");
+  static_assert(!TM || (KS == kTmKs && (MODE == kFp8 || MODE == kNvfp4)), "");
   constexpr int kX = TM ? 0 : kABytes;  // where x begins in a block
   const uint32_t block_bytes = static_cast<uint32_t>(kX + xrows * kBk * 2), stage_bytes = block_bytes * KS;
   const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]), accf0 = Smem(&ctl.acc_full[0]), acce0 = Smem(&ctl.acc_empty[0]);
@@ -622,7 +649,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
 
   if (tid == 0) {
     for (int i = 0; i < p.stages; ++i) {
-      BarInit(full0 + i * 8, 1 + (MODE == kBf16 ? 0 : TM ? kTmWarps : kDqWarps * (PAIR ? 2 : 1)));
+      BarInit(full0 + i * 8, 1 + (MODE == kBf16 ? 0 : (TM ? kTmWarps : kDqWarps) * (PAIR ? 2 : 1)));
       BarInit(empty0 + i * 8, 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -840,7 +867,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
               for (int i = 0; i < kBk / 16; ++i) {
                 const uint32_t at = off + j * (block_bytes >> 4);
                 if constexpr (TM) {
-                  MmaTs(d, a_tm + j * 32 + i * 8, b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
+                  MmaTs<PAIR>(d, a_tm + j * 32 + i * 8, b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
                 } else {
                   MmaSs<PAIR>(d, a0 + at + i * (2048 >> 4), b0 + at + i * (32 >> 4), idesc, k > 0 || i + j > 0);
                 }
@@ -860,7 +887,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
     } else {
       const int w = warp - kFirstDqWarp;
       if constexpr (TM) {
-        DequantTmRole<MODE, SCALED>(p, ctl, w, lane, kcount, first_tile, tile_step, ring, tmem);
+        DequantTmRole<MODE, SCALED, PAIR>(p, ctl, w, lane, rank, kcount, first_tile, tile_step, ring, tmem);
       } else {
         DequantRole<MODE, SCALED, PAIR, KS, kDqGroups>(p, ctl, w % kDqWarps, w / kDqWarps, lane, rank, kcount, first_tile, tile_step, ring, smem, block_bytes);
       }
@@ -1411,9 +1438,9 @@ cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, 
 template <int MODE, bool SCALED>
 cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, bool tm, int ctas, int cluster, size_t smem, cudaStream_t stream) {
   if constexpr (MODE == kFp8 || MODE == kNvfp4) {
-    if (tm)
-      return cluster > 1 ? LaunchOne<MODE, SCALED, false, true, kTmKs, true>(p, ctas, cluster, smem, stream)
-                         : LaunchOne<MODE, SCALED, false, false, kTmKs, true>(p, ctas, 1, smem, stream);
+    if (tm && pair) return LaunchOne<MODE, SCALED, true, false, kTmKs, true>(p, ctas, 2, smem, stream);
+    if (tm && cluster > 1) return LaunchOne<MODE, SCALED, false, true, kTmKs, true>(p, ctas, cluster, smem, stream);
+    if (tm) return LaunchOne<MODE, SCALED, false, false, kTmKs, true>(p, ctas, 1, smem, stream);
   }
   if (pair) return ks == 2 ? LaunchOne<MODE, SCALED, true, false, 2>(p, ctas, 2, smem, stream) : LaunchOne<MODE, SCALED, true, false, 1>(p, ctas, 2, smem, stream);
   if (cluster > 1)
@@ -1458,6 +1485,8 @@ cudaError_t SetUpShape() {
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   if constexpr (KS == kTmKs && (MODE == kFp8 || MODE == kNvfp4)) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
     if (err == cudaSuccess)
@@ -1556,13 +1585,19 @@ cudaError_t ConfigureDenseKernels() {
   return SetUpDevice(&setup);
 }
 
-// Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200;
-// us).  A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair 0.13 + 0.00098 bm
+// Launch shape: rows per tile, CTAs that split K, pairs.  The cheapest by a model fitted to measured launches (one B200; us).
+// A block of 64 k costs a single CTA 0.17 + 0.0011 bm (bm = 48: 0.22, 128: 0.31, 256: 0.45), a pair 0.13 + 0.00098 bm
 // (128: 0.25, 192: 0.32, 256: 0.38) and no less than its dequantisation (0.24); around the blocks 4 + 0.008 bm, 0.9 more for a pair, and 1.8 + 0.01 bm more where ranks add up: with
 // less for those two, as K = 5120 alone had suggested, short K was split and paired where that loses (BF16 146 x 400 x
 // 3728 6.3 us in pairs of 64, 5.5 in single tiles of 48; over 150 random calls the shape chosen took 3.7 % longer than the
 // best one, and takes 1.8).  More row tiles than needed are tried because they can fill the last wave better (509 rows,
 // N = 10240: 3 x 192 56 us, 2 x 256 61 us).
+// Through tensor memory (up to 128 rows of FP8 or NVFP4) a block costs 0.167 + 0.00041 bm, a pair or a small tile 0.175 (scaled 0.2);
+// a seventh more past 40 us, and 0.7 a wave.  Several row tiles of longer calls stay with larger tiles: those of 128
+// rows dequantise the weights more often and run against the power cap (NVFP4 509 rows 5120 x 17408 74.4 us in pairs of 256 rows, 80.4 in
+// tiles of 128).  On 57 calls (rows 9 to 2048, K 320 to 17408, N 512 to 17408) the shape chosen takes 0.1 % longer than the best one tried, 1.8 % at
+// worst.  Tensor memory was tried up to 192 rows, a block a stage: 0.36 a block in pairs, whatever their rows (FP8 400 rows 5120 x
+// 10240 52.8 -> 63.1 us).
 DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_count) {
   const DeviceSetup* setup = nullptr;
   if (SetUpDevice(&setup) != cudaSuccess) throw std::runtime_error("SkinnyGemm(dense): the kernels could not be set up on this device");
@@ -1572,6 +1607,10 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
     bytes += static_cast<double>(p.seg[s].total_bytes);
   }
   const int64_t blocks = (p.K + kBk - 1) / kBk, least = (m + 255) / 256;
+  const int kernel_mode = KernelMode(mode, p);
+  const bool tm_weights = kernel_mode == kFp8 || kernel_mode == kNvfp4;
+  bool scaled = false;
+  for (int s = 0; s < p.nseg; ++s) scaled = scaled || p.seg[s].w_scale != nullptr;
   for (int pair = 0; pair <= 1; ++pair) {
     int64_t n_tiles = 0;
     for (int s = 0; s < p.nseg; ++s) n_tiles += (p.seg[s].n + (pair ? 255 : 127)) / (pair ? 256 : 128);
@@ -1579,14 +1618,18 @@ DenseTcPlan ChooseDenseTcPlan(int mode, const GemmParams& p, int64_t m, int sm_c
       const int bm = static_cast<int>(((m + mt - 1) / mt + 15) / 16 * 16);
       if (bm > 256 || (pair && bm < 64)) continue;
       const int64_t tiles = n_tiles * ((m + bm - 1) / bm);
-      const double step = std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : 0.24);
+      const bool tm = tm_weights && bm <= kTmBm;
+      const double step = tm ? std::max(pair ? 0.0 : 0.167 + 0.00041 * bm, scaled ? 0.199 : 0.175)
+                             : std::max(pair ? 0.13 + 0.00098 * bm : 0.17 + 0.0011 * bm, mode == kBf16 ? 0.0 : 0.24);
       for (int split = 1; split <= (pair ? 1 : 8) && 4 * split <= std::max<int64_t>(blocks, 4); ++split) {
         const int64_t slots = pair ? sm_count / 2 : split == 1 ? sm_count : setup->slots[split];
         if (slots < 1) break;  // the device holds no such cluster
         const int64_t waves = (tiles + slots - 1) / slots;
         if (split > 1 && waves > 1) break;
-        const double work = std::max(static_cast<double>(waves * ((blocks + split - 1) / split)) * step, bytes / 6.3e6);
-        const double cost = work + 4 + 0.008 * bm + (split > 1 ? 1.8 + 0.01 * bm : pair ? 0.9 : 0);
+        double work = static_cast<double>(waves * ((blocks + split - 1) / split)) * step;
+        if (tm && mt > 1 && work > 40.0) continue;
+        if (tm) work += 0.146 * std::max(0.0, work - 40.0) + 0.7 * static_cast<double>(waves - 1);
+        const double cost = std::max(work, bytes / 6.3e6) + 4 + 0.008 * bm + (split > 1 ? 1.8 + 0.01 * bm : pair ? 0.9 : 0);
         if (cost < best_cost) {
           best_cost = cost;
           best.bm = bm;
@@ -1616,7 +1659,7 @@ bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
 }
 
 // Whether a launch shape that does not name its stages hands the weights over in tensor memory.
-bool TakesTm(int mode, const DenseTcPlan& plan) { return (mode == kFp8 || mode == kNvfp4) && !plan.pair && plan.bm <= kTmBm; }
+bool TakesTm(int mode, const DenseTcPlan& plan) { return (mode == kFp8 || mode == kNvfp4) && plan.bm <= kTmBm; }
 
 bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int mode = KernelMode(weights, g);
@@ -1660,7 +1703,7 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   if (p.stages < kDqGroups) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
   size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * ((tm ? 0 : kABytes) + xrows * kBk * 2) + kOutBytes;
   if (tm) {
-    const int slot = mode == kFp8 ? RawRing<kFp8, kTmKs>::kSlot : RawRing<kNvfp4, kTmKs>::kSlot;
+    const int slot = ks * (mode == kFp8 ? RawRing<kFp8, 1>::kSlot : RawRing<kNvfp4, 1>::kSlot);
     p.raw_depth = smem + 2 * kTmGroups * slot <= static_cast<size_t>(kSmemLimit) ? 2 * kTmGroups : kTmGroups;
     smem += static_cast<size_t>(p.raw_depth) * slot;
   } else {

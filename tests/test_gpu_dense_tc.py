@@ -81,10 +81,10 @@ def _check(mode, M, K, seg_widths, plan, seed, x_offset=0, out_offset=0, scale_c
         assert ok.all(), f"weight {i}: {np.count_nonzero(~ok)} of {ok.size} outputs outside tolerance"
 
 
-# tiles of up to 128 rows hand the weights over in tensor memory: one and several stages of a group, a K range shorter than the
-# groups, several tiles per CTA, ranks that add up
+# tiles of up to 128 rows hand the weights over in tensor memory: one and several stages of a group, a K
+# range shorter than the groups, several tiles per CTA, ranks that add up, pairs
 @pytest.mark.parametrize("mode", [1, 2])
-@pytest.mark.parametrize("plan", ["16,1,0", "48,5,0", "80,1,0", "112,2,0", "128,1,0", "128,8,0"])
+@pytest.mark.parametrize("plan", ["16,1,0", "48,5,0", "80,1,0", "112,2,0", "128,1,0", "128,8,0", "64,1,1", "96,1,1", "128,1,1"])
 def test_weights_through_tensor_memory(cuda, mode, plan):
     for i, (M, K, segs) in enumerate([(17, 72, [[256]]), (100, 2504, [[640 + 128], [128, 256 + 128]]), (300, 512, [[512]]), (129, 1096, [[256 * 45]])]):
         _check(mode, M, K, segs, plan, 900 + 10 * mode + i)
