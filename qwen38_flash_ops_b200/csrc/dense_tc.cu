@@ -1,5 +1,5 @@
 // Calls with many rows on the tensor memory path: out[M, N] = x[M, K] @ W[K, N] with BF16, FP8 or NVFP4 weights,
-// dequantised on the way into shared memory.
+// dequantised on the way into tensor memory or shared memory.
 //
 // A CTA computes tiles of 128 columns of W by `bm` rows of x (bm <= 256, a multiple of 16) with tcgen05.mma: the
 // weights are the 128-row operand, read MN-major because a stored row of W is contiguous along N, and the rows of x
@@ -12,20 +12,21 @@
 //   6     FP8 / NVFP4: copies the stored weights into a ring of their own (50-60 KB in flight per SM); 7 idles
 //   8-23  FP8 / NVFP4: sixteen warps in two groups that take the stages in turn; a warp turns eight weight rows of a
 //         stage into BF16, w_scale folded in before the one rounding
-// Rows of x are what the dequantisation is shared by: at bm = 256 a stage takes the tensor core 512 cycles, at
-// bm <= 64 the warps of the third role and the weight stream set the pace.
+// Rows of x are what the dequantisation is shared by: at bm = 256 a stage takes the tensor core 512 cycles.
+// TM, tiles of up to 128 rows of FP8 or NVFP4 (rows on 16 bytes): the weights are dequantised into tensor memory, by four groups of four
+// warps, and the MMA reads its first operand there (DequantTmRole).
 //
 // K is split over the CTAs of a cluster where the tiles alone leave SMs idle; the ranks then add their accumulators
 // through distributed shared memory in rank order.  PAIR: two CTAs of a cluster work on 256 columns with
 // cta_group::2; each holds its own 128 columns of W and half of the rows of x, which halves what the SMs fetch of x
 // from L2 (a 128 x 256 tile fetches 36 KB per 512 cycles, more than an SM's share of L2).
 //
-// What bounds it.  Few rows: the dequantising warps and the barriers between the roles, about 400 cycles a block of 64 k
-// (FP4 at 33 rows, 5120 x 17408: 23.7 us = 2.1 TB/s of weights; the dequantisation pass and the library GEMM that this
-// kernel took the place of, 86.6 us).  Many rows: the tensor core at its rate under load, and the last wave (FP8, 509
-// rows, 5120 x 10240: 65.6 us against 92.5; FP4, 2048 rows, 5120 x 17408: 291 to 302 us against 333).  The tcgen05 operands
-// come from shared memory rather than tensor memory because the rows of x per pass would be limited to 64 there, and the
-// weights are written MN-major because that is how a stored row lies: a nibble byte is two neighbouring columns.
+// What bounds it.  Few rows: MMAs of 64 cycles whatever their rows up to 64 (FP4 at 33 rows, 5120 x 17408: 18.3 us; through shared
+// memory, whose bandwidth the operand written and read back took, 21.5, and the dequantisation pass and the library GEMM that this kernel
+// took the place of, 86.6).  Many rows: the copies from L2 (20 KB a block and SM in pairs of 192 rows, 9.1 TB/s in all), the tensor core
+// at its rate under the power cap, and the last wave (FP8, 509 rows, 5120 x 10240: 62 to 64 us against 92.5; FP4, 2048 rows, 5120 x
+// 17408: 288 to 298 us against 333).  Through shared memory the weights are written MN-major because that is how a stored row
+// lies: a nibble byte is two neighbouring columns.
 //
 // Every wait is bounded.  A CTA that gives up on one writes NaN to the rest of its tiles and leaves: the call then reports
 // no error, but no output keeps what its memory held before.
