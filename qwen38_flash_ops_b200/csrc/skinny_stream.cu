@@ -210,12 +210,13 @@ __device__ __forceinline__ bool StageXByRow(const StreamParams& q, int kbeg, int
   const RowShare rs = ShareOf(q, warp);
   const int chunks = padded >> 3, valid = kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;
   const uint4 zero = make_uint4(0, 0, 0, 0);
+  const uint16_t *const x = BehindWait(p.x), *const x2 = FROM == kSwish ? BehindWait(p.x2) : nullptr;
   auto rows = [&](auto from_tag, bool track) {  // as they are
     constexpr int kFrom = decltype(from_tag)::value;
 #pragma unroll 1
     for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(m) * p.K + kbeg);
-      const uint4* src2 = kFrom == kSwish ? reinterpret_cast<const uint4*>(p.x2 + static_cast<size_t>(m) * p.K + kbeg) : nullptr;
+      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * p.K + kbeg);
+      const uint4* src2 = kFrom == kSwish ? reinterpret_cast<const uint4*>(x2 + static_cast<size_t>(m) * p.K + kbeg) : nullptr;
       uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
       uint32_t mx = 0, mn = 0xFFFFFFFFu;
 #pragma unroll 4
