@@ -162,6 +162,22 @@ __device__ __forceinline__ uint4 ScaleToHalf8(uint4 v, float sc) {
   return make_uint4(ScaleToHalf2(v.x, sc), ScaleToHalf2(v.y, sc), ScaleToHalf2(v.z, sc), ScaleToHalf2(v.w, sc));
 }
 
+// the other way round: FP16 values times a power of two, exact where the products are normal FP16 numbers
+__device__ __forceinline__ uint32_t RescaleHalf2(uint32_t w, float ratio) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  const __half2 h = __floats2half2_rn(f.x * ratio, f.y * ratio);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint4 RescaleHalf8(uint4 v, float ratio) {
+  return make_uint4(RescaleHalf2(v.x, ratio), RescaleHalf2(v.y, ratio), RescaleHalf2(v.z, ratio), RescaleHalf2(v.w, ratio));
+}
+// Whether one of eight FP16 magnitudes is below that of the bits `least`, or not finite.
+__device__ __forceinline__ bool LostInHalf(uint4 v, uint32_t least) {
+  v = make_uint4(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu, v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu);
+  const uint32_t mx = __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w)), mn = __vminu2(__vminu2(v.x, v.y), __vminu2(v.z, v.w));
+  return max(mx & 0xFFFFu, mx >> 16) >= 0x7C00u || min(mn & 0xFFFFu, mn >> 16) < least;
+}
+
 struct StreamScratch {
   uint32_t xmax[kMaxRows][kStreamWarps], xmin[kMaxRows][kStreamWarps];
   float gate[kMaxRows][2];  // SharedExpertDown: the two halves of the gate's sum
@@ -182,10 +198,10 @@ __device__ __forceinline__ RowShare ShareOf(const StreamParams& q, int warp) {
   return r;
 }
 
-// x in FP16, the usual way: times 2^5, in one look at it.  Exact for zero and for magnitudes from 2^-22 (eight significant bits,
-// the last of them FP16's smallest number after the scaling) to 2^11.
-constexpr float kUsualScale = 32.f;
-constexpr uint32_t kUsualLeast = 127 - 22, kUsualMost = 127 + 10;  // exponent fields
+// x in FP16, the usual way: times 2^10, in one look at it.  Exact for zero and for magnitudes from 2^-27 (eight significant bits,
+// the last of them FP16's smallest number after the scaling) to 2^6.
+constexpr float kUsualScale = 1024.f;
+constexpr uint32_t kUsualLeast = 127 - 27, kUsualMost = 127 + 5;  // exponent fields
 __device__ __forceinline__ void Track(const uint4& v, uint32_t& mx, uint32_t& mn) {
   TrackPair(v.x, mx, mn);
   TrackPair(v.y, mx, mn);
@@ -196,81 +212,157 @@ __device__ __forceinline__ bool Unusual(uint32_t mx, uint32_t mn) {  // what Tra
   const uint32_t most = max(mx & 0xFFFFu, mx >> 16), least = min(mn & 0xFFFFu, mn >> 16) + 1u;
   return most != 0 && ((most >> 7) > kUsualMost || (least >> 7) < kUsualLeast);
 }
+// What a warp's lanes saw of row m, for RowScale of all warps behind the next barrier; true: not all of it fits the usual scaling.
+__device__ __forceinline__ bool Publish(StreamScratch& sx, int m, int part, int lane, uint32_t mx, uint32_t mn) {
+  mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
+  mn = __reduce_min_sync(0xffffffffu, min(mn & 0xFFFFu, mn >> 16));
+  if (lane == 0) {
+    sx.xmax[m][part] = mx;
+    sx.xmin[m][part] = mn;
+  }
+  return mx != 0 && ((mx >> 7) > kUsualMost || ((mn + 1u) >> 7) < kUsualLeast);
+}
+// Pieces of eight elements that a lane has on their way at a time, and holds until the slice is known to fit.  Six: four, 0.8 us
+// more for 17408 x 5120 and eight rows (18 us, slices of 5.7 pieces a lane); eight, 0.2 us more for four.
+constexpr int kBatch = 6;
+// The power of two that puts the maximum of row m of a slice in [2^14, 2^15), where every non-zero element then is a normal FP16
+// number: an exponent no more than 28 below the maximum's.  `out`: some element is not.  `low`: one is below the usual window.
+__device__ __forceinline__ float RowScale(const StreamScratch& sx, int m, int wpr, int lane, bool& out, bool& low) {
+  const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < wpr ? sx.xmax[m][lane] : 0u);
+  const uint32_t mn = __reduce_min_sync(0xffffffffu, lane < wpr ? sx.xmin[m][lane] : 0xFFFFu);
+  const int e = static_cast<int>(mx >> 7);  // BF16 exponent field of the row maximum
+  low = ((mn + 1) >> 7) < kUsualLeast;
+  out = mx != 0 && (e < 32 || e >= 255 || static_cast<int>((mn + 1) >> 7) < e - 28);
+  return mx != 0 && !out ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
+}
 
-// x of a slice whose values do not all fit the usual scaling: each row times the power of two that puts the slice's maximum in
-// [2^14, 2^15), where every non-zero element then is a normal FP16 number (an exponent no more than 28 below the maximum's), else
-// all rows as they are, for the BF16 path.  Returns true for the latter.  FROM: where the rows are: in memory, swish_mul of g and u in
-// memory, or copied to shared memory for the head.  `lost`: those copies did not come; the rows are then scaled by NaN and so are
-// the sums: the stages of the weights come all the same, and the loop would take them.
-enum RowSource : int { kRows = 0, kSwish = 1, kCopied = 2 };
-template <int MODE, int FROM>
-__device__ __forceinline__ bool StageXByRow(const StreamParams& q, int kbeg, int kslice, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, bool lost, int padded,
-                                            int warp, int lane) {
+// Eight elements of x, or of swish_mul(g, u).
+template <bool SWISH>
+__device__ __forceinline__ uint4 LoadX8(const uint4* x, const uint4* u, int c) {
+  const uint4 v = __ldg(x + c);
+  if constexpr (SWISH) {
+    const uint4 w = __ldg(u + c);
+    return make_uint4(SwishMul2(v.x, w.x), SwishMul2(v.y, w.y), SwishMul2(v.z, w.z), SwishMul2(v.w, w.w));
+  }
+  return v;
+}
+// All rows as they are, for the BF16 path (rare).
+template <bool SWISH>
+__device__ __forceinline__ void StageXRaw(const StreamParams& q, int kbeg, int kslice, uint16_t* xs, SharedScratch& sh, int padded, const RowShare& rs, int lane) {
+  const GemmParams& p = q.g;
+  const uint16_t *const x = BehindWait(p.x), *const x2 = SWISH ? BehindWait(p.x2) : nullptr;
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * p.K + kbeg);
+    const uint4* src2 = SWISH ? reinterpret_cast<const uint4*>(x2 + static_cast<size_t>(m) * p.K + kbeg) : nullptr;
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 4
+    for (int c = rs.part * 32 + lane; c < padded >> 3; c += rs.wpr * 32) dst[c] = c < kslice >> 3 ? LoadX8<SWISH>(src, src2, c) : make_uint4(0, 0, 0, 0);
+  }
+  if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = 1.f;
+  __syncthreads();
+}
+
+// A slice of x that the usual scaling did not fit, scaled by rows instead: from what the lanes hold of it where that is all, else from
+// what lies in FP16 already.  That is exact wherever it is neither infinite nor, in a row with values below the window, 2^-17 or
+// less (what they round to, or zero), and takes another power of two where it lies; only pieces of eight with something else among
+// them are asked for again.  It costs such calls 0.1 (FP8 5120 x 10240, two rows: 11.6 us) to 2.9 us (NVFP4 5120 x 34816,
+// eight rows: 24.1); staging all of it over again cost 0.8 to 5.5.  Returns true if a row's values are too far apart for FP16: all rows
+// then are staged as they are.
+__device__ __forceinline__ bool RestageX(const StreamParams& q, int kbeg, int kslice, uint16_t* xs, SharedScratch& sh, const StreamScratch& sx,
+                                         const uint4 (&held)[kBatch], int padded, int warp, int lane) {
   const GemmParams& p = q.g;
   const RowShare rs = ShareOf(q, warp);
-  const int chunks = padded >> 3, valid = kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  const uint16_t *const x = BehindWait(p.x), *const x2 = FROM == kSwish ? BehindWait(p.x2) : nullptr;
-  auto rows = [&](auto from_tag, bool track) {  // as they are
-    constexpr int kFrom = decltype(from_tag)::value;
+  const uint16_t* const x = BehindWait(p.x);
+  const int valid = kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // the zeros behind `valid` stay zeros
+  bool bad = p.force_slow != 0;
 #pragma unroll 1
-    for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
-      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * p.K + kbeg);
-      const uint4* src2 = kFrom == kSwish ? reinterpret_cast<const uint4*>(x2 + static_cast<size_t>(m) * p.K + kbeg) : nullptr;
-      uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
-      uint32_t mx = 0, mn = 0xFFFFFFFFu;
-#pragma unroll 4
-      for (int c = c_first; c < chunks; c += step) {
-        uint4 v = c >= valid ? zero : kFrom == kCopied ? dst[c] : __ldg(src + c);
-        if constexpr (kFrom == kSwish) {
-          const uint4 u = c < valid ? __ldg(src2 + c) : zero;
-          v = make_uint4(SwishMul2(v.x, u.x), SwishMul2(v.y, u.y), SwishMul2(v.z, u.z), SwishMul2(v.w, u.w));
-        }
-        if (kFrom != kCopied || c >= valid) dst[c] = v;
-        Track(v, mx, mn);
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    bool out, low;
+    const float sc = RowScale(sx, m, rs.wpr, lane, out, low), ratio = sc / kUsualScale;
+    const uint32_t least = low ? 0x0081u : 0u;  // without such values a zero is a zero
+    if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f / sc;
+    bad = bad || out;
+    if (out) continue;
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+    if (padded >> 3 <= kBatch * step && rs.rpp >= p.M) {  // one batch, of one row
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        if (c_first + i * step < valid) dst[c_first + i * step] = ScaleToHalf8(held[i], sc);
       }
-      if (!track) continue;
-      mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
-      mn = __reduce_min_sync(0xffffffffu, min(mn & 0xFFFFu, mn >> 16));
-      if (lane == 0) {
-        sx.xmax[m][rs.part] = mx;
-        sx.xmin[m][rs.part] = mn;
+      continue;
+    }
+    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * p.K + kbeg);
+#pragma unroll 1
+    for (int c0 = c_first; c0 < valid; c0 += 32 * step) {
+      uint32_t lost = 0;
+      const int n = min(32, (valid - c0 + step - 1) / step);
+#pragma unroll 2
+      for (int i = 0; i < n; ++i) {
+        const uint4 v = dst[c0 + i * step];
+        lost |= LostInHalf(v, least) ? 1u << i : 0u;
+        dst[c0 + i * step] = RescaleHalf8(v, ratio);
+      }
+#pragma unroll 1
+      for (; lost != 0; lost &= lost - 1) {
+        const int c = c0 + (__ffs(lost) - 1) * step;
+        dst[c] = ScaleToHalf8(__ldg(src + c), sc);
       }
     }
-  };
-  rows(std::integral_constant<int, FROM>(), true);
+  }
+  if (!__any_sync(0xffffffffu, __syncthreads_or(bad))) return false;
+  StageXRaw<false>(q, kbeg, kslice, xs, sh, padded, rs, lane);
+  return true;
+}
+
+// The same for swish_mul, which is evaluated again, 1.2 us: what holding pieces or the extremes of the rows for it takes is 0.1 us of
+// every call, of 6 us.
+__device__ __forceinline__ bool RestageSwish(const StreamParams& q, int kbeg, int kslice, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, int padded, int warp,
+                                             int lane) {
+  const GemmParams& p = q.g;
+  const RowShare rs = ShareOf(q, warp);
+  const uint16_t *const g = BehindWait(p.x), *const u = BehindWait(p.x2);
+  const int valid = kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    const size_t at = static_cast<size_t>(m) * p.K + kbeg;
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+    uint32_t mx = 0, mn = 0xFFFFFFFFu;
+#pragma unroll 1
+    for (int c = c_first; c < valid; c += step) {
+      const uint4 v = LoadX8<true>(reinterpret_cast<const uint4*>(g + at), reinterpret_cast<const uint4*>(u + at), c);
+      dst[c] = v;
+      Track(v, mx, mn);
+    }
+    Publish(sx, m, rs.part, lane, mx, mn);
+  }
   __syncthreads();
   bool bad = p.force_slow != 0;
 #pragma unroll 1
   for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
-    const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < rs.wpr ? sx.xmax[m][lane] : 0u);
-    const uint32_t mn = __reduce_min_sync(0xffffffffu, lane < rs.wpr ? sx.xmin[m][lane] : 0xFFFFu);
-    const int e = static_cast<int>(mx >> 7);  // BF16 exponent field of the row maximum
-    const bool out = mx != 0 && (e < 32 || e >= 255 || static_cast<int>((mn + 1) >> 7) < e - 28);
-    bad = bad || out;
-    const float sc = lost ? __uint_as_float(0x7FFFFFFFu) : mx != 0 && !out ? __uint_as_float((268u - (mx >> 7)) << 23) : 1.f;
+    bool out, low;
+    const float sc = RowScale(sx, m, rs.wpr, lane, out, low);
     if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f / sc;
+    bad = bad || out;
     uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
-#pragma unroll 2
-    for (int c = c_first; c < chunks; c += step) dst[c] = ScaleToHalf8(dst[c], sc);
+#pragma unroll 1
+    for (int c = c_first; c < valid; c += step) dst[c] = ScaleToHalf8(dst[c], sc);
   }
   if (!__any_sync(0xffffffffu, __syncthreads_or(bad))) return false;
-  rows(std::integral_constant<int, FROM == kCopied ? kRows : FROM>(), false);  // rare
-  if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = 1.f;
-  __syncthreads();
+  StageXRaw<true>(q, kbeg, kslice, xs, sh, padded, rs, lane);
   return true;
 }
 
 // x of the slice to shared memory, rows padded with zeros to whole stages (so that the K loop needs no end), for the
-// quantised modes scaled by a power of two and converted to FP16 (skinny_common.cuh), as a rule all rows by the same one: one trip
+// quantised modes scaled by a power of two and converted to FP16 (skinny_common.cuh), all rows by the same one: one trip
 // to L2 and one barrier.  (Looking for the rows' maxima first took a second pass and barrier: FP8 5120 x 10240, two rows,
-// 12.6 -> 12.0 us; NVFP4 2560 x 2560, four rows, 6.4 -> 5.9, shared expert 640 x 2560 6.9 -> 6.2.  Slices that do not fit are staged
-// over again, which costs such calls 1 us.)  Returns true if some value does not fit that scaling.
+// 12.6 -> 12.0 us; NVFP4 2560 x 2560, four rows, 6.4 -> 5.9, shared expert 640 x 2560 6.9 -> 6.2.)  Returns true if some value does not
+// fit that scaling (RestageX).
 template <int MODE>
-__device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, int padded, const RowShare& rs, int lane) {
+__device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, uint4 (&held)[kBatch],
+                                             int padded, const RowShare& rs, int lane) {
   const GemmParams& p = q.g;
   const uint16_t* const x = BehindWait(p.x);
-  constexpr int kBatch = 4;
   const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;  // K is a multiple of eight
   bool bad = p.force_slow != 0;
 #pragma unroll 1
@@ -280,16 +372,15 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
     uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
 #pragma unroll 1
     for (int c = c_first; c < chunks; c += kBatch * step) {
-      uint4 v[kBatch];
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) v[i] = c + i * step < valid ? __ldg(src + c + i * step) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < kBatch; ++i) held[i] = c + i * step < valid ? __ldg(src + c + i * step) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int i = 0; i < kBatch; ++i) {
-        if constexpr (MODE != kBf16) Track(v[i], mx, mn);
-        if (c + i * step < chunks) dst[c + i * step] = MODE == kBf16 ? v[i] : ScaleToHalf8(v[i], kUsualScale);
+        if constexpr (MODE != kBf16) Track(held[i], mx, mn);
+        if (c + i * step < chunks) dst[c + i * step] = MODE == kBf16 ? held[i] : ScaleToHalf8(held[i], kUsualScale);
       }
     }
-    if constexpr (MODE != kBf16) bad = bad || Unusual(mx, mn);
+    if constexpr (MODE != kBf16) bad = Publish(sx, m, rs.part, lane, mx, mn) || bad;
   }
   if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = MODE == kBf16 ? 1.f : 1.f / kUsualScale;  // for the epilogue, behind further barriers
   // every warp also sees the mbarriers
@@ -302,24 +393,49 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
 }
 
 // The head's: the producer has the rows copied, and they are only waited for; that gave it 3 us of 85 at four rows and cost calls of 5
-// to 17 us 0.3 us, so the products load them.  Rows are scaled one by one: the usual scaling gained nothing in 90 us.
+// to 17 us 0.3 us, so the products load them.  Rows are scaled one by one: the usual scaling gained nothing in 90 us.  Where the copies
+// did not come, the rows are scaled by NaN and so are the sums: the stages of the weights come all the same, and the loop would
+// take them.  Returns true for the BF16 path.
 template <int MODE>
 __device__ __forceinline__ bool StageXHead(const StreamParams& q, const Tile& tl, uint16_t* xs, SharedScratch& sh, StreamScratch& sx, StreamCtl& ctl, int padded,
-                                           const RowShare& rs, int warp, int lane) {
+                                           const RowShare& rs, int lane) {
   const GemmParams& p = q.g;
+  const int chunks = padded >> 3, valid = tl.kslice >> 3, step = rs.wpr * 32, c_first = rs.part * 32 + lane;
+  const float kNaN = __uint_as_float(0x7FFFFFFFu);
   BarWait(SmemAddr(&ctl.x_full), 0, ctl);
-  if constexpr (MODE != kBf16) {
-    return StageXByRow<MODE, kCopied>(q, tl.kbeg, tl.kslice, xs, sh, sx, ctl.fault != 0, padded, warp, lane);
-  } else {
-    for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
-      uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
-      for (int c = rs.part * 32 + lane; c < padded >> 3; c += rs.wpr * 32) {
-        if (c >= tl.kslice >> 3) dst[c] = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+  for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+    uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+    uint32_t mx = 0, mn = 0xFFFFFFFFu;
+#pragma unroll 4
+    for (int c = c_first; c < chunks; c += step) {
+      if (c >= valid) {
+        dst[c] = make_uint4(0, 0, 0, 0);
+      } else if (MODE != kBf16) {
+        Track(dst[c], mx, mn);
       }
     }
-    if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = ctl.fault ? __uint_as_float(0x7FFFFFFFu) : 1.f;
-    __syncthreads();
+    if constexpr (MODE != kBf16) Publish(sx, m, rs.part, lane, mx, mn);
+  }
+  __syncthreads();
+  if constexpr (MODE == kBf16) {
+    if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = ctl.fault ? kNaN : 1.f;  // for the epilogue, behind further barriers
     return false;
+  } else {
+    bool bad = p.force_slow != 0;
+#pragma unroll 1
+    for (int m = rs.row; rs.any && m < p.M; m += rs.rpp) {
+      bool out, low;
+      const float row_scale = RowScale(sx, m, rs.wpr, lane, out, low), sc = ctl.fault ? kNaN : row_scale;
+      bad = bad || out;
+      if (rs.part == 0 && lane == 0) sh.inv_scale[m] = 1.f / sc;
+      uint4* dst = reinterpret_cast<uint4*>(xs + m * p.xpitch);
+#pragma unroll 2
+      for (int c = c_first; c < chunks; c += step) dst[c] = ScaleToHalf8(dst[c], sc);
+    }
+    if (!__any_sync(0xffffffffu, __syncthreads_or(bad))) return false;
+    StageXRaw<false>(q, tl.kbeg, tl.kslice, xs, sh, padded, rs, lane);
+    return true;
   }
 }
 
@@ -384,16 +500,14 @@ __device__ __forceinline__ bool StageXShared(const StreamParams& q, const Tile& 
     }
     if constexpr (MODE != kBf16) bad = bad || Unusual(mx, mn);
   }
+  if (threadIdx.x < kMaxRows) sh.inv_scale[threadIdx.x] = MODE == kBf16 ? 1.f : 1.f / kUsualScale;  // for the epilogue, behind further barriers
   bool again = false;
   if constexpr (MODE == kBf16) {
     __syncthreads();
   } else {
     again = __syncthreads_or(bad);
   }
-  if (threadIdx.x < p.M) {  // for the epilogue, behind further barriers
-    sh.gate[threadIdx.x] = SigmoidBf16(RoundBf16(sx.gate[threadIdx.x][0] + sx.gate[threadIdx.x][1]));
-    sh.inv_scale[threadIdx.x] = MODE == kBf16 ? 1.f : 1.f / kUsualScale;
-  }
+  if (threadIdx.x < p.M) sh.gate[threadIdx.x] = SigmoidBf16(RoundBf16(sx.gate[threadIdx.x][0] + sx.gate[threadIdx.x][1]));
   return again;
 }
 
@@ -803,14 +917,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   uint16_t* const xs = reinterpret_cast<uint16_t*>(smem + q.x_off);
   const int padded = nst * q.rows;
   Stamp(p, 1);
-  bool usual = true, slow = false;
+  bool unusual = false, slow = false;
+  uint4 held[kBatch];
   if constexpr (KIND == kShared) {
-    usual = !StageXShared<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
+    unusual = StageXShared<MODE>(q, tl, xs, sh, sx, padded, rs, lane);
   } else if constexpr (KIND == kPlain) {
-    usual = !StageXStream<MODE>(q, tl, xs, sh, padded, rs, lane);
+    unusual = StageXStream<MODE>(q, tl, xs, sh, sx, held, padded, rs, lane);
   } else {
     if (warp != q.warps) asm volatile("bar.sync 1, %0;" ::"r"(static_cast<int>(blockDim.x)) : "memory");
-    slow = __any_sync(0xffffffffu, StageXHead<MODE>(q, tl, xs, sh, sx, ctl, padded, rs, warp, lane));
+    slow = StageXHead<MODE>(q, tl, xs, sh, sx, ctl, padded, rs, lane);
   }
   Stamp(p, 2);
 
@@ -819,13 +934,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   // loop's addresses and control leave the uniform registers, 15 instructions more per k-step and warp (NVFP4 5120 x 34816 22.3
   // -> 24.2 us, 17408 x 5120, four rows, 15.9 -> 17.2; `ncu` 12.9 -> 13.8 M warp instructions).
   if constexpr (KIND == kHead || MODE == kBf16) {
-    StreamRest<MODE, KIND>(slow, q, w, sh, ctl);
-  } else if (__all_sync(0xffffffffu, usual)) {
+    StreamRest<MODE, KIND>(__any_sync(0xffffffffu, slow), q, w, sh, ctl);
+  } else if (__all_sync(0xffffffffu, !unusual)) {
     StreamRest<MODE, KIND>(false, q, w, sh, ctl);
-  } else if (__any_sync(0xffffffffu, StageXByRow<MODE, KIND == kShared ? kSwish : kRows>(q, tl.kbeg, tl.kslice, xs, sh, sx, false, padded, warp, lane))) {
-    StreamRest<MODE, KIND>(true, q, w, sh, ctl);
   } else {
-    StreamRest<MODE, KIND>(false, q, w, sh, ctl);
+    if constexpr (KIND == kShared) {
+      slow = RestageSwish(q, tl.kbeg, tl.kslice, xs, sh, sx, padded, warp, lane);
+    } else {
+      slow = RestageX(q, tl.kbeg, tl.kslice, xs, sh, sx, held, padded, warp, lane);
+    }
+    StreamRest<MODE, KIND>(__any_sync(0xffffffffu, slow), q, w, sh, ctl);
   }
 }
 
