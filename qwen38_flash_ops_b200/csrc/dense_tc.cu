@@ -1108,10 +1108,22 @@ struct SwishRole {
   }
 };
 
+// Sixteen products of a row of gx each for rows (g, g + 8) of a lane, added to nothing.
+__device__ __forceinline__ float2 Dot16(uint32_t lo0, uint32_t hi0, uint32_t lo1, uint32_t hi1, uint32_t w0, uint32_t w1) {
+  float d[4];
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(lo0), "r"(hi0), "r"(lo1), "r"(hi1), "r"(w0), "r"(w1), "f"(0.f));
+  return make_float2(d[0], d[2]);
+}
+
 // This CTA's share of the gates, to every CTA of the cluster: asynchronous stores that count their bytes in on the
 // receiver's barrier.  The dot products are MMAs of sixteen rows of gx with gw in every column: a lane reads 16 bytes of two
 // rows, eight k of its own, and the same eight of gw, so that the order of k within an MMA is free (multiplied out they were
 // 24 instructions per 16 bytes, a third of the call).  A warp takes a quarter of k; the quarters are added in order.
+// An MMA adds sixteen products and nothing else: an accumulator that runs through them is cut off at every one, not rounded.  The
+// sums of sixteen go to FP32 sums by ordinary additions, eight of 2560 elements to each.  Gates that are not the 64-bit gate's BF16 number, of
+// 2.5 million of twelve kinds (250 to 4096 elements, of both signs, of one, cancelling): 249 with running accumulators, 79 with FP32
+// multiply-adds, 63 so.
 __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, float (*quarter)[256], uint32_t bar, int warp, int lane, int rank, int m0) {
   const uint16_t *const gx_in = BehindWait(q.gx), *const gw_in = BehindWait(q.gw);
   const int p0 = FirstRow(q, rank), part = FirstRow(q, rank + 1) - p0;
@@ -1126,7 +1138,7 @@ __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, floa
       const uint4* lo_row = reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m) * q.gk);
       const uint4* hi_row = reinterpret_cast<const uint4*>(gx_in + static_cast<size_t>(m + 8) * q.gk);
       const uint4* gw = reinterpret_cast<const uint4*>(gw_in);
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 c[3] = {};
 #pragma unroll 1
       for (int s = warp * steps / kGateWarps; s < s1; s += kAhead) {
         uint4 lo[kAhead], hi[kAhead], w[kAhead];
@@ -1140,15 +1152,14 @@ __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, floa
         }
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo[i].x), "r"(hi[i].x), "r"(lo[i].y), "r"(hi[i].y), "r"(w[i].x), "r"(w[i].y));
-          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo[i].z), "r"(hi[i].z), "r"(lo[i].w), "r"(hi[i].w), "r"(w[i].z), "r"(w[i].w));
+          const float2 a = Dot16(lo[i].x, hi[i].x, lo[i].y, hi[i].y, w[i].x, w[i].y), b = Dot16(lo[i].z, hi[i].z, lo[i].w, hi[i].w, w[i].z, w[i].w);
+          c[i % 3].x += a.x + b.x;
+          c[i % 3].y += a.y + b.y;
         }
       }
       if (t == 0) {
-        quarter[warp][r0 + g] = c[0];
-        if (r0 + 8 < part) quarter[warp][r0 + 8 + g] = c[2];
+        quarter[warp][r0 + g] = (c[0].x + c[1].x) + c[2].x;
+        if (r0 + 8 < part) quarter[warp][r0 + 8 + g] = (c[0].y + c[1].y) + c[2].y;
       }
     }
   } else {
