@@ -123,7 +123,9 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
  * of the LM head is a NaN), the call succeeds and the next one is whole.  "give_up" = 1, for tests, makes every block of
  * an LM head act as if its wait for x had run out.
  * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken;
- * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape. */
+ * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape.  The blocks may be left out.  One sends FP8 and
+ * NVFP4 weights of tiles of up to 128 rows through shared memory, two, like none, through tensor memory; larger tiles have two where
+ * they fit in pairs, BF16 weights wherever they fit, else one is taken.  A shape that does not exist is an error of the call. */
 QFG_API int qfg_skinny_gemm_set_option(qfg_skinny_gemm* op, const char* key, const char* value);
 
 /* Writes a one-line description of the launch plan chosen for these shapes into buf: the general kernels' geometry, then

@@ -1447,6 +1447,11 @@ cudaError_t LaunchOne(const DenseParams& p, int ctas, int cluster, size_t smem, 
   return cudaLaunchKernelEx(&cfg, DenseTcKernel<MODE, SCALED, PAIR, SPLIT, KS, TM>, p);
 }
 
+// Whether there are kernels of two blocks a stage.  The unpaired tiles of FP8 and NVFP4 that do not take tensor memory are too large for
+// enough of those.
+template <int MODE, bool PAIR>
+constexpr bool kTwoBlocks = PAIR || MODE == kBf16 || MODE == kNvfp4Odd;
+
 template <int MODE, bool SCALED>
 cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, bool tm, int ctas, int cluster, size_t smem, cudaStream_t stream) {
   if constexpr (MODE == kFp8 || MODE == kNvfp4) {
@@ -1455,9 +1460,10 @@ cudaError_t LaunchMode(const DenseParams& p, bool pair, int ks, bool tm, int cta
     if (tm) return LaunchOne<MODE, SCALED, false, false, kTmKs, true>(p, ctas, 1, smem, stream);
   }
   if (pair) return ks == 2 ? LaunchOne<MODE, SCALED, true, false, 2>(p, ctas, 2, smem, stream) : LaunchOne<MODE, SCALED, true, false, 1>(p, ctas, 2, smem, stream);
-  if (cluster > 1)
-    return ks == 2 ? LaunchOne<MODE, SCALED, false, true, 2>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, true, 1>(p, ctas, cluster, smem, stream);
-  return ks == 2 ? LaunchOne<MODE, SCALED, false, false, 2>(p, ctas, 1, smem, stream) : LaunchOne<MODE, SCALED, false, false, 1>(p, ctas, 1, smem, stream);
+  if constexpr (kTwoBlocks<MODE, false>) {
+    if (ks == 2) return cluster > 1 ? LaunchOne<MODE, SCALED, false, true, 2>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, false, 2>(p, ctas, 1, smem, stream);
+  }
+  return cluster > 1 ? LaunchOne<MODE, SCALED, false, true, 1>(p, ctas, cluster, smem, stream) : LaunchOne<MODE, SCALED, false, false, 1>(p, ctas, 1, smem, stream);
 }
 
 template <int MODE>
@@ -1491,11 +1497,13 @@ std::atomic<const DeviceSetup*> g_setup_last{nullptr};  // the last one asked fo
 
 template <int MODE, bool SCALED, int KS>
 cudaError_t SetUpShape() {
-  cudaError_t err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  cudaError_t err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  if constexpr (KS == 1 || kTwoBlocks<MODE, false>) {
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, false, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, false, true, KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  }
   if constexpr (KS == kTmKs && (MODE == kFp8 || MODE == kNvfp4)) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(DenseTcKernel<MODE, SCALED, true, false, KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
@@ -1670,8 +1678,8 @@ bool DenseTcEligible(int mode, const GemmParams& p, int64_t m) {
   return TensorMapEncoder() != nullptr;
 }
 
-// Whether a launch shape that does not name its stages hands the weights over in tensor memory.
-bool TakesTm(int mode, const DenseTcPlan& plan) { return (mode == kFp8 || mode == kNvfp4) && plan.bm <= kTmBm; }
+// Whether a launch shape hands the weights over in tensor memory, two blocks a stage; one block goes through shared memory.
+bool TakesTm(int mode, const DenseTcPlan& plan) { return (mode == kFp8 || mode == kNvfp4) && plan.bm <= kTmBm && plan.ks != 1; }
 
 bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int mode = KernelMode(weights, g);
@@ -1683,8 +1691,12 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   p.K = g.K;
   p.bm = plan.bm;
   const int xrows = plan.pair ? p.bm / 2 : p.bm;
-  const bool tm = plan.ks == 0 && TakesTm(mode, plan);
-  const int ks = tm ? kTmKs : plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1, blocks = BlocksFor(mode, xrows, ks);
+  const bool tm = TakesTm(mode, plan);
+  int ks = tm ? kTmKs : plan.ks > 0 ? plan.ks : BlocksFor(mode, xrows, 2) >= 6 ? 2 : 1;
+  // the dequantising groups take the stages in turn: fewer stages than groups would run off the ring
+  if (!tm && BlocksFor(mode, xrows, ks) < kDqGroups * ks) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
+  if (!tm && !plan.pair && (mode == kFp8 || mode == kNvfp4)) ks = 1;  // kTwoBlocks
+  const int blocks = BlocksFor(mode, xrows, ks);
   p.ksteps = (g.K + kBk * ks - 1) / (kBk * ks);
   if (!Encode(&p.xmap, g.x, 2, static_cast<uint64_t>(m), static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.K) * 2, static_cast<uint32_t>(xrows), kBk))
     return false;
@@ -1711,8 +1723,6 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   p.tiles = p.m_tiles * n_tiles;
   const int cluster = plan.pair ? 2 : std::min(plan.split, p.ksteps);
   p.stages = tm ? kTmStages : std::min(kMaxStages, blocks / ks);
-  // the dequantising groups take the stages in turn: fewer stages than groups would run off the ring
-  if (p.stages < kDqGroups) throw std::runtime_error("SkinnyGemm(dense): bad launch shape");
   size_t smem = 1024 + static_cast<size_t>(p.stages) * ks * ((tm ? 0 : kABytes) + xrows * kBk * 2) + kOutBytes;
   if (tm) {
     const int slot = ks * (mode == kFp8 ? RawRing<kFp8, 1>::kSlot : RawRing<kNvfp4, 1>::kSlot);
@@ -1781,7 +1791,8 @@ DenseTcPlan ChooseDenseSharedPlan(const GemmParams& p, int64_t m, int sm_count) 
 bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseTcPlan& plan, cudaStream_t stream) {
   const int mode = KernelMode(weights, g);
   const int C = plan.split;
-  // a pinned shape has even shares in a cluster of up to four, unless it names the blocks per stage, of which there is one
+  // Shares are even and clusters of 1, 2 or 4 where a pinned shape does not name the blocks per stage, of which there is one: "48,4" and "64,3"
+  // have always been errors, and who pins one of them to be told so still is.
   const bool even = (C == 1 || C == 2 || C == 4) && plan.bm % (8 * C) == 0;
   if (C < 1 || C > kMaxCluster || plan.bm < 16 || plan.bm > 256 || plan.bm % 16 != 0 || plan.bm < 8 * C || (!even && plan.ks != 1))
     throw std::runtime_error("SharedExpertDown: bad launch shape");

@@ -272,12 +272,14 @@ constexpr int DenseRowsDefault(int mode) { return mode == kNvfp4 ? 16 : 8; }
 bool DenseEligible(const GemmParams& p);
 void LaunchDenseGemm(int mode, const GemmParams& p, int64_t m, cudaStream_t stream);  // throws std::runtime_error
 
-// dense_tc.cu: the same calls in one kernel, dequantising into shared memory.
+// dense_tc.cu: the same calls in one kernel, dequantising into tensor memory or shared memory.
 struct DenseTcPlan {
   int bm = 0;     // rows of x per tile: a multiple of 16, at most 256
   int split = 1;  // CTAs (a cluster) that share the K range of a tile
   int pair = 0;   // two CTAs per tile of 256 columns
-  int ks = 0;     // blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room
+  // Blocks of 64 k per pipeline stage: 1 or 2, 0 = by the room.  FP8 and NVFP4 weights (rows on 16 bytes) of tiles of up to 128 rows are handed
+  // over in tensor memory, two blocks a stage, unless this is 1; those of larger unpaired tiles one block a stage.
+  int ks = 0;
 };
 cudaError_t ConfigureDenseKernels();  // on the current device
 bool DenseTcEligible(int mode, const GemmParams& p, int64_t m);

@@ -171,3 +171,19 @@ def test_launch_shapes_use_the_clusters_that_the_device_holds(fake, resident, cl
     for code, message, log in out:
         assert code == 0 and len(log) == 1, message
         assert (" cluster=1 " not in log[0]) == clusters, log
+
+
+@pytest.mark.parametrize("dtype", ["FP8", "U8"])
+def test_blocks_per_stage_of_a_pinned_shape(fake, dtype):
+    """Two blocks a stage are what tiles of up to 128 rows have anyway; unpaired tiles above have one, and pinning two takes it where there
+    is room for two and is refused where there never was."""
+    out = fake(f"""
+        def launch(plan):
+            code, error, log = run_gemm(gemm([1], [512], dense_plan=plan), {dtype}, 300, 2048, [[512]])
+            return log if code == 0 else error
+        shapes = ["16,1,0", "48,3,0", "128,1,0", "128,8,0", "64,1,1", "128,1,1"]
+        print(json.dumps([[(launch(p + b), launch(p)) for p in shapes] for b in (",2", ",1")] + [[launch("160,1,0,2"), launch("160,1,0,1"), launch("256,1,0,2")]]))
+        """)
+    assert all(a == b for a, b in out[0])
+    assert all(len(a) == len(b) == 1 and a != b for a, b in out[1])  # one block a stage: through shared memory
+    assert out[2][0] == out[2][1] and "bad launch shape" in out[2][2]
