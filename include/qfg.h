@@ -121,7 +121,7 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
  * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.
  * Every wait of that kernel is bounded; a block whose wait ran out writes NaN for its columns (the winner of such a row
  * of the LM head is a NaN), the call succeeds and the next one is whole.  "give_up" = 1, for tests, makes every block of
- * an LM head act as if its wait for x had run out.
+ * an LM head act as if its wait for x had run out, and lets those of the one-kernel call over more rows wait in vain, and not for long.
  * "dense_rows" moves or disables (0) the row count above which the prefill branch is taken;
  * "dense_plan" = "rows per tile,CTAs that split K,pair,blocks per stage" pins its launch shape.  The blocks may be left out.  One sends FP8 and
  * NVFP4 weights of tiles of up to 128 rows through shared memory, two, like none, through tensor memory; larger tiles have two where

@@ -107,6 +107,7 @@ struct DenseParams {
   int col_begin[kMaxOut], width[kMaxOut];
   int nseg, M, K, ksteps, bm, m_tiles, tiles, stages;
   int raw_depth;  // TM: slots of the raw ring
+  int give_up;    // testing: 1: x never comes and every wait is short
   uint32_t out_vec;  // outputs whose rows can be written 16 bytes at a time
 };
 
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
       BarInit(Smem(&ctl.raw_full[i]), 1);
       BarInit(Smem(&ctl.raw_empty[i]), TM ? kTmWarps : kDqWarps);
     }
-    ctl.fault = 0;
+    ctl.fault = static_cast<uint32_t>(p.give_up);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 4 && lane == 0) {
@@ -803,7 +804,7 @@ __global__ void __launch_bounds__(DenseThreads<MODE>(), 1) DenseTcKernel(const _
   } else if (warp == 4) {
     // ---- x (and BF16 weights)
     int stage = 0, round = 0;
-    bool good = true;
+    bool good = p.give_up == 0;
     const uint32_t mine = static_cast<uint32_t>(KS * (xrows * kBk * 2 + (MODE == kBf16 ? kABytes : 0)));
     for (int tile = first_tile; tile < p.tiles && good; tile += tile_step) {
       const TileAt t = LocateDense<PAIR>(p, tile, rank);
@@ -1054,6 +1055,7 @@ struct SwishRole {
     const DenseParams& p = q.d;
     const uint32_t full0 = Smem(&ctl.full[0]), empty0 = Smem(&ctl.empty[0]);
     const int chunk = lane & 7;
+    if (p.give_up) return;
     while (k < p.ksteps) {
       const int stage = k % p.stages, round = k / p.stages;
       const uint32_t dst = smem + static_cast<uint32_t>(stage) * block_bytes + kABytes;
@@ -1227,7 +1229,7 @@ __global__ void __launch_bounds__(SharedThreads<MODE>(), 1) DenseSharedKernel(co
       BarInit(Smem(&ctl.raw_full[i]), 1);
       BarInit(Smem(&ctl.raw_empty[i]), kDqWarps);
     }
-    ctl.fault = 0;
+    ctl.fault = static_cast<uint32_t>(p.give_up);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 5) {
@@ -1689,6 +1691,7 @@ bool LaunchDenseTc(int weights, const GemmParams& g, int64_t m, const DenseTcPla
   p.nseg = g.nseg;
   p.M = static_cast<int>(m);
   p.K = g.K;
+  p.give_up = g.give_up;
   p.bm = plan.bm;
   const int xrows = plan.pair ? p.bm / 2 : p.bm;
   const bool tm = TakesTm(mode, plan);
@@ -1802,6 +1805,7 @@ bool LaunchDenseShared(int weights, const GemmParams& g, int64_t m, const DenseT
   p.nseg = 1;
   p.M = static_cast<int>(m);
   p.K = g.K;
+  p.give_up = g.give_up;
   p.bm = plan.bm;
   p.ksteps = (g.K + kBk - 1) / kBk;
   p.seg[0] = {sg.w, sg.w_scale, sg.pitch, sg.total_bytes, sg.n, 0, 0, 1};

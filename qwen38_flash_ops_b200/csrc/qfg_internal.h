@@ -125,7 +125,7 @@ struct GemmParams {
   int width[kMaxOut] = {};
   int trigger = 0;
   int pdl_wait = 0;
-  int give_up = 0;     // testing (skinny_stream.cu): 1: every CTA goes on as if its first wait had run out, the LM head's for x
+  int give_up = 0;     // testing: 1: every CTA of the LM head goes on as if its first wait had run out, the one for x; to those of many-row calls x never comes
   int force_slow = 0;  // testing: always take the BF16-MMA path of the quantised modes
   unsigned long long* phase_times = nullptr;  // [CTA][16] timer stamps; written only by builds with -DQFG_PHASE_TIMES
   // plan

@@ -240,3 +240,22 @@ def test_gates_are_fp32_sums(cuda):
         logit = (gx.double() @ gw.double()).bfloat16().float()
         wrong += (op(g, u, w, gx, gw, routed) != torch.sigmoid(logit).bfloat16()).any(dim=1).sum().item()
     assert wrong <= 6  # of 102 400: 42 with the running accumulator
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["32,1", "64,2", "160,7,0,1"])
+def test_waits_that_run_out_give_nan(cuda, mode, plan):
+    """swish_mul never comes: every output is NaN, and the next call is whole."""
+    gen = torch.Generator(device="cuda").manual_seed(mode)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    M, K, N = 170, 648, 1152
+    w = [mk(K, N), mk(K, N).to(torch.float8_e4m3fn), torch.randint(0, 0x70, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)][mode]
+    args = mk(M, K), mk(M, K), w, mk(M, 256), mk(256, 1) * 0.02, mk(M, N)
+    op = SharedExpertDown()
+    op.set_option("dense_plan", plan)
+    first = op(*args)
+    for _ in range(2):
+        op.set_option("give_up", 1)
+        assert torch.isnan(op(*args)).all()
+        op.set_option("give_up", 0)
+        assert torch.equal(op(*args), first)

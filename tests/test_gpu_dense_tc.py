@@ -212,3 +212,27 @@ print("ok")
 """
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("plan", ["48,1,0", "48,1,0,1", "64,4,0", "64,4,0,1", "128,1,1", "96,1,1,1", "256,1,0", "256,1,1"])
+def test_waits_that_run_out_give_nan(cuda, mode, plan):
+    """x never comes: every output is NaN, none keeps what its memory held, and the next call is whole.  Several tiles a CTA."""
+    gen = torch.Generator(device="cuda").manual_seed(mode)
+    M, K, N = 300, 1096, 128 * 46 if "4,0" in plan else 128 * 150
+    x = torch.randn(M, K, generator=gen, device="cuda").bfloat16()
+    w = torch.randn(K, N, generator=gen, device="cuda").bfloat16()
+    if mode == 1:
+        w = w.to(torch.float8_e4m3fn)
+    elif mode == 2:
+        w = torch.randint(0, 0x70, (K, N * 9 // 16), generator=gen, device="cuda", dtype=torch.uint8)
+    op = SkinnyGemm([1], [N])
+    op.set_option("dense_plan", plan)
+    first = op(x, w)[0]
+    for _ in range(2):
+        out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+        op.set_option("give_up", 1)
+        op(x, w, out=[out])
+        assert torch.isnan(out).all()
+        op.set_option("give_up", 0)
+        assert torch.equal(op(x, w)[0], first)
