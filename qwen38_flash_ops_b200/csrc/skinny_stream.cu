@@ -376,8 +376,10 @@ __device__ __forceinline__ bool StageXStream(const StreamParams& q, const Tile& 
       for (int i = 0; i < kBatch; ++i) held[i] = c + i * step < valid ? __ldg(src + c + i * step) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int i = 0; i < kBatch; ++i) {
-        if constexpr (MODE != kBf16) Track(held[i], mx, mn);
-        if (c + i * step < chunks) dst[c + i * step] = MODE == kBf16 ? held[i] : ScaleToHalf8(held[i], kUsualScale);
+        if (c + i * step < chunks) {
+          if constexpr (MODE != kBf16) Track(held[i], mx, mn);
+          dst[c + i * step] = MODE == kBf16 ? held[i] : ScaleToHalf8(held[i], kUsualScale);
+        }
       }
     }
     if constexpr (MODE != kBf16) bad = Publish(sx, m, rs.part, lane, mx, mn) || bad;
@@ -409,11 +411,9 @@ __device__ __forceinline__ bool StageXHead(const StreamParams& q, const Tile& tl
     uint32_t mx = 0, mn = 0xFFFFFFFFu;
 #pragma unroll 4
     for (int c = c_first; c < chunks; c += step) {
-      if (c >= valid) {
-        dst[c] = make_uint4(0, 0, 0, 0);
-      } else if (MODE != kBf16) {
-        Track(dst[c], mx, mn);
-      }
+      const uint4 v = c < valid ? dst[c] : make_uint4(0, 0, 0, 0);
+      if (c >= valid) dst[c] = v;
+      if constexpr (MODE != kBf16) Track(v, mx, mn);
     }
     if constexpr (MODE != kBf16) Publish(sx, m, rs.part, lane, mx, mn);
   }
