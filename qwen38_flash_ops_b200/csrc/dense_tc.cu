@@ -1110,11 +1110,13 @@ struct SwishRole {
   }
 };
 
-// Sixteen products of a row of gx each for rows (g, g + 8) of a lane, added to nothing.
-__device__ __forceinline__ float2 Dot16(uint32_t lo0, uint32_t hi0, uint32_t lo1, uint32_t hi1, uint32_t w0, uint32_t w1) {
+// 32 products of a row of gx each for rows (g, g + 8) of a lane, added to nothing.
+__device__ __forceinline__ float2 Dot32(const uint4& lo, const uint4& hi, const uint4& w) {
   float d[4];
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(lo0), "r"(hi0), "r"(lo1), "r"(hi1), "r"(w0), "r"(w1), "f"(0.f));
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(lo.x), "r"(hi.x), "r"(lo.y), "r"(hi.y), "r"(w.x), "r"(w.y), "f"(0.f));
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(lo.z), "r"(hi.z), "r"(lo.w), "r"(hi.w), "r"(w.z), "r"(w.w));
   return make_float2(d[0], d[2]);
 }
 
@@ -1122,10 +1124,10 @@ __device__ __forceinline__ float2 Dot16(uint32_t lo0, uint32_t hi0, uint32_t lo1
 // receiver's barrier.  The dot products are MMAs of sixteen rows of gx with gw in every column: a lane reads 16 bytes of two
 // rows, eight k of its own, and the same eight of gw, so that the order of k within an MMA is free (multiplied out they were
 // 24 instructions per 16 bytes, a third of the call).  A warp takes a quarter of k; the quarters are added in order.
-// An MMA adds sixteen products and nothing else: an accumulator that runs through them is cut off at every one, not rounded.  The
-// sums of sixteen go to FP32 sums by ordinary additions, eight of 2560 elements to each.  Gates that are not the 64-bit gate's BF16 number, of
-// 2.5 million of twelve kinds (250 to 4096 elements, of both signs, of one, cancelling): 249 with running accumulators, 79 with FP32
-// multiply-adds, 63 so.
+// An accumulator that runs through many MMAs is cut off at every one, not rounded: two add 32 products, and their sums go to FP32 sums by
+// ordinary additions, eight of 2560 elements to each.  Gates that are not the 64-bit gate's BF16 number, of 2.5 million of twelve
+// kinds (250 to 4096 elements, of both signs, of one, cancelling): 249 with running accumulators, 79 with FP32 multiply-adds, 54 so.
+// The additions cost a call 0.03 to 0.25 us (BF16 1912 rows 608 x 1344 18.0 -> 18.3).
 __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, float (*quarter)[256], uint32_t bar, int warp, int lane, int rank, int m0) {
   const uint16_t *const gx_in = BehindWait(q.gx), *const gw_in = BehindWait(q.gw);
   const int p0 = FirstRow(q, rank), part = FirstRow(q, rank + 1) - p0;
@@ -1154,9 +1156,9 @@ __device__ __forceinline__ void GateRole(const DenseShared& q, float* gate, floa
         }
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-          const float2 a = Dot16(lo[i].x, hi[i].x, lo[i].y, hi[i].y, w[i].x, w[i].y), b = Dot16(lo[i].z, hi[i].z, lo[i].w, hi[i].w, w[i].z, w[i].w);
-          c[i % 3].x += a.x + b.x;
-          c[i % 3].y += a.y + b.y;
+          const float2 d = Dot32(lo[i], hi[i], w[i]);
+          c[i % 3].x += d.x;
+          c[i % 3].y += d.y;
         }
       }
       if (t == 0) {
