@@ -115,7 +115,8 @@ QFG_API int qfg_skinny_gemm_compute(const qfg_skinny_gemm* op, const void* x, in
  * with the programmatic-stream-serialisation attribute and wait for their predecessor (griddepcontrol.wait) before they
  * touch memory, so they see what stream order shows them.  That holds for a predecessor that was itself launched with
  * the attribute as long as it executes that wait too, as such kernels have to.  "pdl_wait" = 1 launches the kernel so in
- * captures too and makes it wait only after its first weight tiles are in flight.  "plan" pins the
+ * captures too and makes it wait only after its first weight tiles are in flight; the kernel for more rows of SkinnyGemm takes no
+ * notice of it: it waits first, and in captures its launch is plain.  "plan" pins the
  * geometry of the general kernels ("wn=4,wk=2,ks=1,stages=4,cluster=8,ctas=296") and sends the call to them; "stream_plan"
  * = "width,wk,teams,cluster,tail" pins that of the kernel that streams the weights by tensor copies, "0" sends no call
  * to it, "" gives the choice back.  A geometry that does not exist for the weights is an error of the call.

@@ -182,7 +182,7 @@ def test_a_head_that_gave_up_says_so(cuda, mode, N, plan, pdl_wait):
             assert torch.equal(a, b)
 
 
-# what stands among ordinary values of x: [2^-22, 2^11) is scaled in one look, the rest row by row or not at all
+# what stands among ordinary values of x: [2^-27, 2^6) is scaled in one look, the rest row by row or not at all
 @pytest.mark.parametrize("mode", [1, 2])
 @pytest.mark.parametrize("kind", ["plain", "cluster", "shared", "head"])
 @pytest.mark.parametrize("least,most", [(2.0 ** -22, 1.9921875 * 2.0 ** 10), (1.9921875 * 2.0 ** -23, 1.0), (2.0 ** -10, 2.0 ** 11), (2.0 ** -30, 2.0 ** -4),
