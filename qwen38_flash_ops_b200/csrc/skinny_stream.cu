@@ -590,27 +590,32 @@ enum StreamKind : int { kPlain = 0, kShared = 1, kHead = 2 };
 #define QFG_CLOCK(v)
 #endif
 
-// One lane has stage `s` of the slice copied to place `slot` of the ring.
+// Where a CTA's boxes begin, in elements of eight bytes: the stored values (nibbles), the block scales; and what a row takes.
+struct BoxesAt {
+  int x, scales, pitch;
+};
 template <int MODE>
-__device__ __forceinline__ void IssueStage(const StreamParams& q, int seg, int n0, int kbeg, uint32_t ring, StreamCtl& ctl, int s, int slot) {
-  const Segment& sg = q.g.seg[seg];
-  // where this CTA's boxes begin, in elements of eight bytes
-  const int wpitch8 = static_cast<int>(sg.pitch >> 3);
-  const int x0 = MODE == kBf16 ? n0 >> 2 : MODE == kFp8 ? n0 >> 3 : n0 >> 4;
-  const int sc0 = MODE == kNvfp4 ? ((sg.n >> 1) + (n0 >> 4)) >> 3 : 0;
+__device__ __forceinline__ BoxesAt BoxesOf(const Segment& sg, int n0) {
+  return {MODE == kBf16 ? n0 >> 2 : MODE == kFp8 ? n0 >> 3 : n0 >> 4, MODE == kNvfp4 ? ((sg.n >> 1) + (n0 >> 4)) >> 3 : 0, static_cast<int>(sg.pitch >> 3)};
+}
+// One lane has stage `s` of the slice copied to place `slot` of the ring.  The head makes `at` once: anew for every stage it took 81.5 us
+// instead of 79.7 (5120 x 151936, four rows) and 43.5 instead of 42.6 (2560 x 151936, one).  The products, with few stages
+// past the first round, make it anew: once they took 0.05 to 0.1 us more (NVFP4 17408 x 5120, four rows, 15.67 -> 15.80).
+template <int MODE>
+__device__ __forceinline__ void IssueStage(const StreamParams& q, int seg, const BoxesAt& at, int kbeg, uint32_t ring, StreamCtl& ctl, int s, int slot) {
   const uint32_t bar = SmemAddr(&ctl.full[0]) + static_cast<uint32_t>(slot) * 8u;
   uint32_t dst = ring + static_cast<uint32_t>(slot) * static_cast<uint32_t>(q.g.stage_bytes), sdst = dst + q.scale_off;
   int row = (kbeg + s * q.rows) >> q.odd;
   BarExpect(bar, q.tx);
 #pragma unroll 1
   for (int b = 0; b < q.boxes; ++b) {
-    TmaLoad(dst, &q.wmap[seg], x0, row, bar);
+    TmaLoad(dst, &q.wmap[seg], at.x, row, bar);
 #pragma unroll 1
-    for (int c = 1; c < q.col_boxes; ++c) TmaLoad(dst + c * q.rows * 128, &q.wmap[seg], x0 + c * 16, row, bar);
+    for (int c = 1; c < q.col_boxes; ++c) TmaLoad(dst + c * q.rows * 128, &q.wmap[seg], at.x + c * 16, row, bar);
     if constexpr (MODE == kNvfp4) {
-      if (q.odd) TmaLoad(dst + q.half, &q.wmap[seg], (x0 + wpitch8) & ~1, row, bar);
-      TmaLoad(sdst, &q.smap[seg], sc0 & ~1, row, bar);
-      if (q.odd) TmaLoad(sdst + q.shalf, &q.smap[seg], (sc0 + wpitch8) & ~1, row, bar);
+      if (q.odd) TmaLoad(dst + q.half, &q.wmap[seg], (at.x + at.pitch) & ~1, row, bar);
+      TmaLoad(sdst, &q.smap[seg], at.scales & ~1, row, bar);
+      if (q.odd) TmaLoad(sdst + q.shalf, &q.smap[seg], (at.scales + at.pitch) & ~1, row, bar);
       sdst += q.box_rows * q.spitch;
     }
     dst += q.box_rows * q.pitch;
@@ -731,11 +736,12 @@ __device__ __forceinline__ void StreamRest(bool slow, const StreamParams& q, con
   QFG_CLOCK(loop_begin);
 
   if (warp == q.warps) {
+    const BoxesAt boxes = BoxesOf<MODE>(sg, w.tl.n0);
     int slot = 0;
     uint32_t parity = 0;
     for (int s = p.stages; s < w.nst; ++s) {
       if (!BarWait(empty0 + slot * 8, parity, ctl)) break;
-      if (ElectOne()) IssueStage<MODE>(q, w.tl.seg, w.tl.n0, w.tl.kbeg, ring, ctl, s, slot);
+      if (ElectOne()) IssueStage<MODE>(q, w.tl.seg, KIND == kHead ? boxes : BoxesOf<MODE>(sg, w.tl.n0), w.tl.kbeg, ring, ctl, s, slot);
       __syncwarp();
       if (++slot == p.stages) {
         slot = 0;
@@ -841,7 +847,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
   }
 
   // ---- producer
-  const int wpitch8 = static_cast<int>(sg.pitch >> 3);
   const uint32_t x_smem = ring + q.x_off, x_full = SmemAddr(&ctl.x_full);
   auto issue_x = [&]() {  // one lane
     const uint32_t bytes = static_cast<uint32_t>(tl.kslice) * 2u;
@@ -865,9 +870,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
     if (!p.pdl_wait) GridDependencyWait();  // without the option the weights are the predecessor's to write too
     if (kBulkX) asm volatile("bar.arrive 1, %0;" ::"r"(static_cast<int>(blockDim.x)) : "memory");  // the others may wait on the barriers
     if (ElectOne()) {
+      const BoxesAt boxes = BoxesOf<MODE>(sg, tl.n0);
       // x before the weights, so that it does not queue behind them - unless it may still be the predecessor kernel's to write
       if (kBulkX && !p.pdl_wait) issue_x();
-      for (int s = 0; s < p.stages && s < nst; ++s) IssueStage<MODE>(q, tl.seg, tl.n0, tl.kbeg, ring, ctl, s, s);
+      for (int s = 0; s < p.stages && s < nst; ++s) IssueStage<MODE>(q, tl.seg, KIND == kHead ? boxes : BoxesOf<MODE>(sg, tl.n0), tl.kbeg, ring, ctl, s, s);
       if constexpr (kTail) {
         if (tail_index >= 0) {
           const uint32_t bar = SmemAddr(&ctl.tail_full), dst = ring + q.tail_off, sdst = dst + q.tail_rows * q.tail_pitch;
@@ -876,9 +882,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) SkinnyGemmStreamKernel(cons
           BarExpect(bar, q.tail_tx);
           if (q.odd) {  // even rows, odd rows
             TmaLoad(dst, &q.tail_wmap, tx0, row >> 1, bar);
-            TmaLoad(dst + hw, &q.tail_wmap, (tx0 + wpitch8) & ~1, row >> 1, bar);
+            TmaLoad(dst + hw, &q.tail_wmap, (tx0 + boxes.pitch) & ~1, row >> 1, bar);
             TmaLoad(sdst, &q.tail_smap, tsx & ~1, row >> 1, bar);
-            TmaLoad(sdst + hs, &q.tail_smap, (tsx + wpitch8) & ~1, row >> 1, bar);
+            TmaLoad(sdst + hs, &q.tail_smap, (tsx + boxes.pitch) & ~1, row >> 1, bar);
           } else {      // upper half, lower half
             const int below = row + static_cast<int>(q.tail_rows / 2);
             TmaLoad(dst, &q.tail_wmap, tx0, row, bar);
