@@ -267,8 +267,8 @@ __device__ __forceinline__ void StageXRaw(const StreamParams& q, int kbeg, int k
 // what lies in FP16 already.  That is exact wherever it is neither infinite nor, in a row with values below the window, 2^-17 or
 // less (what they round to, or zero), and takes another power of two where it lies; only pieces of eight with something else among
 // them are asked for again.  It costs such calls 0.1 (FP8 5120 x 10240, two rows: 11.6 us) to 2.9 us (NVFP4 5120 x 34816,
-// eight rows: 24.1); staging all of it over again cost 0.8 to 5.5.  Returns true if a row's values are too far apart for FP16: all rows
-// then are staged as they are.
+// eight rows: 24.1), or 4.6 where most pieces have values past 64 (FP8 5120 x 10240, eight rows: 16.5); staging all of it over again cost
+// 0.8 to 5.5.  Returns true if a row's values are too far apart for FP16: all rows then are staged as they are.
 __device__ __forceinline__ bool RestageX(const StreamParams& q, int kbeg, int kslice, uint16_t* xs, SharedScratch& sh, const StreamScratch& sx,
                                          const uint4 (&held)[kBatch], int padded, int warp, int lane) {
   const GemmParams& p = q.g;
